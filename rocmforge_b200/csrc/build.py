@@ -29,7 +29,7 @@ NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", 
 # module name -> sources (first is the translation unit, the rest are headers it includes)
 MODULES: Dict[str, List[str]] = {
     "elementwise": ["elementwise.cu", "common.cuh"],
-    "gemm_simt": ["gemm_simt.cu", "common.cuh"],
+    "gemm_simt": ["gemm_simt.cu", "gemm_f32_tc.cuh", "f32_parts.cuh", "tcgen05_common.cuh", "common.cuh"],
     "attention_generic": ["attention_generic.cu", "common.cuh"],
     "sampling": ["sampling.cu", "common.cuh"],
     "retention": ["retention.cu", "common.cuh"],

@@ -251,3 +251,6 @@ extern "C" int rf_gemm_simt(int dtype, const void* X, const void* W, const void*
     return dtype == 0 ? launch<float>(X, W, bias, bias_is_f32, Y, M, N, K, ldx, ldy, mode, splits, st)
                       : launch<__nv_bfloat16>(X, W, bias, bias_is_f32, Y, M, N, K, ldx, ldy, mode, splits, st);
 }
+
+// Float32 products on the tensor cores, with the numbers split into bfloat16 parts
+#include "gemm_f32_tc.cuh"

@@ -20,7 +20,7 @@ from .stream import ScaledRows
 @dataclass
 class Options:
     """Switches of the engine (all default to the serving configuration)."""
-    tensor_core_gemm: bool = True        # tcgen05 products on the bfloat16 path where the shape allows
+    tensor_core_gemm: bool = True        # tcgen05 products where the shape allows (in 32-bit: of numbers split into three bfloat16 parts)
     tuned_attention: bool = True         # split-KV decode attention / tiled prefill attention on bfloat16
     tcgen05_attention: bool = True       # prefill attention with tcgen05.mma (else the mma.sync kernel)
     clustered_decode: bool = True        # decode attention by clusters of CTAs (else one CTA per 128-key chunk)
@@ -84,7 +84,15 @@ class StepContext:
             if x.shape[0] <= tc.SKINNY_MAX_TOKENS:
                 return tc.gemm_tc_skinny(x, w, bias, mode=mode, row_ss=row_ss)
             return tc.gemm_tc(x, w, bias, mode=mode)
-        return kernels.gemm_simt(x, w, bias, out_f32=out_f32)
+        return self.gemm_plain(x, w, bias, out_f32=out_f32)
+
+    def plain_splits(self, x, w) -> int:
+        """K splits of a product of few tokens outside the bfloat16 tensor-core path."""
+        return kernels.split_k_for_plain(x, w, self.options.tensor_core_gemm)
+
+    def gemm_plain(self, x, w, bias=None, **kw):
+        """A product outside the bfloat16 tensor-core path."""
+        return kernels.gemm_plain(x, w, bias, tensor_cores=self.options.tensor_core_gemm, **kw)
 
     def matmul_rows_or_parts(self, x, w):
         """x w^T as [M, N] in the compute dtype, or, where few tokens let K be split, as the float32 stack [S, M, N] of partial
@@ -98,9 +106,9 @@ class StepContext:
                 if splits > 1:
                     return tc.gemm_tc_skinny(x, w, mode=tc.PARTIAL, splits=splits)
             elif not self.uses_tensor_cores(x, w, tc.STORE):
-                splits = kernels.split_k_for_simt(w.shape[0], w.shape[1])
+                splits = self.plain_splits(x, w)
                 if splits > 1:
-                    return kernels.gemm_simt(x, w, splits=splits)
+                    return self.gemm_plain(x, w, splits=splits)
         return self.matmul(x, w)
 
     def matmul_f32_parts(self, x, w):
@@ -114,9 +122,9 @@ class StepContext:
                 if splits > 1:
                     return tc.gemm_tc_skinny(x, w, mode=tc.PARTIAL, splits=splits, row_ss=row_ss)
             elif row_ss is None:
-                splits = kernels.split_k_for_simt(w.shape[0], w.shape[1])
+                splits = self.plain_splits(x, w)
                 if splits > 1:
-                    return kernels.gemm_simt(x, w, splits=splits)
+                    return self.gemm_plain(x, w, splits=splits)
         if row_ss is not None:
             x = ScaledRows(x, row_ss[0], row_ss[1], w.shape[1])
         return self.matmul(x, w, out_f32=True)
@@ -149,12 +157,12 @@ class StepContext:
             tc.gemm_tc(x, w, bias, mode=tc.RESIDUAL, out=stream.h)
             return
         if x.shape[0] <= tc.SKINNY_MAX_TOKENS and bias is None:
-            splits = kernels.split_k_for_simt(w.shape[0], w.shape[1])
+            splits = self.plain_splits(x, w)
             if splits > 1:                           # few tokens: K ranges in parallel, summed by the next norm
-                stream.add_pending(kernels.gemm_simt(x, w, splits=splits))
+                stream.add_pending(self.gemm_plain(x, w, splits=splits))
                 return
         stream.flush()
-        kernels.gemm_simt(x, w, bias, out=stream.h, accumulate=True)
+        self.gemm_plain(x, w, bias, out=stream.h, accumulate=True)
 
     def gated_activation(self, y, gate_up, activation: str = "silu", limit: float = 0.0, alpha: float = 0.0):
         """act(gate) * up from the fused, row-interleaved gate/up matrix (act = silu, relu or gelu_tanh), or "clamped_glu":
@@ -170,5 +178,7 @@ class StepContext:
             return tc.gemm_tc(y, w, mode=mode, **glu)
         if row_ss is not None:
             y = ScaledRows(y, row_ss[0], row_ss[1], w.shape[1]).materialize()
+        if mode == tc.SWIGLU and gate_up.bias is None and self.options.tensor_core_gemm and kernels.f32_tc_takes(y, w):
+            return kernels.gemm_f32_tc(y, w, mode=kernels.F32_SWIGLU)
         gu = self.matmul(y, w, gate_up.bias)
         return kernels.clamped_glu(gu, limit, alpha) if mode == tc.CLAMPGLU else kernels.swiglu(gu, activation=activation)

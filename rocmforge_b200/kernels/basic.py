@@ -265,6 +265,93 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None
     return out
 
 
+F32_STORE, F32_ADD, F32_PARTIAL, F32_SWIGLU = 0, 2, 3, 4
+
+
+def gemm_f32_tc(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None, *, mode: int = F32_STORE,
+                out: torch.Tensor | None = None, splits: int = 1, tile_tokens: int = 0) -> torch.Tensor:
+    """The float32 product x @ w.T on the tensor cores, every number split into three bfloat16 parts (csrc/gemm_f32_tc.cuh).
+
+    F32_STORE: [M, N] (+ bias); F32_ADD: out += the product (+ bias); F32_PARTIAL: the stack [splits, M, N] of partial sums over K
+    ranges; F32_SWIGLU: [M, N/2] = silu(gate) * up of row-interleaved gate/up weights."""
+    from .tensor_core import status_word
+    need_cuda(x, w, bias, out)
+    need(x.dim() == 2 and w.dim() == 2 and x.dtype == torch.float32 and w.dtype == torch.float32 and x.stride(1) == 1
+         and w.is_contiguous() and x.shape[1] == w.shape[1], "float32 gemm: x [M,K] and w [N,K] must be float32 and row-major")
+    M, K = x.shape
+    N = w.shape[0]
+    need(f32_tc_operands(x, w), "float32 gemm: rows of whole 16 bytes, aligned")
+    if bias is not None:
+        need(bias.shape == (N,) and bias.dtype in (torch.float32, torch.bfloat16), "gemm: bias must be [N]")
+    need(splits == 1 or mode == F32_PARTIAL, "float32 gemm: several K splits need mode F32_PARTIAL")
+    shape = (splits, M, N) if mode == F32_PARTIAL else (M, N // 2 if mode == F32_SWIGLU else N)
+    if out is None:
+        need(mode != F32_ADD, "gemm: F32_ADD needs the tensor to add into")
+        out = torch.empty(shape, dtype=torch.float32, device=x.device)
+    need(tuple(out.shape) == shape and out.dtype == torch.float32 and out.stride(-1) == 1
+         and (mode != F32_PARTIAL or out.is_contiguous()), "gemm: output has the wrong shape or dtype")
+    bn = tile_tokens or f32_tc_tile(M, N)
+    f = _f("gemm_simt", "rf_gemm_f32_tc", c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int,
+           c_int, c_int, c_int, c_void_p, c_void_p)
+    check(f(ptr(x), x.stride(0), ptr(w), ptr(bias), int(bias is not None and bias.dtype == torch.float32), ptr(out), out.stride(-2),
+            M, N, K, mode, splits, bn, _sms(x.device), ptr(status_word(x.device)), stream()),
+          f"gemm_f32_tc ({M}x{N}x{K}, mode {mode}, {splits} splits)")
+    return out
+
+
+@functools.lru_cache(None)
+def _sms(device) -> int:
+    return device_sm_count(device)
+
+
+def f32_tc_operands(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether TMA can fetch the operands' rows: whole 16-byte pieces on 16-byte boundaries."""
+    return w.shape[1] % 4 == 0 and x.stride(0) % 4 == 0 and x.stride(0) >= x.shape[1] and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
+
+
+def f32_tc_tile(M: int, N: int) -> int:
+    """Tokens of a tile: the next of 16, 32, 64, 128.  A smaller tile fills more CTAs but splits the weights once more for every token
+    tile (64 tokens x 9,728 x 896: tiles of 16, 32, 64 35, 25, 18 us; 1,999 tokens, tiles of 32, 64, 128 343, 221, 194 us)."""
+    return 16 if M <= 16 else 32 if M <= 32 else 64 if M <= 64 else 128
+
+
+@functools.lru_cache(None)
+def split_k_for_f32_tc(N: int, K: int, sm_count: int | None = None) -> int:
+    """K splits of a float32 tensor-core product of few tokens, from N and K alone: at most one CTA per SM, every split at least
+    four stages of 32."""
+    sm_count = sm_count or device_sm_count()
+    tiles = (N + 127) // 128
+    kb = (K + 31) // 32
+    splits = max(1, min(sm_count // tiles, kb // 4))
+    per = (kb + splits - 1) // splits
+    return (kb + per - 1) // per                   # no empty split
+
+
+def f32_tc_takes(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether a product outside the bfloat16 path runs on the tensor cores as well: float32 rows that TMA can fetch, whatever the
+    sizes.  It is faster than the CUDA cores from 3 tokens x 64 x 64 (3.2 against 4.5 us) to 4,096^3 (0.70 against 2.97 ms), and its
+    error is smaller (csrc/gemm_f32_tc.cuh)."""
+    return x.dtype == torch.float32 and w.dtype == torch.float32 and x.shape[0] > 0 and f32_tc_operands(x, w)
+
+
+def split_k_for_plain(x: torch.Tensor, w: torch.Tensor, tensor_cores: bool = True) -> int:
+    """K splits that ``gemm_plain`` wants for a product of few tokens."""
+    if tensor_cores and f32_tc_takes(x, w):
+        return split_k_for_f32_tc(w.shape[0], w.shape[1])
+    return split_k_for_simt(w.shape[0], w.shape[1])
+
+
+def gemm_plain(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None, *, out: torch.Tensor | None = None,
+               out_f32: bool = False, accumulate: bool = False, splits: int = 0, tensor_cores: bool = True) -> torch.Tensor:
+    """``gemm_simt`` with its arguments; float32 operands whose rows TMA can fetch go to the tensor cores."""
+    if not (tensor_cores and f32_tc_takes(x, w)):
+        return gemm_simt(x, w, bias, out=out, out_f32=out_f32, accumulate=accumulate, splits=splits)
+    if splits >= 1:
+        need(not accumulate and out is None and bias is None, "gemm: partial sums take no bias and no output tensor")
+        return gemm_f32_tc(x, w, mode=F32_PARTIAL, splits=splits)
+    return gemm_f32_tc(x, w, bias, mode=F32_ADD if accumulate else F32_STORE, out=out)
+
+
 def key_span(window: int | None, chunk: int | None = None) -> int:
     """The one number by which the attention kernels know which keys a query sees (rf_first_key in csrc/common.cuh):
     the last ``window`` positions (> 0), the positions of the query's own chunk of ``chunk`` positions, chunks counted

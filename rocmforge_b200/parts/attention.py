@@ -264,9 +264,9 @@ class GQAAttention(Mixer):
                 if splits > 1:
                     return kernels.head_norm_kv_write(tc.gemm_tc_skinny(y, w, mode=tc.PARTIAL, splits=splits), *args, **common)
             elif not ctx.uses_tensor_cores(y, w, tc.STORE):
-                splits = kernels.split_k_for_simt(w.shape[0], w.shape[1])
+                splits = ctx.plain_splits(y, w)
                 if splits > 1:
-                    return kernels.head_norm_kv_write(kernels.gemm_simt(y, w, splits=splits), *args, **common)
+                    return kernels.head_norm_kv_write(ctx.gemm_plain(y, w, splits=splits), *args, **common)
         p = ctx.matmul(y, w)
         if self.gate is not None:
             self._gate_cols = p[:, self.gate_col:self.gate_col + self.gate_rows]
@@ -299,9 +299,9 @@ class GQAAttention(Mixer):
         if row_ss is not None:
             y = ScaledRows(y, row_ss[0], row_ss[1], w.shape[1])
         elif y.shape[0] <= tc.SKINNY_MAX_TOKENS and not ctx.uses_tensor_cores(y, w, tc.STORE):
-            splits = kernels.split_k_for_simt(w.shape[0], w.shape[1])
+            splits = ctx.plain_splits(y, w)
             if splits > 1:                           # CUDA-core product of few tokens: the same scheme
-                parts = kernels.gemm_simt(y, w, splits=splits)
+                parts = ctx.gemm_plain(y, w, splits=splits)
                 return kernels.rope_kv_write(parts, self.n_heads, self.n_kv_heads, self.head_dim,
                                              inv_freq, bias=bias, compute_dtype=ctx.compute_dtype,
                                              **rope)
