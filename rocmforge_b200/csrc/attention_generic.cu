@@ -1,6 +1,5 @@
 // Attention of new tokens over the paged cache, for every head size, group size and
-// window: the plain kernel that the true 32-bit path always uses and that the
-// bfloat16 path uses for whatever the tuned kernels refuse.
+// window: the plain kernel for whatever the tuned kernels of the two paths refuse.
 //
 // One block of 128 threads per (query token, kv head): the query heads that share the kv head (eight at a
 // time) are served from one pass over the keys and values, so the cache is read once per group instead of
@@ -338,3 +337,6 @@ extern "C" int rf_attention_generic_rows(int dtype, const void* q, int q_stride,
         : launch<__nv_bfloat16>(q, q_stride, out, out_stride, k_pages, v_pages, tok_seq, tok_pos, seq_slot, block_table,
                                 max_pages, nh, nkv, hd, hdv, scale, 0.f, nullptr, window, T_, st, 0, nullptr, v_row);
 }
+
+// Plain softmax of float32 heads of 32, 64 and 128: prompts on the tensor cores, single tokens by clusters
+#include "attention_f32.cuh"

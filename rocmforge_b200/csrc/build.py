@@ -30,7 +30,7 @@ NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", 
 MODULES: Dict[str, List[str]] = {
     "elementwise": ["elementwise.cu", "common.cuh"],
     "gemm_simt": ["gemm_simt.cu", "gemm_f32_tc.cuh", "f32_parts.cuh", "tcgen05_common.cuh", "common.cuh"],
-    "attention_generic": ["attention_generic.cu", "common.cuh"],
+    "attention_generic": ["attention_generic.cu", "attention_f32.cuh", "f32_parts.cuh", "tcgen05_common.cuh", "common.cuh"],
     "sampling": ["sampling.cu", "common.cuh"],
     "retention": ["retention.cu", "common.cuh"],
     "gla": ["gla.cu", "common.cuh"],

@@ -433,6 +433,88 @@ def attention_generic(q: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: 
     return out
 
 
+def _f32_attention_operands(q, k_pages, v_pages, n_kv_heads, head_dim, what):
+    need_cuda(q, k_pages, v_pages)
+    need(q.dtype == torch.float32 and q.dim() == 2 and q.stride(1) == 1 and q.stride(0) % 4 == 0 and q.data_ptr() % 16 == 0,
+         f"{what}: q must be float32 [T, >= heads*head_dim] with 16-byte rows")
+    need(k_pages.dtype == torch.float32 and v_pages.dtype == torch.float32 and k_pages.is_contiguous() and v_pages.is_contiguous()
+         and tuple(k_pages.shape[1:]) == (n_kv_heads, PAGE, head_dim) and v_pages.shape == k_pages.shape, f"{what}: bad cache page shape or dtype")
+
+
+@functools.lru_cache(None)
+def attention_f32_prompt_supported(n_heads: int, n_kv_heads: int, head_dim: int) -> bool:
+    return bool(_f("attention_generic", "rf_attention_f32_prompt_supported", c_int, c_int, c_int)(n_heads, n_kv_heads, head_dim))
+
+
+def attention_f32_prompt(q: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: int, k_pages, v_pages, tiles, seq_slot, seq_start,
+                         seq_nnew, cu_q, block_table, scale: float, window: int | None, out: torch.Tensor | None = None, *,
+                         chunk: int | None = None) -> torch.Tensor:
+    """Attention of whole stretches of new tokens in 32 bits on the tensor cores (csrc/attention_f32.cuh), heads of 64 or 128, plain
+    softmax.  ``tiles``: (sequence, first row) of every 128 rows, as for ``attention_prefill_tc``."""
+    from .tensor_core import status_word
+    need_cuda(tiles, seq_slot, seq_start, seq_nnew, cu_q, block_table)
+    _f32_attention_operands(q, k_pages, v_pages, n_kv_heads, head_dim, "attention_f32_prompt")
+    need(attention_f32_prompt_supported(n_heads, n_kv_heads, head_dim) and scale > 0,
+         f"attention_f32_prompt: heads={n_heads}, kv_heads={n_kv_heads}, head_dim={head_dim} is not supported")
+    need(q.shape[1] >= n_heads * head_dim and tiles.dtype == torch.int32 and tiles.numel() % 2 == 0, "attention_f32_prompt: bad q or tiles")
+    if out is None:
+        out = torch.empty((q.shape[0], n_heads * head_dim), dtype=torch.float32, device=q.device)
+    f = _f("attention_generic", "rf_attention_f32_prompt", c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_ll, c_void_p, c_int,
+           c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p)
+    check(f(ptr(q), q.stride(0), ptr(out), out.stride(0), ptr(k_pages), ptr(v_pages), k_pages.shape[0], ptr(tiles), tiles.numel() // 2,
+            ptr(seq_slot), ptr(seq_start), ptr(seq_nnew), ptr(cu_q), ptr(block_table), block_table.shape[1], n_heads, n_kv_heads, head_dim,
+            float(scale), key_span(window, chunk), ptr(status_word(q.device)), stream()),
+          f"attention_f32_prompt (heads={n_heads}, kv_heads={n_kv_heads}, head_dim={head_dim})")
+    return out
+
+
+@functools.lru_cache(None)
+def attention_f32_token_supported(n_heads: int, n_kv_heads: int, head_dim: int) -> bool:
+    return bool(_f("attention_generic", "rf_attention_f32_token_supported", c_int, c_int, c_int)(n_heads, n_kv_heads, head_dim))
+
+
+def attention_f32_token(q: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: int, k_pages, v_pages, tok_seq, tok_pos, seq_slot,
+                        block_table, scale: float, window: int | None, splits: int | None = None, out: torch.Tensor | None = None, *,
+                        chunk: int | None = None) -> torch.Tensor:
+    """Attention of single tokens in 32 bits, heads of 32, 64 or 128, plain softmax: ``splits`` CTAs (1, 2, 4 or 8) per (token, kv head)."""
+    need_cuda(tok_seq, tok_pos, seq_slot, block_table)
+    _f32_attention_operands(q, k_pages, v_pages, n_kv_heads, head_dim, "attention_f32_token")
+    need(attention_f32_token_supported(n_heads, n_kv_heads, head_dim) and q.shape[1] >= n_heads * head_dim,
+         f"attention_f32_token: heads={n_heads}, kv_heads={n_kv_heads}, head_dim={head_dim} is not supported")
+    T = q.shape[0]
+    if splits is None:
+        splits = f32_token_splits(T, n_kv_heads)
+    if out is None:
+        out = torch.empty((T, n_heads * head_dim), dtype=torch.float32, device=q.device)
+    f = _f("attention_generic", "rf_attention_f32_token", c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+           c_void_p, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_void_p)
+    check(f(ptr(q), q.stride(0), ptr(out), out.stride(0), ptr(k_pages), ptr(v_pages), ptr(tok_seq), ptr(tok_pos), ptr(seq_slot),
+            ptr(block_table), block_table.shape[1], n_heads, n_kv_heads, head_dim, float(scale), key_span(window, chunk), T, splits, stream()),
+          f"attention_f32_token (heads={n_heads}, kv_heads={n_kv_heads}, head_dim={head_dim}, splits={splits})")
+    return out
+
+
+def f32_token_splits(T: int, n_kv_heads: int, longest: int | None = None, window: int | None = None) -> int:
+    """CTAs per (token, kv head) of ``attention_f32_token``: as many as fit the GPU at two a SM, at most one per page of keys.
+    Measured, us with 1, 2, 4, 8: 64 sequences of 16..1,024 keys, 2 kv heads 29.3, 19.1, 21.5, 31.0; 8 of them 19.3, 13.2, 9.6, 8.2; 8 of
+    512 keys, 4 kv heads of 128 21.9, 17.9, 13.0, 10.3; 20 tokens of one prompt 3.2, 4.9, 5.2, 10.3."""
+    s = 1
+    while s < 8 and T * n_kv_heads * s * 2 <= 2 * device_sm_count():
+        s *= 2
+    if longest is not None:
+        while s > 1 and s > decode_pages(longest, window):
+            s //= 2
+    return s
+
+
+def f32_prompt_pays(T: int, B: int) -> bool:
+    """Whether a step of T tokens of B sequences is a prompt's work (``attention_f32_prompt``) rather than so many single tokens': a
+    query tile of 128 rows costs as much with one row.  Measured, us, prompt and token kernel (14 heads of 64, 2 kv heads): 100 tokens
+    10.1 and 6.1; 4 times 16 tokens after 500 21.7 and 13.0; 16 times 4 38 and 12.5; 8 prompts of 16..1,024 63 and 319; 1,999 tokens
+    68 and 429."""
+    return T > 128 and T > 16 * B
+
+
 def argmax(logits: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
     """Row-wise argmax of float32 logits; of equal maxima the highest index."""
     need_cuda(logits)

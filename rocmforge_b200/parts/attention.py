@@ -325,6 +325,17 @@ class GQAAttention(Mixer):
             return kernels.attention_generic(q, nh, nkv, hd, view.k_pages, view.v_pages, ctx.tok_seq, ctx.tok_pos,
                                              ctx.seq_slot, view.block_table, self.scale, self.window,
                                              v_head_dim=self.v_head_dim, **shaped, **kept)
+        if (ctx.compute_dtype == torch.float32 and ctx.options.tuned_attention and q.data_ptr() % 16 == 0 and q.stride(0) % 4 == 0
+                and view.v_pages.is_contiguous() and view.k_pages.data_ptr() % 16 == 0 and view.v_pages.data_ptr() % 16 == 0):
+            # plain softmax in 32 bits (the options that are not plain went to the generic kernel above)
+            if (tiles128 is not None and tiles128.numel() > 0 and kernels.f32_prompt_pays(ctx.T, ctx.B) and self.scale > 0
+                    and kernels.attention_f32_prompt_supported(nh, nkv, hd)):
+                return kernels.attention_f32_prompt(q, nh, nkv, hd, view.k_pages, view.v_pages, tiles128, ctx.seq_slot, ctx.seq_start,
+                                                    ctx.seq_nnew, ctx.cu_q, view.block_table, self.scale, self.window, chunk=self.chunk)
+            if kernels.attention_f32_token_supported(nh, nkv, hd):
+                return kernels.attention_f32_token(q, nh, nkv, hd, view.k_pages, view.v_pages, ctx.tok_seq, ctx.tok_pos, ctx.seq_slot,
+                                                   view.block_table, self.scale, self.window, chunk=self.chunk,
+                                                   splits=kernels.f32_token_splits(ctx.T, nkv, longest, span))
         if (ctx.is_decode and ctx.compute_dtype == torch.bfloat16 and ctx.options.tuned_attention
                 and kernels.attention_decode_supported(nh, nkv, hd)):
             if ctx.options.clustered_decode:
