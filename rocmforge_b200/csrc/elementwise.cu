@@ -281,14 +281,64 @@ add_rmsnorm_vec_kernel(float* __restrict__ h, const void* __restrict__ pending, 
     }
 }
 
-// The norm of many rows without a pending update (a prompt step: the products add into the stream themselves).  The
-// kernel above keeps a row in registers, and 56 registers a thread leave room for four rows per SM: 56 KB in flight,
-// which one L2 round trip turns into 4 TB/s over the GPU (12 us for 2,048 rows of 3,584).  Here a row is read twice,
-// the second time from L1 (8 rows of 14 KB per SM fit it), so a thread needs 20-odd registers, eight CTAs share an SM
-// and twice the bytes are in flight.  Same sums in the same order as above (block_sum over one float4 per step).
+// The norm of many rows without a pending update (a prompt step: the products add into the stream themselves), up to 8,192 wide.
+// TPR threads share a row and hold it in registers (at most eight 16-byte pieces each, all asked for at once), 256 / TPR rows a
+// block; up to 1,024 wide a row is one warp's, and no barrier stands between a row's loads and its stores.  Memory is the bound
+// (6 or 8 bytes an element).  Measured (us; a block a row, each row read twice): 33,361 x 896 78 -> 27 (6.6 TB/s),
+// 8,192 x 5,120 60 -> 43, 2,048 x 3,584 10.8 -> 10.9.
+// (h without __restrict__: loads through const __restrict__ pointers may be moved up across the wait for the kernel before.)
+template <typename T, int TPR>
+__global__ void __launch_bounds__(256, 5)
+rmsnorm_rows_kernel(const float* h, const void* __restrict__ w, int w_is_f32, float eps, T* y, int H, int n_rows) {
+    constexpr int VPT = 8, RPB = 256 / TPR;
+    __shared__ float part[8];
+    pdl_trigger();
+    const int r = blockIdx.x * RPB + threadIdx.x / TPR, t = threadIdx.x % TPR, nvec = H >> 2;
+    const bool row_ok = r < n_rows;
+    const float4* hrow = reinterpret_cast<const float4*>(h + (size_t)r * H);
+    pdl_wait();
+    float4 a[VPT];
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+        const int c = t + i * TPR;
+        a[i] = row_ok && c < nvec ? hrow[c] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) ss += a[i].x * a[i].x + a[i].y * a[i].y + a[i].z * a[i].z + a[i].w * a[i].w;
+    ss = warp_sum(ss);
+    if constexpr (TPR > 32) {
+        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ss;
+        __syncthreads();
+        ss = 0.f;
+#pragma unroll
+        for (int k = 0; k < TPR / 32; ++k) ss += part[threadIdx.x / TPR * (TPR / 32) + k];
+    }
+    if (!row_ok) return;
+    const float inv = rsqrtf(ss / (float)H + eps);
+    T* yrow = y + (size_t)r * H;
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+        const int c = t + i * TPR;
+        if (c >= nvec) break;
+        float w0, w1, w2, w3;
+        if (w_is_f32) {
+            const float4 u = reinterpret_cast<const float4*>(w)[c];
+            w0 = u.x; w1 = u.y; w2 = u.z; w3 = u.w;
+        } else {                                 // a bfloat16 is the upper half of a float
+            const uint2 two = reinterpret_cast<const uint2*>(w)[c];
+            w0 = __uint_as_float(two.x << 16); w1 = __uint_as_float(two.x & 0xffff0000u);
+            w2 = __uint_as_float(two.y << 16); w3 = __uint_as_float(two.y & 0xffff0000u);
+        }
+        const float ov[4] = {a[i].x * inv * w0, a[i].y * inv * w1, a[i].z * inv * w2, a[i].w * inv * w3};
+        Four<T>::store(yrow + 4 * c, ov);
+    }
+}
+
+// The same for rows wider than that: a block per row, which is read twice, the second time from L1.
 template <typename T>
 __global__ void __launch_bounds__(256, 8)
-rmsnorm_rows_kernel(const float* __restrict__ h, const void* __restrict__ w, int w_is_f32, float eps, T* __restrict__ y,
+rmsnorm_wide_rows_kernel(const float* __restrict__ h, const void* __restrict__ w, int w_is_f32, float eps, T* __restrict__ y,
                     int H) {
     pdl_trigger();
     __shared__ float red[34];
@@ -408,56 +458,68 @@ __global__ void rope_kv_write_kernel(const void* __restrict__ src, int row_strid
     dst[e1] = Cvt<T>::from_f32(x1);
 }
 
-// The same for many tokens (prompts) whose q | k | v rows are one tensor in the compute dtype: a block per
-// token; a thread takes four neighbouring pair indices, computes their sines and cosines once and walks
-// over the heads in steps of blockDim.x / (hd/8) with loads and stores of four elements, so the
-// trigonometry is shared by the heads and every access is 8 or 16 bytes wide.
-template <typename T>
+// The same for many tokens (prompts) whose q | k | v rows are one tensor in the compute dtype: a block takes TB tokens, forms the
+// sines and cosines of each once in shared memory (before it waits for the product: they depend on positions alone), and then walks
+// over (token, head, group of V pairs) with 16-byte loads and stores.  (Each thread with the trigonometry of its own four pairs,
+// one token a block: 33,361 tokens of 18 heads of 64 77 us; now 33, 4.7 TB/s.  8,192 tokens of 56 heads of 128 65 -> 51, with
+// one piece a thread in flight 66.)
+template <typename T, int V>
 __global__ void __launch_bounds__(256)
-rope_kv_write_rows_kernel(const T* __restrict__ src, int row_stride, T* __restrict__ q_out, int q_out_stride,
+rope_kv_write_rows_kernel(const T* src, int row_stride, T* q_out, int q_out_stride,
                           int nh, int nkv, int hd, const float* __restrict__ inv_freq,
                           const int* __restrict__ tok_seq, const int* __restrict__ tok_pos,
                           const int* __restrict__ seq_slot, const int* __restrict__ block_table, int max_pages,
-                          T* __restrict__ k_pages, T* __restrict__ v_pages, int write_kv) {
+                          T* __restrict__ k_pages, T* __restrict__ v_pages, int write_kv, int T_, int TB) {
+    extern __shared__ float2 turn[];                     // [TB][hd / 2] (cosine, sine)
+    __shared__ size_t page_at[8];
     pdl_trigger();
-    const int t = blockIdx.x;
-    const int half = hd >> 1, groups = half >> 2;        // groups of four pairs per head
-    const int g = threadIdx.x % groups, lane_head = threadIdx.x / groups, head_step = blockDim.x / groups;
-    if (lane_head >= head_step) return;                  // threads beyond the last whole row of groups
-    const int pos = tok_pos[t];
-    size_t page_base = 0;
-    if (write_kv) {
-        const int slot = seq_slot[tok_seq[t]];
-        const int page = block_table[(size_t)slot * max_pages + pos / RF_PAGE];
-        page_base = (size_t)page * nkv * RF_PAGE * hd + (size_t)(pos % RF_PAGE) * hd;
+    const int t0 = blockIdx.x * TB, n_tok = min(TB, T_ - t0), half = hd >> 1;
+    if (threadIdx.x < n_tok && write_kv) {
+        const int pos = tok_pos[t0 + threadIdx.x], slot = seq_slot[tok_seq[t0 + threadIdx.x]];
+        page_at[threadIdx.x] = (size_t)block_table[(size_t)slot * max_pages + pos / RF_PAGE] * nkv * RF_PAGE * hd + (size_t)(pos % RF_PAGE) * hd;
     }
-    float sn[4], cs[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) sincosf((float)pos * inv_freq[4 * g + j], &sn[j], &cs[j]);
+    for (int i = threadIdx.x; i < n_tok * half; i += 256) {
+        float sn, cs;
+        sincosf((float)tok_pos[t0 + i / half] * inv_freq[i % half], &sn, &cs);
+        turn[i] = make_float2(cs, sn);
+    }
+    __syncthreads();
     pdl_wait();
-    const T* row = src + (size_t)t * row_stride;
-    const int rotated = write_kv ? nh + nkv : nh;
-    for (int head = lane_head; head < rotated; head += head_step) {
-        float x0[4], x1[4], r0[4], r1[4];
-        Four<T>::load(row + (size_t)head * hd + 4 * g, x0);
-        Four<T>::load(row + (size_t)head * hd + half + 4 * g, x1);
+    const int groups = half / V, heads = write_kv ? nh + 2 * nkv : nh, per_tok = heads * groups;
+    union Piece { uint4 raw[V * sizeof(T) / 16]; T v[V]; };
+    constexpr int W = V * sizeof(T) / 16, N = 2;         // pieces of a thread in flight
+    for (int i0 = threadIdx.x; i0 < n_tok * per_tok; i0 += 256 * N) {
+        Piece x[N], z[N];
+        int at[N];                                       // token, head and group of each
 #pragma unroll
-        for (int j = 0; j < 4; ++j) { r0[j] = x0[j] * cs[j] - x1[j] * sn[j]; r1[j] = x0[j] * sn[j] + x1[j] * cs[j]; }
-        T* dst = head < nh ? q_out + (size_t)t * q_out_stride + (size_t)head * hd
-                           : k_pages + page_base + (size_t)(head - nh) * RF_PAGE * hd;
-        Four<T>::store(dst + 4 * g, r0);
-        Four<T>::store(dst + half + 4 * g, r1);
-    }
-    if (write_kv)
-        for (int vh = lane_head; vh < nkv; vh += head_step) {
-            float a[4], b[4];
-            const T* sv = row + (size_t)(nh + nkv + vh) * hd;
-            Four<T>::load(sv + 4 * g, a);
-            Four<T>::load(sv + half + 4 * g, b);
-            T* dst = v_pages + page_base + (size_t)vh * RF_PAGE * hd;
-            Four<T>::store(dst + 4 * g, a);
-            Four<T>::store(dst + half + 4 * g, b);
+        for (int n = 0; n < N; ++n) {
+            const int i = i0 + n * 256, t = i / per_tok, head = (i - t * per_tok) / groups, g = i - t * per_tok - head * groups;
+            at[n] = i < n_tok * per_tok ? t | head << 4 | g << 20 : -1;
+            if (at[n] < 0) break;
+            const T* from = src + (size_t)(t0 + t) * row_stride + (size_t)head * hd + V * g;
+#pragma unroll
+            for (int u = 0; u < W; ++u) { x[n].raw[u] = reinterpret_cast<const uint4*>(from)[u]; z[n].raw[u] = reinterpret_cast<const uint4*>(from + half)[u]; }
         }
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+            if (at[n] < 0) break;
+            const int t = at[n] & 15, head = at[n] >> 4 & 0xffff, g = at[n] >> 20;
+            if (head < nh + nkv) {
+                const float2* cs = turn + t * half + V * g;
+#pragma unroll
+                for (int j = 0; j < V; ++j) {
+                    const float a = Cvt<T>::to_f32(x[n].v[j]), b = Cvt<T>::to_f32(z[n].v[j]);
+                    x[n].v[j] = Cvt<T>::from_f32(a * cs[j].x - b * cs[j].y);
+                    z[n].v[j] = Cvt<T>::from_f32(a * cs[j].y + b * cs[j].x);
+                }
+            }
+            T* dst = (head < nh ? q_out + (size_t)(t0 + t) * q_out_stride + (size_t)head * hd
+                      : head < nh + nkv ? k_pages + page_at[t] + (size_t)(head - nh) * RF_PAGE * hd
+                                        : v_pages + page_at[t] + (size_t)(head - nh - nkv) * RF_PAGE * hd) + V * g;
+#pragma unroll
+            for (int u = 0; u < W; ++u) { reinterpret_cast<uint4*>(dst)[u] = x[n].raw[u]; reinterpret_cast<uint4*>(dst + half)[u] = z[n].raw[u]; }
+        }
+    }
 }
 
 // ---------------------------------------------------------------- SwiGLU
@@ -994,8 +1056,16 @@ static int launch_add_rmsnorm(float* h, const void* pending, int kind, int n_pen
         !(reinterpret_cast<uintptr_t>(h) & 15) && !(reinterpret_cast<uintptr_t>(w) & 15) && !(reinterpret_cast<uintptr_t>(y) & 15) &&
         !(kind == 1 && (reinterpret_cast<uintptr_t>(pending) & 15))) {
         const int nvec = H / 4;
-        if (kind == 0 && !rows && n_rows >= 512) {       // a prompt step's norm: rows read twice, eight CTAs per SM
-            rf_launch(rmsnorm_rows_kernel<T>, dim3(n_rows), dim3(256), 0, st, (const float*)h, w, w_is_f32, eps, reinterpret_cast<T*>(y), H);
+        if (kind == 0 && !rows && n_rows >= 512) {       // a prompt step's norm
+            T* out = reinterpret_cast<T*>(y);
+            auto go = [&](auto kernel, int per_block) {
+                rf_launch(kernel, dim3((n_rows + per_block - 1) / per_block), dim3(256), 0, st, (const float*)h, w, w_is_f32, eps, out, H, n_rows);
+            };
+            if (H <= 1024) go(rmsnorm_rows_kernel<T, 32>, 8);
+            else if (H <= 2048) go(rmsnorm_rows_kernel<T, 64>, 4);
+            else if (H <= 4096) go(rmsnorm_rows_kernel<T, 128>, 2);
+            else if (H <= 8192) go(rmsnorm_rows_kernel<T, 256>, 1);
+            else rf_launch(rmsnorm_wide_rows_kernel<T>, dim3(n_rows), dim3(256), 0, st, (const float*)h, w, w_is_f32, eps, out, H);
             RF_LAUNCH_CHECK();
             return 0;
         }
@@ -1050,18 +1120,17 @@ static int launch_rope_kv_write(const void* src, int row_stride, int n_partials,
     const int n_pairs = (nh + 2 * nkv) * (hd / 2);
     const dim3 grid(T_, (n_pairs + 255) / 256);
     if (T_ > 2147483647 || grid.y > 65535) return RF_ERR_UNSUPPORTED;
-    // prompts: rows of one tensor, everything aligned for accesses of four elements
-    const size_t four = 4 * sizeof(T);
-    auto aligned = [&](const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) % four) == 0; };
-    if (n_partials == 0 && rot_dim == hd && !interleaved && T_ >= 64 && hd % 8 == 0 && hd / 8 <= 256 && row_stride % 4 == 0 && q_out_stride % 4 == 0 &&
+    // prompts: rows of one tensor, everything aligned for 16-byte accesses, half a head a whole number of them
+    constexpr int V = 16 / sizeof(T);
+    auto aligned = [&](const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) % 16) == 0; };
+    if (n_partials == 0 && rot_dim == hd && !interleaved && T_ >= 64 && hd % (2 * V) == 0 && hd <= 2048 && nh + 2 * nkv <= 65535 && row_stride % V == 0 && q_out_stride % V == 0 &&
         aligned(src) && aligned(q_out) && (!write_kv || (aligned(k_pages) && aligned(v_pages)))) {
-        const int groups = hd / 8;
-        int threads = ((nh + 2 * nkv) * groups + 31) / 32 * 32;        // a row of groups per head, at most 256 threads
-        if (threads > 256) threads = 256;
-        if (threads < groups) threads = (groups + 31) / 32 * 32;
-        rf_launch(rope_kv_write_rows_kernel<T>, dim3(T_), dim3(threads), 0, st, reinterpret_cast<const T*>(src), row_stride,
-            reinterpret_cast<T*>(q_out), q_out_stride, nh, nkv, hd, inv_freq, tok_seq, tok_pos, seq_slot, block_table,
-            max_pages, reinterpret_cast<T*>(k_pages), reinterpret_cast<T*>(v_pages), write_kv);
+        // eight tokens a block; fewer where the step is small (a block per SM before a second token) or the heads are very large
+        int tb = T_ >= 8 * 296 ? 8 : (T_ >= 4 * 296 ? 4 : 2);
+        while (tb * hd > 8192) tb >>= 1;
+        rf_launch(rope_kv_write_rows_kernel<T, V>, dim3((T_ + tb - 1) / tb), dim3(256), (size_t)tb * (hd / 2) * sizeof(float2), st,
+            reinterpret_cast<const T*>(src), row_stride, reinterpret_cast<T*>(q_out), q_out_stride, nh, nkv, hd, inv_freq, tok_seq, tok_pos,
+            seq_slot, block_table, max_pages, reinterpret_cast<T*>(k_pages), reinterpret_cast<T*>(v_pages), write_kv, T_, tb);
         RF_LAUNCH_CHECK();
         return 0;
     }
