@@ -12,7 +12,7 @@
 //                  its rows in registers over the step's tokens; per token their partial r_k and r_q meet by shuffles.
 //                  The order of every sum is fixed by (dim, position) alone: how a prompt is cut into steps and what
 //                  else is in the batch change no bit.
-//   delta_chunk_*  the same recurrence for prompts, with one decay per head and token: chunks of 64 tokens, see below
+//   delta_chunk_*  the same recurrence for prompts: chunks of 64 tokens, see below
 #include <type_traits>
 #include "tcgen05_common.cuh"
 
@@ -247,7 +247,8 @@ int rf_delta_scan(const float* qn, const float* kn, const float* kq, const float
 }
 }
 
-// ---------------------------------------------------------------- prompts: chunks of 64 tokens, one decay per head and token
+// ---------------------------------------------------------------- prompts: chunks of 64 tokens
+// With one decay per head and token (PC = false):
 // With positions t, s inside a chunk of cnt tokens, S0 the state before it, P(s, t) = g_(s+1) ... g_t (P(t, t) = 1) and
 // G_t = g_0 ... g_t, the recurrence above says
 //     u_t = beta_t v_t - beta_t G_t S0^T k_t - sum_(s<t) A_ts u_s,      A_ts = beta_t P(s, t) (k_s . k_t)
@@ -259,6 +260,12 @@ int rf_delta_scan(const float* qn, const float* kn, const float* kq, const float
 //   delta_chunk_carry   (chunk after chunk, a block per sequence, head and 16 value columns)  U = U0 - W S, then the state;
 //                       leaves every chunk's start state and U
 //   delta_chunk_out     (chunks side by side)  o = [M | G q] [U ; S0]
+// With a decay per key channel (PC = true) P and G are vectors over the channels and stay inside the products over them:
+//     A_ts = beta_t sum_d k_s P_d(s, t) k_t,  M_ts likewise with q_t,  (1 + A) W = diag(beta) (G o K),
+//     o_t = (G_t o q_t)^T S0 + sum M_ts u_s,   S_end = diag(G_end) S0 + sum_s (P(s, end) o k_s) u_s^T
+// The solve kernel then walks, for every s, over t with k_s P(s, t) in registers (four lanes share s, 16 channels each at a time),
+// and leaves G o q and P(s, end) o k for the other two kernels, which are the same otherwise.  (16 heads of 128 x 128: 2,048 tokens
+// 669 us token by token, 301 in chunks; three prompts of 1,365, 900 and 513 697 and 421.)
 // Decays are multiplied on as running products, never divided by and never taken the logarithm of: 0 and 1 need no special case.
 // Everything is 32-bit.  The chunk table (built on the host with the step) is first[B+1] (index of each sequence's first
 // chunk), then (sequence, first row) per chunk.
@@ -305,19 +312,20 @@ __device__ __forceinline__ void copies_done() {
 // M [chunk][head][t][s]; gw [chunk][head][2][64]: G_t, then P(s, cnt - 1); and what the carry kernel fetches with one bulk copy
 // each: Kc [chunk][q/k head][64][KD], U0 [chunk][head][ceil(V/DV)][64][DV], Wt [chunk][head][d][64], zeros beyond the chunk's
 // tokens, D and V.
+template <bool PC>
 __global__ void __launch_bounds__(256, 2)
 delta_chunk_solve_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ decay,
                          const float* __restrict__ beta, const float* __restrict__ v, int v_stride, float* __restrict__ M,
                          float* __restrict__ gw, float* __restrict__ Kc, float* __restrict__ U0, float* __restrict__ Wt,
-                         const int* __restrict__ table,
+                         float* __restrict__ Qg, const int* __restrict__ table,
                          const int* __restrict__ cu_q, int B, int H, int G, int D, int V, int region) {
     extern __shared__ __align__(16) float sh[];
-    const int ld = ((D + 3) & ~3) + 4;
+    const int ld = PC ? DC_LD : ((D + 3) & ~3) + 4;
     float* ks = sh;                                   // [64][ld], and later X [64][256]
     float* qs = ks + DC * ld;                         // [64][ld]
     float* X = sh;
     float* at = sh + region;                          // [64 s][DC_LD]: A_ts, zeros for s >= t
-    float* ps = at + DC * DC_LD;                      // [64 s][DC_PLD]: P(s, t) for the tokens t >= s of s's own block of 16
+    float* ps = at + DC * DC_LD;                      // [64 s][DC_PLD]: P(s, t) for the tokens t >= s of s's own block of 16 (PC: [64 s][DC_LD], M_ts)
     __shared__ float sg[DC], sb[DC], sG[DC], sF[DC];  // g, beta, G, and the products from a block's first token on
     pdl_trigger();
     const int c = blockIdx.x, h = blockIdx.y, hg = h / (H / G), tid = threadIdx.x;
@@ -325,81 +333,151 @@ delta_chunk_solve_kernel(const float* __restrict__ qn, const float* __restrict__
     pdl_wait();
     if (tid < DC) {
         const bool in = tid < p.cnt;
-        sg[tid] = in ? decay[(size_t)(p.row0 + tid) * H + h] : 1.f;
+        if constexpr (!PC) sg[tid] = in ? decay[(size_t)(p.row0 + tid) * H + h] : 1.f;
         sb[tid] = in ? beta[(size_t)(p.row0 + tid) * H + h] : 0.f;
     }
     const size_t qk0 = ((size_t)p.row0 * G + hg) * D;
-    chunk_tile(ks, ld, kn + qk0, (size_t)G * D, p.cnt, D, (D & 3) == 0, tid, 256);
-    chunk_tile(qs, ld, qn + qk0, (size_t)G * D, p.cnt, D, (D & 3) == 0, tid, 256);
-    __syncthreads();
-    if (tid < DC) {                                   // thread s multiplies g_(s+1), g_(s+2), ... on, to its block's end
-        const int e = tid | 15;
-        float run = 1.f;
-        ps[tid * DC_PLD + (tid & 15)] = 1.f;
-        for (int t = tid + 1; t <= e; ++t) { run *= sg[t]; ps[tid * DC_PLD + (t & 15)] = run; }
-    } else if (tid < DC + 4) {
-        float run = 1.f;
-        for (int t = (tid - DC) * 16; t < (tid - DC) * 16 + 16; ++t) { run *= sg[t]; sF[t] = run; }
-    }
-    copies_done();
-    __syncthreads();
-    // P(s, t) across blocks: from s to its block's end, the whole blocks between, from t's block's start to t
-    auto between = [&](int s, int t) {
-        const int bs = s >> 4, bt = t >> 4;
-        if (bs == bt) return ps[s * DC_PLD + (t & 15)];
-        float w = ps[s * DC_PLD + 15];
-        for (int b = bs + 1; b < bt; ++b) w *= sF[16 * b + 15];
-        return w * sF[t];
-    };
-    if (tid < DC) {
-        sG[tid] = sg[0] * between(0, tid);
-        float* o = gw + ((size_t)c * H + h) * 2 * DC;
-        o[tid] = sG[tid];
-        o[DC + tid] = tid < p.cnt ? between(tid, p.cnt - 1) : 0.f;
-    }
-    const int tx = tid & 15, ty = tid >> 4;
-    float a[4][4], m[4][4];
-#pragma unroll
-    for (int x = 0; x < 4; ++x)
-#pragma unroll
-        for (int y = 0; y < 4; ++y) { a[x][y] = 0.f; m[x][y] = 0.f; }
     const int D4 = (D + 3) & ~3;
-    if (h % (H / G) == 0) {                               // one of the heads that share these keys leaves them for the carry kernel
-        float* o = Kc + ((size_t)c * G + hg) * DC * D4;
-        for (int i = tid; i < DC * D4 / 4; i += 256) {
-            const int r = i / (D4 >> 2);
-            *reinterpret_cast<float4*>(o + 4 * i) = *reinterpret_cast<const float4*>(ks + r * ld + 4 * (i - r * (D4 >> 2)));
-        }
-    }
-#pragma unroll 2
-    for (int i = 0; i < D4; i += 4) {
-        float4 kt[4], qt[4], kk[4];
+    float* Mo = M + ((size_t)c * H + h) * DC * DC;
+    if constexpr (PC) {
+        float* gs = qs + DC * ld;                     // [64][ld]
+        const size_t g0 = ((size_t)p.row0 * H + h) * D;
+        float* ko = Kc + ((size_t)c * H + h) * DC * D4;
+        float* qo = Qg + ((size_t)c * H + h) * DC * D4;
+        float* go = gw + ((size_t)c * H + h) * D4;
+        for (int i = tid; i < DC * DC_LD; i += 256) { at[i] = 0.f; ps[i] = 0.f; }
+        const int sl = tid >> 2, q4 = tid & 3, first = (tid >> 5) * 8;          // this lane's s, its share of the channels, the warp's first s
+        for (int d0 = 0; d0 < D; d0 += DC) {          // 64 channels at a time
+            const int nd = min(DC, D - d0), nd4 = (nd + 3) & ~3;
+            __syncthreads();                          // the channels before are used up (and at, ps are zero)
+            chunk_tile(ks, ld, kn + qk0 + d0, (size_t)G * D, p.cnt, nd, (D & 3) == 0, tid, 256);
+            chunk_tile(qs, ld, qn + qk0 + d0, (size_t)G * D, p.cnt, nd, (D & 3) == 0, tid, 256);
+            chunk_tile(gs, ld, decay + g0 + d0, (size_t)H * D, p.cnt, nd, (D & 3) == 0, tid, 256);
+            copies_done();
+            __syncthreads();
+            float4 r[4];
 #pragma unroll
-        for (int x = 0; x < 4; ++x) {
-            kt[x] = *reinterpret_cast<const float4*>(ks + (ty + 16 * x) * ld + i);
-            qt[x] = *reinterpret_cast<const float4*>(qs + (ty + 16 * x) * ld + i);
-            kk[x] = *reinterpret_cast<const float4*>(ks + (tx + 16 * x) * ld + i);
+            for (int i = 0; i < 4; ++i) {
+                const int e = 16 * i + 4 * q4;
+                r[i] = e < nd4 ? *reinterpret_cast<const float4*>(ks + sl * ld + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            for (int t = first; t < p.cnt; ++t) {
+                float da = 0.f, dm = 0.f;
+                const bool after = t > sl;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int e = 16 * i + 4 * q4;
+                    if (16 * i < nd4) {               // (whole warps; a lane beyond the last channel multiplies zeros)
+                        const int f = e < nd4 ? e : 0;
+                        const float4 g = *reinterpret_cast<const float4*>(gs + t * ld + f), k = *reinterpret_cast<const float4*>(ks + t * ld + f);
+                        const float4 q = *reinterpret_cast<const float4*>(qs + t * ld + f);
+                        if (after) { r[i].x *= g.x; r[i].y *= g.y; r[i].z *= g.z; r[i].w *= g.w; }
+                        da = fmaf(r[i].x, k.x, fmaf(r[i].y, k.y, fmaf(r[i].z, k.z, fmaf(r[i].w, k.w, da))));
+                        dm = fmaf(r[i].x, q.x, fmaf(r[i].y, q.y, fmaf(r[i].z, q.z, fmaf(r[i].w, q.w, dm))));
+                    }
+                }
+                da += __shfl_xor_sync(0xffffffffu, da, 1); dm += __shfl_xor_sync(0xffffffffu, dm, 1);
+                da += __shfl_xor_sync(0xffffffffu, da, 2); dm += __shfl_xor_sync(0xffffffffu, dm, 2);
+                if (q4 == 0 && t >= sl) {
+                    if (after) at[sl * DC_LD + t] += da;
+                    ps[sl * DC_LD + t] += dm;
+                }
+            }
+            // a thread per channel: G_t o q_t and G_end going forward, P(s, end) o k_s going back
+            const int d = d0 + (tid & 63);
+            if (tid < 64 && d < D) {
+                float run = 1.f;
+#pragma unroll 4
+                for (int t = 0; t < p.cnt; ++t) { run *= gs[t * ld + tid]; qo[t * D4 + d] = qs[t * ld + tid] * run; }
+                go[d] = run;
+            } else if (tid >= 64 && tid < 128 && d < D4) {
+                float run = 1.f;
+                for (int t = p.cnt; t < DC; ++t) ko[t * D4 + d] = 0.f;
+#pragma unroll 4
+                for (int t = p.cnt - 1; t >= 0; --t) {
+                    const float k = d < D ? ks[t * ld + (tid & 63)] : 0.f;
+                    ko[t * D4 + d] = k * run;
+                    run *= d < D ? gs[t * ld + (tid & 63)] : 0.f;
+                }
+                if (d >= D) go[d] = 0.f;
+            }
+        }
+        __syncthreads();
+        for (int i = tid; i < DC * DC; i += 256) {
+            Mo[i] = ps[(i & 63) * DC_LD + (i >> 6)];
+            at[(i >> 6) * DC_LD + (i & 63)] *= sb[i & 63];
+        }
+    } else {
+        chunk_tile(ks, ld, kn + qk0, (size_t)G * D, p.cnt, D, (D & 3) == 0, tid, 256);
+        chunk_tile(qs, ld, qn + qk0, (size_t)G * D, p.cnt, D, (D & 3) == 0, tid, 256);
+        __syncthreads();
+        if (tid < DC) {                                   // thread s multiplies g_(s+1), g_(s+2), ... on, to its block's end
+            const int e = tid | 15;
+            float run = 1.f;
+            ps[tid * DC_PLD + (tid & 15)] = 1.f;
+            for (int t = tid + 1; t <= e; ++t) { run *= sg[t]; ps[tid * DC_PLD + (t & 15)] = run; }
+        } else if (tid < DC + 4) {
+            float run = 1.f;
+            for (int t = (tid - DC) * 16; t < (tid - DC) * 16 + 16; ++t) { run *= sg[t]; sF[t] = run; }
+        }
+        copies_done();
+        __syncthreads();
+        // P(s, t) across blocks: from s to its block's end, the whole blocks between, from t's block's start to t
+        auto between = [&](int s, int t) {
+            const int bs = s >> 4, bt = t >> 4;
+            if (bs == bt) return ps[s * DC_PLD + (t & 15)];
+            float w = ps[s * DC_PLD + 15];
+            for (int b = bs + 1; b < bt; ++b) w *= sF[16 * b + 15];
+            return w * sF[t];
+        };
+        if (tid < DC) {
+            sG[tid] = sg[0] * between(0, tid);
+            float* o = gw + ((size_t)c * H + h) * 2 * DC;
+            o[tid] = sG[tid];
+            o[DC + tid] = tid < p.cnt ? between(tid, p.cnt - 1) : 0.f;
+        }
+        const int tx = tid & 15, ty = tid >> 4;
+        float a[4][4], m[4][4];
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+#pragma unroll
+            for (int y = 0; y < 4; ++y) { a[x][y] = 0.f; m[x][y] = 0.f; }
+        if (h % (H / G) == 0) {                               // one of the heads that share these keys leaves them for the carry kernel
+            float* o = Kc + ((size_t)c * G + hg) * DC * D4;
+            for (int i = tid; i < DC * D4 / 4; i += 256) {
+                const int r = i / (D4 >> 2);
+                *reinterpret_cast<float4*>(o + 4 * i) = *reinterpret_cast<const float4*>(ks + r * ld + 4 * (i - r * (D4 >> 2)));
+            }
+        }
+#pragma unroll 2
+        for (int i = 0; i < D4; i += 4) {
+            float4 kt[4], qt[4], kk[4];
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                kt[x] = *reinterpret_cast<const float4*>(ks + (ty + 16 * x) * ld + i);
+                qt[x] = *reinterpret_cast<const float4*>(qs + (ty + 16 * x) * ld + i);
+                kk[x] = *reinterpret_cast<const float4*>(ks + (tx + 16 * x) * ld + i);
+            }
+#pragma unroll
+            for (int x = 0; x < 4; ++x)
+#pragma unroll
+                for (int y = 0; y <= x; ++y) {
+                    a[x][y] = fmaf(kt[x].x, kk[y].x, a[x][y]); a[x][y] = fmaf(kt[x].y, kk[y].y, a[x][y]);
+                    a[x][y] = fmaf(kt[x].z, kk[y].z, a[x][y]); a[x][y] = fmaf(kt[x].w, kk[y].w, a[x][y]);
+                    m[x][y] = fmaf(qt[x].x, kk[y].x, m[x][y]); m[x][y] = fmaf(qt[x].y, kk[y].y, m[x][y]);
+                    m[x][y] = fmaf(qt[x].z, kk[y].z, m[x][y]); m[x][y] = fmaf(qt[x].w, kk[y].w, m[x][y]);
+                }
         }
 #pragma unroll
         for (int x = 0; x < 4; ++x)
 #pragma unroll
-            for (int y = 0; y <= x; ++y) {
-                a[x][y] = fmaf(kt[x].x, kk[y].x, a[x][y]); a[x][y] = fmaf(kt[x].y, kk[y].y, a[x][y]);
-                a[x][y] = fmaf(kt[x].z, kk[y].z, a[x][y]); a[x][y] = fmaf(kt[x].w, kk[y].w, a[x][y]);
-                m[x][y] = fmaf(qt[x].x, kk[y].x, m[x][y]); m[x][y] = fmaf(qt[x].y, kk[y].y, m[x][y]);
-                m[x][y] = fmaf(qt[x].z, kk[y].z, m[x][y]); m[x][y] = fmaf(qt[x].w, kk[y].w, m[x][y]);
+            for (int y = 0; y < 4; ++y) {
+                const int t = ty + 16 * x, s = tx + 16 * y;
+                const float w = y <= x && s <= t ? between(s, t) : 0.f;
+                at[s * DC_LD + t] = s < t ? sb[t] * w * a[x][y] : 0.f;
+                Mo[t * DC + s] = s <= t ? w * m[x][y] : 0.f;
             }
     }
-    float* Mo = M + ((size_t)c * H + h) * DC * DC;
-#pragma unroll
-    for (int x = 0; x < 4; ++x)
-#pragma unroll
-        for (int y = 0; y < 4; ++y) {
-            const int t = ty + 16 * x, s = tx + 16 * y;
-            const float w = y <= x && s <= t ? between(s, t) : 0.f;
-            at[s * DC_LD + t] = s < t ? sb[t] * w * a[x][y] : 0.f;
-            Mo[t * DC + s] = s <= t ? w * m[x][y] : 0.f;
-        }
     __syncthreads();                                  // A is in place, the tiles of k and q are used up
     const int VP = (V + DV - 1) / DV * DV;
     for (int j0 = 0; j0 < VP + D; j0 += DC_COLS) {
@@ -413,10 +491,16 @@ delta_chunk_solve_kernel(const float* __restrict__ qn, const float* __restrict__
                              : Wt + (((size_t)c * H + h) * D + (j - VP)) * DC;
             // a block's sixteen inputs are asked for while the block before is worked on; rows beyond the chunk's tokens repeat the
             // last one and are multiplied by a beta of zero
-            float next[16];
+            float next[16], gnext[PC ? 16 : 1], run = 1.f;
+            const float* gsrc = PC && !is_v ? decay + ((size_t)p.row0 * H + h) * D + (j - VP) : nullptr;
             auto ask = [&](int t0) {
 #pragma unroll
                 for (int r = 0; r < 16; ++r) next[r] = src[(size_t)min(t0 + r, p.cnt - 1) * stride];
+                if constexpr (PC) {
+                    if (!is_v)
+#pragma unroll
+                        for (int r = 0; r < 16; ++r) gnext[r] = gsrc[(size_t)min(t0 + r, p.cnt - 1) * H * D];
+                }
             };
             ask(0);
             for (int t0 = 0; t0 < DC; t0 += 16) {
@@ -425,8 +509,16 @@ delta_chunk_solve_kernel(const float* __restrict__ qn, const float* __restrict__
                     for (int r = 0; r < 16; ++r) wo[is_v ? (t0 + r) * DV : t0 + r] = 0.f;
                     continue;
                 }
+                if constexpr (PC) {
 #pragma unroll
-                for (int r = 0; r < 16; ++r) x[r] = next[r] * (is_v ? live * sb[t0 + r] : sb[t0 + r] * sG[t0 + r]);
+                    for (int r = 0; r < 16; ++r) {
+                        if (!is_v) run *= gnext[r];
+                        x[r] = next[r] * (is_v ? live * sb[t0 + r] : sb[t0 + r] * run);
+                    }
+                } else {
+#pragma unroll
+                    for (int r = 0; r < 16; ++r) x[r] = next[r] * (is_v ? live * sb[t0 + r] : sb[t0 + r] * sG[t0 + r]);
+                }
                 if (t0 + 16 < p.cnt) ask(t0 + 16);
                 for (int s = 0; s < t0; ++s) {
                     const float xs = X[s * DC_COLS + tid];
@@ -473,7 +565,7 @@ __device__ __forceinline__ void bulk_copy(float* dst, const float* src, uint32_t
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(smem_u32(dst)), "l"(src), "r"(4 * floats), "r"(bar) : "memory");
 }
-template <int TILES>                                  // row tiles of 128 a thread holds: 1 (D <= 128, two stages), 2 (one stage)
+template <int TILES, bool PC>                         // row tiles of 128 a thread holds: 1 (D <= 128, two stages), 2 (one stage)
 __global__ void __launch_bounds__(256, 1)
 delta_chunk_carry_kernel(const float* __restrict__ Kc, const float* __restrict__ U0, const float* __restrict__ Wt,
                          const float* __restrict__ gw, float* __restrict__ state, float* __restrict__ U, float* __restrict__ LS,
@@ -482,7 +574,8 @@ delta_chunk_carry_kernel(const float* __restrict__ Kc, const float* __restrict__
     constexpr int STAGES = TILES == 1 ? 2 : 1;
     extern __shared__ __align__(16) float sh[];
     const int KD = (D + 3) & ~3;
-    const int stage = D * DC + DC * KD + DC * DV + 2 * DC;      // W, keys, U0, the decays' products
+    const int GW = PC ? KD : 2 * DC;
+    const int stage = D * DC + DC * KD + DC * DV + GW;          // W, keys, U0, the decays' products
     float* Ss = sh + STAGES * stage;                  // [KD][DV]
     float* red = Ss + KD * DV;                        // [8][(64 + 16) * DV]
     float* Us = red + 8 * 80 * DV;                    // [64][DV]
@@ -511,9 +604,9 @@ delta_chunk_carry_kernel(const float* __restrict__ Kc, const float* __restrict__
         const uint32_t bar = smem_u32(&bars[buf]);
         mbar_expect_tx(bar, 4u * (uint32_t)stage);
         bulk_copy(w, Wt + ((size_t)c * H + h) * D * DC, D * DC, bar);
-        bulk_copy(w + D * DC, Kc + ((size_t)c * G + hg) * DC * KD, DC * KD, bar);
+        bulk_copy(w + D * DC, Kc + (PC ? (size_t)c * H + h : (size_t)c * G + hg) * DC * KD, DC * KD, bar);
         bulk_copy(w + D * DC + DC * KD, U0 + (((size_t)c * H + h) * gridDim.x + blockIdx.x) * DC * DV, DC * DV, bar);
-        bulk_copy(w + D * DC + DC * KD + DC * DV, gw + ((size_t)c * H + h) * 2 * DC, 2 * DC, bar);
+        bulk_copy(w + D * DC + DC * KD + DC * DV, gw + ((size_t)c * H + h) * GW, GW, bar);
     };
     float s[TILES][4][4];
 #pragma unroll
@@ -605,11 +698,10 @@ delta_chunk_carry_kernel(const float* __restrict__ Kc, const float* __restrict__
                         if (cc + q < nc) uo[q] = xs[q];
                 }
             }
-            const float wt = g[DC + t];                   // P(t, end); 0 beyond the chunk's tokens
+            const float wt = PC ? 1.f : g[DC + t];        // P(t, end); 0 beyond the chunk's tokens (PC: the keys carry it)
             *reinterpret_cast<float4*>(Us + t * DV + cc) = make_float4(x.x * wt, x.y * wt, x.z * wt, x.w * wt);
         }
         __syncthreads();
-        const float gend = g[cnt - 1];
         float x[TILES][4][4];
 #pragma unroll
         for (int i = 0; i < TILES; ++i) {
@@ -644,6 +736,7 @@ delta_chunk_carry_kernel(const float* __restrict__ Kc, const float* __restrict__
                     const int d = dg + r + 128 * i;
                     if (d >= KD) continue;
                     const float4 y = *reinterpret_cast<const float4*>(red + d * DV + cc);
+                    const float gend = PC ? g[d] : g[cnt - 1];
                     s[i][r][0] = fmaf(gend, s[i][r][0], x[i][r][0] + y.x); s[i][r][1] = fmaf(gend, s[i][r][1], x[i][r][1] + y.y);
                     s[i][r][2] = fmaf(gend, s[i][r][2], x[i][r][2] + y.z); s[i][r][3] = fmaf(gend, s[i][r][3], x[i][r][3] + y.w);
                     *reinterpret_cast<float4*>(Ss + d * DV + cc) = make_float4(s[i][r][0], s[i][r][1], s[i][r][2], s[i][r][3]);
@@ -662,6 +755,7 @@ delta_chunk_carry_kernel(const float* __restrict__ Kc, const float* __restrict__
 }
 
 // grid (chunk, head, ceil(V / DO)); 256 threads: thread (ty, tx) owns rows ty + 16 x and columns 4 tx .. 4 tx + 3.
+template <bool PC>                                     // PC: qn holds the chunks' G o q
 __global__ void __launch_bounds__(256)
 delta_chunk_out_kernel(const float* __restrict__ qn, const float* __restrict__ M, const float* __restrict__ gw,
                        const float* __restrict__ U, const float* __restrict__ LS, float* __restrict__ o, const int* __restrict__ table,
@@ -677,8 +771,9 @@ delta_chunk_out_kernel(const float* __restrict__ qn, const float* __restrict__ M
     const int nc = min(DO, V - j0);
     pdl_wait();
     chunk_tile(lhs, ld, M + ((size_t)c * H + h) * DC * DC, DC, p.cnt, DC, true, tid, 256);
-    chunk_tile(lhs + DC, ld, qn + ((size_t)p.row0 * G + hg) * D, (size_t)G * D, p.cnt, D, (D & 3) == 0, tid, 256);
-    if (tid < DC) sG[tid] = gw[((size_t)c * H + h) * 2 * DC + tid];
+    if constexpr (PC) chunk_tile(lhs + DC, ld, qn + ((size_t)c * H + h) * DC * D4, D4, p.cnt, D, (D & 3) == 0, tid, 256);
+    else chunk_tile(lhs + DC, ld, qn + ((size_t)p.row0 * G + hg) * D, (size_t)G * D, p.cnt, D, (D & 3) == 0, tid, 256);
+    if (tid < DC) sG[tid] = PC ? 1.f : gw[((size_t)c * H + h) * 2 * DC + tid];
     const bool vec = (V & 3) == 0;
     const float* us = U + (size_t)p.row0 * H * V + h * V + j0;
     const float* ss = LS + ((size_t)c * H + h) * D * V + j0;
@@ -742,54 +837,73 @@ static int chunk_smem(const void* kernel, size_t bytes, size_t* configured) {
     return 0;
 }
 
-extern "C" {
-// Floats of scratch memory that rf_delta_chunked needs for T_ tokens in n_chunks chunks.
-long long rf_delta_chunked_scratch(int n_chunks, int H, int G, int D, int V, int T_) {
+static long long delta_chunked_floats(bool pc, int n_chunks, int H, int G, int D, int V, int T_) {
     const long long D4 = (D + 3) & ~3, VP = (V + DV - 1) / DV * DV;
-    return (long long)n_chunks * H * (DC * DC + 2 * DC + (long long)D * DC + VP * DC + (long long)D * V) + n_chunks * G * DC * D4 +
-           (long long)T_ * H * V + 16;
+    return (long long)n_chunks * H * (DC * DC + (pc ? D4 : 2 * DC) + (long long)D * DC + VP * DC + (long long)D * V) +
+           (long long)n_chunks * (pc ? 2 * H : G) * DC * D4 + (long long)T_ * H * V + 16;
+}
+
+template <bool PC>
+static int delta_chunked(const float* qn, const float* kn, const float* decay, const float* beta, const float* v, int v_stride,
+                         float* state, float* o, float* scratch, const int* table, int n_chunks, const int* cu_q, const int* seq_slot,
+                         int B, int H, int G, int D, int V, int T_, int* status, cudaStream_t st) {
+    if (B <= 0 || n_chunks <= 0) return 0;
+    if (H <= 0 || G <= 0 || H % G || D <= 0 || V <= 0 || H > 65535 || B > 65535) return RF_ERR_BAD_ARG;
+    if (D > 256 || status == nullptr || (reinterpret_cast<uintptr_t>(scratch) & 15) || (reinterpret_cast<uintptr_t>(kn) & 15) ||
+        (reinterpret_cast<uintptr_t>(qn) & 15) || (PC && (reinterpret_cast<uintptr_t>(decay) & 15)))
+        return RF_ERR_UNSUPPORTED;
+    const size_t ch = (size_t)n_chunks * H;
+    const int D4 = (D + 3) & ~3, VP = (V + DV - 1) / DV * DV, GW = PC ? D4 : 2 * DC;
+    float* M = scratch;
+    float* gw = M + ch * DC * DC;
+    float* Wt = gw + ch * GW;
+    float* U0 = Wt + ch * D * DC;
+    float* Kc = U0 + ch * VP * DC;
+    float* Qg = Kc + (PC ? ch : (size_t)n_chunks * G) * DC * D4;
+    float* U = Qg + (PC ? ch * DC * D4 : 0);
+    float* LS = U + ((size_t)T_ * H * V + 3) / 4 * 4;
+    int region = PC ? 3 * DC * DC_LD : 2 * DC * (D4 + 4);
+    if (region < DC * DC_COLS) region = DC * DC_COLS;
+    const size_t smem1 = ((size_t)region + DC * DC_LD + DC * (PC ? DC_LD : DC_PLD)) * sizeof(float);
+    const int tiles = D4 <= 128 ? 1 : 2;
+    const size_t smem2 = ((size_t)(tiles == 1 ? 2 : 1) * (D * DC + DC * D4 + DC * DV + GW) + D4 * DV + 8 * 80 * DV + DC * DV) * sizeof(float);
+    const size_t smem3 = ((size_t)DC * (DC + D4 + 4) + (DC + D4) * DO) * sizeof(float);
+    static size_t set1 = 48 * 1024, set2[2] = {48 * 1024, 48 * 1024}, set3 = 48 * 1024;
+    const auto solve = delta_chunk_solve_kernel<PC>;
+    const auto carry = tiles == 1 ? delta_chunk_carry_kernel<1, PC> : delta_chunk_carry_kernel<2, PC>;
+    const auto outk = delta_chunk_out_kernel<PC>;
+    int e;
+    if ((e = chunk_smem((const void*)solve, smem1, &set1)) || (e = chunk_smem((const void*)carry, smem2, &set2[tiles - 1])) ||
+        (e = chunk_smem((const void*)outk, smem3, &set3)))
+        return e;
+    rf_launch(solve, dim3(n_chunks, H), dim3(256), smem1, st, qn, kn, decay, beta, v, v_stride, M, gw, Kc, U0, Wt, Qg, table, cu_q, B, H, G, D, V,
+              region);
+    RF_LAUNCH_CHECK();
+    rf_launch(carry, dim3(VP / DV, H, B), dim3(256), smem2, st, (const float*)Kc, (const float*)U0, (const float*)Wt, (const float*)gw,
+              state, U, LS, table, cu_q, seq_slot, B, H, G, D, V, status);
+    RF_LAUNCH_CHECK();
+    rf_launch(outk, dim3(n_chunks, H, (V + DO - 1) / DO), dim3(256), smem3, st, PC ? (const float*)Qg : qn, (const float*)M, (const float*)gw,
+              (const float*)U, (const float*)LS, o, table, cu_q, B, H, G, D, V);
+    RF_LAUNCH_CHECK();
+    return 0;
+}
+
+extern "C" {
+// Floats of scratch memory that rf_delta_chunked (channels: rf_delta_chunked_channels) needs for T_ tokens in n_chunks chunks.
+long long rf_delta_chunked_scratch(int n_chunks, int H, int G, int D, int V, int T_, int channels) {
+    return delta_chunked_floats(channels != 0, n_chunks, H, G, D, V, T_);
 }
 // What rf_delta_scan computes with per_head decays, for prompts (see above).  table: first[B+1], then n_chunks pairs (sequence,
 // first row of the chunk among the sequence's new tokens), in the order of the sequences.
 int rf_delta_chunked(const float* qn, const float* kn, const float* decay, const float* beta, const float* v, int v_stride,
                      float* state, float* o, float* scratch, const int* table, int n_chunks, const int* cu_q, const int* seq_slot,
                      int B, int H, int G, int D, int V, int T_, int* status, cudaStream_t st) {
-    if (B <= 0 || n_chunks <= 0) return 0;
-    if (H <= 0 || G <= 0 || H % G || D <= 0 || V <= 0 || H > 65535 || B > 65535) return RF_ERR_BAD_ARG;
-    if (D > 256 || status == nullptr || (reinterpret_cast<uintptr_t>(scratch) & 15) || (reinterpret_cast<uintptr_t>(kn) & 15) ||
-        (reinterpret_cast<uintptr_t>(qn) & 15))
-        return RF_ERR_UNSUPPORTED;
-    const size_t ch = (size_t)n_chunks * H;
-    const int D4 = (D + 3) & ~3, VP = (V + DV - 1) / DV * DV;
-    float* M = scratch;
-    float* gw = M + ch * DC * DC;
-    float* Wt = gw + ch * 2 * DC;
-    float* U0 = Wt + ch * D * DC;
-    float* Kc = U0 + ch * VP * DC;
-    float* U = Kc + (size_t)n_chunks * G * DC * D4;
-    float* LS = U + ((size_t)T_ * H * V + 3) / 4 * 4;
-    int region = 2 * DC * (D4 + 4);
-    if (region < DC * DC_COLS) region = DC * DC_COLS;
-    const size_t smem1 = ((size_t)region + DC * DC_LD + DC * DC_PLD) * sizeof(float);
-    const int tiles = D4 <= 128 ? 1 : 2;
-    const size_t smem2 = ((size_t)(tiles == 1 ? 2 : 1) * (D * DC + DC * D4 + DC * DV + 2 * DC) + D4 * DV + 8 * 80 * DV + DC * DV) * sizeof(float);
-    const size_t smem3 = ((size_t)DC * (DC + D4 + 4) + (DC + D4) * DO) * sizeof(float);
-    static size_t set1 = 48 * 1024, set2[2] = {48 * 1024, 48 * 1024}, set3 = 48 * 1024;
-    const auto carry = tiles == 1 ? delta_chunk_carry_kernel<1> : delta_chunk_carry_kernel<2>;
-    int e;
-    if ((e = chunk_smem((const void*)delta_chunk_solve_kernel, smem1, &set1)) ||
-        (e = chunk_smem((const void*)carry, smem2, &set2[tiles - 1])) ||
-        (e = chunk_smem((const void*)delta_chunk_out_kernel, smem3, &set3)))
-        return e;
-    rf_launch(delta_chunk_solve_kernel, dim3(n_chunks, H), dim3(256), smem1, st, qn, kn, decay, beta, v, v_stride, M, gw, Kc, U0, Wt, table,
-              cu_q, B, H, G, D, V, region);
-    RF_LAUNCH_CHECK();
-    rf_launch(carry, dim3(VP / DV, H, B), dim3(256), smem2, st, (const float*)Kc, (const float*)U0, (const float*)Wt, (const float*)gw,
-              state, U, LS, table, cu_q, seq_slot, B, H, G, D, V, status);
-    RF_LAUNCH_CHECK();
-    rf_launch(delta_chunk_out_kernel, dim3(n_chunks, H, (V + DO - 1) / DO), dim3(256), smem3, st, qn, (const float*)M, (const float*)gw,
-              (const float*)U, (const float*)LS, o, table, cu_q, B, H, G, D, V);
-    RF_LAUNCH_CHECK();
-    return 0;
+    return delta_chunked<false>(qn, kn, decay, beta, v, v_stride, state, o, scratch, table, n_chunks, cu_q, seq_slot, B, H, G, D, V, T_, status, st);
+}
+// The same with a decay per key channel: decay [T, H*D].
+int rf_delta_chunked_channels(const float* qn, const float* kn, const float* decay, const float* beta, const float* v, int v_stride,
+                              float* state, float* o, float* scratch, const int* table, int n_chunks, const int* cu_q, const int* seq_slot,
+                              int B, int H, int G, int D, int V, int T_, int* status, cudaStream_t st) {
+    return delta_chunked<true>(qn, kn, decay, beta, v, v_stride, state, o, scratch, table, n_chunks, cu_q, seq_slot, B, H, G, D, V, T_, status, st);
 }
 }

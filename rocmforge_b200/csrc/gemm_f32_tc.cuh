@@ -52,9 +52,10 @@ template <int BN> struct FsLayout {
     static constexpr uint32_t stage_bytes = w_bytes + x_bytes;
     static constexpr uint32_t plane_bytes = BN * 64;               // bf16 [BN][32]
     static constexpr int stages = BN == 128 ? 4 : 6;
-    static constexpr uint32_t tmem_cols = BN == 128 ? 512 : (BN == 16 ? 128 : 256);
-    static constexpr int n_bars = 2 * stages + 8;
-    static constexpr size_t smem = (size_t)stages * stage_bytes + 2 * 3 * plane_bytes + n_bars * 8 + 16 + 1024;
+    static constexpr uint32_t tmem_cols = BN >= 64 ? 512 : 256;          // 2 BN + 48 bufs
+    static constexpr int bufs = BN >= 64 ? 4 : 2;                  // split stages on their way to the MMAs (1,999 x 9,728 x 896 with 2: 194 us, with 4: 186)
+    static constexpr int n_bars = 2 * stages + 2 * bufs + 4;
+    static constexpr size_t smem = (size_t)stages * stage_bytes + bufs * 3 * plane_bytes + n_bars * 8 + 16 + 1024;
 };
 
 // K-major tile of 64-byte rows with the 64-byte swizzle: 8-row groups are 512 bytes apart.
@@ -88,19 +89,19 @@ template <int BN>
 __global__ void __launch_bounds__(FsLayout<BN>::threads, FsLayout<BN>::ctas)
 gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const FsParams p) {
     using L = FsLayout<BN>;
-    constexpr int S = L::stages, EW = L::epi_warps, CW = L::conv_warps;
+    constexpr int S = L::stages, EW = L::epi_warps, CW = L::conv_warps, NB = L::bufs;
     constexpr int EC = BN / (EW / 4);                     // columns of an epilogue warp
-    constexpr uint32_t TM_A = 2 * BN;                     // tensor memory: two accumulators, then two stages of weights (3 x 16 columns)
+    constexpr uint32_t TM_A = 2 * BN;                     // tensor memory: two accumulators, then split weights (3 x 16 columns a stage)
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t* planes = smem + S * L::stage_bytes;          // [2 buffers][3 parts][BN rows][64 bytes]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(planes + 2 * 3 * L::plane_bytes);
+    uint8_t* planes = smem + S * L::stage_bytes;          // [NB buffers][3 parts][BN rows][64 bytes]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(planes + NB * 3 * L::plane_bytes);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + L::n_bars);
     __shared__ int abort_flag;
     const uint32_t b_raw_full = smem_u32(bars), b_raw_empty = b_raw_full + 8 * S;
-    const uint32_t b_cv_full = b_raw_empty + 8 * S, b_cv_empty = b_cv_full + 16;
-    const uint32_t b_acc_full = b_cv_empty + 16, b_acc_empty = b_acc_full + 16;
+    const uint32_t b_cv_full = b_raw_empty + 8 * S, b_cv_empty = b_cv_full + 8 * NB;
+    const uint32_t b_acc_full = b_cv_empty + 8 * NB, b_acc_empty = b_acc_full + 16;
 
     pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -110,9 +111,11 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             mbar_init(b_raw_full + 8 * s, 1);
             mbar_init(b_raw_empty + 8 * s, 4);
         }
-        for (int b = 0; b < 2; ++b) {
+        for (int b = 0; b < NB; ++b) {
             mbar_init(b_cv_full + 8 * b, 4);
             mbar_init(b_cv_empty + 8 * b, 1);
+        }
+        for (int b = 0; b < 2; ++b) {
             mbar_init(b_acc_full + 8 * b, 1);
             mbar_init(b_acc_empty + 8 * b, EW);
         }
@@ -178,13 +181,13 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 int m0, n0, kb0, kb1;
                 tile_of(t, m0, n0, kb0, kb1);
                 for (int kb = kb0; kb < kb1; ++kb, ++it) {
-                    const int b = it & 1;
+                    const int b = it & 1, c = it % NB;
                     ok = mbar_wait(b_acc_empty + 8 * b, ((it >> 1) & 1) ^ 1, &abort_flag) &&
-                         mbar_wait(b_cv_full + 8 * b, (it >> 1) & 1, &abort_flag);
+                         mbar_wait(b_cv_full + 8 * c, (it / NB) & 1, &abort_flag);
                     if (!ok) break;
                     tcgen05_fence_after();
-                    const uint32_t d = tmem + b * BN, a = tmem + TM_A + b * 48;
-                    const uint32_t x = smem_u32(planes) + b * 3 * L::plane_bytes;
+                    const uint32_t d = tmem + b * BN, a = tmem + TM_A + c * 48;
+                    const uint32_t x = smem_u32(planes) + c * 3 * L::plane_bytes;
                     // parts (weight, token) of a product, the smallest first
                     constexpr int pw[6] = {2, 1, 0, 1, 0, 0}, px[6] = {0, 1, 2, 0, 1, 0};
 #pragma unroll
@@ -193,7 +196,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                         for (int h = 0; h < 2; ++h)       // 16 k each
                             tcgen05_mma_bf16_ts(d, a + pw[q] * 16 + h * 8, fs_desc(x + px[q] * L::plane_bytes + h * 32), idesc,
                                                 (q | h) ? 1u : 0u);
-                    tcgen05_commit(b_cv_empty + 8 * b);
+                    tcgen05_commit(b_cv_empty + 8 * c);
                     tcgen05_commit(b_acc_full + 8 * b);
                 }
             }
@@ -211,7 +214,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             tile_of(t, m0, n0, kb0, kb1);
             for (int kb = kb0; kb < kb1; ++kb, ++it) {
                 if (GROUPS == 2 && (it & 1) != group) continue;
-                const int s = it % S, b = it & 1;
+                const int s = it % S, b = it % NB;
                 ok = mbar_wait(b_raw_full + 8 * s, (it / S) & 1, &abort_flag);
                 if (!ok) break;
                 const uint32_t w = smem_u32(smem + s * L::stage_bytes) + row * 128, x = smem_u32(smem + s * L::stage_bytes) + L::w_bytes;
@@ -226,7 +229,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                         xv[2 * i + 1] = fs_lds(x + r * 128 + (((2 * c + 1) ^ (r & 7)) << 4));
                     }
                 }
-                ok = mbar_wait(b_cv_empty + 8 * b, ((it >> 1) & 1) ^ 1, &abort_flag);
+                ok = mbar_wait(b_cv_empty + 8 * b, ((it / NB) & 1) ^ 1, &abort_flag);
                 if (!ok) break;
                 tcgen05_fence_after();
                 const uint32_t ta = tmem + TM_A + b * 48 + ((uint32_t)(quarter * 32) << 16);

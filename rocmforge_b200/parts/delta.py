@@ -146,14 +146,16 @@ class GatedDeltaRule(Mixer):
     def cuda_modules(self, compute_dtype):
         return ["elementwise", "retention", "mamba2", "delta"]
 
-    # With one decay per head, prompts run the recurrence in chunks side by side; steps of few tokens per sequence, and decays per
-    # key channel, run it token by token.
+    # Prompts run the recurrence in chunks side by side, steps of few tokens per sequence token by token.
     CHUNKED_FROM = 17            # tokens of the step's longest portion from which the chunk table is built (one table for all parts)
-    CHUNKS_PAY_FROM = 160        # ... and from which this part's chunked kernels are faster (16 heads of 128 x 128 on one sequence:
-                                 # 64 tokens 44 against 26 us, 256 tokens 54 against 77 us, 2,048 tokens 224 against 560 us)
+    # ... and from which the chunked kernels are faster (16 heads of 128 x 128).  One decay per head: 64 tokens 44 against 26 us, 256
+    # tokens 54 against 77, 2,048 tokens 224 against 560.  A decay per key channel: 128 tokens 83 against 45, 256 90 against 87, 512 114
+    # against 170, 2,048 301 against 669, 1,365 + 900 + 513 421 against 697, 16 times 200 540 against 482.
+    CHUNKS_PAY_FROM = 160
+    CHANNEL_CHUNKS_PAY_FROM = 256
 
     def step_table_names(self):
-        return ("retention_chunks",) if self.decay_rank is None else ()
+        return ("retention_chunks",)
 
     def step_table(self, name, batch):
         return recurrence_chunk_table(batch, self.CHUNKED_FROM)
@@ -189,7 +191,8 @@ class GatedDeltaRule(Mixer):
         qn, kn, kq, decay, beta = kernels.delta_prepare(qkv, a, self.dt_bias, self.a_log, b, self.n_heads, self.qk_heads, self.dim,
                                                         self.q_scale, self.unit_eps)
         v = qkv[:, 2 * self.qk_size:]
-        table = ctx.tables.get("retention_chunks") if self.decay_rank is None and ctx.max_new >= self.CHUNKS_PAY_FROM else None
+        pays = self.CHUNKS_PAY_FROM if self.decay_rank is None else self.CHANNEL_CHUNKS_PAY_FROM
+        table = ctx.tables.get("retention_chunks") if ctx.max_new >= pays else None
         if table is not None and table.numel() > 0:
             o = kernels.delta_chunked(qn, kn, decay, beta, v, state_view["S"], table, ctx.cu_q, ctx.seq_slot, self.n_heads,
                                       self.qk_heads, self.dim, self.vdim)
