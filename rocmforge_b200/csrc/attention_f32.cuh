@@ -250,9 +250,10 @@ attention_f32_prompt_kernel(const __grid_constant__ CUtensorMap map_k, const __g
                 for (int j = 0; j < 32; ++j) s[c0 + j] = __uint_as_float(r[j]);
             }
             if (!(key0 + KT - 1 <= pos_first && rows_here == 128 && key0 >= rf_first_key(pos_last, window))) {
+                const int last = row_ok ? pos_i - key0 : -1, low = lo_i - key0;
 #pragma unroll
                 for (int j = 0; j < KT; ++j)
-                    if (!(row_ok && key0 + j <= pos_i && key0 + j >= lo_i)) s[j] = -INFINITY;
+                    if (j > last || j < low) s[j] = -INFINITY;
             }
             float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
