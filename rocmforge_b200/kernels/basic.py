@@ -666,16 +666,23 @@ def attention_prefill(q: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: 
     return out
 
 
-def decode_splits(B: int, n_kv_heads: int, longest: int | None = None, window: int | None = None) -> int:
+def decode_splits(B: int, n_kv_heads: int, longest: int | None = None, window: int | None = None, head_dim: int | None = None) -> int:
     """CTAs that share one (sequence, kv head) in the clustered decode attention, from the batch and the
     longest context the launch may meet (a captured graph keeps its launch shape): about one CTA per SM,
     at most one CTA per page, and clusters of 8 only for very small batches, where nothing else fills the
     GPU.  Measured at 28 layers, 4 kv heads of 7 query heads, ms per decode step: batch 1 / 3,800 keys:
     1, 2, 4, 8 CTAs 3.45, 3.16, 2.92, 2.85; batch 8 / 1,900 keys: 3.21, 3.10, 3.01, 3.05; batch 32 / 512:
-    3.54, 3.54, 3.72; batch 64 / 512: 3.76, 4.04."""
+    3.54, 3.54, 3.72; batch 64 / 512: 3.76, 4.04.
+
+    Heads of at most 64 leave room for three to six CTAs on an SM: contexts of 1,024 and more are then shared further.  14 heads of 64
+    on 2 kv heads, us with 1, 2, 4 CTAs: batch 64 / 16..1,024 10.2, 9.0, 8.4; / 2,048 22.1, 16.6, 15.6; batch 32 / 16..1,024 8.6, 7.4,
+    5.9; but batch 64 / 100 keys 4.3, 5.4, 5.5."""
     pairs = max(1, B * n_kv_heads)
     s = 1
-    while s < 8 and pairs * s * 2 <= device_sm_count() * 7 // 8:          # 128 on the 148 SMs these numbers were taken on
+    most = device_sm_count() * 7 // 8                                     # 129 on the 148 SMs these numbers were taken on
+    if head_dim is not None and head_dim <= 64 and longest is not None and decode_pages(longest, window) >= 16:
+        most *= 4
+    while s < 8 and pairs * s * 2 <= most:
         s *= 2
     if s == 8 and pairs > 8:
         s = 4
@@ -707,7 +714,7 @@ def attention_decode_warps(q: torch.Tensor, n_heads: int, n_kv_heads: int, head_
                            sinks: torch.Tensor | None = None) -> torch.Tensor:
     """One new token per sequence over the bfloat16 paged cache: a cluster of ``splits`` CTAs per (sequence,
     kv head), every warp on its own tiles of keys; merged through distributed shared memory.  ``warps``
-    per CTA: 8 while one CTA per SM is enough for the batch, else 4 (three CTAs fit an SM).  ``softcap``, ``slopes``,
+    per CTA: 8 while one CTA per SM (two with heads of at most 64) is enough for the batch, else 4 (three CTAs fit an SM).  ``softcap``, ``slopes``,
     ``keep_first`` and ``sinks`` as in ``attention_generic``."""
     need_cuda(q, k_pages, v_pages, tok_seq, tok_pos, seq_slot, block_table)
     B = q.shape[0]
@@ -721,7 +728,7 @@ def attention_decode_warps(q: torch.Tensor, n_heads: int, n_kv_heads: int, head_
     if splits is None:
         splits = decode_splits(B, n_kv_heads)
     if warps is None:
-        warps = 8 if B * n_kv_heads * splits <= device_sm_count(q.device) else 4
+        warps = 8 if B * n_kv_heads * splits <= _sms(q.device) * (2 if head_dim <= 64 else 1) else 4
     if out is None:
         out = torch.empty((B, n_heads * head_dim), dtype=torch.bfloat16, device=q.device)
     from .tensor_core import status_word

@@ -344,7 +344,7 @@ class GQAAttention(Mixer):
                 return kernels.attention_decode_warps(
                     q, nh, nkv, hd, view.k_pages, view.v_pages, ctx.tok_seq, ctx.tok_pos, ctx.seq_slot,
                     view.block_table, self.scale, self.window,
-                    splits=kernels.decode_splits(ctx.B, nkv, longest, span), **shaped, **kept)
+                    splits=kernels.decode_splits(ctx.B, nkv, longest, span, hd), **shaped, **kept)
             if (not self.shaped_scores and not self.keep_first and not self.sink
                     and longest <= kernels.DECODE_CHUNK * kernels.DECODE_CHUNK):
                 # the earlier kernel: one CTA per 128-key chunk, partial results merged through scratch memory
