@@ -39,8 +39,9 @@ conv_silu_kernel(const T* __restrict__ src, int row_stride, int col0, const floa
 
 // The same for rows whose channels come in whole groups of four (C, col0 and row_stride multiples of 4): a thread owns
 // four neighbouring channels with their TAPS x 4 weights in registers and walks CV_TOK tokens; the inputs are 8- or
-// 16-byte loads, the result one 16-byte store.  The sum of a channel runs over the taps in the same order as above.
-#define CV_TOK 4
+// 16-byte loads, the result one 16-byte store.  The sum of a channel runs over the taps in the same order as above.  Where the
+// tokens and those before them are one sequence's, all inputs are asked for at once and each is read once (every token looked its
+// sequence up and asked for its taps when the one before was done: 2,778 tokens of 6,144 channels 51 us, now 35).
 
 template <typename T> struct Vec4 {};
 template <> struct Vec4<float> {
@@ -57,10 +58,10 @@ template <> struct Vec4<__nv_bfloat16> {
     }
 };
 
-template <typename T, int TAPS>
+template <typename T, int TAPS, int CV_TOK>
 __global__ void __launch_bounds__(256)
-conv_silu_vec_kernel(const T* __restrict__ src, int row_stride, int col0, const float* __restrict__ state,
-                     const void* __restrict__ w, const void* __restrict__ bias, int w_is_f32, float* __restrict__ out,
+conv_silu_vec_kernel(const T* src, int row_stride, int col0, const float* __restrict__ state,
+                     const void* __restrict__ w, const void* __restrict__ bias, int w_is_f32, float* out,
                      const int* __restrict__ tok_seq, const int* __restrict__ cu_q, const int* __restrict__ seq_slot, int C,
                      int T_) {
     pdl_trigger();
@@ -74,7 +75,27 @@ conv_silu_vec_kernel(const T* __restrict__ src, int row_stride, int col0, const 
 #pragma unroll
         for (int j = 0; j < TAPS; ++j) wt[j][u] = load_vec(w, w_is_f32, (c + u) * TAPS + j);
     }
+    const int b0 = tok_seq[t0];
+    const bool whole = t0 + CV_TOK <= T_ && tok_seq[min(t0 + CV_TOK, T_) - 1] == b0 && t0 - cu_q[b0] >= TAPS - 1;
     pdl_wait();
+    if (whole) {
+        float x[CV_TOK + TAPS - 1][4];
+#pragma unroll
+        for (int i = 0; i < CV_TOK + TAPS - 1; ++i) Vec4<T>::load(src + (size_t)(t0 - (TAPS - 1) + i) * row_stride + col0 + c, x[i]);
+#pragma unroll
+        for (int i = 0; i < CV_TOK; ++i) {
+            float acc[4] = {bs[0], bs[1], bs[2], bs[3]};
+#pragma unroll
+            for (int j = 0; j < TAPS; ++j)
+#pragma unroll
+                for (int u = 0; u < 4; ++u) acc[u] = fmaf(wt[j][u], x[i + j][u], acc[u]);
+            float4 y;
+            y.x = acc[0] / (1.f + expf(-acc[0])); y.y = acc[1] / (1.f + expf(-acc[1]));
+            y.z = acc[2] / (1.f + expf(-acc[2])); y.w = acc[3] / (1.f + expf(-acc[3]));
+            *reinterpret_cast<float4*>(out + (size_t)(t0 + i) * C + c) = y;
+        }
+        return;
+    }
     for (int t = t0; t < t0 + CV_TOK && t < T_; ++t) {
         const int b = tok_seq[t];
         const int r = t - cu_q[b];
@@ -169,8 +190,9 @@ static int launch_conv(const void* src, int row_stride, int col0, float* state, 
     const bool groups_of_four = C % 4 == 0 && col0 % 4 == 0 && row_stride % 4 == 0 && taps <= 4 &&
                                 (reinterpret_cast<uintptr_t>(src) & 15) == 0 && (reinterpret_cast<uintptr_t>(state) & 15) == 0;
     if (groups_of_four && T_ >= 64) {
-        const dim3 grid((T_ + CV_TOK - 1) / CV_TOK, (C / 4 + 255) / 256);
-#define CONV_VEC(TAPS) rf_launch(conv_silu_vec_kernel<T, TAPS>, grid, dim3(256), 0, st, reinterpret_cast<const T*>(src), row_stride, \
+        const int tok = T_ >= 1024 ? 8 : 4;              // eight tokens a thread once that still makes a few blocks per SM
+        const dim3 grid((T_ + tok - 1) / tok, (C / 4 + 255) / 256);
+#define CONV_VEC(TAPS) rf_launch(tok == 8 ? conv_silu_vec_kernel<T, TAPS, 8> : conv_silu_vec_kernel<T, TAPS, 4>, grid, dim3(256), 0, st, reinterpret_cast<const T*>(src), row_stride, \
                                  col0, (const float*)state, w, bias, w_is_f32, out, tok_seq, cu_q, seq_slot, C, T_)
         if (taps == 1) CONV_VEC(1); else if (taps == 2) CONV_VEC(2); else if (taps == 3) CONV_VEC(3); else CONV_VEC(4);
 #undef CONV_VEC
