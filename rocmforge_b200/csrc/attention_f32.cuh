@@ -315,7 +315,7 @@ attention_f32_prompt_kernel(const __grid_constant__ CUtensorMap map_k, const __g
         tcgen05_fence_after();
         tcgen05_dealloc(tmem, 512);
     }
-    if (threadIdx.x == 0 && abort_flag && status) atomicExch(status, 8);
+    if (threadIdx.x == 0 && abort_flag && status) atomicExch(status, 12);
 }
 
 // ---------------------------------------------------------------- single tokens

@@ -353,7 +353,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         tcgen05_fence_after();
         tcgen05_dealloc(tmem, L::tmem_cols);
     }
-    if (threadIdx.x == 0 && abort_flag && p.status) atomicExch(p.status, 7);
+    if (threadIdx.x == 0 && abort_flag && p.status) atomicExch(p.status, 11);
 }
 
 // ---------------------------------------------------------------- host side

@@ -1,7 +1,6 @@
 // CUDA-core matrix product  Y[M,N] = X[M,K] * W[N,K]^T (+ bias), any M, N, K.
 //
-// It is the whole matrix path of the true 32-bit model (FFMA only: the tensor cores'
-// 32-bit mode rounds operands to TF32, which is what that path must not do) and the
+// It serves the true 32-bit model where gemm_f32_tc.cuh cannot (rows that are no whole 16 bytes, routed experts) and is the
 // fallback of the bfloat16 path for shapes the tensor-core kernel refuses.
 //
 // A CTA of 256 threads owns a BM x 128 tile of Y (BM = 16, 32, 64 or 128 tokens, chosen from M) and

@@ -29,15 +29,13 @@ class GatedDeltaRule(Mixer):
 
     One product makes q | k | v | W_b x | W_a1 x | W_g1 x in the compute dtype; the decay's second product stays 32-bit,
     and so do the convolution's result, the unit norms, beta, softplus, the decays, S, o and its norm.  Per sequence the
-    mixer keeps S [heads, dim, vdim] and the convolution's last taps-1 inputs, so a prompt may be cut anywhere; the
-    recurrence runs token by token in prompts too, so its sums do not depend on how a prompt is cut into portions (a token
-    decoded alone takes another kernel form, whose sums differ by rounding).
+    mixer keeps S [heads, dim, vdim] and the convolution's last taps-1 inputs, so a prompt may be cut anywhere; long portions
+    run in chunks (``kernels.delta_chunked``), short ones and decoded tokens token by token, which differs by rounding.
     ``names``: the tensors' names below the part's prefix (keys q, k, v, q_conv, k_conv, v_conv, b, a_log, dt_bias, a1, a2,
     g1, g2, norm, o; a and g in place of the low-rank pairs).
 
     What other designs change: ``decay_rank`` None: ONE decay per head, g = exp(-exp(A_log_h) softplus(W_a x + dt_bias)) with
-    W_a [heads, H] and dt_bias [heads]; W_a and W_b are then a small product of their own whose result stays 32-bit, and
-    prompts run in chunks (``kernels.delta_chunked``), which differs from the token-by-token form by rounding.
+    W_a [heads, H] and dt_bias [heads]; W_a and W_b are then a small product of their own whose result stays 32-bit.
     ``gate_rank`` None: the gate is one full matrix W_g x, part of the first product.  ``gate_fn`` "silu" instead of sigmoid.
     """
 

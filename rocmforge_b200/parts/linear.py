@@ -11,7 +11,8 @@ from .. import kernels
 class Linear:
     """A weight [N, K] (and an optional bias [N]) with the ways a part may apply it.
 
-    On the float32 path every product runs on CUDA cores with 32-bit operands and sums.
+    On the float32 path a product runs on the tensor cores too, every number as three bfloat16 parts (an exact sum), where TMA can
+    fetch the rows, and on CUDA cores otherwise; operands and sums are 32-bit either way.
     On the bfloat16 path the tensor-core kernels are used where the shape allows and the
     CUDA-core kernel otherwise; both accumulate in 32-bit.
     """
