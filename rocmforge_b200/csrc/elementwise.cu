@@ -281,11 +281,48 @@ add_rmsnorm_vec_kernel(float* __restrict__ h, const void* __restrict__ pending, 
     }
 }
 
+// The sum over a row of what 256 threads of a block would each have summed: the value of block_sum, bit for bit, where TPR threads
+// hold the row's pieces c = t + i TPR.  Piece c is thread c mod 256's there, so acc[k] is the part of thread t + k TPR; the 32-thread
+// sums of those are formed by the same pairs (the lanes share out the accumulators as they go) and then folded as block_sum folds
+// its warps': w and w ^ 4, w ^ 2, w ^ 1.  part: 8 floats of shared memory, of which each row of the block uses its own.
+template <int TPR>
+__device__ __forceinline__ float row_sum_256(float (&acc)[256 / TPR], float* part) {
+    constexpr int A = 256 / TPR;
+    const int lane = threadIdx.x & 31;
+    int off = 16;
+#pragma unroll
+    for (int n = A / 2; n >= 1; n >>= 1, off >>= 1) {
+        const bool up = lane & off;
+#pragma unroll
+        for (int k = 0; k < n; ++k) {
+            const float got = __shfl_xor_sync(0xffffffffu, up ? acc[k] : acc[k + n], off);
+            acc[k] = (up ? acc[k + n] : acc[k]) + got;
+        }
+    }
+    float v = acc[0];
+#pragma unroll
+    for (; off >= 1; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    off = 16;
+#pragma unroll
+    for (int n = A / 2; n >= 1; n >>= 1, off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);       // w ^ 4 first
+    if constexpr (TPR > 32) {
+        constexpr int W = TPR / 32;
+        if (lane == 0) part[threadIdx.x >> 5] = v;
+        __syncthreads();
+        const float* p = part + threadIdx.x / TPR * W;
+        if constexpr (W == 2) v = p[0] + p[1];
+        else if constexpr (W == 4) v = (p[0] + p[2]) + (p[1] + p[3]);
+        else v = ((p[0] + p[4]) + (p[2] + p[6])) + ((p[1] + p[5]) + (p[3] + p[7]));
+    }
+    return v;
+}
+
 // The norm of many rows without a pending update (a prompt step: the products add into the stream themselves), up to 8,192 wide.
 // TPR threads share a row and hold it in registers (at most eight 16-byte pieces each, all asked for at once), 256 / TPR rows a
 // block; up to 1,024 wide a row is one warp's, and no barrier stands between a row's loads and its stores.  Memory is the bound
-// (6 or 8 bytes an element).  Measured (us; a block a row, each row read twice): 33,361 x 896 78 -> 27 (6.6 TB/s),
-// 8,192 x 5,120 60 -> 43, 2,048 x 3,584 10.8 -> 10.9.
+// (6 or 8 bytes an element).  The sum is the one of a block of 256 threads a row, which up to 1,024 wide is also the few-row form's:
+// there a token's norm does not depend on the number of rows.  Measured (us; a block a row, each row read twice): 33,361 x 896 78 -> 27
+// (6.6 TB/s), 8,192 x 5,120 60 -> 43, 2,048 x 3,584 10.8 -> 10.9; a sum by one warp's own tree took as long within 1 %.
 // (h without __restrict__: loads through const __restrict__ pointers may be moved up across the wait for the kernel before.)
 template <typename T, int TPR>
 __global__ void __launch_bounds__(256, 5)
@@ -298,22 +335,15 @@ rmsnorm_rows_kernel(const float* h, const void* __restrict__ w, int w_is_f32, fl
     const float4* hrow = reinterpret_cast<const float4*>(h + (size_t)r * H);
     pdl_wait();
     float4 a[VPT];
-    float ss = 0.f;
+    float acc[256 / TPR] = {};
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
         const int c = t + i * TPR;
         a[i] = row_ok && c < nvec ? hrow[c] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) ss += a[i].x * a[i].x + a[i].y * a[i].y + a[i].z * a[i].z + a[i].w * a[i].w;
-    ss = warp_sum(ss);
-    if constexpr (TPR > 32) {
-        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ss;
-        __syncthreads();
-        ss = 0.f;
-#pragma unroll
-        for (int k = 0; k < TPR / 32; ++k) ss += part[threadIdx.x / TPR * (TPR / 32) + k];
-    }
+    for (int i = 0; i < VPT; ++i) acc[i % (256 / TPR)] += a[i].x * a[i].x + a[i].y * a[i].y + a[i].z * a[i].z + a[i].w * a[i].w;
+    const float ss = row_sum_256<TPR>(acc, part);
     if (!row_ok) return;
     const float inv = rsqrtf(ss / (float)H + eps);
     T* yrow = y + (size_t)r * H;

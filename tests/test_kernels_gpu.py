@@ -71,8 +71,8 @@ def test_add_rmsnorm(dt, H):
 @pytest.mark.parametrize("dt", DTS)
 @pytest.mark.parametrize("H", [24, 1000, 3584, 5120, 9000])
 def test_add_rmsnorm_of_a_prompt_step(dt, H):
-    """Many rows without a pending update take a kernel of their own (rows read twice, the second time from L1); with a
-    pending update or a row gather the other one.  All against the plain norm; the two kernels differ by the order of a
+    """Many rows without a pending update take a kernel of their own (rows in registers up to 8,192 wide, read twice beyond); with
+    a pending update or a row gather the other one.  All against the plain norm; the two kernels differ by the order of a
     row's sum of squares at most."""
     from rocmforge_b200 import kernels
     T = 700
@@ -89,6 +89,25 @@ def test_add_rmsnorm_of_a_prompt_step(dt, H):
         rows = torch.arange(0, T, 7, dtype=torch.int32, device=DEV)
         y3 = kernels.add_rmsnorm(h.clone(), w, 1e-6, dt, rows=rows)
         torch.testing.assert_close(y3.double(), P.rms_norm(h[rows.long()].double(), w.double(), 1e-6), **tol(dt))
+
+
+@pytest.mark.parametrize("dt", DTS)
+@pytest.mark.parametrize("H", [4, 124, 896, 1000, 1024, 1028, 1500, 2048, 2052, 3584, 4096])
+def test_a_prompt_steps_norm_has_the_bits_of_the_other_forms(dt, H):
+    """The prompt form (no pending update, 512 rows and more) sums a row as a block of 256 threads does: up to 1,024 wide that is what
+    a few rows get, and up to 4,096 wide what as many rows with a pending update (here of zeros) get.  An odd number of rows leaves
+    the last block with rows of its own."""
+    from rocmforge_b200 import kernels
+    T = 517
+    h = rnd(T, H, seed=H)
+    h[3] *= 1e4
+    h[5] *= 1e-4
+    w = rnd(H, seed=12) + 1.0
+    y = kernels.add_rmsnorm(h.clone(), w, 1e-6, dt)
+    assert torch.equal(y, kernels.add_rmsnorm(h.clone(), w, 1e-6, dt, pending=torch.zeros(1, T, H, device=DEV)))
+    if H <= 1024:
+        for a, b in ((0, 1), (3, 8), (500, T)):
+            assert torch.equal(y[a:b], kernels.add_rmsnorm(h[a:b].clone(), w, 1e-6, dt))
 
 
 @pytest.mark.parametrize("dt", DTS)
