@@ -1017,23 +1017,25 @@ weighted_add_kernel(float* __restrict__ h, const float* __restrict__ a0, int n0,
         y_next[base + c] = Cvt<T>::from_f32(row[c] * r * load_vec(w_next, w_is_f32, c));
 }
 
-// The same for many rows and whole addends (n0 = 1, n1 <= 1): TPR threads share a row, which stays in registers, as in
-// rmsnorm_rows_kernel.  (A block a row, element by element through shared memory: 2,778 rows of 2,048 41 us, now 23.)
-template <typename T, int TPR>
+// The same for many rows of at most 2,048 and whole addends (n0 = 1, n1 <= 1): 64 threads share a row, which stays in registers (VPT
+// 16-byte pieces a thread), four rows a block.  Memory is the bound.  Measured (us, a replayed graph, two addends; element by element
+// through shared memory): 2,778 rows of 2,048 27.7 -> 16.2, of 1,024 13.9 -> 6.4.
+// The sum of squares is that form's, bit for bit: a block of 256 threads gives its thread e mod 256 the element e, which is
+// number e mod 4 of piece t + 64 i here, so each thread carries four of those threads' sums, and they meet by the same pairs.
+template <typename T, int VPT>
 __global__ void __launch_bounds__(256, 4)
 weighted_add_rows_kernel(float* h, const float* a0, float s0, const float* a1, float s1, const void* __restrict__ w_next, int w_is_f32, float eps,
                          T* y_next, int H, int n_rows) {
-    constexpr int VPT = 8, RPB = 256 / TPR;
-    __shared__ float part[8];
+    __shared__ float part[8][4];
     pdl_trigger();
-    const int r = blockIdx.x * RPB + threadIdx.x / TPR, t = threadIdx.x % TPR, nvec = H >> 2;
+    const int r = blockIdx.x * 4 + (threadIdx.x >> 6), t = threadIdx.x & 63, lane = threadIdx.x & 31, nvec = H >> 2;
     const size_t base = (size_t)r * H;
     pdl_wait();
     float4 v[VPT];
-    float ss = 0.f;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
-        const int c = t + i * TPR;
+        const int c = t + i * 64;
         v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (r >= n_rows || c >= nvec) continue;
         const float4 o = reinterpret_cast<const float4*>(h + base)[c], x = reinterpret_cast<const float4*>(a0 + base)[c];
@@ -1042,24 +1044,76 @@ weighted_add_rows_kernel(float* h, const float* a0, float s0, const float* a1, f
     }
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
-        const int c = t + i * TPR;
+        const int c = t + i * 64;
         if (r < n_rows && c < nvec) reinterpret_cast<float4*>(h + base)[c] = v[i];
-        ss += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
+        acc[0] = fmaf(v[i].x, v[i].x, acc[0]); acc[1] = fmaf(v[i].y, v[i].y, acc[1]);
+        acc[2] = fmaf(v[i].z, v[i].z, acc[2]); acc[3] = fmaf(v[i].w, v[i].w, acc[3]);
     }
     if (y_next == nullptr) return;
-    ss = warp_sum(ss);
-    if constexpr (TPR > 32) {
-        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ss;
-        __syncthreads();
-        ss = 0.f;
-#pragma unroll
-        for (int k = 0; k < TPR / 32; ++k) ss += part[threadIdx.x / TPR * (TPR / 32) + k];
-    }
+    // a warp of that block is eight lanes here: lanes 4, 2, 1 apart first (sharing out the four sums), then elements 2 and 1 apart
+    const bool up4 = lane & 4, up2 = lane & 2;
+    const float g0 = __shfl_xor_sync(0xffffffffu, up4 ? acc[0] : acc[2], 4), g1 = __shfl_xor_sync(0xffffffffu, up4 ? acc[1] : acc[3], 4);
+    const float b0 = (up4 ? acc[2] : acc[0]) + g0, b1 = (up4 ? acc[3] : acc[1]) + g1;
+    float ss = (up2 ? b1 : b0) + __shfl_xor_sync(0xffffffffu, up2 ? b0 : b1, 2);
+    ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+    ss += __shfl_xor_sync(0xffffffffu, ss, 4);
+    ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+    // and the eight warps' sums as block_sum folds them: 4 apart (the row's other warp), 2, 1
+    if ((lane & 7) == 0) part[threadIdx.x >> 5][lane >> 3] = ss;
+    __syncthreads();
+    ss += part[(threadIdx.x >> 5) ^ 1][lane >> 3];
+    ss += __shfl_xor_sync(0xffffffffu, ss, 16);
+    ss += __shfl_xor_sync(0xffffffffu, ss, 8);
     if (r >= n_rows) return;
     const float inv = rsqrtf(ss / (float)H + eps);
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
-        const int c = t + i * TPR;
+        const int c = t + i * 64;
+        if (c >= nvec) break;
+        const float ov[4] = {v[i].x * inv * load_vec(w_next, w_is_f32, 4 * c), v[i].y * inv * load_vec(w_next, w_is_f32, 4 * c + 1),
+                             v[i].z * inv * load_vec(w_next, w_is_f32, 4 * c + 2), v[i].w * inv * load_vec(w_next, w_is_f32, 4 * c + 3)};
+        Four<T>::store(y_next + base + 4 * c, ov);
+    }
+}
+
+// The same for rows of up to 8,192: a block a row.  What a thread of the general form sums lies in four threads' pieces here, so the
+// row goes through shared memory once, in 16-byte pieces in and in that form's order out.  Measured (us, as above): 2,048 rows of
+// 4,096 60.4 -> 26.9, 1,000 of 8,192 110 -> 29.0.
+template <typename T, int VPT>
+__global__ void __launch_bounds__(256, 4)
+weighted_add_wide_rows_kernel(float* h, const float* a0, float s0, const float* a1, float s1, const void* __restrict__ w_next, int w_is_f32,
+                              float eps, T* y_next, int H, int) {
+    extern __shared__ __align__(16) float row[];    // [H], 34 for the sums
+    pdl_trigger();
+    const int t = threadIdx.x, nvec = H >> 2;
+    const size_t base = (size_t)blockIdx.x * H;
+    pdl_wait();
+    float4 v[VPT];
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+        const int c = t + i * 256;
+        v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (c >= nvec) continue;
+        const float4 o = reinterpret_cast<const float4*>(h + base)[c], x = reinterpret_cast<const float4*>(a0 + base)[c];
+        const float4 z = a1 != nullptr ? reinterpret_cast<const float4*>(a1 + base)[c] : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[i] = make_float4(o.x + (s0 * x.x + s1 * z.x), o.y + (s0 * x.y + s1 * z.y), o.z + (s0 * x.z + s1 * z.z), o.w + (s0 * x.w + s1 * z.w));
+    }
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+        const int c = t + i * 256;
+        if (c >= nvec) break;
+        reinterpret_cast<float4*>(h + base)[c] = v[i];
+        reinterpret_cast<float4*>(row)[c] = v[i];
+    }
+    if (y_next == nullptr) return;
+    __syncthreads();
+    float ss = 0.f;
+#pragma unroll 8
+    for (int e = t; e < H; e += 256) ss = fmaf(row[e], row[e], ss);
+    const float inv = rsqrtf(block_sum(ss, row + H) / (float)H + eps);
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+        const int c = t + i * 256;
         if (c >= nvec) break;
         const float ov[4] = {v[i].x * inv * load_vec(w_next, w_is_f32, 4 * c), v[i].y * inv * load_vec(w_next, w_is_f32, 4 * c + 1),
                              v[i].z * inv * load_vec(w_next, w_is_f32, 4 * c + 2), v[i].w * inv * load_vec(w_next, w_is_f32, 4 * c + 3)};
@@ -1074,14 +1128,15 @@ static int launch_weighted_add(float* h, const float* a0, int n0, float s0, cons
     if (a0 == nullptr || n0 < 1 || (a1 != nullptr && n1 < 1) || (y_next != nullptr && w_next == nullptr)) return RF_ERR_BAD_ARG;
     if (n0 == 1 && n1 <= 1 && rows >= 512 && H % 4 == 0 && H <= 8192 &&
         !((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(a0) | reinterpret_cast<uintptr_t>(a1) | reinterpret_cast<uintptr_t>(y_next)) & 15)) {
-        auto go = [&](auto kernel, int per_block) {
-            rf_launch(kernel, dim3((rows + per_block - 1) / per_block), dim3(256), 0, st, h, a0, s0, a1, s1, w_next, w_is_f32, eps,
+        auto go = [&](auto kernel, int per_block, size_t row_bytes) {
+            rf_launch(kernel, dim3((rows + per_block - 1) / per_block), dim3(256), row_bytes, st, h, a0, s0, a1, s1, w_next, w_is_f32, eps,
                       reinterpret_cast<T*>(y_next), H, rows);
         };
-        if (H <= 1024) go(weighted_add_rows_kernel<T, 32>, 8);
-        else if (H <= 2048) go(weighted_add_rows_kernel<T, 64>, 4);
-        else if (H <= 4096) go(weighted_add_rows_kernel<T, 128>, 2);
-        else go(weighted_add_rows_kernel<T, 256>, 1);
+        const size_t row_bytes = ((size_t)H + 34) * sizeof(float);
+        if (H <= 1024) go(weighted_add_rows_kernel<T, 4>, 4, 0);
+        else if (H <= 2048) go(weighted_add_rows_kernel<T, 8>, 4, 0);
+        else if (H <= 4096) go(weighted_add_wide_rows_kernel<T, 4>, 1, row_bytes);
+        else go(weighted_add_wide_rows_kernel<T, 8>, 1, row_bytes);
         RF_LAUNCH_CHECK();
         return 0;
     }

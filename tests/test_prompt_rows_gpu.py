@@ -82,6 +82,27 @@ def test_weighted_update(dt, H, two):
 
 
 @pytest.mark.parametrize("dt", DTS)
+@pytest.mark.parametrize("H", [4, 252, 1000, 1028, 2048, 2052, 4096, 4100, 8192])
+@pytest.mark.parametrize("two", [False, True])
+def test_the_weighted_update_of_many_rows_has_the_bits_of_fewer(dt, H, two):
+    """The same rows in a step of 512 and more and in one of fewer (297 to 511, which run the form of 256 threads a row); 517 rows
+    leave the last block with one."""
+    from rocmforge_b200 import kernels
+    torch.manual_seed(H)
+    T = 517
+    h, a, b = (torch.randn(T, H, device=DEV) for _ in range(3))
+    h[7] *= 1e4
+    w = torch.rand(H, device=DEV) + 0.5
+    for nxt in (None, (w, 1e-6), (w.bfloat16(), 1e-6)):
+        def run(rows):
+            got = h[rows].clone()
+            return got, kernels.weighted_add(got, [(a[rows].clone(), 0.7)] + ([(b[rows].clone(), 0.3)] if two else []), dt, next_norm=nxt)
+        big, fewer, rest = run(slice(0, T)), run(slice(0, 300)), run(slice(T - 299, T))
+        for x, y, z in zip(big, fewer, rest):
+            assert x is None or (torch.equal(x[:300], y) and torch.equal(x[T - 299:], z))
+
+
+@pytest.mark.parametrize("dt", DTS)
 @pytest.mark.parametrize("C,taps", [(260, 4), (64, 2), (1028, 3), (8, 1)])
 def test_convolution(dt, C, taps):
     from rocmforge_b200 import kernels
