@@ -762,6 +762,56 @@ head_norm_kv_write_kernel(const void* __restrict__ src, int row_stride, int n_pa
     }
 }
 
+// Four numbers of each of the lanes l, l ^ 8, l ^ 16, l ^ 24: out[k] = number r of the lane 8 k + l % 8, where r = lane / 8.
+__device__ __forceinline__ void quad_trade(const float* x, float* out, int r) {
+    const bool up1 = r & 1, up2 = r & 2;
+    // lanes 8 apart trade odd against even numbers: e[i] is number 2 i + (r & 1) of the even lane, o[i] of the odd one
+    float e[2], o[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const float got = __shfl_xor_sync(0xffffffffu, up1 ? x[2 * i] : x[2 * i + 1], 8);
+        e[i] = up1 ? got : x[2 * i];
+        o[i] = up1 ? x[2 * i + 1] : got;
+    }
+    const float ge = __shfl_xor_sync(0xffffffffu, up2 ? e[0] : e[1], 16), go = __shfl_xor_sync(0xffffffffu, up2 ? o[0] : o[1], 16);
+    out[0] = up2 ? ge : e[0]; out[1] = up2 ? go : o[0];
+    out[2] = up2 ? e[1] : ge; out[3] = up2 ? o[1] : go;
+}
+
+// A head's sum of squares as head_norm_kv_write_kernel's warp forms it, bit for bit: lane L adds elements L, L + 32, L + 64, ... there
+// and the lanes meet 16, 8, 4, 2, 1 apart.  Here a lane holds E neighbours of each half (x, then y), so the lanes E apart in that
+// order first trade elements until each has one such lane's share, and the shuffles follow the bits of L to where they lie now.
+template <int E>
+__device__ __forceinline__ float head_square_sum(const float (&x)[E], const float (&y)[E]) {
+    const int lane = threadIdx.x & 31;
+    float s;
+    if constexpr (E == 1) {
+        s = fmaf(y[0], y[0], x[0] * x[0]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    } else if constexpr (E == 2) {
+        const bool up = lane & 16;                       // lanes 0 .. 15 take the first of the two neighbours, 16 .. 31 the second
+        const float gx = __shfl_xor_sync(0xffffffffu, up ? x[0] : x[1], 16), gy = __shfl_xor_sync(0xffffffffu, up ? y[0] : y[1], 16);
+        const float x0 = up ? gx : x[0], x1 = up ? x[1] : gx, y0 = up ? gy : y[0], y1 = up ? y[1] : gy;
+        s = fmaf(y1, y1, fmaf(y0, y0, fmaf(x1, x1, x0 * x0)));
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        s += __shfl_xor_sync(0xffffffffu, s, 16);
+    } else {
+        const int r = lane >> 3;                         // lanes 8 r .. 8 r + 7 take number r of the four neighbours
+        float v[8];
+        quad_trade(x, v, r); quad_trade(y, v + 4, r);
+        s = v[0] * v[0];
+#pragma unroll
+        for (int k = 1; k < 8; ++k) s = fmaf(v[k], v[k], s);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        s += __shfl_xor_sync(0xffffffffu, s, 16);
+        s += __shfl_xor_sync(0xffffffffu, s, 8);
+    }
+    return s;
+}
+
 // The same for the rows of a prompt step in the compute dtype, heads of 64, 128 or 256 = 64 E wholly rotated as halves (or not at
 // all), keys and values of one size: a warp holds a head in registers, E neighbouring elements of each half a lane, so that a pair's
 // two elements meet in one lane; the sines and cosines of a block's tokens are formed once, in shared memory, before the wait for the
@@ -800,7 +850,7 @@ head_norm_rows_kernel(const T* src, int row_stride, T* q_out, int q_out_stride, 
         const bool is_v = head >= nh + nkv;
         const T* from = src + (size_t)(t0 + t) * row_stride + (size_t)head * HD + lane * E;
         const Piece a = *reinterpret_cast<const Piece*>(from), b = *reinterpret_cast<const Piece*>(from + HALF);
-        float x[E], y[E], ss = 0.f;
+        float x[E], y[E];
 #pragma unroll
         for (int j = 0; j < E; ++j) {
             x[j] = Cvt<T>::to_f32(a.v[j]); y[j] = Cvt<T>::to_f32(b.v[j]);
@@ -808,12 +858,11 @@ head_norm_rows_kernel(const T* src, int row_stride, T* q_out, int q_out_stride, 
                 x[j] += load_vec(ex.bias, ex.bias_is_f32, head * HD + lane * E + j);
                 y[j] += load_vec(ex.bias, ex.bias_is_f32, head * HD + HALF + lane * E + j);
             }
-            ss += x[j] * x[j] + y[j] * y[j];
         }
         const bool normed = unit_norm && !is_v;
         const void* nw = normed ? (head < nh ? q_norm_w : k_norm_w) : nullptr;
         if (normed && !ex.norm_after) {
-            const float r = rsqrtf(warp_sum(ss) / (float)HD + eps);
+            const float r = rsqrtf(head_square_sum<E>(x, y) / (float)HD + eps);
 #pragma unroll
             for (int j = 0; j < E; ++j) {
                 if (nw != nullptr) { x[j] *= load_vec(nw, norm_w_is_f32, lane * E + j); y[j] *= load_vec(nw, norm_w_is_f32, HALF + lane * E + j); }
@@ -830,10 +879,7 @@ head_norm_rows_kernel(const T* src, int row_stride, T* q_out, int q_out_stride, 
             }
         }
         if (normed && ex.norm_after) {
-            float s2 = 0.f;
-#pragma unroll
-            for (int j = 0; j < E; ++j) s2 += x[j] * x[j] + y[j] * y[j];
-            const float r = rsqrtf(warp_sum(s2) / (float)HD + eps);
+            const float r = rsqrtf(head_square_sum<E>(x, y) / (float)HD + eps);
 #pragma unroll
             for (int j = 0; j < E; ++j) {
                 x[j] *= r; y[j] *= r;

@@ -1,6 +1,5 @@
 """The forms that prompt steps take of the per-head writer, the weighted update, the convolution and the delta rule's inputs: the
-same rows in one large step and in small ones, which run the general forms.  Sums of a row may be added in another order: an ulp or two
-of 32 bits, and the rounding to the compute dtype that follows."""
+same rows in one large step and in small ones, which run the general forms."""
 import pytest
 import torch
 
@@ -26,6 +25,8 @@ def near(a, b, dt):
     (6, 2, 64, dict(rot_dim=64, norm_after_rotation=True, unit_norm_eps=1e-6, magnitude=1.2)),
     (5, 1, 128, dict(rot_dim=128, unit_norm_eps=1e-5, weights=True)),
     (3, 3, 256, dict(rot_dim=0, bias=True, q_temperature=(0.1, 64.0), values_are_keys=True)),
+    (3, 1, 256, dict(rot_dim=256, unit_norm_eps=1e-6, weights=True)), (2, 1, 256, dict(rot_dim=256, unit_norm_eps=1e-6, norm_after_rotation=True)),
+    (2, 2, 128, dict(rot_dim=128, unit_norm_eps=1e-6, norm_after_rotation=True, bias=True)),
     (4, 2, 128, dict(rot_dim=0)), (4, 2, 64, dict(rot_dim=32, unit_norm_eps=1e-6)), (4, 4, 128, dict(rot_dim=128, writes=False))])
 def test_head_rows(dt, nh, nkv, hd, opts):
     from rocmforge_b200 import kernels
@@ -60,6 +61,9 @@ def test_head_rows(dt, nh, nkv, hd, opts):
     middle = run([0, 256, 1300])
     for a, b, c in zip(big, small, middle):
         near(a, b, dt), near(c, b, dt)
+        # a head's sums are added in the same order whatever the form, so not a bit differs
+        for p, q in ((a, b), (c, b)):
+            assert torch.equal(p.isnan(), q.isnan()) and torch.equal(p.nan_to_num(0), q.nan_to_num(0))
 
 
 @pytest.mark.parametrize("dt", DTS)
