@@ -34,9 +34,19 @@ delta_prepare_kernel(const float* qkv, int qkv_stride, const float* a, int a_str
             const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
             float4 x = in ? *reinterpret_cast<const float4*>(row + g * D + lane * 4) : zero;
             float4 y = in ? *reinterpret_cast<const float4*>(row + (G + g) * D + lane * 4) : zero;
-            float sq = x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w, sk = y.x * y.x + y.y * y.y + y.z * y.z + y.w * y.w;
-            float dot = x.x * y.x + x.y * y.y + x.z * y.z + x.w * y.w;
-            sq = warp_sum(sq); sk = warp_sum(sk); dot = warp_sum(dot);
+            // the sums as the general form's warp makes them, bit for bit: lane L adds elements L, L + 32, L + 64, L + 96 there, so the
+            // lanes 8 apart trade until each has one such lane's four, and the shuffles follow the bits of L to where they lie now
+            const float xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+            float xv[4], yv[4], sq = 0.f, sk = 0.f, dot = 0.f;
+            quad_trade(xs, xv, lane >> 3); quad_trade(ys, yv, lane >> 3);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) { sq = fmaf(xv[k], xv[k], sq); sk = fmaf(yv[k], yv[k], sk); dot = fmaf(xv[k], yv[k], dot); }
+            constexpr int apart[5] = {4, 2, 1, 16, 8};
+#pragma unroll
+            for (int o = 0; o < 5; ++o) {
+                sq += __shfl_xor_sync(0xffffffffu, sq, apart[o]); sk += __shfl_xor_sync(0xffffffffu, sk, apart[o]);
+                dot += __shfl_xor_sync(0xffffffffu, dot, apart[o]);
+            }
             const float rq = q_scale / sqrtf(sq + unit_eps), rk = 1.f / sqrtf(sk + unit_eps);
             if (in) {
                 *reinterpret_cast<float4*>(qn + ((size_t)t * G + g) * D + lane * 4) = make_float4(x.x * rq, x.y * rq, x.z * rq, x.w * rq);
@@ -254,7 +264,7 @@ int rf_delta_prepare(int dtype, const float* qkv, int qkv_stride, const float* a
     if (H <= 0 || G <= 0 || H % G || D <= 0) return RF_ERR_BAD_ARG;
     int by = T_ >= 512 ? 1 : per_head ? (G + 3) / 4 : (H * D + 511) / 512;           // about four decays a thread when there are few tokens
     if (by > 32) by = 32;
-    // (2,778 tokens of 16 heads of 128, one by one 43 us, so 28)
+    // (2,778 tokens of 16 heads of 128, one by one 43 us, so 28; the same bits)
     const int vec = T_ >= 512 && D % 4 == 0 && D <= 128 && qkv_stride % 4 == 0 && (per_head || a_stride % 4 == 0) &&
                     !((reinterpret_cast<uintptr_t>(qkv) | (per_head ? 0 : reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(decay)) |
                        reinterpret_cast<uintptr_t>(qn) | reinterpret_cast<uintptr_t>(kn)) & 15);

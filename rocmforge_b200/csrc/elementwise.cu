@@ -762,22 +762,6 @@ head_norm_kv_write_kernel(const void* __restrict__ src, int row_stride, int n_pa
     }
 }
 
-// Four numbers of each of the lanes l, l ^ 8, l ^ 16, l ^ 24: out[k] = number r of the lane 8 k + l % 8, where r = lane / 8.
-__device__ __forceinline__ void quad_trade(const float* x, float* out, int r) {
-    const bool up1 = r & 1, up2 = r & 2;
-    // lanes 8 apart trade odd against even numbers: e[i] is number 2 i + (r & 1) of the even lane, o[i] of the odd one
-    float e[2], o[2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const float got = __shfl_xor_sync(0xffffffffu, up1 ? x[2 * i] : x[2 * i + 1], 8);
-        e[i] = up1 ? got : x[2 * i];
-        o[i] = up1 ? x[2 * i + 1] : got;
-    }
-    const float ge = __shfl_xor_sync(0xffffffffu, up2 ? e[0] : e[1], 16), go = __shfl_xor_sync(0xffffffffu, up2 ? o[0] : o[1], 16);
-    out[0] = up2 ? ge : e[0]; out[1] = up2 ? go : o[0];
-    out[2] = up2 ? e[1] : ge; out[3] = up2 ? o[1] : go;
-}
-
 // A head's sum of squares as head_norm_kv_write_kernel's warp forms it, bit for bit: lane L adds elements L, L + 32, L + 64, ... there
 // and the lanes meet 16, 8, 4, 2, 1 apart.  Here a lane holds E neighbours of each half (x, then y), so the lanes E apart in that
 // order first trade elements until each has one such lane's share, and the shuffles follow the bits of L to where they lie now.
