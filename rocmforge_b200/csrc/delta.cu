@@ -360,6 +360,7 @@ __device__ __forceinline__ void copies_done() {
 
 // grid (chunk, head); 256 threads.  Thread (ty, tx) owns rows t = ty + 16 x and columns s = tx + 16 y, x, y = 0 .. 3, of the
 // two score matrices: with y > x every s lies after every t, so ten of the sixteen pairs (x, y) are formed.
+// chunk0: the pass's first chunk; blockIdx.x counts from there, and so do all chunk indices of the scratch memory below.
 // M [chunk][head][t][s]; gw [chunk][head][2][64]: G_t, then P(s, cnt - 1); and what the carry kernel fetches with one bulk copy
 // each: Kc [chunk][q/k head][64][KD], U0 [chunk][head][ceil(V/DV)][64][DV], Wt [chunk][head][d][64], zeros beyond the chunk's
 // tokens, D and V.
@@ -369,7 +370,7 @@ delta_chunk_solve_kernel(const float* __restrict__ qn, const float* __restrict__
                          const float* __restrict__ beta, const float* __restrict__ v, int v_stride, float* __restrict__ M,
                          float* __restrict__ gw, float* __restrict__ Kc, float* __restrict__ U0, float* __restrict__ Wt,
                          float* __restrict__ Qg, const int* __restrict__ table,
-                         const int* __restrict__ cu_q, int B, int H, int G, int D, int V, int region) {
+                         const int* __restrict__ cu_q, int chunk0, int B, int H, int G, int D, int V, int region) {
     extern __shared__ __align__(16) float sh[];
     const int ld = PC ? DC_LD : ((D + 3) & ~3) + 4;
     float* ks = sh;                                   // [64][ld], and later X [64][256]
@@ -380,7 +381,7 @@ delta_chunk_solve_kernel(const float* __restrict__ qn, const float* __restrict__
     __shared__ float sg[DC], sb[DC], sG[DC], sF[DC];  // g, beta, G, and the products from a block's first token on
     pdl_trigger();
     const int c = blockIdx.x, h = blockIdx.y, hg = h / (H / G), tid = threadIdx.x;
-    const ChunkPlace p = chunk_place(table, cu_q, B, c);
+    const ChunkPlace p = chunk_place(table, cu_q, B, chunk0 + c);
     pdl_wait();
     if (tid < DC) {
         const bool in = tid < p.cnt;
@@ -611,7 +612,8 @@ delta_chunk_solve_kernel(const float* __restrict__ qn, const float* __restrict__
 // rows d of its eighth, the eight shares are added in order.  The state's update is cut in two by tokens: the last four warps sum
 // over tokens 32 .. 63 and hand their sums over through shared memory.  A chunk's inputs come as four bulk copies on a barrier per
 // stage, awaited with a limit (issued row by row, as small copies, their issue alone took longer than the arithmetic).
-// LS [chunk][head][d][V]: the state before each chunk; U rows of H*V.
+// LS [chunk][head][d][V]: the state before each chunk; U [chunk][64] rows of H*V.  A sequence whose chunks go on in the next pass
+// leaves its state in its slot, 32 bits like the registers', so passes change no bit.
 __device__ __forceinline__ void bulk_copy(float* dst, const float* src, uint32_t floats, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(smem_u32(dst)), "l"(src), "r"(4 * floats), "r"(bar) : "memory");
@@ -620,8 +622,8 @@ template <int TILES, bool PC>                         // row tiles of 128 a thre
 __global__ void __launch_bounds__(256, 1)
 delta_chunk_carry_kernel(const float* __restrict__ Kc, const float* __restrict__ U0, const float* __restrict__ Wt,
                          const float* __restrict__ gw, float* __restrict__ state, float* __restrict__ U, float* __restrict__ LS,
-                         const int* __restrict__ table, const int* __restrict__ cu_q, const int* __restrict__ seq_slot, int B, int H,
-                         int G, int D, int V, int* __restrict__ status) {
+                         const int* __restrict__ table, const int* __restrict__ cu_q, const int* __restrict__ seq_slot, int chunk0,
+                         int n_chunks, int B, int H, int G, int D, int V, int* __restrict__ status) {
     constexpr int STAGES = TILES == 1 ? 2 : 1;
     extern __shared__ __align__(16) float sh[];
     const int KD = (D + 3) & ~3;
@@ -636,8 +638,9 @@ delta_chunk_carry_kernel(const float* __restrict__ Kc, const float* __restrict__
     const int h = blockIdx.y, b = blockIdx.z, j0 = blockIdx.x * DV, hg = h / (H / G);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nc = min(DV, V - j0);
-    const int c0 = table[b], c1 = table[b + 1];
+    const int first = table[b], c0 = max(first, chunk0), c1 = min(table[b + 1], chunk0 + n_chunks);      // this sequence's chunks in the pass
     const int n_new = cu_q[b + 1] - cu_q[b];
+    if (c0 >= c1) { pdl_wait(); return; }
     const bool owner = tid < 128;                     // holds state
     const int cc = (tid & 3) * 4, dg = ((tid & 127) >> 2) * 4;  // this thread's four columns and its first row
     const bool quad = (V & 3) == 0 && cc + 3 < nc;
@@ -650,7 +653,8 @@ delta_chunk_carry_kernel(const float* __restrict__ Kc, const float* __restrict__
     }
     __syncthreads();
     pdl_wait();
-    auto fetch = [&](int c, int buf) {                // by one thread
+    auto fetch = [&](int chunk, int buf) {            // by one thread
+        const int c = chunk - chunk0;
         float* w = sh + buf * stage;
         const uint32_t bar = smem_u32(&bars[buf]);
         mbar_expect_tx(bar, 4u * (uint32_t)stage);
@@ -669,7 +673,7 @@ delta_chunk_carry_kernel(const float* __restrict__ Kc, const float* __restrict__
             for (int u = 0; u < 4; ++u) s[i][r][u] = (owner && d < D && cc + u < nc) ? S[(size_t)d * V + cc + u] : 0.f;
             if (owner && d < KD) *reinterpret_cast<float4*>(Ss + d * DV + cc) = make_float4(s[i][r][0], s[i][r][1], s[i][r][2], s[i][r][3]);
         }
-    if (STAGES == 2 && c0 < c1 && tid == 0) fetch(c0, 0);
+    if (STAGES == 2 && tid == 0) fetch(c0, 0);
     const int dper = (D + 7) / 8, d0 = warp * dper, d1 = min(D, d0 + dper);
     const int rg = (lane >> 2) * 4, cg = (lane & 3) * 4;
     for (int c = c0; c < c1; ++c) {
@@ -694,9 +698,9 @@ delta_chunk_carry_kernel(const float* __restrict__ Kc, const float* __restrict__
         const float* k = w + D * DC;
         const float* u0 = k + DC * KD;
         const float* g = u0 + DC * DV;
-        const int row0 = cu_q[b] + (c - c0) * DC, cnt = min(DC, n_new - (c - c0) * DC);
+        const int cnt = min(DC, n_new - (c - first) * DC), at = c - chunk0;
         if (owner) {
-            float* ls = LS + ((size_t)c * H + h) * D * V + j0 + cc;
+            float* ls = LS + ((size_t)at * H + h) * D * V + j0 + cc;
 #pragma unroll
             for (int i = 0; i < TILES; ++i)
 #pragma unroll
@@ -740,7 +744,7 @@ delta_chunk_carry_kernel(const float* __restrict__ Kc, const float* __restrict__
                 x.x -= y.x; x.y -= y.y; x.z -= y.z; x.w -= y.w;
             }
             if (t < cnt) {
-                float* uo = U + (size_t)(row0 + t) * H * V + h * V + j0 + cc;
+                float* uo = U + ((size_t)at * DC + t) * H * V + h * V + j0 + cc;
                 if (quad) *reinterpret_cast<float4*>(uo) = x;
                 else {
                     const float xs[4] = {x.x, x.y, x.z, x.w};
@@ -810,7 +814,7 @@ template <bool PC>                                     // PC: qn holds the chunk
 __global__ void __launch_bounds__(256)
 delta_chunk_out_kernel(const float* __restrict__ qn, const float* __restrict__ M, const float* __restrict__ gw,
                        const float* __restrict__ U, const float* __restrict__ LS, float* __restrict__ o, const int* __restrict__ table,
-                       const int* __restrict__ cu_q, int B, int H, int G, int D, int V) {
+                       const int* __restrict__ cu_q, int chunk0, int B, int H, int G, int D, int V) {
     extern __shared__ __align__(16) float sh[];
     const int D4 = (D + 3) & ~3, ld = DC + D4 + 4;
     float* lhs = sh;                                  // [64][ld]: M_ts, then q
@@ -818,7 +822,7 @@ delta_chunk_out_kernel(const float* __restrict__ qn, const float* __restrict__ M
     __shared__ float sG[DC];
     pdl_trigger();
     const int c = blockIdx.x, h = blockIdx.y, j0 = blockIdx.z * DO, hg = h / (H / G), tid = threadIdx.x;
-    const ChunkPlace p = chunk_place(table, cu_q, B, c);
+    const ChunkPlace p = chunk_place(table, cu_q, B, chunk0 + c);
     const int nc = min(DO, V - j0);
     pdl_wait();
     chunk_tile(lhs, ld, M + ((size_t)c * H + h) * DC * DC, DC, p.cnt, DC, true, tid, 256);
@@ -826,7 +830,7 @@ delta_chunk_out_kernel(const float* __restrict__ qn, const float* __restrict__ M
     else chunk_tile(lhs + DC, ld, qn + ((size_t)p.row0 * G + hg) * D, (size_t)G * D, p.cnt, D, (D & 3) == 0, tid, 256);
     if (tid < DC) sG[tid] = PC ? 1.f : gw[((size_t)c * H + h) * 2 * DC + tid];
     const bool vec = (V & 3) == 0;
-    const float* us = U + (size_t)p.row0 * H * V + h * V + j0;
+    const float* us = U + (size_t)c * DC * H * V + h * V + j0;
     const float* ss = LS + ((size_t)c * H + h) * D * V + j0;
     const int per = vec ? DO / 4 : DO, step = vec ? 4 : 1;
     for (int i = tid; i < (DC + D4) * per; i += 256) {
@@ -888,31 +892,42 @@ static int chunk_smem(const void* kernel, size_t bytes, size_t* configured) {
     return 0;
 }
 
-static long long delta_chunked_floats(bool pc, int n_chunks, int H, int G, int D, int V, int T_) {
+// Scratch memory of a pass.  All of a step's chunks at once took 53,000 numbers a chunk and head (a decay per channel, 128 x 128): 1.7 GB
+// for 32,000 tokens of 16 heads.  Passes of at most 512 MB (152 such chunks) keep the GPU full:
+// 32,000 tokens in one pass 4.21 ms, so 4.31; 16 prompts of 2,000 4.10 and 4.37 (passes of 128 MB 4.58 and 4.78).
+#define DC_PASS_FLOATS (128LL << 20)
+static long long chunk_floats(bool pc, int H, int G, int D, int V) {
     const long long D4 = (D + 3) & ~3, VP = (V + DV - 1) / DV * DV;
-    return (long long)n_chunks * H * (DC * DC + (pc ? D4 : 2 * DC) + (long long)D * DC + VP * DC + (long long)D * V) +
-           (long long)n_chunks * (pc ? 2 * H : G) * DC * D4 + (long long)T_ * H * V + 16;
+    return (long long)H * (DC * DC + (pc ? D4 : 2 * DC) + (long long)D * DC + VP * DC + (long long)D * V + DC * (long long)V) +
+           (long long)(pc ? 2 * H : G) * DC * D4;
+}
+static int pass_chunks(bool pc, int n_chunks, int H, int G, int D, int V, int most) {
+    const long long fit = DC_PASS_FLOATS / chunk_floats(pc, H, G, D, V);
+    long long n = fit < 1 ? 1 : fit;
+    if (most > 0 && most < n) n = most;
+    return n < n_chunks ? (int)n : n_chunks;
 }
 
 template <bool PC>
 static int delta_chunked(const float* qn, const float* kn, const float* decay, const float* beta, const float* v, int v_stride,
                          float* state, float* o, float* scratch, const int* table, int n_chunks, const int* cu_q, const int* seq_slot,
-                         int B, int H, int G, int D, int V, int T_, int* status, cudaStream_t st) {
+                         int B, int H, int G, int D, int V, int most, int* status, cudaStream_t st) {
     if (B <= 0 || n_chunks <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G || D <= 0 || V <= 0 || H > 65535 || B > 65535) return RF_ERR_BAD_ARG;
     if (D > 256 || status == nullptr || (reinterpret_cast<uintptr_t>(scratch) & 15) || (reinterpret_cast<uintptr_t>(kn) & 15) ||
         (reinterpret_cast<uintptr_t>(qn) & 15) || (PC && (reinterpret_cast<uintptr_t>(decay) & 15)))
         return RF_ERR_UNSUPPORTED;
-    const size_t ch = (size_t)n_chunks * H;
+    const int pass = pass_chunks(PC, n_chunks, H, G, D, V, most);
+    const size_t ch = (size_t)pass * H;
     const int D4 = (D + 3) & ~3, VP = (V + DV - 1) / DV * DV, GW = PC ? D4 : 2 * DC;
     float* M = scratch;
     float* gw = M + ch * DC * DC;
     float* Wt = gw + ch * GW;
     float* U0 = Wt + ch * D * DC;
     float* Kc = U0 + ch * VP * DC;
-    float* Qg = Kc + (PC ? ch : (size_t)n_chunks * G) * DC * D4;
+    float* Qg = Kc + (PC ? ch : (size_t)pass * G) * DC * D4;
     float* U = Qg + (PC ? ch * DC * D4 : 0);
-    float* LS = U + ((size_t)T_ * H * V + 3) / 4 * 4;
+    float* LS = U + ch * DC * V;
     int region = PC ? 3 * DC * DC_LD : 2 * DC * (D4 + 4);
     if (region < DC * DC_COLS) region = DC * DC_COLS;
     const size_t smem1 = ((size_t)region + DC * DC_LD + DC * (PC ? DC_LD : DC_PLD)) * sizeof(float);
@@ -927,34 +942,38 @@ static int delta_chunked(const float* qn, const float* kn, const float* decay, c
     if ((e = chunk_smem((const void*)solve, smem1, &set1)) || (e = chunk_smem((const void*)carry, smem2, &set2[tiles - 1])) ||
         (e = chunk_smem((const void*)outk, smem3, &set3)))
         return e;
-    rf_launch(solve, dim3(n_chunks, H), dim3(256), smem1, st, qn, kn, decay, beta, v, v_stride, M, gw, Kc, U0, Wt, Qg, table, cu_q, B, H, G, D, V,
-              region);
-    RF_LAUNCH_CHECK();
-    rf_launch(carry, dim3(VP / DV, H, B), dim3(256), smem2, st, (const float*)Kc, (const float*)U0, (const float*)Wt, (const float*)gw,
-              state, U, LS, table, cu_q, seq_slot, B, H, G, D, V, status);
-    RF_LAUNCH_CHECK();
-    rf_launch(outk, dim3(n_chunks, H, (V + DO - 1) / DO), dim3(256), smem3, st, PC ? (const float*)Qg : qn, (const float*)M, (const float*)gw,
-              (const float*)U, (const float*)LS, o, table, cu_q, B, H, G, D, V);
-    RF_LAUNCH_CHECK();
+    for (int c = 0; c < n_chunks; c += pass) {
+        const int n = pass < n_chunks - c ? pass : n_chunks - c;
+        rf_launch(solve, dim3(n, H), dim3(256), smem1, st, qn, kn, decay, beta, v, v_stride, M, gw, Kc, U0, Wt, Qg, table, cu_q, c, B, H, G, D, V,
+                  region);
+        RF_LAUNCH_CHECK();
+        rf_launch(carry, dim3(VP / DV, H, B), dim3(256), smem2, st, (const float*)Kc, (const float*)U0, (const float*)Wt, (const float*)gw,
+                  state, U, LS, table, cu_q, seq_slot, c, n, B, H, G, D, V, status);
+        RF_LAUNCH_CHECK();
+        rf_launch(outk, dim3(n, H, (V + DO - 1) / DO), dim3(256), smem3, st, PC ? (const float*)Qg : qn, (const float*)M, (const float*)gw,
+                  (const float*)U, (const float*)LS, o, table, cu_q, c, B, H, G, D, V);
+        RF_LAUNCH_CHECK();
+    }
     return 0;
 }
 
 extern "C" {
-// Floats of scratch memory that rf_delta_chunked (channels: rf_delta_chunked_channels) needs for T_ tokens in n_chunks chunks.
-long long rf_delta_chunked_scratch(int n_chunks, int H, int G, int D, int V, int T_, int channels) {
-    return delta_chunked_floats(channels != 0, n_chunks, H, G, D, V, T_);
+// Floats of scratch memory that rf_delta_chunked (channels: rf_delta_chunked_channels) needs for n_chunks chunks.  most: chunks of a
+// pass at most (0: as many as 512 MB hold), the same number there.
+long long rf_delta_chunked_scratch(int n_chunks, int H, int G, int D, int V, int channels, int most) {
+    return pass_chunks(channels != 0, n_chunks, H, G, D, V, most) * chunk_floats(channels != 0, H, G, D, V) + 16;
 }
 // What rf_delta_scan computes with per_head decays, for prompts (see above).  table: first[B+1], then n_chunks pairs (sequence,
-// first row of the chunk among the sequence's new tokens), in the order of the sequences.
+// first row of the chunk among the sequence's new tokens), in the order of the sequences; a sequence without chunks is left alone.
 int rf_delta_chunked(const float* qn, const float* kn, const float* decay, const float* beta, const float* v, int v_stride,
                      float* state, float* o, float* scratch, const int* table, int n_chunks, const int* cu_q, const int* seq_slot,
-                     int B, int H, int G, int D, int V, int T_, int* status, cudaStream_t st) {
-    return delta_chunked<false>(qn, kn, decay, beta, v, v_stride, state, o, scratch, table, n_chunks, cu_q, seq_slot, B, H, G, D, V, T_, status, st);
+                     int B, int H, int G, int D, int V, int most, int* status, cudaStream_t st) {
+    return delta_chunked<false>(qn, kn, decay, beta, v, v_stride, state, o, scratch, table, n_chunks, cu_q, seq_slot, B, H, G, D, V, most, status, st);
 }
 // The same with a decay per key channel: decay [T, H*D].
 int rf_delta_chunked_channels(const float* qn, const float* kn, const float* decay, const float* beta, const float* v, int v_stride,
                               float* state, float* o, float* scratch, const int* table, int n_chunks, const int* cu_q, const int* seq_slot,
-                              int B, int H, int G, int D, int V, int T_, int* status, cudaStream_t st) {
-    return delta_chunked<true>(qn, kn, decay, beta, v, v_stride, state, o, scratch, table, n_chunks, cu_q, seq_slot, B, H, G, D, V, T_, status, st);
+                              int B, int H, int G, int D, int V, int most, int* status, cudaStream_t st) {
+    return delta_chunked<true>(qn, kn, decay, beta, v, v_stride, state, o, scratch, table, n_chunks, cu_q, seq_slot, B, H, G, D, V, most, status, st);
 }
 }

@@ -1626,11 +1626,12 @@ def _delta_scratch():
 
 def delta_chunked(qn: torch.Tensor, kn: torch.Tensor, decay: torch.Tensor, beta: torch.Tensor, v: torch.Tensor, state: torch.Tensor,
                   table: torch.Tensor, cu_q: torch.Tensor, seq_slot: torch.Tensor, heads: int, qk_heads: int, dim: int,
-                  vdim: int) -> torch.Tensor:
-    """What ``delta_scan`` computes, with one decay per head (decay [T, heads]) or per key channel (decay [T, heads*dim]), for prompts: chunks of 64 tokens whose corrected
-    values come from one triangular system each, side by side; then the states between the chunks one after the other; then
-    every chunk's outputs.  All in 32-bit.  ``table``: the chunk table of ``retention_chunked``.  Differs from the scan by
-    rounding only."""
+                  vdim: int, *, chunks_per_pass: int = 0) -> torch.Tensor:
+    """What ``delta_scan`` computes, with one decay per head (decay [T, heads]) or per key channel (decay [T, heads*dim]), for prompts:
+    chunks of 64 tokens whose corrected values come from one triangular system each, side by side; then the states between the
+    chunks one after the other; then every chunk's outputs.  All in 32-bit.  ``table``: the chunk table of ``retention_chunked``.
+    Differs from the scan by rounding only.  Chunks are taken in passes whose scratch memory stays below 512 MB
+    (``chunks_per_pass``: fewer, for tests); the passes change no bit."""
     need_cuda(qn, kn, decay, beta, v, state, table, cu_q, seq_slot)
     T, B = qn.shape[0], seq_slot.shape[0]
     need(all(x.dtype == torch.float32 and x.is_contiguous() for x in (qn, kn, decay, beta, state)), "delta_chunked: float32 inputs")
@@ -1643,11 +1644,12 @@ def delta_chunked(qn: torch.Tensor, kn: torch.Tensor, decay: torch.Tensor, beta:
     need(table.dtype == torch.int32 and (table.numel() - (B + 1)) % 2 == 0 and table.numel() > B + 1,
          "delta_chunked: the chunk table must hold first[B+1] and a pair per chunk")
     n_chunks = (table.numel() - (B + 1)) // 2
-    scratch = torch.empty((_delta_scratch()(n_chunks, heads, qk_heads, dim, vdim, T, int(channels)),), dtype=torch.float32, device=qn.device)
+    scratch = torch.empty((_delta_scratch()(n_chunks, heads, qk_heads, dim, vdim, int(channels), chunks_per_pass),), dtype=torch.float32,
+                          device=qn.device)
     o = torch.empty((T, heads * vdim), dtype=torch.float32, device=qn.device)
     f = _f("delta", "rf_delta_chunked_channels" if channels else "rf_delta_chunked", c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
            c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p)
     from .tensor_core import status_word
     check(f(ptr(qn), ptr(kn), ptr(decay), ptr(beta), ptr(v), v.stride(0), ptr(state), ptr(o), ptr(scratch), ptr(table), n_chunks,
-            ptr(cu_q), ptr(seq_slot), B, heads, qk_heads, dim, vdim, T, ptr(status_word(qn.device)), stream()), f"delta_chunked (heads={heads}, dim={dim}, vdim={vdim})")
+            ptr(cu_q), ptr(seq_slot), B, heads, qk_heads, dim, vdim, chunks_per_pass, ptr(status_word(qn.device)), stream()), f"delta_chunked (heads={heads}, dim={dim}, vdim={vdim})")
     return o

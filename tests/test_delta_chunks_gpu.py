@@ -66,3 +66,48 @@ def test_chunks_with_a_decay_per_channel(H, G, dim, vdim):
                 size = x.norm() + 1e-6
                 assert (y.double().cpu() - x).norm() < 2e-5 * size and (z.double().cpu() - x).norm() < 2e-5 * size, (i, h)
     assert not state[2].any() and not state[5].any()
+
+
+def ragged(lens, H, G, dim, vdim, per_head, seed):
+    torch.manual_seed(seed)
+    T = sum(lens)
+    q, k = (torch.nn.functional.normalize(torch.randn(T, G, dim, device=DEV), dim=-1).reshape(T, G * dim).contiguous() for _ in range(2))
+    v, beta = torch.randn(T, H * vdim, device=DEV), torch.rand(T, H, device=DEV)
+    decay = torch.rand(T, H if per_head else H * dim, device=DEV) ** 0.1
+    return q, k, (q.view(T, G, dim) * k.view(T, G, dim)).sum(-1), decay, beta, v
+
+
+def chunk_table(lens):
+    counts = [(n + 63) // 64 for n in lens]
+    return i32(*([sum(counts[:j]) for j in range(len(lens) + 1)] + [x for j, n in enumerate(lens) for r in range(0, n, 64) for x in (j, r)]))
+
+
+@pytest.mark.parametrize("per_head", [False, True])
+@pytest.mark.parametrize("H,G,dim,vdim", [(4, 2, 24, 12), (2, 1, 128, 40), (1, 1, 200, 20)])
+def test_passes_over_the_chunks_change_no_bit(per_head, H, G, dim, vdim):
+    """Chunks are taken in passes of bounded scratch memory: passes of 1, 3 and 7 chunks, which cut sequences anywhere, against one pass."""
+    from rocmforge_b200 import kernels
+    lens, slots = [300, 64, 1, 130, 449], [3, 0, 5, 1, 2]
+    q, k, kq, decay, beta, v = ragged(lens, H, G, dim, vdim, per_head, dim)
+    cu = i32(*[sum(lens[:j]) for j in range(6)])
+    begin = torch.randn(6, H, dim, vdim, device=DEV)
+    got = []
+    for most in (0, 1, 3, 7):
+        state = begin.clone()
+        got.append((kernels.delta_chunked(q, k, decay, beta, v, state, chunk_table(lens), cu, i32(*slots), H, G, dim, vdim, chunks_per_pass=most), state))
+    for o, state in got[1:]:
+        assert torch.equal(o, got[0][0]) and torch.equal(state, got[0][1])
+
+
+@pytest.mark.parametrize("per_head", [False, True])
+def test_the_chunks_scratch_memory_is_bounded(per_head):
+    """30,000 tokens of 16 heads of 128 x 128: beyond its result the call holds 512 MB and a little, not a size that grows with the prompt."""
+    from rocmforge_b200 import kernels
+    lens, H, dim = [17000, 13000], 16, 128
+    q, k, kq, decay, beta, v = ragged(lens, H, H, dim, dim, per_head, 1)
+    state, table, cu = torch.zeros(2, H, dim, dim, device=DEV), chunk_table(lens), i32(0, 17000, 30000)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    o = kernels.delta_chunked(q, k, decay, beta, v, state, table, cu, i32(0, 1), H, H, dim, dim)
+    assert torch.cuda.max_memory_allocated() - before < o.numel() * 4 + (520 << 20)
