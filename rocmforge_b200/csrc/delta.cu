@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(DL_WARPS * 32)
 delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ kq,
                   const float* __restrict__ decay, const float* __restrict__ beta, const float* __restrict__ v, int v_stride,
                   float* __restrict__ state, float* __restrict__ o, const int* __restrict__ cu_q,
-                  const int* __restrict__ seq_slot, int H, int G, int D, int V) {
+                  const int* __restrict__ seq_slot, int H, int G, int D, int V, int below) {
     constexpr int DP = LPC * ROWS;                                   // rows of the padded state
     constexpr int COLS = DL_WARPS * 32 / LPC;                        // value columns of a block
     constexpr int TOK = DP <= 64 ? 16 : (DP <= 128 ? 8 : 4);         // tokens of a stage
@@ -134,6 +134,7 @@ delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
     const int rg = lane % LPC, cl = warp * (32 / LPC) + lane / LPC;            // this lane's rows inside every 16, its column in the block
     const int hg = h / (H / G);
     const int t0 = cu_q[b], n = cu_q[b + 1] - t0;
+    if (below > 0 && n >= below) { pdl_wait(); return; }                       // another kernel's sequence
     const int col = j0 + cl;
     const bool live = col < V;
     float* S = state + ((size_t)seq_slot[b] * H + h) * D * V;
@@ -245,10 +246,10 @@ delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
 template <int ROWS, int LPC, bool PER_HEAD>
 static int launch_scan(const float* qn, const float* kn, const float* kq, const float* decay, const float* beta, const float* v,
                        int v_stride, float* state, float* o, const int* cu_q, const int* seq_slot, int B, int H, int G, int D,
-                       int V, cudaStream_t st) {
+                       int V, int below, cudaStream_t st) {
     constexpr int COLS = DL_WARPS * 32 / LPC;
     rf_launch(delta_scan_kernel<ROWS, LPC, PER_HEAD>, dim3((V + COLS - 1) / COLS, H, B), dim3(DL_WARPS * 32), 0, st, qn, kn, kq, decay,
-              beta, v, v_stride, state, o, cu_q, seq_slot, H, G, D, V);
+              beta, v, v_stride, state, o, cu_q, seq_slot, H, G, D, V, below);
     RF_LAUNCH_CHECK();
     return 0;
 }
@@ -277,14 +278,15 @@ int rf_delta_prepare(int dtype, const float* qkv, int qkv_stride, const float* a
     RF_LAUNCH_CHECK();
     return 0;
 }
-// decay float [T, H*D], or (per_head) [T, H]; state float [slots, H, D, V]; v float [T, v_stride] with head h's values at columns h*V..; o float [T, H*V]; cu_q [B+1]
+// decay float [T, H*D], or (per_head) [T, H]; state float [slots, H, D, V]; v float [T, v_stride] with head h's values at columns h*V..; o float [T, H*V]; cu_q [B+1].
+// below > 0: sequences that bring as many tokens or more are left alone.
 int rf_delta_scan(const float* qn, const float* kn, const float* kq, const float* decay, const float* beta, const float* v,
                   int v_stride, float* state, float* o, const int* cu_q, const int* seq_slot, int B, int H, int G, int D, int V,
-                  int per_head, int one_token, int lanes, cudaStream_t st) {
+                  int per_head, int one_token, int lanes, int below, cudaStream_t st) {
     if (B <= 0) return 0;
     if (lanes != 0 && lanes != 4 && lanes != 8) return RF_ERR_BAD_ARG;
     if (H <= 0 || G <= 0 || H % G || D <= 0 || V <= 0 || H > 65535 || B > 65535) return RF_ERR_BAD_ARG;
-#define DL_GO(ROWS, LPC) return (per_head ? launch_scan<ROWS, LPC, true> : launch_scan<ROWS, LPC, false>)(qn, kn, kq, decay, beta, v, v_stride, state, o, cu_q, seq_slot, B, H, G, D, V, st)
+#define DL_GO(ROWS, LPC) return (per_head ? launch_scan<ROWS, LPC, true> : launch_scan<ROWS, LPC, false>)(qn, kn, kq, decay, beta, v, v_stride, state, o, cu_q, seq_slot, B, H, G, D, V, below, st)
     // Steps of one token a sequence (the state is read and written once, nothing else): four lanes a column.  Steps with
     // longer portions: eight lanes a column (twice the blocks, half the chain of each; fetching the next token's operands
     // into registers ahead of the chain was measured and cost more in registers than it hid).  The two forms add a column's products in another order: a difference of rounding between a token

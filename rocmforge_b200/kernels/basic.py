@@ -1592,14 +1592,15 @@ def delta_prepare(qkv: torch.Tensor, a: torch.Tensor, dt_bias: torch.Tensor, a_l
 
 def delta_scan(qn: torch.Tensor, kn: torch.Tensor, kq: torch.Tensor, decay: torch.Tensor, beta: torch.Tensor, v: torch.Tensor,
                state: torch.Tensor, cu_q: torch.Tensor, seq_slot: torch.Tensor, heads: int, qk_heads: int, dim: int,
-               vdim: int, one_token: bool = False, lanes: int = 0) -> torch.Tensor:
+               vdim: int, one_token: bool = False, lanes: int = 0, below: int = 0, out: torch.Tensor | None = None) -> torch.Tensor:
     """The gated delta rule, token by token for every sequence of the step, per head (head h reads q/k head h // (heads /
     qk_heads)):  S <- diag(decay_t) S (decay [T, heads*dim], or [T, heads]: one number per head);  u = beta_t (v_t - S^T k_t);  S <- S + k_t u^T;  o_t = S^T q_t.
 
     ``state`` float32 [slots, heads, dim, vdim] is read and replaced; ``v`` float32 [T, >= heads*vdim] view; returns o float32
     [T, heads*vdim].  The sums' order depends on (dim, position) alone.  ``one_token``: every sequence of the
     step brings exactly one token (the kernel form for decoding: four lanes a value column instead of eight, which adds a
-    column's products in another order; ``lanes`` 4 or 8 forces a form, for measurements)."""
+    column's products in another order; ``lanes`` 4 or 8 forces a form, for measurements).  ``below`` > 0: sequences that bring so
+    many tokens or more are left alone, their rows of ``out`` and their states untouched."""
     need_cuda(qn, kn, kq, decay, beta, v, state, cu_q, seq_slot)
     T = qn.shape[0]
     B = seq_slot.shape[0]
@@ -1609,11 +1610,12 @@ def delta_scan(qn: torch.Tensor, kn: torch.Tensor, kq: torch.Tensor, decay: torc
     need(v.dtype == torch.float32 and v.dim() == 2 and v.stride(1) == 1 and v.shape == (T, heads * vdim), "delta_scan: v must be float32 [T, heads*vdim]")
     need(tuple(state.shape[1:]) == (heads, dim, vdim), "delta_scan: state must be [slots, heads, dim, vdim]")
     need(dim <= 256, "delta_scan: at most 256 key channels a head")
-    o = torch.empty((T, heads * vdim), dtype=torch.float32, device=qn.device)
+    need(out is None or (out.shape == (T, heads * vdim) and out.dtype == torch.float32 and out.is_contiguous()), "delta_scan: out must be float32 [T, heads*vdim]")
+    o = out if out is not None else torch.empty((T, heads * vdim), dtype=torch.float32, device=qn.device)
     f = _f("delta", "rf_delta_scan", c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
-           c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p)
+           c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p)
     check(f(ptr(qn), ptr(kn), ptr(kq), ptr(decay), ptr(beta), ptr(v), v.stride(0), ptr(state), ptr(o), ptr(cu_q), ptr(seq_slot),
-            B, heads, qk_heads, dim, vdim, int(decay.shape[1] == heads and dim != 1), int(bool(one_token)), int(lanes), stream()), f"delta_scan (heads={heads}, dim={dim}, vdim={vdim})")
+            B, heads, qk_heads, dim, vdim, int(decay.shape[1] == heads and dim != 1), int(bool(one_token)), int(lanes), int(below), stream()), f"delta_scan (heads={heads}, dim={dim}, vdim={vdim})")
     return o
 
 
@@ -1630,7 +1632,7 @@ def delta_chunked(qn: torch.Tensor, kn: torch.Tensor, decay: torch.Tensor, beta:
     """What ``delta_scan`` computes, with one decay per head (decay [T, heads]) or per key channel (decay [T, heads*dim]), for prompts:
     chunks of 64 tokens whose corrected values come from one triangular system each, side by side; then the states between the
     chunks one after the other; then every chunk's outputs.  All in 32-bit.  ``table``: the chunk table of ``retention_chunked``.
-    Differs from the scan by rounding only.  Chunks are taken in passes whose scratch memory stays below 512 MB
+    Sequences without chunks in the table are left alone.  Differs from the scan by rounding only.  Chunks are taken in passes whose scratch memory stays below 512 MB
     (``chunks_per_pass``: fewer, for tests); the passes change no bit."""
     need_cuda(qn, kn, decay, beta, v, state, table, cu_q, seq_slot)
     T, B = qn.shape[0], seq_slot.shape[0]

@@ -29,13 +29,15 @@ class GatedDeltaRule(Mixer):
 
     One product makes q | k | v | W_b x | W_a1 x | W_g1 x in the compute dtype; the decay's second product stays 32-bit,
     and so do the convolution's result, the unit norms, beta, softplus, the decays, S, o and its norm.  Per sequence the
-    mixer keeps S [heads, dim, vdim] and the convolution's last taps-1 inputs, so a prompt may be cut anywhere; long portions
-    run in chunks (``kernels.delta_chunked``), short ones and decoded tokens token by token, which differs by rounding.
+    mixer keeps S [heads, dim, vdim] and the convolution's last taps-1 inputs, so a prompt may be cut anywhere; portions of a
+    sequence from 512 tokens on (heads of more than 64 key channels) run in chunks (``kernels.delta_chunked``), shorter ones and
+    decoded tokens token by token, which differs by rounding.
     ``names``: the tensors' names below the part's prefix (keys q, k, v, q_conv, k_conv, v_conv, b, a_log, dt_bias, a1, a2,
     g1, g2, norm, o; a and g in place of the low-rank pairs).
 
     What other designs change: ``decay_rank`` None: ONE decay per head, g = exp(-exp(A_log_h) softplus(W_a x + dt_bias)) with
-    W_a [heads, H] and dt_bias [heads]; W_a and W_b are then a small product of their own whose result stays 32-bit.
+    W_a [heads, H] and dt_bias [heads]; W_a and W_b are then a small product of their own whose result stays 32-bit, and
+    prompts run in chunks from 160 tokens of the step's longest portion on.
     ``gate_rank`` None: the gate is one full matrix W_g x, part of the first product.  ``gate_fn`` "silu" instead of sigmoid.
     """
 
@@ -146,17 +148,26 @@ class GatedDeltaRule(Mixer):
 
     # Prompts run the recurrence in chunks side by side, steps of few tokens per sequence token by token.
     CHUNKED_FROM = 17            # tokens of the step's longest portion from which the chunk table is built (one table for all parts)
-    # ... and from which the chunked kernels are faster (16 heads of 128 x 128).  One decay per head: 64 tokens 44 against 26 us, 256
-    # tokens 54 against 77, 2,048 tokens 224 against 560.  A decay per key channel: 128 tokens 83 against 45, 256 90 against 87, 512 114
-    # against 170, 2,048 301 against 669, 1,365 + 900 + 513 421 against 697, 16 times 200 540 against 482.
+    # ... and from which the chunked kernels are faster with one decay per head (16 heads of 128 x 128): 64 tokens 44 against 26 us, 256
+    # tokens 54 against 77, 2,048 tokens 224 against 560.
     CHUNKS_PAY_FROM = 160
-    CHANNEL_CHUNKS_PAY_FROM = 256
+    # With a decay per key channel each sequence goes by its own number of new tokens, so its sums do not depend on what else is in the
+    # step.  us, chunks against scan, 16 heads of 128 x 128, prompts x tokens: 1 x 256 90, 87; 4 x 320 240, 206; 16 x 200 536, 484; 64 x 384
+    # 3226, 3285; 1 x 512 114, 170; 4 x 512 307, 327; 16 x 512 1078, 1251; 64 x 512 4246, 4387; 1 x 2,048 300, 672; 16 x 2,048 4144, 5028.
+    # Heads of at most 64 channels leave the scan more blocks per SM and never chunk (64 x 64: 1 x 512 73, 110, but 4 x 512 142, 141;
+    # 16 x 512 482, 306; 16 x 2,048 1835, 1209); 96 x 96 is like 128 (8 x 1,024 867, 1262), 256 x 256 too (8 x 1,024 3528, 4803).
+    CHANNEL_CHUNKS_FROM = 512
+    CHANNEL_CHUNKS_MIN_DIM = 65
+
+    @property
+    def chunks_channels(self) -> bool:
+        return self.decay_rank is not None and self.dim >= self.CHANNEL_CHUNKS_MIN_DIM
 
     def step_table_names(self):
-        return ("retention_chunks",)
+        return ("retention_chunks",) if self.decay_rank is None else ("channel_chunks",) if self.chunks_channels else ()
 
     def step_table(self, name, batch):
-        return recurrence_chunk_table(batch, self.CHUNKED_FROM)
+        return recurrence_chunk_table(batch, self.CHUNKED_FROM if name == "retention_chunks" else self.CHANNEL_CHUNKS_FROM, name == "channel_chunks")
 
     def cache_request(self):
         named = dict(S=((self.n_heads, self.dim, self.vdim), torch.float32))
@@ -188,16 +199,19 @@ class GatedDeltaRule(Mixer):
                                 ctx.seq_slot)                                # float32 [T, q | k | v]
         qn, kn, kq, decay, beta = kernels.delta_prepare(qkv, a, self.dt_bias, self.a_log, b, self.n_heads, self.qk_heads, self.dim,
                                                         self.q_scale, self.unit_eps)
-        v = qkv[:, 2 * self.qk_size:]
-        pays = self.CHUNKS_PAY_FROM if self.decay_rank is None else self.CHANNEL_CHUNKS_PAY_FROM
-        table = ctx.tables.get("retention_chunks") if ctx.max_new >= pays else None
-        if table is not None and table.numel() > 0:
-            o = kernels.delta_chunked(qn, kn, decay, beta, v, state_view["S"], table, ctx.cu_q, ctx.seq_slot, self.n_heads,
-                                      self.qk_heads, self.dim, self.vdim)
-        else:
-            o = kernels.delta_scan(qn, kn, kq, decay, beta, v, state_view["S"], ctx.cu_q, ctx.seq_slot, self.n_heads, self.qk_heads,
-                                   self.dim, self.vdim, one_token=ctx.is_decode)
+        o = self.recurrence(ctx, qn, kn, kq, decay, beta, qkv[:, 2 * self.qk_size:], state_view["S"])
         return kernels.retention_gate(o, gate, self.n_heads, self.vdim, self.eps, weight=self.norm_w, gate_fn=self.gate_fn)
+
+    def recurrence(self, ctx, qn, kn, kq, decay, beta, v, S):
+        """o float32 [T, heads*vdim] of the step's tokens, the sequences' states S brought on."""
+        where = (ctx.cu_q, ctx.seq_slot, self.n_heads, self.qk_heads, self.dim, self.vdim)
+        table = ctx.tables.get("channel_chunks" if self.decay_rank is not None else "retention_chunks")
+        if table is None or table.numel() == 0 or (self.decay_rank is None and ctx.max_new < self.CHUNKS_PAY_FROM):
+            return kernels.delta_scan(qn, kn, kq, decay, beta, v, S, *where, one_token=ctx.is_decode)
+        o = kernels.delta_chunked(qn, kn, decay, beta, v, S, table, *where)
+        if self.decay_rank is not None and (ctx.host is None or int(ctx.host.n_new.min()) < self.CHANNEL_CHUNKS_FROM):
+            kernels.delta_scan(qn, kn, kq, decay, beta, v, S, *where, below=self.CHANNEL_CHUNKS_FROM, out=o)      # the sequences without chunks
+        return o
 
     def forward(self, ctx, y, cache_view, stream):
         self.o.add_to_stream(ctx, self.gated(ctx, y, cache_view), stream)

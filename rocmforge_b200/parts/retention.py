@@ -14,16 +14,17 @@ from .base import MIXERS, Mixer
 from .linear import Linear
 
 
-def recurrence_chunk_table(batch, chunked_from: int) -> np.ndarray:
+def recurrence_chunk_table(batch, chunked_from: int, own: bool = False) -> np.ndarray:
     """The table of the recurrences' chunked kernels: first[B+1] (index of each sequence's first chunk), then (sequence,
     first row) of every chunk of 64 new tokens; empty for steps that take the token-by-token kernel (decoding, and
-    portions whose longest is below ``chunked_from`` tokens)."""
+    portions whose longest is below ``chunked_from`` tokens).  ``own``: every sequence goes by its own number of new tokens, and
+    one below ``chunked_from`` has no chunks, whatever the others bring."""
     if batch.is_decode or batch.max_new < chunked_from:
         return np.zeros((0,), dtype=np.int32)
     C = kernels.RETENTION_CHUNK
-    counts = [(int(n) + C - 1) // C for n in batch.n_new]
+    counts = [(int(n) + C - 1) // C if not own or n >= chunked_from else 0 for n in batch.n_new]
     first = np.concatenate([[0], np.cumsum(counts)])
-    pairs = [(b, q0) for b in range(batch.B) for q0 in range(0, int(batch.n_new[b]), C)]
+    pairs = [(b, C * i) for b in range(batch.B) for i in range(counts[b])]
     return np.concatenate([first, np.asarray(pairs, dtype=np.int64).reshape(-1)]).astype(np.int32)
 
 

@@ -111,3 +111,29 @@ def test_the_chunks_scratch_memory_is_bounded(per_head):
     before = torch.cuda.memory_allocated()
     o = kernels.delta_chunked(q, k, decay, beta, v, state, table, cu, i32(0, 1), H, H, dim, dim)
     assert torch.cuda.max_memory_allocated() - before < o.numel() * 4 + (520 << 20)
+
+
+def test_a_sequences_sums_do_not_depend_on_the_others():
+    """Sequences of 20, 511, 512, 700 and 1 tokens in one step and alone in theirs: the same outputs and states, bit for bit, through
+    the mixer's own choice of kernels."""
+    from types import SimpleNamespace
+    from rocmforge_b200.engine.batch import StepBatch, StepRequest
+    from rocmforge_b200.parts.delta import GatedDeltaRule
+    H, G, dim, vdim = 2, 1, 128, 40
+    part = GatedDeltaRule(256, H, G, dim, vdim, 4, 8, 8, 1e-6)
+    lens, slots = [20, 511, 512, 700, 1], [2, 0, 4, 1, 3]
+    data = ragged(lens, H, G, dim, vdim, False, 5)
+    begin = torch.randn(5, H, dim, vdim, device=DEV)
+
+    def run(which):
+        batch = StepBatch([StepRequest(slots[i], [1] * lens[i]) for i in which], [0] * len(which), 10,
+                          {n: (lambda b, n=n: part.step_table(n, b)) for n in part.step_table_names()})
+        rows = torch.cat([torch.arange(sum(lens[:i]), sum(lens[:i + 1])) for i in which]).to(DEV)
+        ctx = SimpleNamespace(cu_q=i32(*batch.cu_q.tolist()), seq_slot=i32(*batch.slots), max_new=batch.max_new, is_decode=False, host=batch,
+                              tables={n: torch.from_numpy(t).to(DEV) for n, t in batch.tables.items()})
+        state = begin.clone()
+        return part.recurrence(ctx, *(x[rows] for x in data), state), state, rows
+    whole, state, _ = run(range(5))
+    for i in range(5):
+        o, alone, rows = run([i])
+        assert torch.equal(o, whole[rows]) and torch.equal(alone[slots[i]], state[slots[i]]), lens[i]

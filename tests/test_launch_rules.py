@@ -19,3 +19,25 @@ def test_splits_of_the_32_bit_product_are_never_empty():
             s = basic.split_k_for_f32_tc(N, K, 148)
             kb = (K + 31) // 32
             assert 1 <= s and (s - 1) * ((kb + s - 1) // s) < kb and (s == 1 or s * ((N + 127) // 128) <= 148)
+
+
+def test_channel_decays_chunk_by_each_sequences_own_length():
+    """A sequence's chunks, and with them the order of its sums, must not depend on what the others of its step bring."""
+    import numpy as np
+    from rocmforge_b200.engine.batch import StepBatch, StepRequest
+    from rocmforge_b200.parts.delta import GatedDeltaRule
+    part = GatedDeltaRule(256, 2, 2, 128, 128, 4, 8, 8, 1e-6)
+    few = GatedDeltaRule(256, 2, 2, 64, 128, 4, 8, 8, 1e-6)
+    assert part.step_table_names() == ("channel_chunks",) and few.step_table_names() == ()
+    tables = {"channel_chunks": lambda b: part.step_table("channel_chunks", b)}
+    n = [20, 512, 511, 1, 700]
+    t = StepBatch([StepRequest(i, [1] * k) for i, k in enumerate(n)], [0] * 5, 10, tables).tables["channel_chunks"]
+    first, pairs = t[:6].tolist(), t[6:].reshape(-1, 2).tolist()
+    assert first == [0, 0, 8, 8, 8, 19]
+    assert pairs == [[1, 64 * i] for i in range(8)] + [[4, 64 * i] for i in range(11)]
+    for alone in ([20], [511, 400], [1, 1]):
+        assert StepBatch([StepRequest(i, [1] * k) for i, k in enumerate(alone)], [0] * len(alone), 10, tables).tables["channel_chunks"].size == 0
+    # chunks of all sequences of a step whose longest is long enough: the table of the other recurrences
+    t = StepBatch([StepRequest(i, [1] * k) for i, k in enumerate([20, 65])], [0, 0], 10,
+                  {"x": lambda b: part.step_table("retention_chunks", b)}).tables["x"]
+    assert np.array_equal(t, [0, 1, 3, 0, 0, 1, 0, 1, 64])
