@@ -17,8 +17,8 @@
 // so with the queries of the token kernel).
 //
 // Measured (us, the generic kernel's in brackets; 14 heads of 64 on 2 kv heads): a prompt of 1,999 tokens 68 [1,775], 8 of 16..1,024
-// 63 [1,205]; 28 heads of 128, 1,024 tokens 66 [1,886]; single tokens of 64 sequences of 16..1,024 keys 19 [142], of one with 20,000
-// 59 [2,240].  Error against 64 bits 1.7e-7 [2.6e-7], 1.4e-7 [2.6e-7] for single tokens.  A prompt's tile of 64 keys takes 2.7 us
+// 63 [1,205]; 28 heads of 128, 1,024 tokens 66 [1,886]; single tokens of 64 sequences of 16..1,024 keys 22.5 [142], of one with 20,000
+// 56 [2,240].  Error against 64 bits 1.7e-7 [2.6e-7], 1.4e-7 [2.6e-7] for single tokens.  A prompt's tile of 64 keys takes 2.7 us
 // where its MMAs need 0.8: one softmax warp a scheduler forms, splits and writes 64 weights a row with nothing beside it.
 #pragma once
 #include "f32_parts.cuh"
@@ -322,27 +322,54 @@ attention_f32_prompt_kernel(const __grid_constant__ CUtensorMap map_k, const __g
 
 #define FD_WARPS 8
 #define FD_U 4                                       // loads of a batch: 4 * 32 / LPK keys
+#define FD_SHARES 8
+
+__device__ __forceinline__ float eight_max(float v) {        // over eight neighbouring lanes (whole warps)
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+__device__ __forceinline__ float eight_sum(float v) {
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+// (rows of the output need no alignment)
+__device__ __forceinline__ void fd_store(float* out, float4 O, float L) {
+    out[0] = L > 0.f ? O.x / L : 0.f; out[1] = L > 0.f ? O.y / L : 0.f; out[2] = L > 0.f ? O.z / L : 0.f; out[3] = L > 0.f ? O.w / L : 0.f;
+}
 
 // LPK: lanes per key (head size / 4); GP: query heads of a pass.  gridDim.x = tokens * splits (a cluster of `splits`), y = kv heads,
 // z = passes over the group's heads.
+//
+// The keys a token sees are dealt to 1 .. 8 shares by their number alone (a share is at least a batch a warp), so its sums do not
+// depend on what else is in the step; the CTAs, whose number follows the step's size, take the shares in turn and their results
+// meet in the shares' order.  us, 14 heads of 64 on 2 kv heads, and with one share a CTA, whose sums followed the step's size: 1
+// sequence of 1,023 keys 6.9 and 7.1, 8 of 16..1,024 7.9 and 8.0, 64 of them 22.5 and 19.4 (two CTAs take four shares each there).
+// Tried: two batches a warp (64 sequences 22.6, 8 8.6); a number of CTAs that follows the keys alone, 256 a CTA (23.1 and 9.8:
+// a cluster waits for the room of its idle CTAs too).
 template <int LPK, int GP>
 __global__ void __launch_bounds__(FD_WARPS * 32, 2)
 attention_f32_token_kernel(const float* q, int q_stride, float* out, int out_stride,
                            const float* k_pages, const float* v_pages, const int* __restrict__ tok_seq,
                            const int* __restrict__ tok_pos, const int* __restrict__ seq_slot, const int* __restrict__ block_table,
-                           int max_pages, int nh, int nkv, float scale, int window, int splits) {
+                           int max_pages, int nh, int nkv, float scale, int window, int splits, int slots) {
     constexpr int HD = LPK * 4, KPL = 32 / LPK, BATCH = FD_U * KPL;
+    extern __shared__ __align__(16) float wo[];      // [slots][warps][GP][HD]: a warp's sums of a share; then the shares' own
+    float* co = wo + slots * FD_WARPS * GP * HD;     // [8 / splits, rounded up][GP][HD]
     __shared__ __align__(16) float pbuf[FD_WARPS][BATCH][GP];
-    __shared__ __align__(16) float wm[FD_WARPS][GP], wl[FD_WARPS][GP];
-    __shared__ __align__(16) float wo[FD_WARPS][GP][HD];
-    __shared__ float cm[GP], cl[GP];
-    __shared__ __align__(16) float co[GP][HD];
+    __shared__ __align__(16) float wc[FD_WARPS][GP], wm[FD_SHARES][FD_WARPS][GP], wl[FD_SHARES][FD_WARPS][GP];
+    __shared__ float cm[FD_SHARES][GP], cl[FD_SHARES][GP], factor[FD_SHARES][8][GP], all_l[GP];
+    constexpr int FOLD = GP * 8;                     // threads that fold the factors of a share: eight lanes a head
+    static_assert(FD_WARPS == 8 && FD_SHARES == 8, "eight lanes fold the warps' and the shares' factors");
     pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane / LPK, part = lane % LPK;
     const int rank = blockIdx.x % splits, t = blockIdx.x / splits, kvh = blockIdx.y;
     const int G = nh / nkv, g0 = blockIdx.z * GP, gb = min(GP, G - g0);
     const int pos = tok_pos[t], lo = rf_first_key(pos, window);
     const int* bt = block_table + (size_t)seq_slot[tok_seq[t]] * max_pages;
+    const int shares = min(FD_SHARES, (pos - lo + FD_WARPS * BATCH) / (FD_WARPS * BATCH)), ctas = min(splits, shares);
+    if (rank >= shares) return;                      // (rank 0 waits for the kernel before; a cluster's barriers do not wait for who has left)
     pdl_wait();
     float4 qv[GP];
 #pragma unroll
@@ -356,13 +383,18 @@ attention_f32_token_kernel(const float* q, int q_stride, float* out, int out_str
     bool writes = true;
 #pragma unroll
     for (int o = LPK / GP / 2; o >= 1; o >>= 1) if (lane & o) writes = false;
+    for (int share0 = rank; share0 < shares; share0 += splits * slots) {
+    if (share0 > rank) __syncthreads();              // the shares before have been summed up
+    // the warps go through up to `slots` shares without waiting for each other
+    int n_slots = 0;
+    for (int share = share0; share < shares && n_slots < slots; share += splits, ++n_slots) {
     float m = -INFINITY, l = 0.f;                    // of my_head, over this lane's keys (m over the warp's)
     float4 o[GP];
 #pragma unroll
     for (int g = 0; g < GP; ++g) o[g] = make_float4(0.f, 0.f, 0.f, 0.f);
 
-    const int u_last = pos / BATCH, stride = splits * FD_WARPS;
-    for (int u = lo / BATCH + rank * FD_WARPS + warp; u <= u_last; u += stride) {
+    const int u_last = pos / BATCH, stride = shares * FD_WARPS;
+    for (int u = lo / BATCH + share * FD_WARPS + warp; u <= u_last; u += stride) {
         const int key0 = u * BATCH;                  // a batch lies in one page
         const size_t base = (((size_t)bt[key0 / RF_PAGE] * nkv + kvh) * RF_PAGE + key0 % RF_PAGE) * HD + part * 4;
         float4 kv[FD_U], vv[FD_U];
@@ -412,11 +444,11 @@ attention_f32_token_kernel(const float* q, int q_stride, float* out, int out_str
         }
         l = l * corr + sum;
         if (__any_sync(0xffffffffu, corr != 1.f)) {
-            if (writes && sub == 0) wm[warp][my_head] = corr;
+            if (writes && sub == 0) wc[warp][my_head] = corr;
             __syncwarp();
 #pragma unroll
             for (int g = 0; g < GP; ++g) {
-                const float c = wm[warp][g];
+                const float c = wc[warp][g];
                 o[g].x *= c; o[g].y *= c; o[g].z *= c; o[g].w *= c;
             }
         }
@@ -445,57 +477,78 @@ attention_f32_token_kernel(const float* q, int q_stride, float* out, int out_str
     }
     __syncwarp();
     if (sub == 0) {
-        if (writes) { wm[warp][my_head] = m; wl[warp][my_head] = l; }
+        if (writes) { wm[n_slots][warp][my_head] = m; wl[n_slots][warp][my_head] = l; }
 #pragma unroll
-        for (int g = 0; g < GP; ++g) *reinterpret_cast<float4*>(&wo[warp][g][part * 4]) = o[g];
+        for (int g = 0; g < GP; ++g) *reinterpret_cast<float4*>(wo + ((n_slots * FD_WARPS + warp) * GP + g) * HD + part * 4) = o[g];
+    }
     }
     __syncthreads();
-    // ---- the CTA's, warps in index order
-    for (int i = threadIdx.x; i < GP * HD; i += FD_WARPS * 32) {
-        const int g = i / HD, d = i % HD;
-        float M = wm[0][g];
-#pragma unroll
-        for (int w = 1; w < FD_WARPS; ++w) M = fmaxf(M, wm[w][g]);
-        float L = 0.f, O = 0.f;
+    // ---- each share's, warps in index order: their factors first, then the sums, four dimensions a thread
+    const int at0 = share0 / splits;
+    for (int i = threadIdx.x; i < (n_slots * FOLD + 31) / 32 * 32; i += FD_WARPS * 32) {      // (whole warps)
+        const int k = min(i / FOLD, n_slots - 1), g = i / FD_WARPS % GP, w = i % FD_WARPS;
+        const float mw = wm[k][w][g], M = eight_max(mw), f = mw == -INFINITY ? 0.f : expf(mw - M), L = eight_sum(f * wl[k][w][g]);
+        if (i < n_slots * FOLD) {
+            factor[k][w][g] = f;
+            if (w == 0) { cm[at0 + k][g] = M; cl[at0 + k][g] = L; }
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x * 4; i < n_slots * GP * HD; i += FD_WARPS * 128) {
+        const int k = i / (GP * HD), e = i % (GP * HD), g = e / HD;
+        float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int w = 0; w < FD_WARPS; ++w) {
-            const float f = wm[w][g] == -INFINITY ? 0.f : expf(wm[w][g] - M);
-            L += f * wl[w][g];
-            O += f * wo[w][g][d];
+            const float f = factor[k][w][g];
+            const float4 x = *reinterpret_cast<const float4*>(wo + (k * FD_WARPS + w) * GP * HD + e);
+            O.x = fmaf(f, x.x, O.x); O.y = fmaf(f, x.y, O.y); O.z = fmaf(f, x.z, O.z); O.w = fmaf(f, x.w, O.w);
         }
-        if (splits == 1) {
-            if (g < gb) out[(size_t)t * out_stride + (size_t)(kvh * G + g0 + g) * HD + d] = L > 0.f ? O / L : 0.f;
-        } else {
-            co[g][d] = O;
-            if (d == 0) { cm[g] = M; cl[g] = L; }
-        }
+        if (shares == 1) {
+            if (g < gb) fd_store(out + (size_t)t * out_stride + (size_t)(kvh * G + g0) * HD + e, O, cl[0][g]);
+        } else *reinterpret_cast<float4*>(co + at0 * GP * HD + i) = O;
     }
-    if (splits == 1) return;
-    // ---- the cluster's, CTAs in rank order; each writes a share of the dimensions
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    const int share = HD / splits;
-    auto peer = [&](const float* p, int r) {
+    }
+    if (shares == 1) return;
+    // ---- all shares, in their order, the same way; each CTA writes some of the dimensions
+    if (ctas > 1) {
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    } else __syncthreads();
+    auto place = [&](const float* p, int r) {
         uint32_t a;
-        float v;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(r));
-        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
-        return v;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(r % splits));
+        return a;
     };
-    for (int i = threadIdx.x; i < gb * share; i += FD_WARPS * 32) {
-        const int g = i / share, d = rank * share + i % share;
-        float M = -INFINITY;
-        for (int r = 0; r < splits; ++r) M = fmaxf(M, peer(&cm[g], r));
-        float L = 0.f, O = 0.f;
-        for (int r = 0; r < splits; ++r) {
-            const float mr = peer(&cm[g], r), f = mr == -INFINITY ? 0.f : expf(mr - M);
-            L += f * peer(&cl[g], r);
-            O += f * peer(&co[g][d], r);
+    for (int i = threadIdx.x; i < (FOLD + 31) / 32 * 32; i += FD_WARPS * 32) {
+        const int g = i / FD_SHARES % GP, r = i % FD_SHARES;
+        float mr = -INFINITY, lr = 0.f;
+        if (r < shares) {
+            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(mr) : "r"(place(&cm[r / splits][g], r)) : "memory");
+            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(lr) : "r"(place(&cl[r / splits][g], r)) : "memory");
         }
-        out[(size_t)t * out_stride + (size_t)(kvh * G + g0 + g) * HD + d] = L > 0.f ? O / L : 0.f;
+        const float M = eight_max(mr), f = mr == -INFINITY ? 0.f : expf(mr - M), L = eight_sum(f * lr);
+        if (i < FOLD) {
+            factor[0][r][g] = f;
+            if (r == 0) all_l[g] = L;
+        }
     }
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");        // nobody's memory goes while a peer reads it
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    __syncthreads();
+    for (int i = (rank * FD_WARPS * 32 + threadIdx.x) * 4; i < gb * HD; i += ctas * FD_WARPS * 128) {
+        const int g = i / HD;
+        float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int r = 0; r < shares; ++r) {
+            const float f = factor[0][r][g];
+            float4 x;
+            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w)
+                         : "r"(place(co + (r / splits) * GP * HD + i, r)) : "memory");
+            O.x = fmaf(f, x.x, O.x); O.y = fmaf(f, x.y, O.y); O.z = fmaf(f, x.z, O.z); O.w = fmaf(f, x.w, O.w);
+        }
+        fd_store(out + (size_t)t * out_stride + (size_t)(kvh * G + g0) * HD + i, O, all_l[g]);
+    }
+    if (ctas > 1) {
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");    // nobody's memory goes while a peer reads it
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
 }
 
 // ---------------------------------------------------------------- host side
@@ -528,11 +581,17 @@ static int fd_launch(const float* q, int q_stride, float* out, int out_stride, c
                      int T, int splits, cudaStream_t st) {
     const int G = nh / nkv;
     dim3 grid(T * splits, nkv, (G + GP - 1) / GP);
+    // the shares of a CTA, and how many of them its warps may go through before their sums meet: as many as 64 KB hold
+    const size_t share = (size_t)GP * LPK * 4 * sizeof(float);
+    const int most = (FD_SHARES + splits - 1) / splits, fit = (int)((64 << 10) / (FD_WARPS * share)), slots = most < fit ? most : fit;
+    const size_t smem = (slots * FD_WARPS + most) * share;
+    static SmemLimit limit;
+    if (int e = limit.allow((const void*)attention_f32_token_kernel<LPK, GP>, smem)) return e;
     cudaError_t le = splits > 1
-        ? rf_launch_cluster(attention_f32_token_kernel<LPK, GP>, grid, dim3(FD_WARPS * 32), 0, st, splits, q, q_stride, out, out_stride, k_pages,
-                            v_pages, tok_seq, tok_pos, seq_slot, block_table, max_pages, nh, nkv, scale, window, splits)
-        : rf_launch(attention_f32_token_kernel<LPK, GP>, grid, dim3(FD_WARPS * 32), 0, st, q, q_stride, out, out_stride, k_pages, v_pages,
-                    tok_seq, tok_pos, seq_slot, block_table, max_pages, nh, nkv, scale, window, splits);
+        ? rf_launch_cluster(attention_f32_token_kernel<LPK, GP>, grid, dim3(FD_WARPS * 32), smem, st, splits, q, q_stride, out, out_stride, k_pages,
+                            v_pages, tok_seq, tok_pos, seq_slot, block_table, max_pages, nh, nkv, scale, window, splits, slots)
+        : rf_launch(attention_f32_token_kernel<LPK, GP>, grid, dim3(FD_WARPS * 32), smem, st, q, q_stride, out, out_stride, k_pages, v_pages,
+                    tok_seq, tok_pos, seq_slot, block_table, max_pages, nh, nkv, scale, window, splits, slots);
     if (le != cudaSuccess) return (int)le;
     RF_LAUNCH_CHECK();
     return 0;

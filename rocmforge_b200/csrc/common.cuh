@@ -71,6 +71,21 @@ static cudaError_t rf_launch_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 b
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// A kernel's dynamic shared memory beyond the 48 KB that need no asking for: the limit is set once for each device that launches it.
+struct SmemLimit {
+    size_t set[64] = {};
+    int allow(const void* kernel, size_t bytes) {
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e != cudaSuccess) return (int)e;
+        if (dev >= 0 && dev < 64 && bytes <= set[dev]) return 0;
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (e != cudaSuccess) return (int)e;
+        if (dev >= 0 && dev < 64) set[dev] = bytes;
+        return 0;
+    }
+};
+
 #define RF_LAUNCH_CHECK()                         \
     do {                                          \
         cudaError_t e__ = cudaGetLastError();     \

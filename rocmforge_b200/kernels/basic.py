@@ -476,7 +476,8 @@ def attention_f32_token_supported(n_heads: int, n_kv_heads: int, head_dim: int) 
 def attention_f32_token(q: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: int, k_pages, v_pages, tok_seq, tok_pos, seq_slot,
                         block_table, scale: float, window: int | None, splits: int | None = None, out: torch.Tensor | None = None, *,
                         chunk: int | None = None) -> torch.Tensor:
-    """Attention of single tokens in 32 bits, heads of 32, 64 or 128, plain softmax: ``splits`` CTAs (1, 2, 4 or 8) per (token, kv head)."""
+    """Attention of single tokens in 32 bits, heads of 32, 64 or 128, plain softmax: ``splits`` CTAs (1, 2, 4 or 8) per (token, kv
+    head), which change no bit: a token's sums follow the keys it sees alone."""
     need_cuda(tok_seq, tok_pos, seq_slot, block_table)
     _f32_attention_operands(q, k_pages, v_pages, n_kv_heads, head_dim, "attention_f32_token")
     need(attention_f32_token_supported(n_heads, n_kv_heads, head_dim) and q.shape[1] >= n_heads * head_dim,
@@ -496,8 +497,8 @@ def attention_f32_token(q: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim
 
 def f32_token_splits(T: int, n_kv_heads: int, longest: int | None = None, window: int | None = None) -> int:
     """CTAs per (token, kv head) of ``attention_f32_token``: as many as fit the GPU at two a SM, at most one per page of keys.
-    Measured, us with 1, 2, 4, 8: 64 sequences of 16..1,024 keys, 2 kv heads 29.3, 19.1, 21.5, 31.0; 8 of them 19.3, 13.2, 9.6, 8.2; 8 of
-    512 keys, 4 kv heads of 128 21.9, 17.9, 13.0, 10.3; 20 tokens of one prompt 3.2, 4.9, 5.2, 10.3."""
+    Measured, us with 1, 2, 4, 8: 64 sequences of 16..1,024 keys, 2 kv heads 38.0, 22.5, 24.9, 30.9; 8 of them 27.2, 16.2, 10.2, 7.9; 8 of
+    512 keys, 4 kv heads of 128 28.4, 19.5, 13.3, 9.8."""
     s = 1
     while s < 8 and T * n_kv_heads * s * 2 <= 2 * device_sm_count():
         s *= 2

@@ -88,6 +88,17 @@ def test_single_tokens(nh, nkv, hd, span):
         close(run(b, "token", splits=splits, **span), want)
 
 
+@pytest.mark.parametrize("span", [dict(), dict(window=65), dict(chunk=300)], ids=str)
+@pytest.mark.parametrize("nh,nkv,hd", [(6, 2, 32), (7, 1, 64), (9, 1, 64), (10, 2, 128)])
+def test_a_tokens_sums_do_not_depend_on_the_number_of_ctas(nh, nkv, hd, span):
+    """How many CTAs share a token follows the step's size; its sums must not, so every number gives the same bits.  Contexts at the
+    edges of the shares: 31 to 1,025 keys."""
+    b = batch([0, 30, 31, 63, 64, 127, 128, 255, 256, 511, 700, 1000, 1024], [1] * 13, nh, nkv, hd, seed=hd)
+    want = run(b, "token", splits=8, **span)
+    for splits in (1, 2, 4):
+        assert torch.equal(run(b, "token", splits=splits, **span), want)
+
+
 def test_no_larger_error_than_the_generic_kernel():
     for kind, b in (("prompt", batch([0, 700], [900, 400], 4, 2, 64)), ("token", batch([900] * 4, [1] * 4, 14, 2, 64)),
                     ("prompt", batch([0], [700], 4, 1, 128)), ("token", batch([500] * 4, [1] * 4, 10, 2, 128))):
