@@ -340,7 +340,7 @@ __device__ __forceinline__ void fd_store(float* out, float4 O, float L) {
 }
 
 // LPK: lanes per key (head size / 4); GP: query heads of a pass.  gridDim.x = tokens * splits (a cluster of `splits`), y = kv heads,
-// z = passes over the group's heads.
+// z = passes over the group's heads.  rows: the step's tokens that are taken (null: all).
 //
 // The keys a token sees are dealt to 1 .. 8 shares by their number alone (a share is at least a batch a warp), so its sums do not
 // depend on what else is in the step; the CTAs, whose number follows the step's size, take the shares in turn and their results
@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(FD_WARPS * 32, 2)
 attention_f32_token_kernel(const float* q, int q_stride, float* out, int out_stride,
                            const float* k_pages, const float* v_pages, const int* __restrict__ tok_seq,
                            const int* __restrict__ tok_pos, const int* __restrict__ seq_slot, const int* __restrict__ block_table,
-                           int max_pages, int nh, int nkv, float scale, int window, int splits, int slots) {
+                           int max_pages, int nh, int nkv, float scale, int window, int splits, int slots, const int* __restrict__ rows) {
     constexpr int HD = LPK * 4, KPL = 32 / LPK, BATCH = FD_U * KPL;
     extern __shared__ __align__(16) float wo[];      // [slots][warps][GP][HD]: a warp's sums of a share; then the shares' own
     float* co = wo + slots * FD_WARPS * GP * HD;     // [8 / splits, rounded up][GP][HD]
@@ -364,7 +364,7 @@ attention_f32_token_kernel(const float* q, int q_stride, float* out, int out_str
     static_assert(FD_WARPS == 8 && FD_SHARES == 8, "eight lanes fold the warps' and the shares' factors");
     pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane / LPK, part = lane % LPK;
-    const int rank = blockIdx.x % splits, t = blockIdx.x / splits, kvh = blockIdx.y;
+    const int rank = blockIdx.x % splits, t = rows != nullptr ? rows[blockIdx.x / splits] : blockIdx.x / splits, kvh = blockIdx.y;
     const int G = nh / nkv, g0 = blockIdx.z * GP, gb = min(GP, G - g0);
     const int pos = tok_pos[t], lo = rf_first_key(pos, window);
     const int* bt = block_table + (size_t)seq_slot[tok_seq[t]] * max_pages;
@@ -578,7 +578,7 @@ static int fa_launch(const float* q, int q_stride, float* out, int out_stride, c
 template <int LPK, int GP>
 static int fd_launch(const float* q, int q_stride, float* out, int out_stride, const float* k_pages, const float* v_pages, const int* tok_seq,
                      const int* tok_pos, const int* seq_slot, const int* block_table, int max_pages, int nh, int nkv, float scale, int window,
-                     int T, int splits, cudaStream_t st) {
+                     int T, int splits, const int* rows, cudaStream_t st) {
     const int G = nh / nkv;
     dim3 grid(T * splits, nkv, (G + GP - 1) / GP);
     // the shares of a CTA, and how many of them its warps may go through before their sums meet: as many as 64 KB hold
@@ -589,9 +589,9 @@ static int fd_launch(const float* q, int q_stride, float* out, int out_stride, c
     if (int e = limit.allow((const void*)attention_f32_token_kernel<LPK, GP>, smem)) return e;
     cudaError_t le = splits > 1
         ? rf_launch_cluster(attention_f32_token_kernel<LPK, GP>, grid, dim3(FD_WARPS * 32), smem, st, splits, q, q_stride, out, out_stride, k_pages,
-                            v_pages, tok_seq, tok_pos, seq_slot, block_table, max_pages, nh, nkv, scale, window, splits, slots)
+                            v_pages, tok_seq, tok_pos, seq_slot, block_table, max_pages, nh, nkv, scale, window, splits, slots, rows)
         : rf_launch(attention_f32_token_kernel<LPK, GP>, grid, dim3(FD_WARPS * 32), smem, st, q, q_stride, out, out_stride, k_pages, v_pages,
-                    tok_seq, tok_pos, seq_slot, block_table, max_pages, nh, nkv, scale, window, splits, slots);
+                    tok_seq, tok_pos, seq_slot, block_table, max_pages, nh, nkv, scale, window, splits, slots, rows);
     if (le != cudaSuccess) return (int)le;
     RF_LAUNCH_CHECK();
     return 0;
@@ -623,10 +623,10 @@ int rf_attention_f32_token_supported(int nh, int nkv, int hd) {
     return nkv > 0 && nkv <= 65535 && nh % nkv == 0 && (hd == 32 || hd == 64 || hd == 128);
 }
 
-// splits: CTAs that share one (token, kv head), 1, 2, 4 or 8.
+// splits: CTAs that share one (token, kv head), 1, 2, 4 or 8.  rows: T indices of the step's tokens, or null for the first T.
 int rf_attention_f32_token(const float* q, int q_stride, float* out, int out_stride, const float* k_pages, const float* v_pages,
                            const int* tok_seq, const int* tok_pos, const int* seq_slot, const int* block_table, int max_pages, int nh, int nkv,
-                           int hd, float scale, int window, int T, int splits, cudaStream_t st) {
+                           int hd, float scale, int window, int T, int splits, const int* rows, cudaStream_t st) {
     if (T <= 0) return 0;
     if (!rf_attention_f32_token_supported(nh, nkv, hd)) return RF_ERR_UNSUPPORTED;
     if (splits != 1 && splits != 2 && splits != 4 && splits != 8) return RF_ERR_BAD_ARG;
@@ -635,7 +635,7 @@ int rf_attention_f32_token(const float* q, int q_stride, float* out, int out_str
         return RF_ERR_BAD_ARG;
     const int G = nh / nkv;
 #define FD_GO(LPK, GP) fd_launch<LPK, GP>(q, q_stride, out, out_stride, k_pages, v_pages, tok_seq, tok_pos, seq_slot, block_table, max_pages, \
-                                          nh, nkv, scale, window, T, splits, st)
+                                          nh, nkv, scale, window, T, splits, rows, st)
     if (hd == 32) return G <= 2 ? FD_GO(8, 2) : (G <= 4 ? FD_GO(8, 4) : FD_GO(8, 8));
     if (hd == 64) return G <= 2 ? FD_GO(16, 2) : (G <= 4 ? FD_GO(16, 4) : FD_GO(16, 8));
     return G <= 2 ? FD_GO(32, 2) : (G <= 4 ? FD_GO(32, 4) : FD_GO(32, 8));

@@ -1,6 +1,6 @@
 from ._ffi import KernelError
 from .basic import (PAGE, embed, add_rmsnorm, rope_kv_write, swiglu, gemm_simt, split_k_for_simt, gemm_plain, split_k_for_plain, gemm_f32_tc, f32_tc_takes, F32_SWIGLU, attention_generic, attention_f32_prompt, attention_f32_prompt_supported, attention_f32_token,
-                    attention_f32_token_supported, f32_token_splits, f32_prompt_pays, argmax, sample, set_sample_cached, advance_decode, gather_tokens,
+                    attention_f32_token_supported, f32_token_splits, F32_PROMPT_FROM, argmax, sample, set_sample_cached, advance_decode, gather_tokens,
                     attention_decode, attention_decode_supported, attention_decode_scratch, DECODE_CHUNK,
                     attention_prefill, attention_prefill_supported, PREFILL_TILE,
                     attention_decode_warps, decode_splits, decode_pages,

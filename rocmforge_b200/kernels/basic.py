@@ -475,22 +475,24 @@ def attention_f32_token_supported(n_heads: int, n_kv_heads: int, head_dim: int) 
 
 def attention_f32_token(q: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: int, k_pages, v_pages, tok_seq, tok_pos, seq_slot,
                         block_table, scale: float, window: int | None, splits: int | None = None, out: torch.Tensor | None = None, *,
-                        chunk: int | None = None) -> torch.Tensor:
+                        chunk: int | None = None, rows: torch.Tensor | None = None) -> torch.Tensor:
     """Attention of single tokens in 32 bits, heads of 32, 64 or 128, plain softmax: ``splits`` CTAs (1, 2, 4 or 8) per (token, kv
-    head), which change no bit: a token's sums follow the keys it sees alone."""
-    need_cuda(tok_seq, tok_pos, seq_slot, block_table)
+    head), which change no bit: a token's sums follow the keys it sees alone.  ``rows`` (int32): only these tokens of the step."""
+    need_cuda(tok_seq, tok_pos, seq_slot, block_table, rows)
+    need(rows is None or (rows.dtype == torch.int32 and rows.is_contiguous()), "attention_f32_token: rows must be int32")
     _f32_attention_operands(q, k_pages, v_pages, n_kv_heads, head_dim, "attention_f32_token")
     need(attention_f32_token_supported(n_heads, n_kv_heads, head_dim) and q.shape[1] >= n_heads * head_dim,
          f"attention_f32_token: heads={n_heads}, kv_heads={n_kv_heads}, head_dim={head_dim} is not supported")
-    T = q.shape[0]
+    T = q.shape[0] if rows is None else rows.numel()
     if splits is None:
         splits = f32_token_splits(T, n_kv_heads)
     if out is None:
-        out = torch.empty((T, n_heads * head_dim), dtype=torch.float32, device=q.device)
+        out = torch.empty((q.shape[0], n_heads * head_dim), dtype=torch.float32, device=q.device)
     f = _f("attention_generic", "rf_attention_f32_token", c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-           c_void_p, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_void_p)
+           c_void_p, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_void_p, c_void_p)
     check(f(ptr(q), q.stride(0), ptr(out), out.stride(0), ptr(k_pages), ptr(v_pages), ptr(tok_seq), ptr(tok_pos), ptr(seq_slot),
-            ptr(block_table), block_table.shape[1], n_heads, n_kv_heads, head_dim, float(scale), key_span(window, chunk), T, splits, stream()),
+            ptr(block_table), block_table.shape[1], n_heads, n_kv_heads, head_dim, float(scale), key_span(window, chunk), T, splits,
+            ptr(rows), stream()),
           f"attention_f32_token (heads={n_heads}, kv_heads={n_kv_heads}, head_dim={head_dim}, splits={splits})")
     return out
 
@@ -508,12 +510,12 @@ def f32_token_splits(T: int, n_kv_heads: int, longest: int | None = None, window
     return s
 
 
-def f32_prompt_pays(T: int, B: int) -> bool:
-    """Whether a step of T tokens of B sequences is a prompt's work (``attention_f32_prompt``) rather than so many single tokens': a
-    query tile of 128 rows costs as much with one row.  Measured, us, prompt and token kernel (14 heads of 64, 2 kv heads): 100 tokens
-    10.1 and 6.1; 4 times 16 tokens after 500 21.7 and 13.0; 16 times 4 38 and 12.5; 8 prompts of 16..1,024 63 and 319; 1,999 tokens
-    68 and 429."""
-    return T > 128 and T > 16 * B
+# New tokens of a sequence from which its attention in 32 bits is a prompt's work (``attention_f32_prompt``) rather than so many single
+# tokens'.  The sequence's own number decides, so its sums do not depend on the others of its step.  A query tile of 128 rows costs as
+# much with one row.  Measured, us, prompt and token kernel (14 heads of 64, 2 kv heads), sequences x new tokens after cached ones:
+# 1 x 64 7.8 and 4.7; 1 x 100 9.8, 6.4; 1 x 200 12.3, 13.8; 64 x 30 46.4, 45.9; 64 x 63 50, 105; 1 x 64 after 2,000 61, 35; 1 x 128
+# after 2,000 55, 64; 16 x 32 after 500 41, 67; 16 x 64 after 500 43, 129; 8 x 100 after 1,000 40, 183; 1,999 tokens 68, 429.
+F32_PROMPT_FROM = 64
 
 
 def argmax(logits: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:

@@ -15,12 +15,12 @@ from .base import MIXERS, Mixer, POSITIONS
 from .linear import Linear
 
 
-def query_tiles(batch, rows: int) -> np.ndarray:
+def query_tiles(batch, rows: int, at_least: int = 1) -> np.ndarray:
     """(sequence, first row) pairs of the step's query tiles of ``rows`` rows, by the keys a tile sees (none for steps of one token
-    per sequence)."""
+    per sequence), of the sequences that bring ``at_least`` tokens."""
     if batch.is_decode:
         return np.zeros((0,), dtype=np.int32)
-    tiles = [(i, q0) for i in range(batch.B) for q0 in range(0, int(batch.n_new[i]), rows)]
+    tiles = [(i, q0) for i in range(batch.B) if batch.n_new[i] >= at_least for q0 in range(0, int(batch.n_new[i]), rows)]
     tiles.sort(key=lambda t: int(batch.starts[t[0]]) + t[1])
     return np.asarray(tiles, dtype=np.int32).reshape(-1)
 
@@ -166,6 +166,7 @@ class GQAAttention(Mixer):
 
     def bind(self, params, compute_dtype):
         n = self.names
+        self.compute_dtype = compute_dtype
         # one product for everything that reads the mixer's input: q | k | v | gate (k, v absent with a borrowed cache)
         blocks = [params[n["q"]]] + ([] if self.shares_kv else [params[n["k"]]] + ([] if self.values_are_keys else [params[n["v"]]]))
         self.gate_col = self.q_size + (0 if self.shares_kv else self.kv_size + self.v_size)
@@ -217,15 +218,24 @@ class GQAAttention(Mixer):
     # rows of the query tiles of the two tiled prefill kernels (csrc/attention_prefill.cu, attention_prefill_tc.cu)
     TILE_ROWS = {"attention_tiles64": 64, "attention_tiles128": 128}
 
+    compute_dtype: Optional[torch.dtype] = None           # known once the part is bound
+
     def step_table_names(self):
         if self.v_head_dim != self.head_dim:
             return ()
+        if self.compute_dtype == torch.float32:
+            return ("f32_prompt_tiles", "f32_token_rows")
         return ("attention_tiles128",) if self.keep_first or self.sink else tuple(self.TILE_ROWS)
 
     def step_table(self, name, batch):
         """(sequence, first row) of every query tile of the step's new tokens, sorted by the keys a tile sees (the
         kernels start with the heaviest): decided on the host so that the device never searches.  Steps of one token
         per sequence need none."""
+        if name == "f32_prompt_tiles":                    # the sequences whose attention in 32 bits is a prompt's work ...
+            return query_tiles(batch, 128, kernels.F32_PROMPT_FROM)
+        if name == "f32_token_rows":                      # ... and the tokens of the others, where a step has both
+            few = batch.n_new < kernels.F32_PROMPT_FROM
+            return np.nonzero(few[batch.tok_seq])[0].astype(np.int32) if few.any() and not few.all() else np.zeros((0,), dtype=np.int32)
         return query_tiles(batch, self.TILE_ROWS[name])
 
     def forward(self, ctx, y, cache_view, stream):
@@ -328,14 +338,17 @@ class GQAAttention(Mixer):
         if (ctx.compute_dtype == torch.float32 and ctx.options.tuned_attention and q.data_ptr() % 16 == 0 and q.stride(0) % 4 == 0
                 and view.v_pages.is_contiguous() and view.k_pages.data_ptr() % 16 == 0 and view.v_pages.data_ptr() % 16 == 0):
             # plain softmax in 32 bits (the options that are not plain went to the generic kernel above)
-            if (tiles128 is not None and tiles128.numel() > 0 and kernels.f32_prompt_pays(ctx.T, ctx.B) and self.scale > 0
-                    and kernels.attention_f32_prompt_supported(nh, nkv, hd)):
-                return kernels.attention_f32_prompt(q, nh, nkv, hd, view.k_pages, view.v_pages, tiles128, ctx.seq_slot, ctx.seq_start,
-                                                    ctx.seq_nnew, ctx.cu_q, view.block_table, self.scale, self.window, chunk=self.chunk)
+            tiles, rows, out = ctx.tables.get("f32_prompt_tiles"), None, None
+            if tiles is not None and tiles.numel() > 0 and self.scale > 0 and kernels.attention_f32_prompt_supported(nh, nkv, hd):
+                out = kernels.attention_f32_prompt(q, nh, nkv, hd, view.k_pages, view.v_pages, tiles, ctx.seq_slot, ctx.seq_start,
+                                                   ctx.seq_nnew, ctx.cu_q, view.block_table, self.scale, self.window, chunk=self.chunk)
+                rows = ctx.tables["f32_token_rows"]
+                if rows.numel() == 0:
+                    return out
             if kernels.attention_f32_token_supported(nh, nkv, hd):
                 return kernels.attention_f32_token(q, nh, nkv, hd, view.k_pages, view.v_pages, ctx.tok_seq, ctx.tok_pos, ctx.seq_slot,
-                                                   view.block_table, self.scale, self.window, chunk=self.chunk,
-                                                   splits=kernels.f32_token_splits(ctx.T, nkv, longest, span))
+                                                   view.block_table, self.scale, self.window, chunk=self.chunk, rows=rows, out=out,
+                                                   splits=kernels.f32_token_splits(ctx.T if rows is None else rows.numel(), nkv, longest, span))
         if (ctx.is_decode and ctx.compute_dtype == torch.bfloat16 and ctx.options.tuned_attention
                 and kernels.attention_decode_supported(nh, nkv, hd)):
             if ctx.options.clustered_decode:

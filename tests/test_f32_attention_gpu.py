@@ -99,6 +99,42 @@ def test_a_tokens_sums_do_not_depend_on_the_number_of_ctas(nh, nkv, hd, span):
         assert torch.equal(run(b, "token", splits=splits, **span), want)
 
 
+@pytest.mark.parametrize("hd", [64, 128, 32])
+def test_a_sequences_kernel_does_not_depend_on_the_others(hd):
+    """Sequences that bring 1 to 200 tokens in one step and each alone in its own: the same bits, through the mixer's own choice; and
+    some tokens of a step by their indices, the others' rows left as they were."""
+    from test_parts_gpu import context
+    from rocmforge_b200 import kernels
+    from rocmforge_b200.cache import SequenceCache
+    from rocmforge_b200.parts import MIXERS, POSITIONS
+    nh, nkv, lens, starts = 4, 2, [200, 1, 64, 63, 17], [0, 300, 70, 5, 0]
+    mixer = MIXERS.build("gqa_attention", hidden=32, n_heads=nh, n_kv_heads=nkv, head_dim=hd, qkv_bias=False,
+                         position=POSITIONS.build("rope_neox", head_dim=hd, theta=1e4))
+    g = torch.Generator().manual_seed(hd)
+    mixer.bind({n: torch.randn(*sp.shape, generator=g).to(DEV) for n, sp in mixer.param_specs().items()}, torch.float32)
+    cache = SequenceCache({0: mixer.cache_request()}, max_tokens=2048, dtype=torch.float32, device=DEV)
+    slots = [cache.alloc_slot() for _ in lens]
+    cache.prepare(slots, [a + b for a, b in zip(starts, lens)])
+    view = cache.view(0)
+    for pages in (view.k_pages, view.v_pages):
+        pages.copy_(torch.randn(pages.shape, generator=g))
+    q = torch.randn(sum(lens), nh * hd, generator=g).to(DEV)
+
+    def attend(which):
+        ctx = context(torch.float32, [(slots[i], [0] * lens[i], []) for i in which], [starts[i] for i in which], parts=[mixer])
+        rows = torch.cat([torch.arange(sum(lens[:i]), sum(lens[:i + 1])) for i in which])
+        return mixer.attend(ctx, q[rows.to(DEV)].contiguous(), view), rows
+    whole, _ = attend(range(len(lens)))
+    assert whole.isfinite().all()
+    for i in range(len(lens)):
+        o, rows = attend([i])
+        assert torch.equal(o, whole[rows.to(DEV)]), lens[i]
+    b = batch([0, 9, 100], [3, 1, 2], nh, nkv, hd)
+    want, out = run(b, "token"), torch.full((6, nh * hd), 7.0, device=DEV)
+    assert run(b, "token", rows=i32([5, 0, 3]), out=out) is out
+    assert torch.equal(out[[5, 0, 3]], want[[5, 0, 3]]) and (out[[1, 2, 4]] == 7).all()
+
+
 def test_no_larger_error_than_the_generic_kernel():
     for kind, b in (("prompt", batch([0, 700], [900, 400], 4, 2, 64)), ("token", batch([900] * 4, [1] * 4, 14, 2, 64)),
                     ("prompt", batch([0], [700], 4, 1, 128)), ("token", batch([500] * 4, [1] * 4, 10, 2, 128))):
@@ -129,7 +165,6 @@ def test_rules():
     from rocmforge_b200 import kernels
     assert kernels.f32_token_splits(1, 1) == 8 and kernels.f32_token_splits(1, 1, longest=100) == 2
     assert kernels.f32_token_splits(300, 2) == 1 and kernels.f32_token_splits(1, 1, 5000, 64) == 2
-    assert kernels.f32_prompt_pays(129, 1) and not kernels.f32_prompt_pays(128, 1) and not kernels.f32_prompt_pays(1024, 64)
     for nh, nkv, hd in [(4, 2, 48), (4, 2, 16), (4, 2, 256)]:
         assert not kernels.attention_f32_prompt_supported(nh, nkv, hd) and not kernels.attention_f32_token_supported(nh, nkv, hd)
     b = batch([0], [3], 4, 2, 16)

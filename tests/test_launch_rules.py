@@ -41,3 +41,23 @@ def test_channel_decays_chunk_by_each_sequences_own_length():
     t = StepBatch([StepRequest(i, [1] * k) for i, k in enumerate([20, 65])], [0, 0], 10,
                   {"x": lambda b: part.step_table("retention_chunks", b)}).tables["x"]
     assert np.array_equal(t, [0, 1, 3, 0, 0, 1, 0, 1, 64])
+
+
+def test_attention_in_32_bits_goes_by_each_sequences_own_tokens():
+    """Which kernel a sequence takes must not depend on what the others of its step bring."""
+    import torch
+    from rocmforge_b200.engine.batch import StepBatch, StepRequest
+    from rocmforge_b200.kernels import F32_PROMPT_FROM as many
+    from rocmforge_b200.parts import MIXERS, POSITIONS
+    part = MIXERS.build("gqa_attention", hidden=32, n_heads=2, n_kv_heads=1, head_dim=64, qkv_bias=False,
+                        position=POSITIONS.build("rope_neox", head_dim=64, theta=1e4))
+    part.bind({n: torch.zeros(*sp.shape) for n, sp in part.param_specs().items()}, torch.float32)
+    assert part.step_table_names() == ("f32_prompt_tiles", "f32_token_rows")
+
+    def tables(n, starts=None):
+        t = StepBatch([StepRequest(i, [1] * k) for i, k in enumerate(n)], starts or [0] * len(n), 10,
+                      {name: (lambda b, name=name: part.step_table(name, b)) for name in part.step_table_names()}).tables
+        return t["f32_prompt_tiles"].reshape(-1, 2).tolist(), t["f32_token_rows"].tolist()
+    assert tables([1, many, 2, 130]) == ([[1, 0], [3, 0], [3, 128]], [0, many + 1, many + 2])
+    assert tables([130, many], [0, 500]) == ([[0, 0], [0, 128], [1, 0]], [])
+    assert tables([many - 1, 5]) == ([], []) and tables([1, 1, 1]) == ([], [])
