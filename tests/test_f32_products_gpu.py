@@ -104,3 +104,53 @@ def test_what_the_route_leaves_to_the_cuda_cores():
     for bad in [dict(x=x, w=w[:, :4]), dict(x=x.double(), w=w.double()), dict(x=x.cpu(), w=w)]:
         with pytest.raises(kernels.KernelError):
             kernels.gemm_plain(bad["x"], bad["w"])
+
+
+def us(f, n=5):
+    f()
+    a, b = torch.cuda.Event(True), torch.cuda.Event(True)
+    a.record()
+    for _ in range(n):
+        f()
+    b.record()
+    torch.cuda.synchronize()
+    return a.elapsed_time(b) / n * 1e3
+
+
+@pytest.mark.parametrize("M,N,K,mode", [(1999, 896, 4864, "store"), (300, 512, 896, "swiglu"), (64, 512, 896, "partial"), (140, 130, 132, "add")])
+def test_whatever_is_not_finite_costs_a_bounded_time(M, N, K, mode):
+    """A NaN, an infinity or a sum that overflows in one token and in every token: the CUDA-core kernel's kinds of results, the other
+    tokens' bits as they were, no status, and no more than sixteen times the CUDA-core kernel's time (it reads both operands once
+    for 128 x 128 results; here a result reads its two rows, 128 numbers at a time)."""
+    from rocmforge_b200 import kernels
+    from rocmforge_b200.kernels import basic, tensor_core
+    kw = dict(store={}, swiglu=dict(mode=basic.F32_SWIGLU), partial=dict(mode=basic.F32_PARTIAL, splits=4), add=dict(mode=basic.F32_ADD))[mode]
+
+    def call(x, w):
+        if mode != "add":
+            return kernels.gemm_f32_tc(x, w, **kw)
+        return kernels.gemm_f32_tc(x, w, out=torch.ones(M, N, device=DEV), **kw)
+
+    def plain(x, w):
+        y = kernels.gemm_simt(x, w)
+        return kernels.swiglu(y) if mode == "swiglu" else y
+    x, w = operands(M, N, K, seed=1)
+    fine = call(x, w)
+    limit = 16 * us(lambda: plain(x, w)) + 200
+    for kind, value in (("nan", float("nan")), ("inf", float("inf")), ("overflow", 3e38)):
+        for rows in ([M // 2], range(M)):
+            y = x.clone()
+            rows = torch.tensor(list(rows), device=DEV)
+            y[rows, (rows * 7) % K] = value
+            if kind == "overflow":
+                y[rows] = y[rows].sign() * value
+            got, want = call(y, w), plain(y, w)
+            flat = got.sum(0) if mode == "partial" else got
+            if kind != "overflow":                  # (where a sum overflows follows its order)
+                assert torch.equal(flat.isnan(), want.isnan()) and torch.equal(flat.isinf(), want.isinf()) and not want[rows].isfinite().any()
+                assert torch.equal(flat[flat.isinf()], want[want.isinf()])
+            if len(rows) == 1:
+                keep = [i for i in range(M) if i != M // 2]
+                assert torch.equal(got[..., keep, :], fine[..., keep, :])
+            assert us(lambda: call(y, w)) < limit, (kind, len(rows))
+    assert int(tensor_core.status_word(torch.device(DEV))[0]) == 0
