@@ -37,23 +37,75 @@ template <int HD> struct FaLayout {
     static constexpr uint32_t tm_s = 0, tm_p = 2 * KT, tm_o = tm_p + 3 * KT / 2, tm_q = tm_o + HD;     // 512 columns at most
 };
 
-// One row of a prompt's attention again, in ascending key order: what a row that is not finite gets.
+// Rows of a warp's 32 again (a bit each in `rows`), key after key in ascending order, by the whole warp: what rows that are not finite
+// get.  A lane holds HD / 32 dimensions.  A row's sum of weights that is no number stays so and gives zeros, as in the generic kernel,
+// so the walk ends there.  (One thread a row with its sums in memory: 1,999 tokens of 14 heads with an infinite value
+// 250 ms, now 7.3, and 0.09 with a key that is not a number; without either 0.067, the generic kernel 1.8.)
 template <int HD>
-__device__ __noinline__ void fa_again(const float* qr, float* o, const float* k_pages, const float* v_pages, const int* bt, int kvh, int nkv,
-                                      int lo, int pos, float scale) {
-    float m = -INFINITY, l = 0.f;
-    for (int d = 0; d < HD; ++d) o[d] = 0.f;
-    for (int j = lo; j <= pos; ++j) {
-        const size_t at = (((size_t)bt[j / RF_PAGE] * nkv + kvh) * RF_PAGE + (j % RF_PAGE)) * HD;
-        float s = 0.f;
-        for (int d = 0; d < HD; ++d) s = fmaf(qr[d], k_pages[at + d], s);
-        s *= scale;
-        const float mn = fmaxf(m, s), c = m == -INFINITY ? 0.f : expf(m - mn), p = expf(s - mn);
-        l = l * c + p;
-        for (int d = 0; d < HD; ++d) o[d] = o[d] * c + p * v_pages[at + d];
-        m = mn;
+__device__ __noinline__ void fa_again(uint32_t rows, const float* q, int q_stride, float* out, int out_stride, const float* k_pages,
+                                      const float* v_pages, const int* bt, int kvh, int nkv, int window, int pos_first, float scale) {
+    constexpr int E = HD / 32, U = 4, R = 4;             // four rows and four keys at a time
+    struct alignas(4 * E) Piece { float v[E]; };
+    const int lane = threadIdx.x & 31;
+    while (rows) {
+        int row[R];
+        Piece qv[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {                    // (the last row again where fewer are left: the same numbers, written twice)
+            row[r] = rows ? __ffs(rows) - 1 : row[r > 0 ? r - 1 : 0];
+            rows &= rows - 1;
+            qv[r] = *reinterpret_cast<const Piece*>(q + (size_t)row[r] * q_stride + lane * E);
+        }
+        const int first = rf_first_key(pos_first + row[0], window), last = pos_first + row[R - 1];       // (rows ascend)
+        float m[R], l[R], o[R][E] = {};
+        int lo[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) { m[r] = -INFINITY; l[r] = 0.f; lo[r] = rf_first_key(pos_first + row[r], window); }
+#pragma unroll 1
+        for (int j0 = first; j0 <= last; j0 += U) {
+            float s[R][U];
+            Piece vv[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int j = min(j0 + u, last);
+                const size_t at = (((size_t)bt[j / RF_PAGE] * nkv + kvh) * RF_PAGE + (j % RF_PAGE)) * HD + lane * E;
+                const Piece kk = *reinterpret_cast<const Piece*>(k_pages + at);
+                vv[u] = *reinterpret_cast<const Piece*>(v_pages + at);
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    s[r][u] = 0.f;
+#pragma unroll
+                    for (int d = 0; d < E; ++d) s[r][u] = fmaf(qv[r].v[d], kk.v[d], s[r][u]);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int u = 0; u < U; ++u) s[r][u] = warp_sum(s[r][u]) * scale;
+            bool more = false;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    if (j0 + u < lo[r] || j0 + u > pos_first + row[r]) continue;
+                    const float mn = fmaxf(m[r], s[r][u]), c = m[r] == -INFINITY ? 0.f : expf(m[r] - mn), p = expf(s[r][u] - mn);
+                    l[r] = l[r] * c + p;
+#pragma unroll
+                    for (int d = 0; d < E; ++d) o[r][d] = o[r][d] * c + p * vv[u].v[d];
+                    m[r] = mn;
+                }
+                more = more || !isnan(l[r]);
+            }
+            if (!more) break;
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            Piece y;
+#pragma unroll
+            for (int d = 0; d < E; ++d) y.v[d] = l[r] > 0.f ? o[r][d] / l[r] : 0.f;
+            *reinterpret_cast<Piece*>(out + (size_t)row[r] * out_stride + lane * E) = y;
+        }
     }
-    for (int d = 0; d < HD; ++d) o[d] = l > 0.f ? o[d] / l : 0.f;
 }
 
 template <int HD>
@@ -306,7 +358,14 @@ attention_f32_prompt_kernel(const __grid_constant__ CUtensorMap map_k, const __g
                 fine = fine && fabsf(y.x) <= 3.402823466e38f && fabsf(y.y) <= 3.402823466e38f && fabsf(y.z) <= 3.402823466e38f && fabsf(y.w) <= 3.402823466e38f;
                 if (row_ok) *reinterpret_cast<float4*>(o + d) = y;
             }
-            if (row_ok && !fine) fa_again<HD>(qr, o, k_pages, v_pages, bt, kvh, nkv, lo_i, pos_i, scale);
+            const uint32_t again = __ballot_sync(0xffffffffu, row_ok && !fine);
+            if (again) {
+                __syncwarp();                                   // what is written over comes after what was written
+                const int row0 = warp * 32;
+                fa_again<HD>(again, q + (size_t)(row_base + row0) * q_stride + (size_t)head * HD, q_stride,
+                             out + (size_t)(row_base + row0) * out_stride + (size_t)head * HD, out_stride, k_pages, v_pages, bt, kvh, nkv, window,
+                             pos_first + row0, scale);
+            }
         }
     }
     tcgen05_fence_before();

@@ -161,6 +161,31 @@ def test_large_scores_and_what_is_not_finite():
         assert (y - want).abs()[fine].max() <= 2.0 ** -19 * want.abs()[fine].max()
 
 
+def test_whatever_is_not_finite_costs_a_bounded_time():
+    """1,999 tokens with a value, or a key, that is infinite or not a number at the first position, so that every row of its kv head
+    meets it: the generic kernel's kinds of results in at most eight times its time.  (A warp forms four rows at once and the generic
+    kernel a token's seven heads: 4.1 times its time with every row formed again, where one thread a row took 140 times.)"""
+    def us(f):
+        f()
+        a, e = torch.cuda.Event(True), torch.cuda.Event(True)
+        a.record()
+        for _ in range(3):
+            f()
+        e.record()
+        torch.cuda.synchronize()
+        return a.elapsed_time(e) / 3 * 1e3
+    for hd, nh, nkv in ((64, 14, 2), (128, 4, 4)):
+        for what, value in (("vp", float("inf")), ("vp", float("nan")), ("kp", float("nan")), ("kp", float("inf"))):
+            b = batch([0], [1999], nh, nkv, hd, seed=9)
+            b["q"].mul_(0.1)
+            b[what][int(b["table"][0, 0]), :, 0, 7] = value
+            y, want = run(b, "prompt"), run(b, "generic")
+            assert torch.equal(y.isnan(), want.isnan()) and torch.equal(y.isinf(), want.isinf())
+            fine = want.isfinite()
+            assert (y - want).abs()[fine].max() <= 2.0 ** -19 * want.abs()[fine].max()
+            assert us(lambda: run(b, "prompt")) < 8 * us(lambda: run(b, "generic")), (hd, what, value)
+
+
 def test_rules():
     from rocmforge_b200 import kernels
     assert kernels.f32_token_splits(1, 1) == 8 and kernels.f32_token_splits(1, 1, longest=100) == 2
