@@ -327,11 +327,16 @@ def split_k_for_f32_tc(N: int, K: int, sm_count: int | None = None) -> int:
     return (kb + per - 1) // per                   # no empty split
 
 
+F32_TC_FROM_K = 20
+
+
 def f32_tc_takes(x: torch.Tensor, w: torch.Tensor) -> bool:
-    """Whether a product outside the bfloat16 path runs on the tensor cores as well: float32 rows that TMA can fetch, whatever the
-    sizes.  It is faster than the CUDA cores from 3 tokens x 64 x 64 (3.2 against 4.5 us) to 4,096^3 (0.70 against 2.97 ms), and its
-    error is smaller (csrc/gemm_f32_tc.cuh)."""
-    return x.dtype == torch.float32 and w.dtype == torch.float32 and x.shape[0] > 0 and f32_tc_operands(x, w)
+    """Whether a product outside the bfloat16 path runs on the tensor cores as well: float32 rows that TMA can fetch, of 20 numbers and
+    more.  It is then faster than the CUDA cores (us, 3 and 500 tokens x 600: K = 8 3.1 against 2.1 and 6.3 each, K = 16 3.1, 2.0 and 6.3
+    each, K = 20 3.0, 2.9 and 6.5, 7.9, K = 64 3.4, 4.8 and 6.8, 11.1; 4,096^3 0.70 against 2.97 ms), and its error against 64 bits is
+    smaller, which it is not for the shortest sums (K = 8 5.54e-8 against 5.35e-8, K = 12 5.5e-8 and 6.5e-8, K = 20 6.2e-8 and 8.2e-8)."""
+    return (x.dtype == torch.float32 and w.dtype == torch.float32 and x.shape[0] > 0 and w.shape[1] >= F32_TC_FROM_K
+            and f32_tc_operands(x, w))
 
 
 def split_k_for_plain(x: torch.Tensor, w: torch.Tensor, tensor_cores: bool = True) -> int:
