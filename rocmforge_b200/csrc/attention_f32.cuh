@@ -88,7 +88,7 @@ __device__ __noinline__ void fa_again(uint32_t rows, const float* q, int q_strid
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     if (j0 + u < lo[r] || j0 + u > pos_first + row[r]) continue;
-                    const float mn = fmaxf(m[r], s[r][u]), c = m[r] == -INFINITY ? 0.f : expf(m[r] - mn), p = expf(s[r][u] - mn);
+                    const float mn = fmaxf(m[r], s[r][u]), c = m[r] == -INFINITY ? 0.f : expf(m[r] - mn), p = s[r][u] == -INFINITY ? 0.f : expf(s[r][u] - mn);
                     l[r] = l[r] * c + p;
 #pragma unroll
                     for (int d = 0; d < E; ++d) o[r][d] = o[r][d] * c + p * vv[u].v[d];
