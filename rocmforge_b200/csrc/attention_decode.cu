@@ -708,7 +708,8 @@ static int launch_warps(const void* q, int q_stride, void* out, int out_stride, 
     constexpr int HD = EPL * 32;
     const size_t smem = (size_t)WARPS * 2 * ROWS * HD * 2 +
                         (size_t)(WARPS * DEC_GP + 2 * DEC_GP + 16 * 2 * DEC_GP + DEC_GP * HD) * sizeof(float) + WARPS * 2 * 8 + 16 + 1024;
-    static bool configured = false;
+    static PerDevice<bool> devices;
+    bool& configured = devices.here();
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(attention_decode_warps_kernel<EPL, ROWS, WARPS>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -758,7 +759,8 @@ static int launch(const void* q, int q_stride, void* out, int out_stride, const 
                   float* part_o, float* part_ml, int* counters, int* status, cudaStream_t st) {
     constexpr int HD = EPL * 32;
     const size_t smem = (size_t)2 * DEC_CHUNK * HD * 2 + (DEC_GP * DEC_CHUNK + DEC_WARPS * DEC_GP) * sizeof(float) + 16;
-    static bool configured = false;
+    static PerDevice<bool> devices;
+    bool& configured = devices.here();
     if (!configured && smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(attention_decode_kernel<EPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);

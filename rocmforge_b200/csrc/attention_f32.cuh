@@ -616,7 +616,8 @@ static int fa_launch(const float* q, int q_stride, float* out, int out_stride, c
                      const int* tiles, int n_tiles, const int* seq_slot, const int* seq_start, const int* seq_nnew, const int* cu_q,
                      const int* block_table, int max_pages, int nh, int nkv, float scale, int window, int* status, cudaStream_t st) {
     using L = FaLayout<HD>;
-    static bool configured = false;
+    static PerDevice<bool> devices;
+    bool& configured = devices.here();
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(attention_f32_prompt_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::smem);
         if (e != cudaSuccess) return (int)e;
@@ -644,8 +645,13 @@ static int fd_launch(const float* q, int q_stride, float* out, int out_stride, c
     const size_t share = (size_t)GP * LPK * 4 * sizeof(float);
     const int most = (FD_SHARES + splits - 1) / splits, fit = (int)((64 << 10) / (FD_WARPS * share)), slots = most < fit ? most : fit;
     const size_t smem = (slots * FD_WARPS + most) * share;
-    static SmemLimit limit;
-    if (int e = limit.allow((const void*)attention_f32_token_kernel<LPK, GP>, smem)) return e;
+    static PerDevice<size_t> devices;
+    size_t& configured = devices.here();
+    if (smem > configured) {
+        cudaError_t e = cudaFuncSetAttribute(attention_f32_token_kernel<LPK, GP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+        configured = smem;
+    }
     cudaError_t le = splits > 1
         ? rf_launch_cluster(attention_f32_token_kernel<LPK, GP>, grid, dim3(FD_WARPS * 32), smem, st, splits, q, q_stride, out, out_stride, k_pages,
                             v_pages, tok_seq, tok_pos, seq_slot, block_table, max_pages, nh, nkv, scale, window, splits, slots, rows)

@@ -237,7 +237,8 @@ static int launch_ck(const void* q, int q_stride, void* out, int out_stride, con
                      const float* slopes, int window, int T_, cudaStream_t st, int keep_first, const float* sinks, int v_row) {
     const int hm = hd > hdv ? hd : hdv;
     const size_t smem = ((size_t)GB * hd + (size_t)CK * (hm + 1) + GB * CK + ATT_WARPS * GB) * sizeof(float);
-    static size_t configured = 0;
+    static PerDevice<size_t> devices;
+    size_t& configured = devices.here();
     if (smem > configured) {
         cudaError_t e = cudaFuncSetAttribute(attention_generic_kernel<T, CK, GB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);

@@ -485,7 +485,8 @@ static bool ld_plan(int heads, int rank, int ld, LatentDecodePlan* p) {
 
 template <int NH>
 static int ld_launch(const CUtensorMap& mq, const CUtensorMap& mc, const LatentDecode& a, int T, int groups, size_t smem, cudaStream_t st) {
-    static size_t configured = 0;
+    static PerDevice<size_t> devices;
+    size_t& configured = devices.here();
     if (smem > configured) {
         cudaError_t e = cudaFuncSetAttribute(attention_latent_decode_kernel<NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;

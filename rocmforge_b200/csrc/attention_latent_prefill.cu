@@ -336,7 +336,8 @@ int rf_attention_latent_prefill(const void* q, int q_stride, int T, const void* 
         for (int f = 0; f < 4 && a.k_stages == 0; ++f)
             if (lp_smem(nb, a.nv, forms[f][0], forms[f][1]) <= limit) { a.k_stages = forms[f][0]; a.v_stages = forms[f][1]; }
     const size_t smem = lp_smem(nb, a.nv, a.k_stages, a.v_stages);
-    static size_t configured = 0;
+    static PerDevice<size_t> devices;
+    size_t& configured = devices.here();
     if (smem > configured) {
         cudaError_t ce = cudaFuncSetAttribute(attention_latent_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (ce != cudaSuccess) return (int)ce;

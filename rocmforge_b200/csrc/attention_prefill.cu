@@ -318,7 +318,8 @@ static int pf_launch(const CUtensorMap& mk, const CUtensorMap& mv, const void* q
                      const int* seq_nnew, const int* cu_q, const int* block_table, int max_pages, int nh, int nkv,
                      float scale, int window, int* status, cudaStream_t st) {
     constexpr size_t smem = 2 * 2 * (HD / 64) * 64 * 128 + 2 * 8 + 1024;
-    static bool configured = false;
+    static PerDevice<bool> devices;
+    bool& configured = devices.here();
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(attention_prefill_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);

@@ -352,7 +352,8 @@ static int at_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
                      const int* cu_q, const int* block_table, int max_pages, int nh, int nkv, float scale, int window,
                      int* status, float softcap, const float* slopes, int keep_first, const float* sinks, cudaStream_t st) {
     constexpr size_t smem = (size_t)(HD / 64) * AT_BM * 128 + 4 * (size_t)(HD / 64) * AT_BN * 128 + 15 * 8 + 16;
-    static bool configured = false;
+    static PerDevice<bool> devices;
+    bool& configured = devices.here();
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);

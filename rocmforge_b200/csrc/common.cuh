@@ -71,18 +71,15 @@ static cudaError_t rf_launch_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 b
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
-// A kernel's dynamic shared memory beyond the 48 KB that need no asking for: the limit is set once for each device that launches it.
-struct SmemLimit {
-    size_t set[64] = {};
-    int allow(const void* kernel, size_t bytes) {
+// A host-side note of what has been set on each device: a kernel's attributes (its limit of shared memory, the cluster sizes it may
+// have) hold for the device that was current when they were set, and a process may run models on several.
+template <typename T>
+struct PerDevice {
+    T at[64] = {};
+    T& here() {
         int dev = 0;
-        cudaError_t e = cudaGetDevice(&dev);
-        if (e != cudaSuccess) return (int)e;
-        if (dev >= 0 && dev < 64 && bytes <= set[dev]) return 0;
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        if (e != cudaSuccess) return (int)e;
-        if (dev >= 0 && dev < 64) set[dev] = bytes;
-        return 0;
+        cudaGetDevice(&dev);
+        return at[dev & 63];
     }
 };
 

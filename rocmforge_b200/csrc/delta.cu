@@ -936,13 +936,13 @@ static int delta_chunked(const float* qn, const float* kn, const float* decay, c
     const int tiles = D4 <= 128 ? 1 : 2;
     const size_t smem2 = ((size_t)(tiles == 1 ? 2 : 1) * (D * DC + DC * D4 + DC * DV + GW) + D4 * DV + 8 * 80 * DV + DC * DV) * sizeof(float);
     const size_t smem3 = ((size_t)DC * (DC + D4 + 4) + (DC + D4) * DO) * sizeof(float);
-    static size_t set1 = 48 * 1024, set2[2] = {48 * 1024, 48 * 1024}, set3 = 48 * 1024;
+    static PerDevice<size_t> set1, set2[2], set3;
     const auto solve = delta_chunk_solve_kernel<PC>;
     const auto carry = tiles == 1 ? delta_chunk_carry_kernel<1, PC> : delta_chunk_carry_kernel<2, PC>;
     const auto outk = delta_chunk_out_kernel<PC>;
     int e;
-    if ((e = chunk_smem((const void*)solve, smem1, &set1)) || (e = chunk_smem((const void*)carry, smem2, &set2[tiles - 1])) ||
-        (e = chunk_smem((const void*)outk, smem3, &set3)))
+    if ((e = chunk_smem((const void*)solve, smem1, &set1.here())) || (e = chunk_smem((const void*)carry, smem2, &set2[tiles - 1].here())) ||
+        (e = chunk_smem((const void*)outk, smem3, &set3.here())))
         return e;
     for (int c = 0; c < n_chunks; c += pass) {
         const int n = pass < n_chunks - c ? pass : n_chunks - c;

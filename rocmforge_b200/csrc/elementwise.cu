@@ -1171,7 +1171,8 @@ static int launch_weighted_add(float* h, const float* a0, int n0, float s0, cons
         return 0;
     }
     const size_t smem = ((size_t)H + 34) * sizeof(float);
-    static size_t configured = 48 * 1024;
+    static PerDevice<size_t> devices;
+    size_t& configured = devices.here();
     if (smem > configured) {
         cudaError_t e = cudaFuncSetAttribute(weighted_add_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
@@ -1239,7 +1240,8 @@ static int launch_scaled_add(float* h, const float* a0, int n0, const void* w0, 
     if (y_next != nullptr && (alpha == nullptr || w_next == nullptr || b_next == nullptr)) return RF_ERR_BAD_ARG;
     const size_t smem = (size_t)(2 * H + 34) * sizeof(float);
     if (smem > 200 * 1024) return RF_ERR_UNSUPPORTED;
-    static size_t configured = 48 * 1024;
+    static PerDevice<size_t> devices;
+    size_t& configured = devices.here();
     if (smem > configured) {
         cudaError_t e = cudaFuncSetAttribute(scaled_add_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
@@ -1454,7 +1456,8 @@ static int launch_branch_norm_add(float* h, const float* a0, int n0, const void*
     if (n0 < 1 || (a1 != nullptr && n1 < 1)) return RF_ERR_BAD_ARG;
     const size_t smem = (size_t)(2 * H + 34) * sizeof(float);
     if (smem > 200 * 1024) return RF_ERR_UNSUPPORTED;
-    static size_t configured = 48 * 1024;
+    static PerDevice<size_t> devices;
+    size_t& configured = devices.here();
     if (smem > configured) {
         cudaError_t e = cudaFuncSetAttribute(branch_norm_add_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;

@@ -419,7 +419,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 template <int BN>
 static int fs_launch(FsParams p, int sms, cudaStream_t st) {
     using L = FsLayout<BN>;
-    static bool configured = false;
+    static PerDevice<bool> devices;
+    bool& configured = devices.here();
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(gemm_f32_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::smem);
         if (e != cudaSuccess) return (int)e;

@@ -340,7 +340,8 @@ template <int BN, bool SWAP, int STAGES, bool NORM = false, bool GROUPED = false
 static int launch_cfg(const CUtensorMap& ma, const CUtensorMap& mb, const TcParams& p, dim3 grid, cudaStream_t st,
                       const TcNorm* norm = nullptr, int cluster_z = 1, const TcGroup* group = nullptr) {
     constexpr size_t smem = (size_t)STAGES * (TC_BM * TC_BK * 2 + BN * TC_BK * 2) + (2 * STAGES + 1) * 8 + 16 + 1024;
-    static bool configured = false;
+    static PerDevice<bool> devices;
+    bool& configured = devices.here();
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN, SWAP, STAGES, NORM, GROUPED>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -456,8 +456,9 @@ static int make_out_map(CUtensorMap* map, const void* base, long long rows, long
 template <int CL, bool PAIR>
 static int cluster_width() {
     constexpr size_t smem = ClusterLayout<PAIR>::smem;
-    static int max_clusters = -1;
-    if (max_clusters < 0) {
+    static PerDevice<int> devices;
+    int& max_clusters = devices.here();
+    if (max_clusters == 0) {
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;

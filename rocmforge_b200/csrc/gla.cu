@@ -340,7 +340,8 @@ static int launch_scan_cols(const float* q, const float* k, const float* alpha, 
     if (gz > 65535) return RF_ERR_UNSUPPORTED;
     const size_t smem = (size_t)((SCALAR ? 4 : 6) * GL_TOK * slices * ROWS + (SCALAR ? 4 * GL_TOK : 0) + 2 * GL_TOK * COLS +
                                  GL_TOK * slices * (ROWS / GL_SLICE) * COLS) * sizeof(float);
-    static size_t configured = 48 * 1024;
+    static PerDevice<size_t> devices;
+    size_t& configured = devices.here();
     if (smem > configured) {
         cudaError_t e = cudaFuncSetAttribute(gla_scan_kernel<T, COLS, ROWS, SCALAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
@@ -682,7 +683,8 @@ static int launch_gated_chunked(const float* q, const float* k, int qk_heads, in
     const int vz = (vdim + GV - 1) / GV;
     const size_t smem1 = (size_t)(GC * ((dim + 3) & ~3) + GC * GV + 2 * GC + 4) * sizeof(float);
     const size_t smem3 = (size_t)(2 * dim * GC_LD + GC * GV + GC * GC_LD + 3 * GC) * sizeof(float);
-    static size_t set1 = 48 * 1024, set3 = 48 * 1024;
+    static PerDevice<size_t> devices1, devices3;
+    size_t &set1 = devices1.here(), &set3 = devices3.here();
     if (smem1 > set1) {
         cudaError_t e = cudaFuncSetAttribute(gated_chunk_state_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
         if (e != cudaSuccess) return (int)e;

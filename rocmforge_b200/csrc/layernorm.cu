@@ -309,7 +309,8 @@ static int go_update(float* h, const int* rows, const RoutedRows& rt, const Dens
                      int H, cudaStream_t st) {
     const size_t smem = ((size_t)(H + 3) / 4 * 4 + 34) * sizeof(float);
     if (smem > 200 * 1024) return RF_ERR_UNSUPPORTED;
-    static size_t configured = 48 * 1024;
+    static PerDevice<size_t> devices;
+    size_t& configured = devices.here();
     if (smem > configured) {
         cudaError_t e = cudaFuncSetAttribute(stream_update_kernel<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;

@@ -431,7 +431,8 @@ static int launch_chunked(const float* q, const float* k, int qk_stride, const v
     const int vz = (vdim + RV - 1) / RV;
     const size_t smem1 = (size_t)(RC * ((dim + 3) & ~3) + RC * RV + RC) * sizeof(float);
     const size_t smem3 = (size_t)(2 * dim * RC_LD + RC * RV + RC * RC_LD + RC + 4) * sizeof(float);
-    static size_t set1 = 48 * 1024, set3 = 48 * 1024;
+    static PerDevice<size_t> devices1, devices3;
+    size_t &set1 = devices1.here(), &set3 = devices3.here();
     if (smem1 > set1) {
         cudaError_t e = cudaFuncSetAttribute(retention_chunk_state_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
         if (e != cudaSuccess) return (int)e;

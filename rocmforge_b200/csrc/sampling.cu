@@ -103,7 +103,8 @@ extern "C" int rf_argmax(const float* logits, int rows, int V, long long row_str
     int slices = 16;
     while (slices > 1 && ((long long)rows * slices > 320 || V / slices < 4096)) slices >>= 1;
     if (row_stride % 4) slices = 1;                  // rows that do not start on 16-byte borders: one CTA, scalar loads
-    static bool configured = false;
+    static PerDevice<bool> devices;
+    bool& configured = devices.here();
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(argmax_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return (int)e;
@@ -862,7 +863,8 @@ static int launch_sample_cached(const float* logits, int rows, int V, long long 
                                 int top_k, const unsigned long long* seeds, const int* draw_counter, int* out, int cl,
                                 cudaStream_t st) {
     const size_t smem = (size_t)SMP2_CAP * 10;
-    static bool configured = false;
+    static PerDevice<bool> devices;
+    bool& configured = devices.here();
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(sample_cached_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return (int)e;
@@ -908,7 +910,8 @@ extern "C" int rf_sample(const float* logits, int rows, int V, long long row_str
     // in clusters of 16, 0.19 ms in clusters of 8; one row 0.14 against 0.19 ms)
     int cl = rows <= 4 ? 16 : 8;
     while (cl > 1 && (long long)rows * cl > 160) cl >>= 1;
-    static bool configured = false;
+    static PerDevice<bool> devices;
+    bool& configured = devices.here();
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return (int)e;

@@ -200,7 +200,8 @@ static int st_launch(const StreamsArgs& a, int rows, int cluster, int threads, c
     const int share = ((a.W / V + cluster - 1) / cluster) * V;
     const size_t smem = (size_t)(share + 34 + ST_MAX_CLUSTER + (S_ == 0 ? a.S * threads : 0)) * sizeof(float);
     if (smem > 200 * 1024) return RF_ERR_UNSUPPORTED;
-    static size_t configured = 48 * 1024;
+    static PerDevice<size_t> devices;
+    size_t& configured = devices.here();
     if (smem > configured) {
         cudaError_t e = cudaFuncSetAttribute(streams_update_kernel<T, V, S_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
@@ -317,11 +318,12 @@ static int launch_pair_embed(const void* table, const void* pairs, const int* id
     auto whole = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
     const bool vec = H % 4 == 0 && whole(table) && whole(pairs) && whole(w) && whole(out);
     auto kernel = vec ? pair_embed_kernel<T, 4> : pair_embed_kernel<T, 1>;
-    static size_t configured[2] = {48 * 1024, 48 * 1024};
-    if (smem > configured[vec]) {
+    static PerDevice<size_t> devices[2];
+    size_t& configured = devices[vec].here();
+    if (smem > configured) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
-        configured[vec] = smem;
+        configured = smem;
     }
     int threads = ((vec ? H / 4 : H) + 31) / 32 * 32;
     threads = threads < 64 ? 64 : (threads > 512 ? 512 : threads);
