@@ -608,11 +608,10 @@ def other_shapes(pk, seed, only=None):
             out[key + "_e2e_tok_s"] = round(e2e_rate(llm, prompts, 128 if elem == 2 else 32, warmup=8)["value"], 1)
             del llm
             if elem == 4:
-                # the 32-bit products run on the CUDA cores: 148 SMs x 128 lanes x 2 flops at the highest SM clock
-                ffma = 148 * 128 * 2 * pk.get("sm_max_mhz", 1965.0) * 1e6
+                # the 32-bit products are six bfloat16 products of exact parts on the tensor cores
                 ms = prefill_rate(model, PREFILL_TOKENS, 2, seed + 13)
                 out["qwen0.5b_fp32_prefill2048_tok_s"] = round(PREFILL_TOKENS / (ms / 1e3), 1)
-                out["qwen0.5b_fp32_prefill2048_ffma_frac"] = round(prefill_flops(cfg, PREFILL_TOKENS) / (ms / 1e3) / ffma, 4)
+                out["qwen0.5b_fp32_prefill2048_frac_of_six_bf16"] = round(6 * prefill_flops(cfg, PREFILL_TOKENS) / (ms / 1e3) / (tf * 1e12), 4)
             del model
             torch.cuda.empty_cache()
     if only in (None, "14b"):
