@@ -67,7 +67,7 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, __nv_
 
     // positions, slots and block tables are not written by any kernel of the step; the queries and the
     // newest keys and values are: wait for the kernel before us
-    pdl_wait();
+    pdl_wait(q, k_pages, v_pages);
     // ---- bring the chunk's pages in: all copies in flight at once
     const uint32_t bar_a = dec_smem_u32(bar);
     if (tid == 0) {
@@ -437,7 +437,7 @@ attention_decode_warps_kernel(const __grid_constant__ CUtensorMap map_k, const _
     int u = next_tile(warp - WARPS);
     const bool early = u < n_units && first_key(u) / RF_PAGE < p_hi;
     if (lane == 0 && early) { issue(u, true); issue(u, false); }
-    pdl_wait();                                         // queries and the newest keys/values come from the kernel before us
+    pdl_wait(q);                                         // queries and the newest keys/values come from the kernel before us
     if (lane == 0 && !early && u < n_units) { issue(u, true); issue(u, false); }
 
     uint32_t qb[HD / 16][2];                            // Q^T as the B operand: head gid, dims ks*16 + tig*2 (+8)

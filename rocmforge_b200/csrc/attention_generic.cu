@@ -44,7 +44,7 @@ attention_generic_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ 
                          const float* __restrict__ sinks, int v_row) {
     constexpr int ACC = GB * (CK == 128 ? 256 : (CK == 64 ? 512 : ATT_MAX_HD)) / ATT_THREADS;     // (head, dim) pairs of a thread at most
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(q, k_pages, v_pages);
     extern __shared__ float smem[];
     const int ldk = hd + 1, ldv = hdv + 1;          // a key row per thread: odd stride, no bank conflicts
     float* qs = smem;                               // [GB][hd]

@@ -86,7 +86,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_v) : "memory");
     }
     __syncthreads();
-    pdl_wait();                                        // queries, keys and values come from the kernel before us
+    pdl_wait(q);                                        // queries, keys and values come from the kernel before us
 
     auto issue = [&](int it) {                          // thread 0: bring page kt_lo + it into stage it & 1
         const int stage = it & 1;

@@ -28,7 +28,28 @@ __host__ __device__ __forceinline__ int rf_first_key(int pos, int span) {
 // library calls pdl_wait() before it reads anything another kernel of the step wrote and before it
 // writes anything at all; what it touches earlier is only weights, the step descriptor and block
 // tables, which no kernel of a step writes.  Launched without the attribute, both calls do nothing.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+//
+// Pointers to what another kernel of the step wrote are named in the call (or are not __restrict__): the compiler takes loads
+// through a const __restrict__ parameter for loads of what nobody writes, and may move them up across the wait.  The call hands the
+// pointer back as a new one that it knows nothing of but that it is global, so what is read through it is read after the wait; the
+// parameters that kernels write through keep their __restrict__.  A pointer formed from the parameter before the wait is named itself.
+template <typename T>
+__device__ __forceinline__ void rf_read_from_here(T*& p) {
+    size_t g = __cvta_generic_to_global(p);
+    asm volatile("" : "+l"(g));
+    p = static_cast<T*>(__cvta_global_to_generic(g));
+}
+template <typename T>
+__device__ __forceinline__ void rf_read_from_here(const T* __restrict__& p) {
+    size_t g = __cvta_generic_to_global(p);
+    asm volatile("" : "+l"(g));
+    p = static_cast<const T*>(__cvta_global_to_generic(g));
+}
+template <typename... P>
+__device__ __forceinline__ void pdl_wait(P&... written_before) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    (rf_read_from_here(written_before), ...);
+}
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 static int g_rf_pdl = 0;

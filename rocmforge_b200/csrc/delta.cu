@@ -149,7 +149,7 @@ delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
     for (int i = tid; i < 2 * TOK * COLS; i += NT)
         if (j0 + i % COLS >= V) (&sv[0][0][0])[i] = 0.f;
     const bool vec = (D & 3) == 0;
-    pdl_wait();
+    pdl_wait(qn, kn, kq, decay, beta, v);
     auto stage_in = [&](int base, int buf) {
         const int cnt = min(TOK, n - base);
         if (vec) {
@@ -384,7 +384,7 @@ delta_chunk_solve_kernel(const float* __restrict__ qn, const float* __restrict__
     pdl_trigger();
     const int c = blockIdx.x, h = blockIdx.y, hg = h / (H / G), tid = threadIdx.x;
     const ChunkPlace p = chunk_place(table, cu_q, B, chunk0 + c);
-    pdl_wait();
+    pdl_wait(qn, kn, decay, beta, v);
     if (tid < DC) {
         const bool in = tid < p.cnt;
         if constexpr (!PC) sg[tid] = in ? decay[(size_t)(p.row0 + tid) * H + h] : 1.f;
@@ -654,7 +654,7 @@ delta_chunk_carry_kernel(const float* __restrict__ Kc, const float* __restrict__
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    pdl_wait();
+    pdl_wait(Kc, U0, Wt, gw);
     auto fetch = [&](int chunk, int buf) {            // by one thread
         const int c = chunk - chunk0;
         float* w = sh + buf * stage;
@@ -826,7 +826,7 @@ delta_chunk_out_kernel(const float* __restrict__ qn, const float* __restrict__ M
     const int c = blockIdx.x, h = blockIdx.y, j0 = blockIdx.z * DO, hg = h / (H / G), tid = threadIdx.x;
     const ChunkPlace p = chunk_place(table, cu_q, B, chunk0 + c);
     const int nc = min(DO, V - j0);
-    pdl_wait();
+    pdl_wait(qn, M, gw, U, LS);
     chunk_tile(lhs, ld, M + ((size_t)c * H + h) * DC * DC, DC, p.cnt, DC, true, tid, 256);
     if constexpr (PC) chunk_tile(lhs + DC, ld, qn + ((size_t)c * H + h) * DC * D4, D4, p.cnt, D, (D & 3) == 0, tid, 256);
     else chunk_tile(lhs + DC, ld, qn + ((size_t)p.row0 * G + hg) * D, (size_t)G * D, p.cnt, D, (D & 3) == 0, tid, 256);

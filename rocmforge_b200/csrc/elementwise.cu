@@ -42,7 +42,7 @@ __global__ void embed_kernel(const T* __restrict__ table, const int* __restrict_
                              float* __restrict__ out, int H, int V, const T* __restrict__ pos_table,
                              const int* __restrict__ tok_pos, int P, T* __restrict__ rounded, float scale) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(ids);
     const int t = blockIdx.x;
     int id = ids[t];
     id = id < 0 ? 0 : (id >= V ? V - 1 : id);   // ids are validated on the host; never read outside
@@ -84,7 +84,7 @@ __global__ void add_rmsnorm_kernel(float* __restrict__ h, const void* __restrict
                                    const void* __restrict__ w, int w_is_f32, float eps,
                                    T* __restrict__ y, const int* __restrict__ rows, int H) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(pending);
     extern __shared__ float row_buf[];          // H floats + 33 for the reduction
     float* red = row_buf + H;
     const int r = blockIdx.x;
@@ -211,7 +211,7 @@ add_rmsnorm_vec_kernel(float* __restrict__ h, const void* __restrict__ pending, 
             }
         }
     }
-    pdl_wait();
+    pdl_wait(pending);
     float4* hrow = reinterpret_cast<float4*>(h + (size_t)t * H);
     float4 v[NV];
     float ss = 0.f;
@@ -373,7 +373,7 @@ rmsnorm_wide_rows_kernel(const float* __restrict__ h, const void* __restrict__ w
     pdl_trigger();
     __shared__ float red[34];
     const int r = blockIdx.x, nvec = H >> 2;
-    pdl_wait();
+    pdl_wait(h);
     const float4* hrow = reinterpret_cast<const float4*>(h + (size_t)r * H);
     float ss = 0.f;
     for (int c0 = threadIdx.x; c0 < nvec; c0 += 4 * blockDim.x) {          // four loads in flight per thread
@@ -456,7 +456,7 @@ __global__ void rope_kv_write_kernel(const void* __restrict__ src, int row_strid
     }
     float s = 0.f, c = 1.f;
     if (rotated) sincosf((float)pos * inv_freq[i], &s, &c);
-    pdl_wait();
+    pdl_wait(src);
     float x0, x1;
     if (PARTIALS) {
         const float* p = reinterpret_cast<const float*>(src) + (size_t)t * row_stride;
@@ -558,7 +558,7 @@ rope_kv_write_rows_kernel(const T* src, int row_stride, T* q_out, int q_out_stri
 template <typename T, int ACT>
 __global__ void swiglu_kernel(const T* __restrict__ gu, T* __restrict__ a, size_t n_out, int I) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(gu);
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n_out;
          idx += (size_t)gridDim.x * blockDim.x) {
         const size_t t = idx / I, j = idx - t * I;
@@ -577,7 +577,7 @@ __global__ void swiglu_kernel(const T* __restrict__ gu, T* __restrict__ a, size_
 template <typename T>
 __global__ void relu2_kernel(const T* __restrict__ x, T* __restrict__ a, size_t n) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(x);
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += (size_t)gridDim.x * blockDim.x) {
         const float v = fmaxf(Cvt<T>::to_f32(x[idx]), 0.f);
         a[idx] = Cvt<T>::from_f32(v * v);
@@ -588,7 +588,7 @@ __global__ void relu2_kernel(const T* __restrict__ x, T* __restrict__ a, size_t 
 template <typename T>
 __global__ void add_row_kernel(float* __restrict__ h, const T* __restrict__ vec, size_t n, int H) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(vec);
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += (size_t)gridDim.x * blockDim.x)
         h[idx] += Cvt<T>::to_f32(vec[idx % H]);
 }
@@ -614,7 +614,7 @@ branch_norm_add_kernel(float* __restrict__ h, const float* __restrict__ a0, int 
     pdl_trigger();
     const size_t base = (size_t)blockIdx.x * H;
     const float invH = 1.f / (float)H;
-    pdl_wait();
+    pdl_wait(a0, a1, extra);
     if (a1 != nullptr) {
         float s0 = 0.f, s1 = 0.f;
         for (int c = threadIdx.x; c < H; c += blockDim.x) {
@@ -700,7 +700,7 @@ head_norm_kv_write_kernel(const void* __restrict__ src, int row_stride, int n_pa
     const int rh = rot_dim >> 1;
     // a query's temperature grows with its position in steps of q_every positions
     const float q_temp = ex.q_every > 0.f ? 1.f + ex.q_coef * logf(floorf((float)(pos + 1) / ex.q_every) + 1.f) : 1.f;
-    pdl_wait();
+    pdl_wait(src);
     const int n_heads_all = write_kv ? nh + (ex.v_is_k ? 1 : 2) * nkv : nh;
     for (int head = blockIdx.y * nwarp + warp; head < n_heads_all; head += gridDim.y * nwarp) {
         const bool is_v = head >= nh + nkv;
@@ -890,7 +890,7 @@ template <typename T>
 __global__ void clamped_glu_kernel(const T* __restrict__ gu, T* __restrict__ a, size_t n_out, int I, float limit, float alpha,
                                    const float* __restrict__ row_scale) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(gu, row_scale);
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n_out; idx += (size_t)gridDim.x * blockDim.x) {
         const size_t t = idx / I, j = idx - t * I;
         const float sc = row_scale != nullptr ? row_scale[t] : 1.f;
@@ -906,7 +906,7 @@ template <typename T>
 __global__ void sigmoid_gate_kernel(const T* __restrict__ x, int x_stride, const T* __restrict__ gate, int gate_stride,
                                     T* __restrict__ out, size_t n, int W, int group) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(x, gate);
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += (size_t)gridDim.x * blockDim.x) {
         const size_t t = idx / W, c = idx - t * W;
         const float g = Cvt<T>::to_f32(gate[t * gate_stride + c / group]);
@@ -921,7 +921,7 @@ __global__ void sigmoid_gate_vec_kernel(const T* __restrict__ x, int x_stride, c
                                         T* __restrict__ out, size_t n_vec, int Wv, int group) {
     constexpr int V = 16 / sizeof(T);
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(x, gate);
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n_vec; idx += (size_t)gridDim.x * blockDim.x) {
         const size_t t = idx / Wv;
         const int c = (int)(idx - t * Wv) * V;
@@ -945,7 +945,7 @@ __global__ void sigmoid_gate_vec_kernel(const T* __restrict__ x, int x_stride, c
 template <typename T>
 __global__ void round_rows_kernel(const float* __restrict__ h, T* __restrict__ out, size_t n) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(h);
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += (size_t)gridDim.x * blockDim.x)
         out[idx] = Cvt<T>::from_f32(h[idx]);
 }
@@ -958,7 +958,7 @@ __global__ void dyt_rows_kernel(const float* __restrict__ h, const int* __restri
                                 const float* __restrict__ w, const float* __restrict__ b, T* __restrict__ y, int H) {
     pdl_trigger();
     const float a = alpha[0];
-    pdl_wait();
+    pdl_wait(h);
     const size_t src = (size_t)(rows != nullptr ? rows[blockIdx.x] : (int)blockIdx.x) * H, dst = (size_t)blockIdx.x * H;
     for (int c = threadIdx.x; c < H; c += blockDim.x) y[dst + c] = Cvt<T>::from_f32(fmaf(tanhf(a * h[src + c]), w[c], b[c]));
 }
@@ -985,7 +985,7 @@ scaled_add_kernel(float* __restrict__ h, const float* __restrict__ a0, int n0, c
     const size_t base = (size_t)blockIdx.x * H;
     const float invH = 1.f / (float)H;
     const float a = y_next != nullptr ? alpha[0] : 0.f;
-    pdl_wait();
+    pdl_wait(a0, a1);
     float s0 = 0.f, s1 = 0.f;
     for (int c = threadIdx.x; c < H; c += blockDim.x) {
         float x = 0.f, z = 0.f;
@@ -1026,7 +1026,7 @@ weighted_add_kernel(float* __restrict__ h, const float* __restrict__ a0, int n0,
     float* red = row + H;
     pdl_trigger();
     const size_t base = (size_t)blockIdx.x * H;
-    pdl_wait();
+    pdl_wait(a0, a1);
     float ss = 0.f;
     for (int c = threadIdx.x; c < H; c += blockDim.x) {
         float x = 0.f, z = 0.f;
@@ -1203,7 +1203,7 @@ stretch_norm_kernel(const T* __restrict__ src, int src_stride, NormStretch a, No
     const NormStretch s = blockIdx.y == 0 ? a : b;
     const T* x = src + (size_t)blockIdx.x * src_stride + s.col;
     T* y = reinterpret_cast<T*>(s.out) + (size_t)blockIdx.x * s.out_stride;
-    pdl_wait();
+    pdl_wait(x);
     float ss = 0.f;
     for (int c = threadIdx.x; c < s.n; c += blockDim.x) { const float v = Cvt<T>::to_f32(x[c]); ss += v * v; }
     const float r = rsqrtf(block_sum(ss, red) / (float)s.n + eps);

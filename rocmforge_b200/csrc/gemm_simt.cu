@@ -70,7 +70,7 @@ gemm_simt_kernel(const T* __restrict__ X, const T* __restrict__ W, const void* _
     const int n0 = blockIdx.x * GS_BN;
     __shared__ int src_row[GROUPED ? BM : 1];
     if constexpr (GROUPED) {
-        pdl_wait();                                   // the tile table and the row map are the sort kernel's
+        pdl_wait(X, tiles, row_map);                  // the tile table and the row map are the sort kernel's
         if ((int)blockIdx.y >= tiles[0]) return;
         const int* tl = tiles + 1 + 3 * blockIdx.y;
         W += (size_t)tl[0] * w_stride;
@@ -123,7 +123,7 @@ gemm_simt_kernel(const T* __restrict__ X, const T* __restrict__ W, const void* _
         for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
     // weights do not depend on the kernel before this one; activations (and the output) do
     if (k_begin < k_end) fetch_w(k_begin);
-    pdl_wait();
+    pdl_wait(X);
     if (k_begin < k_end) {
         fetch_x(k_begin);
         stash(0);

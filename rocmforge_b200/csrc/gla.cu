@@ -22,7 +22,7 @@ __global__ void gla_prepare_kernel(const T* __restrict__ src, int row_stride, in
                                    const float* __restrict__ z, float* __restrict__ qka, int width, float q_scale,
                                    float inv_tau, int T_) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(src, z);
     const size_t n = (size_t)T_ * width;
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += (size_t)gridDim.x * blockDim.x) {
         const size_t t = idx / width, c = idx - t * width;
@@ -138,7 +138,7 @@ gla_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, const 
         qs[tt * dimP + i] = 0.f; ks[tt * dimP + i] = 0.f;
         if (!SCALAR) as[tt * dimP + i] = 0.f;
     }
-    pdl_wait();
+    pdl_wait(q, k, alpha, v);
     float s[ROWS];
 #pragma unroll
     for (int r = 0; r < ROWS; ++r)
@@ -258,7 +258,7 @@ gla_decode_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
     float* S = state + ((size_t)seq_slot[b] * heads + h) * dim * vdim;
     const bool ncol = SCALAR && nstate != nullptr && j == vdim;
     float* Nn = ncol ? nstate + ((size_t)seq_slot[b] * heads + h) * dim : nullptr;
-    pdl_wait();
+    pdl_wait(q, k, alpha, v);
     float s[ROWS];
 #pragma unroll
     for (int r = 0; r < ROWS; ++r)
@@ -445,7 +445,7 @@ gated_chunk_state_kernel(const float* __restrict__ k, int qk_heads, int qk_strid
     const int hq = h / (heads / qk_heads);
     const int b = table[B + 1 + 2 * c], q0 = table[B + 2 + 2 * c];
     const int row0 = cu_q[b] + q0, cnt = min(GC, cu_q[b + 1] - row0);
-    pdl_wait();
+    pdl_wait(k, ab, v);
     if (threadIdx.x < cnt) {
         const float2 g = *reinterpret_cast<const float2*>(&ab[((size_t)(row0 + threadIdx.x) * heads + h) * 2]);
         as[threadIdx.x] = g.x;
@@ -526,7 +526,7 @@ gated_chunk_carry_kernel(float* __restrict__ LS, float* __restrict__ NL, const f
     const size_t step = (size_t)heads * (of_n ? dim : ne);
     float* p = of_n ? NL + ((size_t)c0 * heads + h) * dim + (e - ne) : LS + ((size_t)c0 * heads + h) * ne + e;
     const float* cd = CD + (size_t)c0 * heads + h;
-    pdl_wait();
+    pdl_wait(cd);
     float s = *S;
     for (int c = c0; c < c1; c += 8) {                   // eight chunks' sums on their way at once; the chain is the FMAs alone
         float l[8], d[8];
@@ -567,7 +567,7 @@ gated_chunk_out_kernel(const float* __restrict__ q, const float* __restrict__ k,
     const int hq = h / (heads / qk_heads);
     const int b = table[B + 1 + 2 * c], q0 = table[B + 2 + 2 * c];
     const int row0 = cu_q[b] + q0, cnt = min(GC, cu_q[b + 1] - row0);
-    pdl_wait();
+    pdl_wait(q, k, ab, v, LS, NL);
     if (threadIdx.x < GC) {
         float2 g = make_float2(1.f, 0.f);
         if (threadIdx.x < cnt) g = *reinterpret_cast<const float2*>(&ab[((size_t)(row0 + threadIdx.x) * heads + h) * 2]);

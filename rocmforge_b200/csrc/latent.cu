@@ -154,7 +154,7 @@ latent_gather_kernel(const uint4* __restrict__ pages, const int* __restrict__ cu
     const int pos = row - cu[lo];
     const int page = block_table[(size_t)seq_slot[lo] * max_pages + pos / RF_PAGE];
     const uint4* src = pages + ((size_t)page * RF_PAGE + pos % RF_PAGE) * n16;
-    pdl_wait();
+    pdl_wait(src);
     for (int i = threadIdx.x; i < n16; i += blockDim.x) out[(size_t)row * n16 + i] = src[i];
 }
 

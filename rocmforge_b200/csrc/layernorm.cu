@@ -356,7 +356,7 @@ side_gate_kernel(const void* __restrict__ z, int n_partials, long long part_stri
                  long long table_stride, int col0, const int* __restrict__ tokens, T* __restrict__ out, int out_stride, int dim,
                  int vocab, size_t n) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(z, tokens);
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const size_t t = i / out_stride;
         const int j = (int)(i - t * out_stride);

@@ -24,7 +24,7 @@ conv_silu_kernel(const T* __restrict__ src, int row_stride, int col0, const floa
     const int b = tok_seq[t];
     const int r = t - cu_q[b];                       // the token's index among its sequence's new tokens
     const float* old = state + (size_t)seq_slot[b] * (taps - 1) * C;
-    pdl_wait();
+    pdl_wait(src, old);
     for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < C; c += gridDim.y * blockDim.x) {
         float acc = load_vec(bias, w_is_f32, c);
         for (int j = 0; j < taps; ++j) {
@@ -77,7 +77,7 @@ conv_silu_vec_kernel(const T* src, int row_stride, int col0, const float* __rest
     }
     const int b0 = tok_seq[t0];
     const bool whole = t0 + CV_TOK <= T_ && tok_seq[min(t0 + CV_TOK, T_) - 1] == b0 && t0 - cu_q[b0] >= TAPS - 1;
-    pdl_wait();
+    pdl_wait(state);
     if (whole) {
         float x[CV_TOK + TAPS - 1][4];
 #pragma unroll
@@ -125,7 +125,7 @@ conv_state_update_kernel(const T* __restrict__ src, int row_stride, int col0, fl
     const int b = blockIdx.x;
     const int row0 = cu_q[b], n = cu_q[b + 1] - row0;
     float* st = state + (size_t)seq_slot[b] * (taps - 1) * C;
-    pdl_wait();
+    pdl_wait(src);
     for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < C; c += gridDim.y * blockDim.x) {
         float keep[MB_MAX_TAPS];
 #pragma unroll
@@ -145,7 +145,7 @@ conv_state_update_kernel(const T* __restrict__ src, int row_stride, int col0, fl
 __global__ void mamba_gates_kernel(const float* __restrict__ z, const void* __restrict__ dt_bias, const void* __restrict__ a_log,
                                    int v_is_f32, float* __restrict__ ab, int heads, size_t n) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(z);
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += (size_t)gridDim.x * blockDim.x) {
         const int h = (int)(idx % heads);
         const float x = z[idx] + load_vec(dt_bias, v_is_f32, h);
@@ -166,7 +166,7 @@ mamba_finish_kernel(const float* __restrict__ y, const float* __restrict__ x, in
     float* red = row + len;
     pdl_trigger();
     const int t = blockIdx.x, c0 = blockIdx.y * len;
-    pdl_wait();
+    pdl_wait(y, x, gate);
     float ss = 0.f;
     for (int i = threadIdx.x; i < len; i += blockDim.x) {
         const int c = c0 + i;

@@ -22,7 +22,7 @@ template <typename T>
 __global__ void mlstm_prepare_kernel(const T* __restrict__ src, int row_stride, int q_col, int k_col, float* __restrict__ qk,
                                      int width, float q_scale, int T_) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(src);
     const size_t n = (size_t)T_ * width;
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += (size_t)gridDim.x * blockDim.x) {
         const size_t t = idx / width, c = idx - t * width;
@@ -42,7 +42,7 @@ mlstm_gates_kernel(const float* __restrict__ z, float* __restrict__ ab, float* _
     const int b = blockIdx.x, h = blockIdx.y;
     const int row0 = cu_q[b], row1 = cu_q[b + 1];
     float* mslot = mstate + (size_t)seq_slot[b] * heads + h;
-    pdl_wait();
+    pdl_wait(z);
     if (threadIdx.x == 0) mm[0] = *mslot;
     for (int t0 = row0; t0 < row1; t0 += ML_TOK) {
         const int cnt = min(ML_TOK, row1 - t0);

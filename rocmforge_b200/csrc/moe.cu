@@ -21,7 +21,7 @@
 __global__ void moe_route_kernel(const float* __restrict__ logits, int E, int top, int* __restrict__ idx,
                                  float* __restrict__ w, int T_, int scoring) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(logits);
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= T_) return;
     const float* z = logits + (size_t)t * E;
@@ -87,7 +87,7 @@ moe_route_grouped_kernel(const float* __restrict__ logits, long long z_stride, c
     float* s = sh + (size_t)warp * (2 * E + groups);
     float* c = s + E;
     float* gs = c + E;
-    pdl_wait();
+    pdl_wait(logits);
     if (t >= T_) return;
     const float* z = logits + (size_t)t * z_stride;
     float largest = -INFINITY, sum = 0.f;
@@ -146,7 +146,7 @@ moe_sort_kernel(const int* __restrict__ idx, int n, int E, int active, int BM, i
     __shared__ int counts[1024];
     __shared__ int cursor[1024];
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(idx, w);
     for (int e = threadIdx.x; e < E; e += blockDim.x) counts[e] = 0;
     __syncthreads();
     for (int i = threadIdx.x; i < n; i += blockDim.x) atomicAdd(&counts[idx[i]], 1);
@@ -182,7 +182,7 @@ __global__ void moe_combine_kernel(const float* __restrict__ y, const int* __res
                                    float* __restrict__ out, int top, int H, size_t n, const int* __restrict__ idx, int experts,
                                    const T* __restrict__ x, long long x_stride) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(y, inv, w, idx, x);
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const size_t t = i / H, c = i - t * H;
         float acc = 0.f;
@@ -201,7 +201,7 @@ __global__ void moe_gather_kernel(const uint8_t* __restrict__ x, long long x_str
                                   int top, uint8_t* __restrict__ out, int row_bytes, int vec,
                                   const int* __restrict__ n_active) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(x, perm, n_active);
     const int r = blockIdx.x;
     if (n_active != nullptr && r >= *n_active) return;       // the pairs of passive experts: nobody reads these rows
     const uint8_t* src = x + (size_t)(perm[r] / top) * x_stride_bytes;

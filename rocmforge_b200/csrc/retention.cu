@@ -33,7 +33,7 @@ __global__ void retention_prepare_kernel(const T* __restrict__ src, int row_stri
     const int pos = tok_pos[t];
     const int rh = rot_dim >> 1;
     const int units = rh + (dim - rot_dim);               // per head
-    pdl_wait();
+    pdl_wait(src);
     const T* qrow = src + (size_t)t * row_stride + q_col;
     const T* krow = src + (size_t)t * row_stride + k_col;
     float* qo = qk + (size_t)t * width;
@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(256)
 silu_columns_kernel(const void* __restrict__ src, int n_partials, long long part_stride, int row_stride, float* __restrict__ out,
                     int W, size_t n) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(src);
     const int per_row = W / V;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const size_t t = i / per_row;
@@ -107,7 +107,7 @@ row_norm_gate_kernel(const float* __restrict__ o, const void* __restrict__ gate,
                      int sigmoid) {
     __shared__ float red[34];
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(o, gate);
     const size_t t = blockIdx.x;
     const float* orow = o + t * W;
     float ss = 0.f;
@@ -143,7 +143,7 @@ retention_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, 
     const int slot = seq_slot[b];
     const float d = decay[h];
     float* S = state + (((size_t)slot * heads + h) * vdim + (j < vdim ? j : 0)) * dim;      // this warp's column
-    pdl_wait();
+    pdl_wait(q, k, v);
     float s[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -195,7 +195,7 @@ __global__ void retention_gate_kernel(const float* __restrict__ o, const T* __re
                                       const void* __restrict__ norm_w, int w_is_f32, int w_per_head, int sigmoid,
                                       const float* __restrict__ qn, const float* __restrict__ mt) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(o, gate, qn, mt);
     const int lane = threadIdx.x & 31;
     const long long total = (long long)T_ * heads;
     for (long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < total;
@@ -247,7 +247,7 @@ retention_chunk_state_kernel(const float* __restrict__ k, int qk_stride, const T
     const int b = table[B + 1 + 2 * c], q0 = table[B + 2 + 2 * c];
     const int row0 = cu_q[b] + q0, cnt = min(RC, cu_q[b + 1] - row0);
     if (threadIdx.x < RC) pw[threadIdx.x] = powf(decay[h], (float)threadIdx.x);
-    pdl_wait();
+    pdl_wait(k, v);
     __syncthreads();
     for (int idx = threadIdx.x; idx < cnt * dimP; idx += 256) {
         const int s = idx / dimP, i = idx - s * dimP;
@@ -342,7 +342,7 @@ retention_chunk_out_kernel(const float* __restrict__ q, const float* __restrict_
     const int row0 = cu_q[b] + q0, cnt = min(RC, cu_q[b + 1] - row0);
     const float d = decay[h];
     if (threadIdx.x <= RC) pw[threadIdx.x] = powf(d, (float)threadIdx.x);
-    pdl_wait();
+    pdl_wait(q, k, v, LS);
     for (int idx = threadIdx.x; idx < RC * dim; idx += 256) {
         const int s = idx / dim, i = idx - s * dim;
         const bool in = s < cnt;

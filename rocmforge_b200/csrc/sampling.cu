@@ -33,7 +33,7 @@ argmax_kernel(const float* __restrict__ logits, int V, long long row_stride, int
     int per = (V + slices - 1) / slices;
     per = (per + 3) & ~3;                                                 // slices start on 16-byte borders of the row
     const int i0 = min(V, rank * per), i1 = min(V, i0 + per);
-    pdl_wait();
+    pdl_wait(x);
     float best = -INFINITY;
     int bi = -1;
     if ((reinterpret_cast<uintptr_t>(x) & 15) == 0) {
@@ -415,7 +415,7 @@ sample_kernel(const float* __restrict__ logits, int V, long long row_stride, flo
               int top_k, const unsigned long long* __restrict__ seeds, const int* __restrict__ draw_counter,
               int* __restrict__ out) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(logits, draw_counter);
     __shared__ SampleShared s;
     const int cl = (int)smp_nranks();
     const int row = blockIdx.x / cl;
@@ -617,7 +617,7 @@ sample_cached_kernel(const float* __restrict__ logits, int V, long long row_stri
                      int top_k, const unsigned long long* __restrict__ seeds, const int* __restrict__ draw_counter,
                      int* __restrict__ out) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(logits, draw_counter);
     extern __shared__ __align__(16) uint8_t smp_dyn[];
     __shared__ Sample2Shared s;
     float* xs = reinterpret_cast<float*>(smp_dyn);                       // the slice's logits

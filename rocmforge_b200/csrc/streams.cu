@@ -256,7 +256,7 @@ pair_embed_kernel(const T* __restrict__ table, const T* __restrict__ pairs, cons
     __shared__ int row_s;
     float* red = sm + H;
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(pairs, ids);
     const int t = blockIdx.x;
     int id = ids[t];
     id = id < 0 ? 0 : (id >= V ? V - 1 : id);        // ids are validated on the host; never read outside
