@@ -488,11 +488,63 @@ __global__ void rope_kv_write_kernel(const void* __restrict__ src, int row_strid
     dst[e1] = Cvt<T>::from_f32(x1);
 }
 
-// The same for many tokens (prompts) whose q | k | v rows are one tensor in the compute dtype: a block takes TB tokens, forms the
-// sines and cosines of each once in shared memory (before it waits for the product: they depend on positions alone), and then walks
-// over (token, head, group of V pairs) with 16-byte loads and stores.  (Each thread with the trigonometry of its own four pairs,
-// one token a block: 33,361 tokens of 18 heads of 64 77 us; now 33, 4.7 TB/s.  8,192 tokens of 56 heads of 128 65 -> 51, with
-// one piece a thread in flight 66.)
+// The same for prompts whose q | k | v rows are one tensor in the compute dtype: a block per token, a thread owns the four pairs
+// of its group in every head it walks over and forms their sines and cosines once.
+template <typename T>
+__global__ void __launch_bounds__(256)
+rope_kv_write_token_kernel(const T* src, int row_stride, T* q_out, int q_out_stride,
+                          int nh, int nkv, int hd, const float* __restrict__ inv_freq,
+                          const int* __restrict__ tok_seq, const int* __restrict__ tok_pos,
+                          const int* __restrict__ seq_slot, const int* __restrict__ block_table, int max_pages,
+                          T* __restrict__ k_pages, T* __restrict__ v_pages, int write_kv) {
+    pdl_trigger();
+    const int t = blockIdx.x;
+    const int half = hd >> 1, groups = half >> 2;        // groups of four pairs per head
+    const int g = threadIdx.x % groups, lane_head = threadIdx.x / groups, head_step = blockDim.x / groups;
+    if (lane_head >= head_step) return;                  // threads beyond the last whole row of groups
+    const int pos = tok_pos[t];
+    size_t page_base = 0;
+    if (write_kv) {
+        const int slot = seq_slot[tok_seq[t]];
+        const int page = block_table[(size_t)slot * max_pages + pos / RF_PAGE];
+        page_base = (size_t)page * nkv * RF_PAGE * hd + (size_t)(pos % RF_PAGE) * hd;
+    }
+    float sn[4], cs[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sincosf((float)pos * inv_freq[4 * g + j], &sn[j], &cs[j]);
+    pdl_wait();
+    const T* row = src + (size_t)t * row_stride;
+    const int rotated = write_kv ? nh + nkv : nh;
+    for (int head = lane_head; head < rotated; head += head_step) {
+        float x0[4], x1[4], r0[4], r1[4];
+        Four<T>::load(row + (size_t)head * hd + 4 * g, x0);
+        Four<T>::load(row + (size_t)head * hd + half + 4 * g, x1);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { r0[j] = x0[j] * cs[j] - x1[j] * sn[j]; r1[j] = x0[j] * sn[j] + x1[j] * cs[j]; }
+        T* dst = head < nh ? q_out + (size_t)t * q_out_stride + (size_t)head * hd
+                           : k_pages + page_base + (size_t)(head - nh) * RF_PAGE * hd;
+        Four<T>::store(dst + 4 * g, r0);
+        Four<T>::store(dst + half + 4 * g, r1);
+    }
+    if (write_kv)
+        for (int vh = lane_head; vh < nkv; vh += head_step) {
+            float a[4], b[4];
+            const T* sv = row + (size_t)(nh + nkv + vh) * hd;
+            Four<T>::load(sv + 4 * g, a);
+            Four<T>::load(sv + half + 4 * g, b);
+            T* dst = v_pages + page_base + (size_t)vh * RF_PAGE * hd;
+            Four<T>::store(dst + 4 * g, a);
+            Four<T>::store(dst + half + 4 * g, b);
+        }
+}
+
+// The same for many tokens: a block takes TB of them, forms the sines and cosines of each once in shared memory (before it waits
+// for the product: they depend on positions alone), and then walks over (token, head, group of V pairs) with 16-byte loads and
+// stores, 8-byte ones where heads, strides or addresses allow no more (bfloat16 heads of 72, 104, 120).  33,361 tokens of 18 heads of
+// 64 33 us, 4.7 TB/s (a block per token 77); 8,192 tokens of 56 heads of 128 51 (65), with one piece a thread in flight 66.
+template <int BYTES> struct Wide { typedef uint4 type; };
+template <> struct Wide<8> { typedef uint2 type; };
+
 template <typename T, int V>
 __global__ void __launch_bounds__(256)
 rope_kv_write_rows_kernel(const T* src, int row_stride, T* q_out, int q_out_stride,
@@ -516,8 +568,9 @@ rope_kv_write_rows_kernel(const T* src, int row_stride, T* q_out, int q_out_stri
     __syncthreads();
     pdl_wait();
     const int groups = half / V, heads = write_kv ? nh + 2 * nkv : nh, per_tok = heads * groups;
-    union Piece { uint4 raw[V * sizeof(T) / 16]; T v[V]; };
-    constexpr int W = V * sizeof(T) / 16, N = 2;         // pieces of a thread in flight
+    typedef typename Wide<V * sizeof(T)>::type Raw;
+    union Piece { Raw raw; T v[V]; };
+    constexpr int N = 2;                                 // pieces of a thread in flight
     for (int i0 = threadIdx.x; i0 < n_tok * per_tok; i0 += 256 * N) {
         Piece x[N], z[N];
         int at[N];                                       // token, head and group of each
@@ -527,8 +580,8 @@ rope_kv_write_rows_kernel(const T* src, int row_stride, T* q_out, int q_out_stri
             at[n] = i < n_tok * per_tok ? t | head << 4 | g << 20 : -1;
             if (at[n] < 0) break;
             const T* from = src + (size_t)(t0 + t) * row_stride + (size_t)head * hd + V * g;
-#pragma unroll
-            for (int u = 0; u < W; ++u) { x[n].raw[u] = reinterpret_cast<const uint4*>(from)[u]; z[n].raw[u] = reinterpret_cast<const uint4*>(from + half)[u]; }
+            x[n].raw = *reinterpret_cast<const Raw*>(from);
+            z[n].raw = *reinterpret_cast<const Raw*>(from + half);
         }
 #pragma unroll
         for (int n = 0; n < N; ++n) {
@@ -546,8 +599,8 @@ rope_kv_write_rows_kernel(const T* src, int row_stride, T* q_out, int q_out_stri
             T* dst = (head < nh ? q_out + (size_t)(t0 + t) * q_out_stride + (size_t)head * hd
                       : head < nh + nkv ? k_pages + page_at[t] + (size_t)(head - nh) * RF_PAGE * hd
                                         : v_pages + page_at[t] + (size_t)(head - nh - nkv) * RF_PAGE * hd) + V * g;
-#pragma unroll
-            for (int u = 0; u < W; ++u) { reinterpret_cast<uint4*>(dst)[u] = x[n].raw[u]; reinterpret_cast<uint4*>(dst + half)[u] = z[n].raw[u]; }
+            *reinterpret_cast<Raw*>(dst) = x[n].raw;
+            *reinterpret_cast<Raw*>(dst + half) = z[n].raw;
         }
     }
 }
@@ -1390,17 +1443,36 @@ static int launch_rope_kv_write(const void* src, int row_stride, int n_partials,
     const int n_pairs = (nh + 2 * nkv) * (hd / 2);
     const dim3 grid(T_, (n_pairs + 255) / 256);
     if (T_ > 2147483647 || grid.y > 65535) return RF_ERR_UNSUPPORTED;
-    // prompts: rows of one tensor, everything aligned for 16-byte accesses, half a head a whole number of them
+    // prompts: rows of one tensor, half a head a whole number of accesses of v elements, everything aligned for them
+    auto fits = [&](int v) {
+        auto aligned = [&](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr) % (v * sizeof(T)) == 0; };
+        return n_partials == 0 && rot_dim == hd && !interleaved && T_ >= 64 && hd % (2 * v) == 0 && hd <= 2048 && row_stride % v == 0 &&
+            q_out_stride % v == 0 && aligned(src) && aligned(q_out) && (!write_kv || (aligned(k_pages) && aligned(v_pages)));
+    };
+    const T* from = reinterpret_cast<const T*>(src);
+    T *q_to = reinterpret_cast<T*>(q_out), *k_to = reinterpret_cast<T*>(k_pages), *v_to = reinterpret_cast<T*>(v_pages);
+    // Several tokens a block from sixteen tokens an SM on, where that still leaves blocks enough.  us, a block per token against
+    // 2 / 4 / 8 tokens, bfloat16, q + kv heads: 296 tokens of 28 + 4 heads of 128 2.0, 2.7 / 3.9 / 6.0; 1,200 7.6, 7.0 / 9.9 / 10.6; 2,400 12.3,
+    // 11.7 / 10.7 / 16.9; 5,000 24.7, 22.2 / 18.9 / 18.6; 14 + 2 of 64 1,200 2.6, 2.5 / 3.4 / 3.4; 2,400 5.4, 4.9 / 3.8 / 5.7; 5,000 11.0, 10.0
+    // / 7.2 / 7.0; 16 + 8 of 104 (8-byte accesses) 5,000 21.6, 17.3 / 16.6 / 19.8.  float32: 28 + 4 of 128 5,000 33.5, 31.1 / 32.1 / 35.4.
     constexpr int V = 16 / sizeof(T);
-    auto aligned = [&](const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) % 16) == 0; };
-    if (n_partials == 0 && rot_dim == hd && !interleaved && T_ >= 64 && hd % (2 * V) == 0 && hd <= 2048 && nh + 2 * nkv <= 65535 && row_stride % V == 0 && q_out_stride % V == 0 &&
-        aligned(src) && aligned(q_out) && (!write_kv || (aligned(k_pages) && aligned(v_pages)))) {
-        // eight tokens a block; fewer where the step is small (a block per SM before a second token) or the heads are very large
-        int tb = T_ >= 8 * 296 ? 8 : (T_ >= 4 * 296 ? 4 : 2);
-        while (tb * hd > 8192) tb >>= 1;
-        rf_launch(rope_kv_write_rows_kernel<T, V>, dim3((T_ + tb - 1) / tb), dim3(256), (size_t)tb * (hd / 2) * sizeof(float2), st,
-            reinterpret_cast<const T*>(src), row_stride, reinterpret_cast<T*>(q_out), q_out_stride, nh, nkv, hd, inv_freq, tok_seq, tok_pos,
-            seq_slot, block_table, max_pages, reinterpret_cast<T*>(k_pages), reinterpret_cast<T*>(v_pages), write_kv, T_, tb);
+    if (T_ >= 16 * 148 && nh + 2 * nkv <= 65535 && (fits(V) || fits(4))) {
+        const bool wide = fits(V), light = sizeof(T) == 2 || (nh + 2 * nkv) * (hd / 2 / V) <= 256;
+        int tb = !light ? 2 : (wide && T_ >= 32 * 148 ? 8 : 4);
+        while (tb * hd > 8192) tb >>= 1;                  // (the sines and cosines take tb * hd * 4 bytes)
+        rf_launch(wide ? rope_kv_write_rows_kernel<T, V> : rope_kv_write_rows_kernel<T, 4>, dim3((T_ + tb - 1) / tb), dim3(256),
+            (size_t)tb * (hd / 2) * sizeof(float2), st, from, row_stride, q_to, q_out_stride, nh, nkv, hd, inv_freq, tok_seq, tok_pos,
+            seq_slot, block_table, max_pages, k_to, v_to, write_kv, T_, tb);
+        RF_LAUNCH_CHECK();
+        return 0;
+    }
+    if (fits(4)) {
+        const int groups = hd / 8;
+        int threads = ((nh + 2 * nkv) * groups + 31) / 32 * 32;        // a row of groups per head, at most 256 threads
+        if (threads > 256) threads = 256;
+        if (threads < groups) threads = (groups + 31) / 32 * 32;
+        rf_launch(rope_kv_write_token_kernel<T>, dim3(T_), dim3(threads), 0, st, from, row_stride, q_to, q_out_stride, nh, nkv, hd,
+            inv_freq, tok_seq, tok_pos, seq_slot, block_table, max_pages, k_to, v_to, write_kv);
         RF_LAUNCH_CHECK();
         return 0;
     }
