@@ -127,7 +127,7 @@ row_norm_gate_kernel(const float* __restrict__ o, const void* __restrict__ gate,
 
 // grid (sequence, head, ceil(vdim / RT_COLS)); block RT_COLS warps.  R = ceil(dim / 32) rows of a column per lane.
 template <typename T, int R>
-__global__ void __launch_bounds__(RT_COLS * 32)
+__global__ void __launch_bounds__(RT_COLS * 32, R <= 4 ? 2048 / (RT_COLS * 32) : 1)      // (as many blocks as an SM has threads for)
 retention_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, int qk_stride, const T* __restrict__ v, int v_stride,
                       float* __restrict__ state, const float* __restrict__ decay, float* __restrict__ o,
                       const int* __restrict__ cu_q, const int* __restrict__ seq_slot, int heads, int dim, int vdim) {
