@@ -161,6 +161,16 @@ def test_large_scores_and_what_is_not_finite():
         assert (y - want).abs()[fine].max() <= 2.0 ** -19 * want.abs()[fine].max()
 
 
+@pytest.mark.parametrize("kind", ["prompt", "token"])
+def test_large_scores_against_64_bits(kind):
+    """A score of some hundreds carries an error of 2^-22 of the sum of its 64 products' sizes, of up to a thousand: 2^-12 in the
+    exponent, and so in a weight."""
+    b = batch([0, 40], [200, 100], 4, 2, 64, seed=5)
+    b["q"].mul_(30.0)
+    want = exact(b)
+    assert (run(b, kind).double() - want).abs().max() <= 2.0 ** -12 * want.abs().max()
+
+
 def test_whatever_is_not_finite_costs_a_bounded_time():
     """1,999 tokens with a value, or a key, that is infinite or not a number at the first position, so that every row of its kv head
     meets it: the generic kernel's kinds of results in at most eight times its time.  (A warp forms four rows at once and the generic
