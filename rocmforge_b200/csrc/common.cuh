@@ -33,6 +33,8 @@ __host__ __device__ __forceinline__ int rf_first_key(int pos, int span) {
 // through a const __restrict__ parameter for loads of what nobody writes, and may move them up across the wait.  The call hands the
 // pointer back as a new one that it knows nothing of but that it is global, so what is read through it is read after the wait; the
 // parameters that kernels write through keep their __restrict__.  A pointer formed from the parameter before the wait is named itself.
+// What it costs (ms a step, before and after): 7B decoding 2.45, 2.45 at batch 1 and 3.35, 3.35 at batch 64, Rifizen at batch 64 0.737,
+// 0.749, a Vilulorn prompt of 2,048 tokens 2.78, 2.89 (width 2,048).
 template <typename T>
 __device__ __forceinline__ void rf_read_from_here(T*& p) {
     size_t g = __cvta_generic_to_global(p);
