@@ -35,15 +35,18 @@
 // Row tile y of the grid is (group, first row, end row) of grp.tiles (grp.tiles[0] tiles exist; the others return at
 // once); its rows of X, sorted by group, meet rows group * group_n + ... of the stacked weights W [groups * group_n, K];
 // rows of the tile beyond its end belong to the next group and are computed but not stored.
-template <int BN, bool SWAP, int STAGES, bool NORM = false, bool GROUPED = false>
-__global__ void __launch_bounds__(TC_THREADS, SWAP ? (STAGES <= 4 && BN == 16 ? 3 : 2) : 1)
+// BM (weights as rows): weight rows of a tile, 128 or 64.  EW: epilogue warps, 4, or 8 that share the tile's columns.
+template <int BN, bool SWAP, int STAGES, bool NORM = false, bool GROUPED = false, int BM = TC_BM, int EW = 4>
+__global__ void __launch_bounds__(64 + 32 * EW, SWAP ? (BN == 16 && STAGES <= 4 ? 3 : 2) : 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, TcParams p,
                typename std::conditional<NORM, TcNorm, TcNoNorm>::type norm_arg,
                typename std::conditional<GROUPED, TcGroup, TcNoNorm>::type grp_arg) {
     static_assert(!(GROUPED && (SWAP || NORM)), "grouped products are tokens-as-rows and carry no norm");
+    static_assert(BM == TC_BM || (SWAP && !NORM && BM == 64), "tiles of 64 weight rows");
+    static_assert(EW == 4 || (SWAP && !NORM && EW == 8 && BN >= 32), "eight epilogue warps share the columns");
     // the variant without the norm never looks at this (every use below sits behind ``NORM &&``)
     const TcNorm& pn = *reinterpret_cast<const TcNorm*>(&norm_arg);
-    constexpr uint32_t A_BYTES = TC_BM * TC_BK * 2;
+    constexpr uint32_t A_BYTES = BM * TC_BK * 2;
     constexpr uint32_t B_BYTES = BN * TC_BK * 2;
     constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
     constexpr uint32_t TMEM_COLS = BN < 32 ? 32 : BN;
@@ -59,7 +62,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tile_a = blockIdx.y, tile_b = blockIdx.x, split = blockIdx.z;
-    int coord_a = tile_a * TC_BM, coord_b = tile_b * BN;            // first rows of the two operands' tiles
+    int coord_a = tile_a * BM, coord_b = tile_b * BN;            // first rows of the two operands' tiles
     if constexpr (GROUPED) {
         const TcGroup& grp = *reinterpret_cast<const TcGroup*>(&grp_arg);
         pdl_wait();                                     // the tile table is the sorting kernel's
@@ -132,7 +135,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     } else if (warp == 1) {
         // ---------------- MMA issuer: one thread, accumulator in tensor memory
         if (elect_one()) {
-            constexpr uint32_t idesc = make_idesc(BN);
+            constexpr uint32_t idesc = make_idesc(BN, BM);
             bool ok = true;
             for (int i = 0; i < n_kb && ok; ++i) {
                 const int s = i % STAGES;
@@ -168,11 +171,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const bool ok = mbar_wait(smem_u32(&bars[2 * STAGES]), 0, &abort_flag);
         tcgen05_fence_after();
         if (ok && n_kb > 0 && !(NORM && p.mode == EPI_RESNORM)) {
-            const int row_a = coord_a + quarter * 32 + lane;               // index along map A's rows
+            // index along map A's rows (64 rows lie in the first 16 lanes of each quarter; the other lanes hold nothing)
+            const int row_a = BM == 64 ? (lane < 16 ? coord_a + quarter * 16 + lane : p.N) : coord_a + quarter * 32 + lane;
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16);
-            constexpr int CH = BN < 32 ? 16 : 32;
+            constexpr int COLS = BN / (EW / 4), CH = COLS < 32 ? 16 : 32;
+            const int c_first = EW == 8 ? ((warp - 2) >> 2) * COLS : 0;
 #pragma unroll 1
-            for (int c0 = 0; c0 < BN; c0 += CH) {
+            for (int c0 = c_first; c0 < c_first + COLS; c0 += CH) {
                 uint32_t r[32];
                 if (CH == 32) tcgen05_ld32(taddr + c0, r); else tcgen05_ld16(taddr + c0, r);
                 tcgen05_wait_ld();
@@ -336,14 +341,25 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 }
 
 // ---------------------------------------------------------------- host side
-template <int BN, bool SWAP, int STAGES, bool NORM = false, bool GROUPED = false>
+static int sm_count() {
+    static PerDevice<int> devices;
+    int& n = devices.here();
+    if (n == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) n = 0;
+    }
+    return n;
+}
+
+template <int BN, bool SWAP, int STAGES, bool NORM = false, bool GROUPED = false, int BM = TC_BM, int EW = 4>
 static int launch_cfg(const CUtensorMap& ma, const CUtensorMap& mb, const TcParams& p, dim3 grid, cudaStream_t st,
                       const TcNorm* norm = nullptr, int cluster_z = 1, const TcGroup* group = nullptr) {
-    constexpr size_t smem = (size_t)STAGES * (TC_BM * TC_BK * 2 + BN * TC_BK * 2) + (2 * STAGES + 1) * 8 + 16 + 1024;
+    constexpr size_t smem = (size_t)STAGES * (BM * TC_BK * 2 + BN * TC_BK * 2) + (2 * STAGES + 1) * 8 + 16 + 1024;
     static PerDevice<bool> devices;
     bool& configured = devices.here();
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN, SWAP, STAGES, NORM, GROUPED>,
+        cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN, SWAP, STAGES, NORM, GROUPED, BM, EW>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         configured = true;
@@ -355,7 +371,7 @@ static int launch_cfg(const CUtensorMap& ma, const CUtensorMap& mb, const TcPara
     if (cluster_z > 1) {                             // the K splits of a tile as one cluster
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = grid;
-        cfg.blockDim = dim3(TC_THREADS);
+        cfg.blockDim = dim3(64 + 32 * EW);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = st;
         cudaLaunchAttribute attr[2];
@@ -365,12 +381,12 @@ static int launch_cfg(const CUtensorMap& ma, const CUtensorMap& mb, const TcPara
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = g_rf_pdl ? 2 : 1;
-        cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<BN, SWAP, STAGES, NORM, GROUPED>, ma, mb, p, extra, grp);
+        cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<BN, SWAP, STAGES, NORM, GROUPED, BM, EW>, ma, mb, p, extra, grp);
         if (e != cudaSuccess) return (int)e;
         RF_LAUNCH_CHECK();
         return 0;
     }
-    rf_launch(gemm_tc_kernel<BN, SWAP, STAGES, NORM, GROUPED>, grid, dim3(TC_THREADS), smem, st, ma, mb, p, extra, grp);
+    rf_launch(gemm_tc_kernel<BN, SWAP, STAGES, NORM, GROUPED, BM, EW>, grid, dim3(64 + 32 * EW), smem, st, ma, mb, p, extra, grp);
     RF_LAUNCH_CHECK();
     return 0;
 }
@@ -480,22 +496,44 @@ static int gemm_skinny(const void* X, int ldx, const void* W, const void* bias, 
     CUtensorMap ma, mb;
     int e;
     const int bn = M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128));
-    if ((e = make_map(&ma, W, N, K, K, TC_BM)) || (e = make_map(&mb, X, M, K, ldx, bn))) return e;
-    dim3 grid((M + bn - 1) / bn, (N + TC_BM - 1) / TC_BM, splits);      // token tiles fastest: they share a weight tile in L2
+    const bool normed_rows = ss_in || mode == EPI_RESNORM;
+    // Tiles of 64 weight rows where tiles of 128 leave SMs without one and K is whole (us with the norm before it, 128 and 64 rows:
+    // 64 tokens x 9,728 x 896 8.7, 8.4; 8 tokens x 9,728 x 896 8.1, 7.2, x 16,384 x 2,048 15.6, 14.2, x 4,096 x 2,048 12.3, 9.6).  Beyond
+    // a tile an SM they cost: half a tile's rows meet as many token bytes (8 tokens x 32,000 x 2,048 23.4, 27.7; 64 x 37,888 x 3,584
+    // 46.6, 50.7; 8 x 27,648 x 5,120 48.2, 48.3).
+    const bool half_tiles = !normed_rows && splits == 1 && (N + TC_BM - 1) / TC_BM * ((M + bn - 1) / bn) <= sm_count();
+    const int bm = half_tiles ? 64 : TC_BM;
+    // Eight epilogue warps where a number costs more than an add and a store to a whole line (us, four and eight: 64 tokens x 9,728 x 896
+    // gated 10.0, 8.7, 128 tokens 14.0, 11.6; 64 tokens x 37,888 x 3,584 47.8, 46.6; 64 x 8,192 x 2,048 in bfloat16 15.3, 14.3; but
+    // partial sums, 64 x 4,608 x 3,584 9.9, 10.4, 64 x 896 x 896 5.1, 5.4, and a head's 32-bit rows, 64 x 151,936 x 896 55.8, 56.6)
+    const bool wide_epilogue = epi_gated(mode) || mode == EPI_STORE;
+    if ((e = make_map(&ma, W, N, K, K, bm)) || (e = make_map(&mb, X, M, K, ldx, bn))) return e;
+    dim3 grid((M + bn - 1) / bn, (N + bm - 1) / bm, splits);      // token tiles fastest: they share a weight tile in L2
     // stage counts chosen so that two CTAs share an SM (three with up to 16 tokens: 3 x 4 stages hold as many weight
     // bytes as 2 x 6, and the third place takes a CTA of the next product while this one still runs: 2.791 against
     // 2.802 ms a decode step of the 7B shape at batch 8, 2.737 against 2.756 ms at batch 1): their pipelines overlap each
     // other's start-up and epilogue, and 2 x stages x 16 KB of weight bytes are in flight per SM.  (128 tokens:
     // two CTAs with three 32 KB stages each, 5.09 ms a decode step of the 7B shape; one CTA with six
     // stages 6.46 ms; two tiles of 64 tokens sharing the weight tile through L2 5.65 ms.)
-    if (ss_in || mode == EPI_RESNORM) {
+    if (normed_rows) {
         const int cz = mode == EPI_RESNORM ? splits : 1;
         if (bn == 16) return launch_cfg<16, true, 6, true>(ma, mb, p, grid, st, &nrm, cz);
         if (bn == 32) return launch_cfg<32, true, 5, true>(ma, mb, p, grid, st, &nrm, cz);
         if (bn == 64) return launch_cfg<64, true, 4, true>(ma, mb, p, grid, st, &nrm, cz);
         return launch_cfg<128, true, 3, true>(ma, mb, p, grid, st, &nrm, cz);
     }
+    if (half_tiles) {
+        if (bn == 16) return launch_cfg<16, true, 11, false, false, 64>(ma, mb, p, grid, st);
+        if (bn == 32) return launch_cfg<32, true, 9, false, false, 64, 8>(ma, mb, p, grid, st);
+        if (bn == 64) return launch_cfg<64, true, 6, false, false, 64, 8>(ma, mb, p, grid, st);
+        return launch_cfg<128, true, 4, false, false, 64, 8>(ma, mb, p, grid, st);
+    }
     if (bn == 16) return launch_cfg<16, true, 4>(ma, mb, p, grid, st);
+    if (wide_epilogue) {
+        if (bn == 32) return launch_cfg<32, true, 5, false, false, TC_BM, 8>(ma, mb, p, grid, st);
+        if (bn == 64) return launch_cfg<64, true, 4, false, false, TC_BM, 8>(ma, mb, p, grid, st);
+        return launch_cfg<128, true, 3, false, false, TC_BM, 8>(ma, mb, p, grid, st);
+    }
     if (bn == 32) return launch_cfg<32, true, 5>(ma, mb, p, grid, st);
     if (bn == 64) return launch_cfg<64, true, 4>(ma, mb, p, grid, st);
     return launch_cfg<128, true, 3>(ma, mb, p, grid, st);

@@ -224,9 +224,9 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t addr) {
     d |= (uint64_t)2 << 61;                          // 128-byte swizzle
     return d;
 }
-// Instruction descriptor: bf16 x bf16 -> f32, both operands K-major, M = 128, N = n.
-__host__ __device__ constexpr uint32_t make_idesc(int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
+// Instruction descriptor: bf16 x bf16 -> f32, both operands K-major, M = m (128 or 64), N = n.
+__host__ __device__ constexpr uint32_t make_idesc(int n, int m = TC_BM) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
 
