@@ -108,9 +108,9 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-// grid.x = n_clusters * CL (cluster dimension CL along x).  Work item w -> row group w % groups_m,
-// column tile (w / groups_m) % tiles_n, K part w / (groups_m * tiles_n); CTA `rank` of the cluster owns
-// row tile group * CL + rank.
+// grid.x = n_clusters * CL (cluster dimension CL along x).  Work items go K part by K part, in a part band by band of `band` row
+// groups, in a band column tile by column tile, rows fastest; CTA `rank` of the cluster owns row tile group * CL + rank.
+// A band's activations are read again for every column tile, so the host makes bands that L2 keeps.
 //
 // K parts (p.splits > 1, residual epilogue only).  The persistent clusters work in rounds, and a last round
 // that is half empty costs as much as a full one (2,048 x 3,584 outputs: 112 tiles on 74 clusters).  The
@@ -134,7 +134,7 @@ template <bool PAIR> struct ClusterLayout {
 template <int CL, bool PAIR>
 __global__ void __launch_bounds__(CG_THREADS, 1)
 gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                       const __grid_constant__ CUtensorMap map_out, TcParams p, int groups_m, int tiles_n, int bn,
+                       const __grid_constant__ CUtensorMap map_out, TcParams p, int groups_m, int tiles_n, int bn, int band,
                        int* __restrict__ flags) {
     // bn: columns of a tile (a multiple of 32, at most CG_BN; the host picks the width that wastes least of the last
     // round of clusters); the ring and the accumulators are laid out for CG_BN
@@ -164,6 +164,11 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     const int kb_all = (p.K + TC_BK - 1) / TC_BK;
     const int kb_part = (kb_all + p.splits - 1) / p.splits;         // k blocks per K part (the host leaves none empty)
     const uint16_t all = (uint16_t)((1u << CL) - 1);
+    auto place_of = [&](int w, int& group, int& tile_n) {               // row group and column tile of work item w
+        const int i = w % n_tiles, first = i / (band * tiles_n) * band, rows = min(band, groups_m - first), at = i - first * tiles_n;
+        group = first + at % rows;
+        tile_n = at / rows;
+    };
 
     if (threadIdx.x == 0) {
         abort_flag = 0;
@@ -218,7 +223,8 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             };
             const bool arms = !PAIR || rank == 0;        // who tells the barrier how many bytes to expect
             if (cluster_id < n_work) {
-                const int tile_n = (cluster_id / groups_m) % tiles_n;
+                int group, tile_n;
+                place_of(cluster_id, group, tile_n);
                 const int kb0 = (cluster_id / n_tiles) * kb_part, kb1 = min(kb_all, kb0 + kb_part);
                 pre = min(S, kb1 - kb0);
                 for (int i = 0; i < pre; ++i) {
@@ -229,7 +235,9 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             pdl_wait();
             int it = 0;                                  // running k-block count across work items
             for (int w = cluster_id; w < n_work && !abort_flag; w += n_clusters) {
-                const int tile_m = (w % groups_m) * CL + (int)rank, tile_n = (w / groups_m) % tiles_n;
+                int group, tile_n;
+                place_of(w, group, tile_n);
+                const int tile_m = group * CL + (int)rank;
                 const int kb0 = (w / n_tiles) * kb_part, kb1 = min(kb_all, kb0 + kb_part);
                 for (int kb = kb0; kb < kb1; ++kb, ++it) {
                     const int s = it % S;
@@ -287,7 +295,9 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         int local = 0, slab = 0;
         for (int w = cluster_id; w < n_work; w += n_clusters, ++local) {
             const int buf = local & 1;
-            const int tile_m = (w % groups_m) * CL + (int)rank, tile_n = (w / groups_m) % tiles_n;
+            int group, tile_n;
+            place_of(w, group, tile_n);
+            const int tile_m = group * CL + (int)rank;
             const int part = w / n_tiles;                // K part: only the first one adds the bias
             const int mode = p.mode;
             const CUtensorMap* omap = &map_out;
@@ -480,6 +490,17 @@ static int cluster_width() {
     return max_clusters;
 }
 
+static long long l2_bytes() {
+    static PerDevice<int> devices;
+    int& n = devices.here();
+    if (n == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrL2CacheSize, dev) != cudaSuccess) n = 0;
+    }
+    return n;
+}
+
 template <int CL, bool PAIR>
 static int launch_cluster(const void* X, int ldx, const void* W, TcParams p, int parts, int* flags, int n_flags,
                           cudaStream_t st) {
@@ -549,7 +570,15 @@ static int launch_cluster(const void* X, int ldx, const void* W, TcParams p, int
     if (n_clusters > max_clusters) n_clusters = max_clusters;
     cfg.gridDim = dim3(n_clusters * CL);
     cfg.numAttrs = g_rf_pdl ? 2 : 1;
-    cudaError_t le = cudaLaunchKernelEx(&cfg, gemm_tc_cluster_kernel<CL, PAIR>, ma, mb, mo, p, groups_m, tiles_n, bn, flags);
+    // Bands of row groups whose activations (of a K part) take at most a quarter of L2, all alike.  With the rows fastest over the whole
+    // matrix, activations beyond L2 came from memory once for every column tile: the down projection of 33,361 tokens x 896 x 4,864 read
+    // its 324 MB four times.  Whole prompts (ms, with bands of 24, 48, 80 MB and without): 14B of 8,192 tokens 210.7,
+    // 209.5, 219.5, 222.9, 0.5B of 33,361 29.2, 29.1, 30.5, 31.4.  Activations that fit (7B, 2,048 tokens) keep the one band.
+    const long long group_bytes = (long long)CL * TC_BM * ((kb_all + p.splits - 1) / p.splits) * TC_BK * 2;
+    long long most = l2_bytes() / 4 / group_bytes;
+    most = most < 1 ? 1 : most > groups_m ? groups_m : most;
+    const int n_bands = (int)((groups_m + most - 1) / most), band = (groups_m + n_bands - 1) / n_bands;
+    cudaError_t le = cudaLaunchKernelEx(&cfg, gemm_tc_cluster_kernel<CL, PAIR>, ma, mb, mo, p, groups_m, tiles_n, bn, band, flags);
     if (le != cudaSuccess) return (int)le;
     RF_LAUNCH_CHECK();
     return 0;
