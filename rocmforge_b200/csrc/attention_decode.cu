@@ -15,6 +15,7 @@
 // the chunks in index order, so the result does not depend on which CTA that was.  The grid
 // may be larger than the context needs (a replayed CUDA graph keeps its launch shape): CTAs
 // beyond the sequence's last chunk, or wholly before its window, leave at once.
+#include <type_traits>
 #include <cuda.h>
 #include "common.cuh"
 
@@ -326,15 +327,35 @@ __device__ __forceinline__ void dcl_cluster_sync() {
 // the slice of output dimensions that this peer owns (remote stores into a slot per sender); after ONE cluster
 // barrier each CTA folds the slots of its slice in rank order and writes it.  No CTA reads a peer's memory,
 // so none has to wait for its peers before it exits.
-template <int EPL, int ROWS, int WARPS>
+//
+// FORM: the kernel before this one is the q|k|v product itself, its K split into 32-bit partial sums.  Every CTA adds up the sums
+// (and bias) of its group's query heads and turns them; the CTA whose pages hold the newest position does so with that position's key
+// and value too, puts them into the tile that TMA brought in (its row there is not written yet) and, once that copy has landed, into
+// the cache.  Elements are added and turned as rope_kv_write_kernel does it.  No tile then holds anything that this step's other
+// kernels write, so the first tiles of all warps are on their way while the product still runs.
+struct DecShaped {              // the kernel's own arguments for queries that another kernel has made
+    const __nv_bfloat16* q;
+    const float* slopes;
+    const float* sinks;
+    int q_stride, keep_first;
+    float softcap;
+};
+struct DecFormed {              // ... and for those it forms itself (with two tensor maps and the rest 384 bytes: more cost a launch 4 us)
+    const float* parts;         // [n_parts][B][(nh + 2 nkv) HD]
+    const void* bias;           // [(nh + 2 nkv) HD] or null
+    const float* inv_freq;      // [HD / 2]: heads turn as pairs (i, i + HD / 2)
+    __nv_bfloat16* k_pages;
+    __nv_bfloat16* v_pages;
+    int n_parts, bias_is_f32;
+};
+template <int EPL, int ROWS, int WARPS, bool FORM>
 __global__ void __launch_bounds__(WARPS * 32)
 attention_decode_warps_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-                              const __nv_bfloat16* __restrict__ q, int q_stride, __nv_bfloat16* __restrict__ out,
+                              __nv_bfloat16* __restrict__ out,
                               int out_stride, const int* __restrict__ tok_seq, const int* __restrict__ tok_pos,
                               const int* __restrict__ seq_slot, const int* __restrict__ block_table, int max_pages,
                               int nh, int nkv, float scale, int window, int splits, int* __restrict__ status,
-                              float softcap, const float* __restrict__ slopes, int keep_first,
-                              const float* __restrict__ sinks) {
+                              typename std::conditional<FORM, DecFormed, DecShaped>::type own) {
     constexpr int HD = EPL * 32;
     constexpr int NT = WARPS * 32;
     constexpr int HALVES = HD / 64;                             // 128-byte column blocks of a row
@@ -353,6 +374,8 @@ attention_decode_warps_kernel(const __grid_constant__ CUtensorMap map_k, const _
     float* slots = c_l + DEC_GP;                                // [splits][2*GP + GP * HD/splits]: what the peers push
     uint64_t* bars = reinterpret_cast<uint64_t*>(slots + splits * 2 * DEC_GP + DEC_GP * HD);     // [warp][K | V]
     __shared__ int gave_up;
+    // FORM: queries, then the newest key and value, rows of HD + 8 (16 bytes apart from a multiple of 128: no bank conflicts)
+    __shared__ __align__(16) __nv_bfloat16 formed[FORM ? (DEC_GP + 2) * (HD + 8) : 1];
 
     pdl_trigger();
     const int G = nh / nkv;
@@ -361,6 +384,11 @@ attention_decode_warps_kernel(const __grid_constant__ CUtensorMap map_k, const _
     const int rank = splits > 1 ? (int)dcl_cluster_rank() : 0;
     const int pos = tok_pos[b];
     const int lo = rf_first_key(pos, window);
+    const float* slopes = nullptr;
+    const float* sinks = nullptr;
+    float softcap = 0.f;
+    int keep_first = 0;
+    if constexpr (!FORM) { slopes = own.slopes; sinks = own.sinks; softcap = own.softcap; keep_first = own.keep_first; }
     // designs that cap their scores (softcap * tanh(score / softcap)) and lower them by slope * distance afterwards
     const bool shaped = softcap > 0.f || slopes != nullptr;
     const float inv_cap = softcap > 0.f ? 1.f / softcap : 0.f;
@@ -432,24 +460,88 @@ attention_decode_warps_kernel(const __grid_constant__ CUtensorMap map_k, const _
         return __all_sync(0xffffffffu, ok != 0);
     };
 
-    // Only the page of the newest position is written in this step (by the kernel before this one); the
-    // older pages were written by earlier steps, which are complete: their copies start before the wait.
+    // Only the newest position is written in this step (by the kernel before this one, or below); what is older was written by
+    // earlier steps, which are complete: the copies of older pages (FORM: of all pages) start before the wait.
     int u = next_tile(warp - WARPS);
-    const bool early = u < n_units && first_key(u) / RF_PAGE < p_hi;
+    const bool early = u < n_units && (FORM || first_key(u) / RF_PAGE < p_hi);
     if (lane == 0 && early) { issue(u, true); issue(u, false); }
-    pdl_wait(q);                                         // queries and the newest keys/values come from the kernel before us
-    if (lane == 0 && !early && u < n_units) { issue(u, true); issue(u, false); }
-
+    const bool newest_here = FORM && (n_listed - 1) % splits == rank;       // the newest position's page is this CTA's
     uint32_t qb[HD / 16][2];                            // Q^T as the B operand: head gid, dims ks*16 + tig*2 (+8)
+    if constexpr (FORM) {
+        // item i: four pairs of head i / (HD / 8) of this CTA: the group's queries, then the newest key and value
+        constexpr int PER = HD / 8, HALF = HD / 2;
+        const int items = (newest_here ? G + 2 : G) * PER, width = (nh + 2 * nkv) * HD;
+        float b0[4], b1[4], cs[4], sn[4];
+        auto column = [&](int i) {
+            const int h = i / PER;
+            return (h < G ? kvh * G + h : (h == G ? nh : nh + nkv) + kvh) * HD + 4 * (i % PER);
+        };
+        auto lead = [&](int i) {                         // what does not depend on the product
+            const int c = column(i);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                b0[j] = own.bias != nullptr ? load_vec(own.bias, own.bias_is_f32, c + j) : 0.f;
+                b1[j] = own.bias != nullptr ? load_vec(own.bias, own.bias_is_f32, c + HALF + j) : 0.f;
+                if (i < (G + 1) * PER) sincosf((float)pos * own.inv_freq[4 * (i % PER) + j], &sn[j], &cs[j]);
+            }
+        };
+        if (tid < items) lead(tid);
+        pdl_wait();
+        const float* rows = own.parts + (size_t)b * width;
+        const size_t stride = (size_t)gridDim.z * width;
+        for (int i = tid; i < items; i += NT) {
+            if (i != tid) lead(i);
+            const float* p = rows + column(i);
+            for (int sp = 0; sp < own.n_parts; sp += 8) {        // eight pairs of loads in flight at once, added in index order
+                float4 u0[8], u1[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    if (sp + k < own.n_parts) {
+                        u0[k] = *reinterpret_cast<const float4*>(p + (sp + k) * stride);
+                        u1[k] = *reinterpret_cast<const float4*>(p + (sp + k) * stride + HALF);
+                    }
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    if (sp + k < own.n_parts) {
+                        b0[0] += u0[k].x; b0[1] += u0[k].y; b0[2] += u0[k].z; b0[3] += u0[k].w;
+                        b1[0] += u1[k].x; b1[1] += u1[k].y; b1[2] += u1[k].z; b1[3] += u1[k].w;
+                    }
+            }
+            if (i < (G + 1) * PER)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float x0 = b0[j], x1 = b1[j];
+                    b0[j] = x0 * cs[j] - x1 * sn[j]; b1[j] = x0 * sn[j] + x1 * cs[j];
+                }
+            __nv_bfloat162* to = reinterpret_cast<__nv_bfloat162*>(formed + (i / PER) * (HD + 8) + 4 * (i % PER));
+            to[0] = __floats2bfloat162_rn(b0[0], b0[1]); to[1] = __floats2bfloat162_rn(b0[2], b0[3]);
+            to[HALF / 2] = __floats2bfloat162_rn(b1[0], b1[1]); to[HALF / 2 + 1] = __floats2bfloat162_rn(b1[2], b1[3]);
+        }
+        __syncthreads();
+    } else {
+        pdl_wait();                                      // queries and the newest keys/values come from the kernel before us
+        if (lane == 0 && !early && u < n_units) { issue(u, true); issue(u, false); }
+    }
 #pragma unroll
     for (int ks = 0; ks < HD / 16; ++ks) {
         qb[ks][0] = qb[ks][1] = 0u;
         if (gid < G) {
-            const __nv_bfloat16* qrow = q + (size_t)b * q_stride + (size_t)(kvh * G + gid) * HD + ks * 16 + tig * 2;
+            const __nv_bfloat16* qrow;
+            if constexpr (FORM) qrow = formed + gid * (HD + 8) + ks * 16 + tig * 2;
+            else qrow = own.q + (size_t)b * own.q_stride + (size_t)(kvh * G + gid) * HD + ks * 16 + tig * 2;
             qb[ks][0] = *reinterpret_cast<const uint32_t*>(qrow);
             qb[ks][1] = *reinterpret_cast<const uint32_t*>(qrow + 8);
         }
     }
+    // FORM: the newest key or value (rows G, G + 1 of what was formed) into its row of this warp's tile; 16 bytes a lane
+    auto place_newest = [&](uint32_t tile, int row, int which) {
+        if (lane < HD / 8) {
+            const uint4 x = *reinterpret_cast<const uint4*>(formed + (G + which) * (HD + 8) + lane * 8);
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};"
+                         ::"r"(tile + (lane >> 3) * HALF_BYTES + row * 128 + (((lane & 7) ^ (row & 7)) << 4)), "r"(x.x), "r"(x.y), "r"(x.z), "r"(x.w) : "memory");
+        }
+        __syncwarp();
+    };
     // O^T: block mt of 16 dimensions: [0] (dim gid, head tig*2), [1] (dim gid, head tig*2+1), [2], [3] the same for dim gid + 8
     float oc[HD / 16][4];
 #pragma unroll
@@ -466,6 +558,9 @@ attention_decode_warps_kernel(const __grid_constant__ CUtensorMap map_k, const _
         int k_kept = keep_first - key0; if (k_kept > k_last + 1) k_kept = k_last + 1;  // rows below it are kept first positions
         if (k_kept < 0) k_kept = 0;
         if (!wait(bar_k, it & 1)) { failed = true; break; }
+        // (the newest position's tile is the last of its warp: nothing is copied over the row again)
+        const bool newest = newest_here && pos - key0 < ROWS;
+        if (newest) place_newest(k_t, pos - key0, 0);
         // ---- scores, transposed: [0] (key gid, head tig*2), [1] (key gid, head tig*2+1), [2], [3] the same for key gid + 8
         float sc[NB][4];
 #pragma unroll
@@ -538,6 +633,15 @@ attention_decode_warps_kernel(const __grid_constant__ CUtensorMap map_k, const _
             oc[mt][0] *= corr[0]; oc[mt][1] *= corr[1]; oc[mt][2] *= corr[0]; oc[mt][3] *= corr[1];
         }
         if (!wait(bar_v, it & 1)) { failed = true; break; }
+        if constexpr (FORM)
+            if (newest) {
+                place_newest(v_t, pos - key0, 1);
+                if (lane < HD / 8) {                     // both copies of the row's place have landed
+                    const size_t at = (((size_t)bt[pos / RF_PAGE] * nkv + kvh) * RF_PAGE + pos % RF_PAGE) * HD + lane * 8;
+                    *reinterpret_cast<uint4*>(own.k_pages + at) = *reinterpret_cast<const uint4*>(formed + G * (HD + 8) + lane * 8);
+                    *reinterpret_cast<uint4*>(own.v_pages + at) = *reinterpret_cast<const uint4*>(formed + (G + 1) * (HD + 8) + lane * 8);
+                }
+            }
         if ((k_begin > 0 && k_kept < ROWS) || k_last < ROWS - 1) {
             // rows outside the sequence get weight zero, but 0 * (whatever bits lie there) must be 0
             // (the swizzle permutes 16-byte pieces inside a row: clearing whole rows needs no address math)
@@ -699,23 +803,22 @@ static int dec_make_map(CUtensorMap* map, const void* pages, long long rows, int
     return r == CUDA_SUCCESS ? 0 : RF_ERR_BAD_ARG;
 }
 
-template <int EPL, int ROWS, int WARPS>
-static int launch_warps(const void* q, int q_stride, void* out, int out_stride, const void* k_pages,
+template <int EPL, int ROWS, int WARPS, bool FORM, typename Own>
+static int launch_warps(const Own& own, void* out, int out_stride, const void* k_pages,
                         const void* v_pages, long long n_pages, const int* tok_seq, const int* tok_pos,
                         const int* seq_slot, const int* block_table, int max_pages, int nh, int nkv, float scale,
-                        int window, int B, int splits, int* status, float softcap, const float* slopes, int keep_first,
-                        const float* sinks, cudaStream_t st) {
+                        int window, int B, int splits, int* status, cudaStream_t st) {
     constexpr int HD = EPL * 32;
     const size_t smem = (size_t)WARPS * 2 * ROWS * HD * 2 +
                         (size_t)(WARPS * DEC_GP + 2 * DEC_GP + 16 * 2 * DEC_GP + DEC_GP * HD) * sizeof(float) + WARPS * 2 * 8 + 16 + 1024;
     static PerDevice<bool> devices;
     bool& configured = devices.here();
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attention_decode_warps_kernel<EPL, ROWS, WARPS>,
+        cudaError_t e = cudaFuncSetAttribute(attention_decode_warps_kernel<EPL, ROWS, WARPS, FORM>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         // clusters of 16 (one sequence with a long context: 4 kv heads x 16 CTAs) are beyond the portable size
-        e = cudaFuncSetAttribute(attention_decode_warps_kernel<EPL, ROWS, WARPS>,
+        e = cudaFuncSetAttribute(attention_decode_warps_kernel<EPL, ROWS, WARPS, FORM>,
                                  cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return (int)e;
         configured = true;
@@ -744,9 +847,9 @@ static int launch_warps(const void* q, int q_stride, void* out, int out_stride, 
     if ((me = dec_make_map(&mk, k_pages, n_pages * nkv * RF_PAGE, HD, ROWS)) ||
         (me = dec_make_map(&mv, v_pages, n_pages * nkv * RF_PAGE, HD, ROWS)))
         return me;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, attention_decode_warps_kernel<EPL, ROWS, WARPS>, mk, mv,
-        reinterpret_cast<const __nv_bfloat16*>(q), q_stride, reinterpret_cast<__nv_bfloat16*>(out), out_stride, tok_seq,
-        tok_pos, seq_slot, block_table, max_pages, nh, nkv, scale, window, splits, status, softcap, slopes, keep_first, sinks);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, attention_decode_warps_kernel<EPL, ROWS, WARPS, FORM>, mk, mv,
+        reinterpret_cast<__nv_bfloat16*>(out), out_stride, tok_seq, tok_pos, seq_slot, block_table, max_pages, nh, nkv, scale, window,
+        splits, status, own);
     if (e != cudaSuccess) return (int)e;
     RF_LAUNCH_CHECK();
     return 0;
@@ -795,7 +898,34 @@ void rf_attention_decode_scratch(int B, int nh, int nkv, int hd, int max_chunks,
     *n_counters = (long long)B * nkv;
 }
 
+}   // extern "C"
+
 // A warp per tile of keys, `warps` (4 or 8) warps per CTA.
+template <bool FORM, typename Own>
+static int decode_warps(const Own& own, void* out, int out_stride, const void* k_pages, const void* v_pages, long long n_pages,
+                        const int* tok_seq, const int* tok_pos, const int* seq_slot, const int* block_table, int max_pages, int nh, int nkv,
+                        int hd, float scale, int window, int B, int splits, int warps, int* status, cudaStream_t st) {
+    if (!rf_attention_decode_supported(nh, nkv, hd)) return RF_ERR_UNSUPPORTED;
+    if (nkv > 65535 || B > 65535) return RF_ERR_UNSUPPORTED;
+    if (splits != 1 && splits != 2 && splits != 4 && splits != 8 && splits != 16) return RF_ERR_BAD_ARG;
+    if (warps != 4 && warps != 8) return RF_ERR_BAD_ARG;
+#define GOW(EPL, ROWS, WARPS) return launch_warps<EPL, ROWS, WARPS, FORM>(own, out, out_stride, k_pages, v_pages, n_pages, tok_seq, tok_pos, \
+                              seq_slot, block_table, max_pages, nh, nkv, scale, window, B, splits, status, st)
+    if (hd == 64) { if (warps == 8) GOW(2, 32, 8); GOW(2, 32, 4); }
+    if constexpr (FORM) {
+        if (hd != 128) return RF_ERR_UNSUPPORTED;
+        if (warps == 8) GOW(4, 16, 8);
+        GOW(4, 16, 4);
+    } else {
+        if (hd == 128) { if (warps == 8) GOW(4, 32, 8); GOW(4, 32, 4); }
+        if (warps == 8) GOW(8, 16, 8);
+        GOW(8, 16, 4);
+    }
+#undef GOW
+}
+
+extern "C" {
+
 // softcap > 0: scores become softcap * tanh(score / softcap); slopes (float [nh] or null): after the cap a score is
 // lowered by slopes[head] * (query position - key position).  keep_first: with a window (window > 0), the first keep_first
 // positions of a sequence stay visible as well.  sinks (float [nh] or null): exp(sinks[head]) counts once in the softmax's
@@ -807,18 +937,23 @@ int rf_attention_decode_warps_sink(const void* q, int q_stride, void* out, int o
                                    int keep_first, const float* sinks, int* status, cudaStream_t st) {
     if (B <= 0) return 0;
     if (keep_first < 0 || (keep_first > 0 && window <= 0)) return RF_ERR_BAD_ARG;
-    if (!rf_attention_decode_supported(nh, nkv, hd)) return RF_ERR_UNSUPPORTED;
-    if (nkv > 65535 || B > 65535) return RF_ERR_UNSUPPORTED;
-    if (splits != 1 && splits != 2 && splits != 4 && splits != 8 && splits != 16) return RF_ERR_BAD_ARG;
-    if (warps != 4 && warps != 8) return RF_ERR_BAD_ARG;
     if ((reinterpret_cast<uintptr_t>(q) & 15) || (q_stride * 2) % 16) return RF_ERR_BAD_ARG;
-#define GOW(EPL, ROWS, WARPS) return launch_warps<EPL, ROWS, WARPS>(q, q_stride, out, out_stride, k_pages, v_pages, n_pages, tok_seq, \
-                              tok_pos, seq_slot, block_table, max_pages, nh, nkv, scale, window, B, splits, status, softcap, slopes, keep_first, sinks, st)
-    if (hd == 64) { if (warps == 8) GOW(2, 32, 8); GOW(2, 32, 4); }
-    if (hd == 128) { if (warps == 8) GOW(4, 32, 8); GOW(4, 32, 4); }
-    if (warps == 8) GOW(8, 16, 8);
-    GOW(8, 16, 4);
-#undef GOW
+    return decode_warps<false>(DecShaped{reinterpret_cast<const __nv_bfloat16*>(q), slopes, sinks, q_stride, keep_first, softcap}, out, out_stride,
+                               k_pages, v_pages, n_pages, tok_seq, tok_pos, seq_slot, block_table, max_pages, nh, nkv, hd, scale, window, B,
+                               splits, warps, status, st);
+}
+
+// From the q|k|v product's partial sums [n_parts][B][(nh + 2 nkv) hd] (and a bias): queries and the newest key and value are formed,
+// turned as pairs (i, i + hd / 2) by position * inv_freq[i] and, key and value, written to their place in the pages.  Heads of 64 or 128.
+int rf_attention_decode_warps_formed(const float* parts, int n_parts, const void* bias, int bias_is_f32, const float* inv_freq, void* out,
+                                     int out_stride, void* k_pages, void* v_pages, long long n_pages, const int* tok_seq, const int* tok_pos,
+                                     const int* seq_slot, const int* block_table, int max_pages, int nh, int nkv, int hd, float scale,
+                                     int window, int B, int splits, int warps, int* status, cudaStream_t st) {
+    if (B <= 0) return 0;
+    if (!parts || n_parts < 1 || !inv_freq || (reinterpret_cast<uintptr_t>(parts) & 15)) return RF_ERR_BAD_ARG;
+    return decode_warps<true>(DecFormed{parts, bias, inv_freq, reinterpret_cast<__nv_bfloat16*>(k_pages), reinterpret_cast<__nv_bfloat16*>(v_pages),
+                                        n_parts, bias_is_f32}, out, out_stride, k_pages, v_pages, n_pages, tok_seq, tok_pos, seq_slot, block_table,
+                              max_pages, nh, nkv, hd, scale, window, B, splits, warps, status, st);
 }
 
 int rf_attention_decode_warps_ext(const void* q, int q_stride, void* out, int out_stride, const void* k_pages,

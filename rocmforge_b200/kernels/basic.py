@@ -756,6 +756,42 @@ def attention_decode_warps(q: torch.Tensor, n_heads: int, n_kv_heads: int, head_
     return out
 
 
+def attention_decode_formed(parts: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: int, inv_freq: torch.Tensor, k_pages, v_pages,
+                            tok_seq, tok_pos, seq_slot, block_table, scale: float, window: int | None, *, splits: int,
+                            warps: int | None = None, bias: torch.Tensor | None = None, chunk: int | None = None) -> torch.Tensor:
+    """``attention_decode_warps`` on the q|k|v product's own output: ``parts`` is the float32 stack [S, B, (heads + 2 kv_heads) *
+    head_dim] of its partial sums, to which ``bias`` is added; queries and keys turn as in ``rope_kv_write`` (whole heads, pairs
+    (i, i + head_dim / 2)), and the new keys and values are written to their pages.  Heads of 64, in tiles of
+    32 keys a warp (then the bits are those of the two kernels), or of 128, in tiles of 16."""
+    need_cuda(parts, inv_freq, k_pages, v_pages, tok_seq, tok_pos, seq_slot, block_table, bias)
+    width = (n_heads + 2 * n_kv_heads) * head_dim
+    need(parts.dim() == 3 and parts.dtype == torch.float32 and parts.is_contiguous() and parts.data_ptr() % 16 == 0
+         and parts.shape[2] == width,
+         "attention_decode: partial sums must be a contiguous float32 [S, B, (heads + 2 kv_heads) * head_dim] stack")
+    S, B = parts.shape[:2]
+    need(k_pages.dtype == torch.bfloat16 and tuple(k_pages.shape[1:]) == (n_kv_heads, PAGE, head_dim)
+         and k_pages.is_contiguous() and v_pages.dtype == torch.bfloat16 and v_pages.shape == k_pages.shape and v_pages.is_contiguous(),
+         "attention_decode: bad cache page shape or dtype")
+    need(attention_decode_supported(n_heads, n_kv_heads, head_dim) and head_dim <= 128,
+         f"attention_decode: heads={n_heads}, kv_heads={n_kv_heads}, head_dim={head_dim} is not supported")
+    need(inv_freq.dtype == torch.float32 and inv_freq.numel() == head_dim // 2 and inv_freq.is_contiguous(),
+         "attention_decode: inv_freq must hold head_dim/2 float32 frequencies")
+    need(bias is None or (bias.shape == (width,) and bias.dtype in (torch.float32, torch.bfloat16) and bias.is_contiguous()),
+         "attention_decode: the bias must be [(heads + 2 kv_heads) * head_dim]")
+    if warps is None:
+        warps = 8 if B * n_kv_heads * splits <= _sms(parts.device) * (2 if head_dim <= 64 else 1) else 4
+    out = torch.empty((B, n_heads * head_dim), dtype=torch.bfloat16, device=parts.device)
+    from .tensor_core import status_word
+    f = _f("attention_decode", "rf_attention_decode_warps_formed", c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p,
+           c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_int,
+           c_void_p, c_void_p)
+    check(f(ptr(parts), S, ptr(bias), int(bias is not None and bias.dtype == torch.float32), ptr(inv_freq), ptr(out), out.stride(0),
+            ptr(k_pages), ptr(v_pages), k_pages.shape[0], ptr(tok_seq), ptr(tok_pos), ptr(seq_slot), ptr(block_table), block_table.shape[1],
+            n_heads, n_kv_heads, head_dim, float(scale), key_span(window, chunk), B, splits, warps, ptr(status_word(parts.device)), stream()),
+          f"attention_decode_formed (heads={n_heads}, kv_heads={n_kv_heads}, head_dim={head_dim}, splits={splits})")
+    return out
+
+
 PREFILL_TC_TILE = 128
 
 
