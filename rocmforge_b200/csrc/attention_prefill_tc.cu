@@ -135,7 +135,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc_s = at_idesc(AT_BN, 0), idesc_o = at_idesc(HD, 1);
             // S has two buffers in tensor memory: the scores of page t + 1 are computed while the softmax
             // warps are still busy with page t, so they find their next input ready when they come back.
@@ -252,9 +252,9 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             }
             float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-            for (int j = 0; j < AT_BN; j += 4) {
-                mx4[0] = fmaxf(mx4[0], sc[j]); mx4[1] = fmaxf(mx4[1], sc[j + 1]);
-                mx4[2] = fmaxf(mx4[2], sc[j + 2]); mx4[3] = fmaxf(mx4[3], sc[j + 3]);
+            for (int j = 0; j < AT_BN; j += 8) {
+                mx4[0] = max3(mx4[0], sc[j], sc[j + 4]); mx4[1] = max3(mx4[1], sc[j + 1], sc[j + 5]);
+                mx4[2] = max3(mx4[2], sc[j + 2], sc[j + 6]); mx4[3] = max3(mx4[3], sc[j + 3], sc[j + 7]);
             }
             const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * sl2;      // in units of log2 e (sl2 > 0)
             // move the reference only when the maximum has grown by more than 8: then O and l are rescaled
@@ -264,17 +264,27 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 m_ref = mx;
             }
             const float nref = (m_ref == -INFINITY) ? 0.f : -m_ref;
-            float sum4[4] = {0.f, 0.f, 0.f, 0.f};
+            // Two numbers an instruction wherever there is one, rounded to bfloat16 by it: the softmax warps' own stream of instructions is
+            // what a page takes.  (us, with one number an instruction, rounded by integer additions, and so: 64 prompts of 16..1,024
+            // tokens, 14 heads of 64 166.5, 152.5; one of 8,192 227, 208; 2,048 tokens, 28 heads of 128 42.9, 38.9.  Four CTAs an SM in
+            // place of two, heads of 64 and halves of a page at a time, changed nothing; pages left out for warps that see none
+            // of their keys cost 3 %.)
+            Two sum01 = two(0.f, 0.f), sum23 = sum01;
+            const Two sl22 = two(sl2, sl2), nref2 = two(nref, nref);
             uint32_t pk[AT_BN / 2];
 #pragma unroll
             for (int j = 0; j < AT_BN; j += 4) {
-                // weight = 2^(raw * scale * log2 e - reference): one FMA and one ex2 each; ex2(-inf) = 0
-                const float p0 = at_exp2(fmaf(sc[j], sl2, nref)), p1 = at_exp2(fmaf(sc[j + 1], sl2, nref));
-                const float p2 = at_exp2(fmaf(sc[j + 2], sl2, nref)), p3 = at_exp2(fmaf(sc[j + 3], sl2, nref));
-                sum4[0] += p0; sum4[1] += p1; sum4[2] += p2; sum4[3] += p3;
-                pk[j >> 1] = at_pack_bf16x2(p0, p1);
-                pk[(j >> 1) + 1] = at_pack_bf16x2(p2, p3);
+                // weight = 2^(raw * scale * log2 e - reference): half an FMA and one ex2 each; ex2(-inf) = 0
+                float p0, p1, p2, p3;
+                one(fma2(two(sc[j], sc[j + 1]), sl22, nref2), p0, p1);
+                one(fma2(two(sc[j + 2], sc[j + 3]), sl22, nref2), p2, p3);
+                p0 = at_exp2(p0); p1 = at_exp2(p1); p2 = at_exp2(p2); p3 = at_exp2(p3);
+                sum01 = add2(sum01, two(p0, p1)); sum23 = add2(sum23, two(p2, p3));
+                pk[j >> 1] = pack_bf16x2(p0, p1);
+                pk[(j >> 1) + 1] = pack_bf16x2(p2, p3);
             }
+            float sum4[4];
+            one(sum01, sum4[0], sum4[1]); one(sum23, sum4[2], sum4[3]);
             const float sum = (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
             // P takes the place of this page's scores in tensor memory: 64 bfloat16 = 32 columns of this thread's lane, the
             // A operand of P V as they lie (no way through shared memory, no proxy fence, and nothing of the previous P V

@@ -159,13 +159,37 @@ __device__ __forceinline__ float at_exp2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// Weights are rounded to bfloat16 with integer arithmetic (add half an ulp, keep the upper 16 bits): the
+// (The latent attention's) weights are rounded to bfloat16 with integer arithmetic (add half an ulp, keep the upper 16 bits): the
 // conversion instruction shares the special-function unit with ex2.  Two variants that measured SLOWER here
 // and were dropped: a share of the exponentials as a polynomial on the FMA pipe (763 -> 734 TFLOP/s at 8,192
 // tokens), and two softmax threads per row (763 -> 435): the softmax warps lack neither ex2 throughput nor
 // threads; what helped was letting the next page's scores be computed while they work (see issue_s).
 __device__ __forceinline__ uint32_t at_pack_bf16x2(float a, float b) {      // a, b >= 0 and finite
     return __byte_perm(__float_as_uint(a) + 0x8000u, __float_as_uint(b) + 0x8000u, 0x7632);
+}
+
+// Two numbers in a pair of registers, worked on by one instruction (each as by its own: same roundings).
+typedef unsigned long long Two;
+__device__ __forceinline__ Two two(float a, float b) {
+    Two r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void one(Two t, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(t)); }
+__device__ __forceinline__ Two fma2(Two a, Two b, Two c) {
+    Two r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ Two add2(Two a, Two b) {
+    Two r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
 }
 
 __device__ __forceinline__ void tcgen05_st32(uint32_t taddr, const uint32_t* r) {
