@@ -318,7 +318,10 @@ int rf_delta_scan(const float* qn, const float* kn, const float* kq, const float
 //     o_t = (G_t o q_t)^T S0 + sum M_ts u_s,   S_end = diag(G_end) S0 + sum_s (P(s, end) o k_s) u_s^T
 // The solve kernel then walks, for every s, over t with k_s P(s, t) in registers (four lanes share s, 16 channels each at a time),
 // and leaves G o q and P(s, end) o k for the other two kernels, which are the same otherwise.  (16 heads of 128 x 128: 2,048 tokens
-// 669 us token by token, 301 in chunks; three prompts of 1,365, 900 and 513 697 and 421.)
+// 669 us token by token, 284 in chunks; three prompts of 1,365, 700 and 500 373.)
+// A warp's own stream of instructions bounds all three (issue slots 40 to 60 % busy), so they work on two numbers an instruction wherever
+// there is one, and the solve kernel on two tokens at a time (us, one number and one token at a time: 309 and 413; one decay per head,
+// 2,048 tokens 224, now 220).
 // Decays are multiplied on as running products, never divided by and never taken the logarithm of: 0 and 1 need no special case.
 // Everything is 32-bit.  The chunk table (built on the host with the step) is first[B+1] (index of each sequence's first
 // chunk), then (sequence, first row) per chunk.
@@ -409,33 +412,46 @@ delta_chunk_solve_kernel(const float* __restrict__ qn, const float* __restrict__
             chunk_tile(gs, ld, decay + g0 + d0, (size_t)H * D, p.cnt, nd, (D & 3) == 0, tid, 256);
             copies_done();
             __syncthreads();
-            float4 r[4];
+            ulonglong2 r[4];                          // k_s P(s, t): channels in pairs
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int e = 16 * i + 4 * q4;
-                r[i] = e < nd4 ? *reinterpret_cast<const float4*>(ks + sl * ld + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+                r[i] = e < nd4 ? *reinterpret_cast<const ulonglong2*>(ks + sl * ld + e) : make_ulonglong2(0ull, 0ull);
             }
-            for (int t = first; t < p.cnt; ++t) {
-                float da = 0.f, dm = 0.f;
-                const bool after = t > sl;
+            // two tokens at a time (rows from cnt on are zeros); their four sums over the lanes of s end in one lane each
+            for (int t = first; t < p.cnt; t += 2) {
+                Two sum[4][2];                        // A and M at t, A and M at t + 1
+#pragma unroll
+                for (int u = 0; u < 4; ++u) sum[u][0] = sum[u][1] = two(0.f, 0.f);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const int e = 16 * i + 4 * q4;
                     if (16 * i < nd4) {               // (whole warps; a lane beyond the last channel multiplies zeros)
                         const int f = e < nd4 ? e : 0;
-                        const float4 g = *reinterpret_cast<const float4*>(gs + t * ld + f), k = *reinterpret_cast<const float4*>(ks + t * ld + f);
-                        const float4 q = *reinterpret_cast<const float4*>(qs + t * ld + f);
-                        if (after) { r[i].x *= g.x; r[i].y *= g.y; r[i].z *= g.z; r[i].w *= g.w; }
-                        da = fmaf(r[i].x, k.x, fmaf(r[i].y, k.y, fmaf(r[i].z, k.z, fmaf(r[i].w, k.w, da))));
-                        dm = fmaf(r[i].x, q.x, fmaf(r[i].y, q.y, fmaf(r[i].z, q.z, fmaf(r[i].w, q.w, dm))));
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) {
+                            const ulonglong2 g = *reinterpret_cast<const ulonglong2*>(gs + (t + u) * ld + f);
+                            const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(ks + (t + u) * ld + f);
+                            const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(qs + (t + u) * ld + f);
+                            if (t + u > sl) { r[i].x = mul2(r[i].x, g.x); r[i].y = mul2(r[i].y, g.y); }
+                            sum[2 * u][0] = fma2(r[i].x, k.x, sum[2 * u][0]); sum[2 * u][1] = fma2(r[i].y, k.y, sum[2 * u][1]);
+                            sum[2 * u + 1][0] = fma2(r[i].x, q.x, sum[2 * u + 1][0]); sum[2 * u + 1][1] = fma2(r[i].y, q.y, sum[2 * u + 1][1]);
+                        }
                     }
                 }
-                da += __shfl_xor_sync(0xffffffffu, da, 1); dm += __shfl_xor_sync(0xffffffffu, dm, 1);
-                da += __shfl_xor_sync(0xffffffffu, da, 2); dm += __shfl_xor_sync(0xffffffffu, dm, 2);
-                if (q4 == 0 && t >= sl) {
-                    if (after) at[sl * DC_LD + t] += da;
-                    ps[sl * DC_LD + t] += dm;
+                float d[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    float x, y;
+                    one(add2(sum[u][0], sum[u][1]), x, y);
+                    d[u] = x + y;
                 }
+                const bool up = q4 & 1, high = q4 & 2;
+                const float e0 = (up ? d[1] : d[0]) + __shfl_xor_sync(0xffffffffu, up ? d[0] : d[1], 1);
+                const float e1 = (up ? d[3] : d[2]) + __shfl_xor_sync(0xffffffffu, up ? d[2] : d[3], 1);
+                const float mine = (high ? e1 : e0) + __shfl_xor_sync(0xffffffffu, high ? e0 : e1, 2);
+                const int tm = t + (high ? 1 : 0);    // lane q4 holds A (even) or M of token t + q4 / 2
+                if (up ? tm >= sl : tm > sl) (up ? ps : at)[sl * DC_LD + tm] += mine;
             }
             // a thread per channel: G_t o q_t and G_end going forward, P(s, end) o k_s going back
             const int d = d0 + (tid & 63);
@@ -574,26 +590,41 @@ delta_chunk_solve_kernel(const float* __restrict__ qn, const float* __restrict__
                     for (int r = 0; r < 16; ++r) x[r] = next[r] * (is_v ? live * sb[t0 + r] : sb[t0 + r] * sG[t0 + r]);
                 }
                 if (t0 + 16 < p.cnt) ask(t0 + 16);
-                for (int s = 0; s < t0; ++s) {
-                    const float xs = X[s * DC_COLS + tid];
+                Two x2[8];                            // rows in pairs
 #pragma unroll
-                    for (int r = 0; r < 16; r += 4) {
-                        const float4 av = *reinterpret_cast<const float4*>(at + s * DC_LD + t0 + r);
-                        x[r] = fmaf(-av.x, xs, x[r]); x[r + 1] = fmaf(-av.y, xs, x[r + 1]);
-                        x[r + 2] = fmaf(-av.z, xs, x[r + 2]); x[r + 3] = fmaf(-av.w, xs, x[r + 3]);
+                for (int r = 0; r < 8; ++r) x2[r] = two(x[2 * r], x[2 * r + 1]);
+                for (int s = 0; s < t0; ++s) {
+                    const float xs = -X[s * DC_COLS + tid];
+                    const Two xx = two(xs, xs);
+#pragma unroll
+                    for (int r = 0; r < 8; r += 2) {
+                        const ulonglong2 av = *reinterpret_cast<const ulonglong2*>(at + s * DC_LD + t0 + 2 * r);
+                        x2[r] = fma2(av.x, xx, x2[r]); x2[r + 1] = fma2(av.y, xx, x2[r + 1]);
                     }
                 }
 #pragma unroll
                 for (int s = 0; s < 15; ++s) {
-                    float av[16];
+                    Two av[8];
 #pragma unroll
-                    for (int r = (s + 1) & ~3; r < 16; r += 4) {
-                        const float4 f = *reinterpret_cast<const float4*>(at + (t0 + s) * DC_LD + t0 + r);
-                        av[r] = f.x; av[r + 1] = f.y; av[r + 2] = f.z; av[r + 3] = f.w;
+                    for (int r = (s + 1) / 4 * 2; r < 8; r += 2) {
+                        const ulonglong2 f = *reinterpret_cast<const ulonglong2*>(at + (t0 + s) * DC_LD + t0 + 2 * r);
+                        av[r] = f.x; av[r + 1] = f.y;
                     }
+                    float lo, hi;
+                    one(x2[s / 2], lo, hi);
+                    if (s % 2 == 0) {                 // the pair's other row still wants this one
+                        float a0, a1;
+                        one(av[s / 2], a0, a1);
+                        hi = fmaf(-a1, lo, hi);
+                        x2[s / 2] = two(lo, hi);
+                    }
+                    const float xs = s % 2 == 0 ? -lo : -hi;
+                    const Two xx = two(xs, xs);
 #pragma unroll
-                    for (int r = s + 1; r < 16; ++r) x[r] = fmaf(-av[r], x[s], x[r]);
+                    for (int r = s / 2 + 1; r < 8; ++r) x2[r] = fma2(av[r], xx, x2[r]);
                 }
+#pragma unroll
+                for (int r = 0; r < 8; ++r) one(x2[r], x[2 * r], x[2 * r + 1]);
 #pragma unroll
                 for (int r = 0; r < 16; ++r) X[(t0 + r) * DC_COLS + tid] = x[r];
                 if (is_v) {
@@ -716,20 +747,26 @@ delta_chunk_carry_kernel(const float* __restrict__ Kc, const float* __restrict__
                             if (cc + u < nc) ls[(size_t)d * V + u] = s[i][r][u];
                 }
         }
-        float acc[8][4];
+        Two acc2[4][4];                                   // rows in pairs
 #pragma unroll
-        for (int r = 0; r < 8; ++r) { acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f; }
+        for (int r = 0; r < 4; ++r) acc2[r][0] = acc2[r][1] = acc2[r][2] = acc2[r][3] = two(0.f, 0.f);
 #pragma unroll 4
         for (int d = d0; d < d1; ++d) {
-            const float4 w0 = *reinterpret_cast<const float4*>(w + d * DC + rg), w1 = *reinterpret_cast<const float4*>(w + d * DC + 32 + rg);
+            const ulonglong2 w0 = *reinterpret_cast<const ulonglong2*>(w + d * DC + rg), w1 = *reinterpret_cast<const ulonglong2*>(w + d * DC + 32 + rg);
             const float4 sv = *reinterpret_cast<const float4*>(Ss + d * DV + cg);
-            const float wr[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+            const Two wr[4] = {w0.x, w0.y, w1.x, w1.y};
+            const Two s0 = two(sv.x, sv.x), s1 = two(sv.y, sv.y), s2 = two(sv.z, sv.z), s3 = two(sv.w, sv.w);
 #pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                acc[r][0] = fmaf(wr[r], sv.x, acc[r][0]); acc[r][1] = fmaf(wr[r], sv.y, acc[r][1]);
-                acc[r][2] = fmaf(wr[r], sv.z, acc[r][2]); acc[r][3] = fmaf(wr[r], sv.w, acc[r][3]);
+            for (int r = 0; r < 4; ++r) {
+                acc2[r][0] = fma2(wr[r], s0, acc2[r][0]); acc2[r][1] = fma2(wr[r], s1, acc2[r][1]);
+                acc2[r][2] = fma2(wr[r], s2, acc2[r][2]); acc2[r][3] = fma2(wr[r], s3, acc2[r][3]);
             }
         }
+        float acc[8][4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) one(acc2[r][u], acc[2 * r][u], acc[2 * r + 1][u]);
         // a row's place in red leaves a gap of one row after every four: the warp's 16-byte stores then spread over all banks
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
@@ -767,17 +804,23 @@ delta_chunk_carry_kernel(const float* __restrict__ Kc, const float* __restrict__
             for (int r = 0; r < 4; ++r) { x[i][r][0] = x[i][r][1] = x[i][r][2] = x[i][r][3] = 0.f; }
             if (d < KD) {
                 const int t0 = owner ? 0 : DC / 2;
+                Two x2[2][4];
+#pragma unroll
+                for (int r = 0; r < 2; ++r) x2[r][0] = x2[r][1] = x2[r][2] = x2[r][3] = two(0.f, 0.f);
 #pragma unroll 8
                 for (int t = t0; t < t0 + DC / 2; ++t) {
-                    const float4 kk = *reinterpret_cast<const float4*>(k + t * KD + d);
+                    const ulonglong2 kk = *reinterpret_cast<const ulonglong2*>(k + t * KD + d);
                     const float4 uu = *reinterpret_cast<const float4*>(Us + t * DV + cc);
-                    const float kv[4] = {kk.x, kk.y, kk.z, kk.w};
-#pragma unroll
-                    for (int r = 0; r < 4; ++r) {
-                        x[i][r][0] = fmaf(kv[r], uu.x, x[i][r][0]); x[i][r][1] = fmaf(kv[r], uu.y, x[i][r][1]);
-                        x[i][r][2] = fmaf(kv[r], uu.z, x[i][r][2]); x[i][r][3] = fmaf(kv[r], uu.w, x[i][r][3]);
-                    }
+                    const Two u0 = two(uu.x, uu.x), u1 = two(uu.y, uu.y), u2 = two(uu.z, uu.z), u3 = two(uu.w, uu.w);
+                    x2[0][0] = fma2(kk.x, u0, x2[0][0]); x2[0][1] = fma2(kk.x, u1, x2[0][1]);
+                    x2[0][2] = fma2(kk.x, u2, x2[0][2]); x2[0][3] = fma2(kk.x, u3, x2[0][3]);
+                    x2[1][0] = fma2(kk.y, u0, x2[1][0]); x2[1][1] = fma2(kk.y, u1, x2[1][1]);
+                    x2[1][2] = fma2(kk.y, u2, x2[1][2]); x2[1][3] = fma2(kk.y, u3, x2[1][3]);
                 }
+#pragma unroll
+                for (int r = 0; r < 2; ++r)
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) one(x2[r][u], x[i][2 * r][u], x[i][2 * r + 1][u]);
                 if (!owner)                               // (the shares of W S are used up: their place takes these sums)
 #pragma unroll
                     for (int r = 0; r < 4; ++r)
@@ -849,40 +892,42 @@ delta_chunk_out_kernel(const float* __restrict__ qn, const float* __restrict__ M
     copies_done();
     __syncthreads();
     const int tx = tid & 15, ty = tid >> 4;
-    float a[4][4], e[4][4];
+    Two a2[4][2], e2[4][2];                            // columns in pairs
 #pragma unroll
-    for (int x = 0; x < 4; ++x)
-#pragma unroll
-        for (int y = 0; y < 4; ++y) { a[x][y] = 0.f; e[x][y] = 0.f; }
+    for (int x = 0; x < 4; ++x) a2[x][0] = a2[x][1] = e2[x][0] = e2[x][1] = two(0.f, 0.f);
     // four inner positions i .. i + 3 for the rows x >= x0: 4 (4 - x0) + 16 loads' worth of FMAs
-    auto block = [&](float (&acc)[4][4], int i, auto x0) {
-        float4 r[4];
+    auto block = [&](Two (&acc)[4][2], int i, auto x0) {
+        ulonglong2 r[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) r[q] = *reinterpret_cast<const float4*>(rhs + (i + q) * DO + 4 * tx);
+        for (int q = 0; q < 4; ++q) r[q] = *reinterpret_cast<const ulonglong2*>(rhs + (i + q) * DO + 4 * tx);
 #pragma unroll
         for (int x = decltype(x0)::value; x < 4; ++x) {
             const float4 l = *reinterpret_cast<const float4*>(lhs + (ty + 16 * x) * ld + i);
-            acc[x][0] = fmaf(l.x, r[0].x, acc[x][0]); acc[x][1] = fmaf(l.x, r[0].y, acc[x][1]); acc[x][2] = fmaf(l.x, r[0].z, acc[x][2]); acc[x][3] = fmaf(l.x, r[0].w, acc[x][3]);
-            acc[x][0] = fmaf(l.y, r[1].x, acc[x][0]); acc[x][1] = fmaf(l.y, r[1].y, acc[x][1]); acc[x][2] = fmaf(l.y, r[1].z, acc[x][2]); acc[x][3] = fmaf(l.y, r[1].w, acc[x][3]);
-            acc[x][0] = fmaf(l.z, r[2].x, acc[x][0]); acc[x][1] = fmaf(l.z, r[2].y, acc[x][1]); acc[x][2] = fmaf(l.z, r[2].z, acc[x][2]); acc[x][3] = fmaf(l.z, r[2].w, acc[x][3]);
-            acc[x][0] = fmaf(l.w, r[3].x, acc[x][0]); acc[x][1] = fmaf(l.w, r[3].y, acc[x][1]); acc[x][2] = fmaf(l.w, r[3].z, acc[x][2]); acc[x][3] = fmaf(l.w, r[3].w, acc[x][3]);
+            const Two l0 = two(l.x, l.x), l1 = two(l.y, l.y), l2 = two(l.z, l.z), l3 = two(l.w, l.w);
+            acc[x][0] = fma2(l0, r[0].x, acc[x][0]); acc[x][1] = fma2(l0, r[0].y, acc[x][1]);
+            acc[x][0] = fma2(l1, r[1].x, acc[x][0]); acc[x][1] = fma2(l1, r[1].y, acc[x][1]);
+            acc[x][0] = fma2(l2, r[2].x, acc[x][0]); acc[x][1] = fma2(l2, r[2].y, acc[x][1]);
+            acc[x][0] = fma2(l3, r[3].x, acc[x][0]); acc[x][1] = fma2(l3, r[3].y, acc[x][1]);
         }
     };
     // the scores of tokens s in 16 y .. 16 y + 15 are zero for the rows x < y
-    for (int i = 0; i < 16; i += 4) block(a, i, std::integral_constant<int, 0>{});
-    for (int i = 16; i < 32; i += 4) block(a, i, std::integral_constant<int, 1>{});
-    for (int i = 32; i < 48; i += 4) block(a, i, std::integral_constant<int, 2>{});
-    for (int i = 48; i < 64; i += 4) block(a, i, std::integral_constant<int, 3>{});
-    for (int i = DC; i < DC + D4; i += 4) block(e, i, std::integral_constant<int, 0>{});
+    for (int i = 0; i < 16; i += 4) block(a2, i, std::integral_constant<int, 0>{});
+    for (int i = 16; i < 32; i += 4) block(a2, i, std::integral_constant<int, 1>{});
+    for (int i = 32; i < 48; i += 4) block(a2, i, std::integral_constant<int, 2>{});
+    for (int i = 48; i < 64; i += 4) block(a2, i, std::integral_constant<int, 3>{});
+    for (int i = DC; i < DC + D4; i += 4) block(e2, i, std::integral_constant<int, 0>{});
 #pragma unroll
     for (int x = 0; x < 4; ++x) {
         const int t = ty + 16 * x;
         if (t >= p.cnt) continue;
+        float a[4], e[4];
+#pragma unroll
+        for (int y = 0; y < 2; ++y) { one(a2[x][y], a[2 * y], a[2 * y + 1]); one(e2[x][y], e[2 * y], e[2 * y + 1]); }
         float* out = o + (size_t)(p.row0 + t) * H * V + h * V + j0 + 4 * tx;
         const float g = sG[t];
 #pragma unroll
         for (int y = 0; y < 4; ++y)
-            if (4 * tx + y < nc) out[y] = fmaf(g, e[x][y], a[x][y]);
+            if (4 * tx + y < nc) out[y] = fmaf(g, e[y], a[y]);
     }
 }
 
