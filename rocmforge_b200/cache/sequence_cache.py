@@ -18,6 +18,8 @@ from typing import Dict, List, Optional, Sequence
 import numpy as np
 import torch
 
+from ..kernels._ffi import record
+
 from .pages import CacheError, FreeList
 from .requests import KVRequest, StateRequest
 
@@ -129,19 +131,26 @@ class KVGroup:
         if not self._dirty:
             return
         if self.table_dev.is_cuda:
-            n = sum(hi - lo for lo, hi in self._dirty.values())
-            if self._upload_done is not None:
+            # the changed entries and what lies between them in one copy, unless that is far more than they are
+            W = self.max_pages_per_seq
+            spans = [(slot * W + lo, slot * W + hi) for slot, (lo, hi) in self._dirty.items()]
+            first, last = min(a for a, _ in spans), max(b for _, b in spans)
+            if last - first <= 4096 + 4 * sum(b - a for a, b in spans):
+                spans = [(first, last)]
+            n = sum(b - a for a, b in spans)
+            if self._upload_done is None:
+                self._upload_done = torch.cuda.Event()
+            else:
                 self._upload_done.synchronize()         # the staging buffer may still be read
             if self._staging is None or self._staging.numel() < n:
                 self._staging = torch.empty((max(n, 1024),), dtype=torch.int32).pin_memory()
-            off = 0
-            for slot, (lo, hi) in self._dirty.items():
-                k = hi - lo
-                self._staging[off:off + k] = torch.from_numpy(self.table[slot, lo:hi])
-                self.table_dev[slot, lo:hi].copy_(self._staging[off:off + k], non_blocking=True)
+            host, device, off = self.table.reshape(-1), self.table_dev.view(-1), 0
+            for a, b in spans:
+                k = b - a
+                self._staging[off:off + k] = torch.from_numpy(host[a:b])
+                device[a:b].copy_(self._staging[off:off + k], non_blocking=True)
                 off += k
-            self._upload_done = torch.cuda.Event()
-            self._upload_done.record()
+            record(self._upload_done)
         else:
             for slot, (lo, hi) in self._dirty.items():
                 self.table_dev[slot, lo:hi] = torch.from_numpy(self.table[slot, lo:hi].copy())

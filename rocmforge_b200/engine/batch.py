@@ -15,6 +15,8 @@ from typing import List, Optional, Sequence
 import numpy as np
 import torch
 
+from ..kernels._ffi import record
+
 
 class BatchError(ValueError):
     pass
@@ -126,6 +128,7 @@ class DeviceDescriptor:
                 self._done = torch.cuda.Event()
         self._pinned_np = self.pinned.numpy()          # the same memory, written without a tensor per call
         self._slices = {}                              # n -> (device slice, pinned slice)
+        self._views = {}                               # arguments of ``views`` -> what it returned, for decode steps
         self._busy = False
 
     def upload(self, packed: np.ndarray) -> None:
@@ -145,9 +148,17 @@ class DeviceDescriptor:
             pair = self._slices[n] = (self.dev[:n], self.pinned[:n])
         pair[0].copy_(pair[1], non_blocking=True)
         if self._done is not None:
-            self._done.record()
+            record(self._done)
             self._busy = True
 
     def views(self, T: int, B: int, R: int, extras=(), decode_extras: bool = False):
-        lay, _ = StepBatch.layout(T, B, R, extras, decode_extras)
-        return {name: self.dev[o:o + n] for name, (o, n) in lay.items()}
+        key = (T, B, R, extras, decode_extras)
+        got = self._views.get(key)
+        if got is None:
+            lay, _ = StepBatch.layout(T, B, R, extras, decode_extras)
+            got = {name: self.dev[o:o + n] for name, (o, n) in lay.items()}
+            if T == B:                                 # a decode step's: prompts' sizes hardly ever come again
+                if len(self._views) >= 64:
+                    self._views.clear()
+                self._views[key] = got
+        return got

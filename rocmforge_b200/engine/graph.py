@@ -17,6 +17,7 @@ import torch
 import numpy as np
 
 from ..cache import CacheError
+from ..kernels._ffi import record
 from .batch import BatchError, DeviceDescriptor, StepBatch, StepRequest
 from .context import StepContext
 
@@ -264,7 +265,7 @@ class DecodeRunner:
         self.replays += 1
         pinned, host, event = self._pinned(B)
         pinned[:B].copy_(cap.ids, non_blocking=True)
-        event.record()
+        record(event)
         return dict(slots=list(slots), gens=[self.cache.generation(s) for s in slots], starts=list(starts), cap=cap,
                     host=host, event=event, sampling=sampling, requests=list(requests), draws=list(draws), B=B)
 

@@ -7,6 +7,7 @@ import torch
 
 from .. import kernels
 from ..cache import pages_for
+from ..kernels._ffi import record
 from ..sampling import DeviceSampler, SamplingParams
 from .batch import StepRequest
 from .generate import StepEngine
@@ -50,7 +51,7 @@ class ModelEngine(StepEngine):
             self._host_np = self._host_ids.numpy()
             self._host_done = torch.cuda.Event()
         self._host_ids[:n].copy_(out.reshape(-1), non_blocking=True)
-        self._host_done.record()
+        record(self._host_done)
         self._host_done.synchronize()
         return self._host_np[:n].tolist()
 

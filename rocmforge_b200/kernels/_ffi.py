@@ -44,20 +44,40 @@ def dtype_code(dt: torch.dtype) -> int:
     raise KernelError(f"compute dtype {dt} is not supported (float32 or bfloat16)")
 
 
-def ptr(t) -> c_void_p:
-    return c_void_p(0) if t is None else c_void_p(t.data_ptr())
+def ptr(t):
+    """The address of a tensor's data for a launcher's pointer argument (None: null)."""
+    return None if t is None else t.data_ptr()
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_device = getattr(torch._C, "_cuda_getDevice", None)
 
 
-def stream() -> c_void_p:
+def stream() -> int:
     """torch's current stream of the current device as a raw handle.  Asked at every launch (the current
     stream changes under ``torch.cuda.stream`` and during graph capture), so through the cheapest call there is:
     ``torch.cuda.current_stream()`` builds a Stream object and costs about 15 us, a third of a launch's host time."""
-    if _raw_stream is not None:
-        return c_void_p(_raw_stream(torch.cuda.current_device()))
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    if _raw_stream is not None and _device is not None:
+        return _raw_stream(_device())
+    return torch.cuda.current_stream().cuda_stream
+
+
+_streams = {}
+
+
+def record(event) -> None:
+    """``event.record()`` on the current stream, without a Stream object built for it where one of that stream is at hand."""
+    if _raw_stream is None or _device is None:
+        event.record()
+        return
+    dev = _device()
+    key = (dev, _raw_stream(dev))
+    s = _streams.get(key)
+    if s is None:
+        if len(_streams) >= 64:
+            _streams.clear()
+        s = _streams[key] = torch.cuda.current_stream()
+    event.record(s)
 
 
 def need_cuda(*tensors) -> None:

@@ -6,6 +6,7 @@ from typing import Optional, Sequence
 import torch
 
 from .. import kernels
+from ..kernels._ffi import record
 from .params import SamplingParams, as_int64, draw_seed
 
 
@@ -37,7 +38,7 @@ class DeviceSampler:
         self._pinned_np[:n] = values
         self._dev[:n].copy_(self._pinned[:n], non_blocking=True)
         if self._copied is not None:
-            self._copied.record()
+            record(self._copied)
             self._busy = True
         return self._dev[:n]
 
