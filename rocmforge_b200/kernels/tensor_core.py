@@ -224,7 +224,9 @@ def gemm_tc_grouped(x: torch.Tensor, w: torch.Tensor, tiles: torch.Tensor, max_t
 
 def split_k_for(N: int, K: int, sm_count: Optional[int] = None, tokens: Optional[int] = None) -> int:
     """K splits of a skinny product, from N and K (never from the batch's content), so that about two CTAs per SM stream
-    the weight and every split keeps at least 4 blocks of 64.  ``tokens``: a step of at most 16 tokens fits three CTAs on an
+    the weight and every split keeps at least 4 blocks of 64, of a K of at most 16 blocks 8 / 3 (the products of 14 blocks of the
+    0.5B shape in 3, 4, 5, 7 splits, a decode step, us: batch 1 676, 645, 629, 624, batch 16 723, 677, 662, 666, batch 64 922, 880, 862,
+    864; longer K in finer splits gains nothing, K of 2,048 in 8, 10, 12: Ludusun batch 8 275, 275, 281).  ``tokens``: a step of at most 16 tokens fits three CTAs on an
     SM, and a weight with long K ranges is then cut for three per SM (splits of at least 16 blocks; the down projection of
     the 7B shape 10 -> 15: a decode step at batch 8 2.624 -> 2.603 ms, at batch 1 2.560 -> 2.530 ms; with 32 or 64 tokens,
     two CTAs per SM, the same cut costs 0.16 ms).  The short K ranges of q|k|v and o gain nothing from more splits."""
@@ -234,7 +236,7 @@ def split_k_for(N: int, K: int, sm_count: Optional[int] = None, tokens: Optional
     if tiles >= 2 * sm_count or kb < 8:
         return 1
     want = max(1, (2 * sm_count) // tiles)
-    splits = max(1, min(want, kb // 4))
+    splits = max(1, min(want, kb // 4 if kb > 16 else kb * 3 // 8))
     if tokens is not None and tokens <= 16:
         splits = max(splits, min((3 * sm_count) // tiles, kb // 16))
     per = (kb + splits - 1) // splits
