@@ -316,9 +316,11 @@ int rf_delta_scan(const float* qn, const float* kn, const float* kq, const float
 // With a decay per key channel (PC = true) P and G are vectors over the channels and stay inside the products over them:
 //     A_ts = beta_t sum_d k_s P_d(s, t) k_t,  M_ts likewise with q_t,  (1 + A) W = diag(beta) (G o K),
 //     o_t = (G_t o q_t)^T S0 + sum M_ts u_s,   S_end = diag(G_end) S0 + sum_s (P(s, end) o k_s) u_s^T
-// The solve kernel then walks, for every s, over t with k_s P(s, t) in registers (four lanes share s, 16 channels each at a time),
-// and leaves G o q and P(s, end) o k for the other two kernels, which are the same otherwise.  (16 heads of 128 x 128: 2,048 tokens
-// 669 us token by token, 284 in chunks; three prompts of 1,365, 700 and 500 373.)
+// The solve kernel then takes the tokens in blocks of 16.  Inside a block it walks, for every s, over t with k_s P(s, t) in registers
+// (four lanes share s, 16 channels each at a time).  Between two blocks P(s, t) is the product from s to its block's end, times that of
+// the whole blocks between, times that from t's block's start to t: keys and queries are scaled so once, and what remains are plain
+// products over the channels.  It leaves G o q and P(s, end) o k for the other two kernels, which are the same otherwise.  (16 heads of 128 x 128: 2,048 tokens
+// 669 us token by token, 250 in chunks; three prompts of 1,365, 700 and 500 321; walking over all later tokens, not a block's, 284, 370.)
 // A warp's own stream of instructions bounds all three (issue slots 40 to 60 % busy), so they work on two numbers an instruction wherever
 // there is one, and the solve kernel on two tokens at a time (us, one number and one token at a time: 309 and 413; one decay per head,
 // 2,048 tokens 224, now 220).
@@ -383,6 +385,7 @@ delta_chunk_solve_kernel(const float* __restrict__ qn, const float* __restrict__
     float* X = sh;
     float* at = sh + region;                          // [64 s][DC_LD]: A_ts, zeros for s >= t
     float* ps = at + DC * DC_LD;                      // [64 s][DC_PLD]: P(s, t) for the tokens t >= s of s's own block of 16 (PC: [64 s][DC_LD], M_ts)
+    __shared__ __align__(16) float between_blocks[PC ? 3 : 1][PC ? DC : 1];   // PC: products of the decays of blocks 1, 2, and both
     __shared__ float sg[DC], sb[DC], sG[DC], sF[DC];  // g, beta, G, and the products from a block's first token on
     pdl_trigger();
     const int c = blockIdx.x, h = blockIdx.y, hg = h / (H / G), tid = threadIdx.x;
@@ -404,6 +407,14 @@ delta_chunk_solve_kernel(const float* __restrict__ qn, const float* __restrict__
         float* go = gw + ((size_t)c * H + h) * D4;
         for (int i = tid; i < DC * DC_LD; i += 256) { at[i] = 0.f; ps[i] = 0.f; }
         const int sl = tid >> 2, q4 = tid & 3, first = (tid >> 5) * 8;          // this lane's s, its share of the channels, the warp's first s
+        // between blocks: thread (four tokens s, tokens t and t + 8), 16, 32 and 48 tokens s for the second, third and fourth block of t
+        float* ends = gs + DC * ld;                   // [48][ld]
+        const int group = tid >> 3, j_at = group < 4 ? 1 : group < 12 ? 2 : 3, s_at = 4 * (group - (j_at == 1 ? 0 : j_at == 2 ? 4 : 12));
+        const int t_at = 16 * j_at + (tid & 7), apart = j_at - (s_at >> 4);
+        const int gap = apart == 1 ? -1 : apart == 3 ? 2 : (s_at >> 4);          // the blocks between: none, both, or the one after s's
+        Two fa[4][2], fm[4][2];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) fa[x][0] = fa[x][1] = fm[x][0] = fm[x][1] = two(0.f, 0.f);
         for (int d0 = 0; d0 < D; d0 += DC) {          // 64 channels at a time
             const int nd = min(DC, D - d0), nd4 = (nd + 3) & ~3;
             __syncthreads();                          // the channels before are used up (and at, ps are zero)
@@ -418,8 +429,9 @@ delta_chunk_solve_kernel(const float* __restrict__ qn, const float* __restrict__
                 const int e = 16 * i + 4 * q4;
                 r[i] = e < nd4 ? *reinterpret_cast<const ulonglong2*>(ks + sl * ld + e) : make_ulonglong2(0ull, 0ull);
             }
-            // two tokens at a time (rows from cnt on are zeros); their four sums over the lanes of s end in one lane each
-            for (int t = first; t < p.cnt; t += 2) {
+            // inside s's block: two tokens at a time (rows from cnt on are zeros); their four sums over the lanes of s end in one lane each
+            const int block_end = min(p.cnt, (first & ~15) + 16);
+            for (int t = first; t < block_end; t += 2) {
                 Two sum[4][2];                        // A and M at t, A and M at t + 1
 #pragma unroll
                 for (int u = 0; u < 4; ++u) sum[u][0] = sum[u][1] = two(0.f, 0.f);
@@ -453,6 +465,13 @@ delta_chunk_solve_kernel(const float* __restrict__ qn, const float* __restrict__
                 const int tm = t + (high ? 1 : 0);    // lane q4 holds A (even) or M of token t + q4 / 2
                 if (up ? tm >= sl : tm > sl) (up ? ps : at)[sl * DC_LD + tm] += mine;
             }
+            // k_s P(s, its block's end), of the blocks that others follow
+            if (sl < 48)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int e = 16 * i + 4 * q4;
+                    if (e < nd4) *reinterpret_cast<ulonglong2*>(ends + sl * ld + e) = r[i];
+                }
             // a thread per channel: G_t o q_t and G_end going forward, P(s, end) o k_s going back
             const int d = d0 + (tid & 63);
             if (tid < 64 && d < D) {
@@ -471,7 +490,54 @@ delta_chunk_solve_kernel(const float* __restrict__ qn, const float* __restrict__
                 }
                 if (d >= D) go[d] = 0.f;
             }
+                    __syncthreads();                          // keys, queries and decays have been read as they are
+            if (tid < 192) {                          // a thread per channel and block after the first: k_t and q_t times the decays from its start
+                const int j = 1 + (tid >> 6), e = tid & 63;
+                float run = 1.f;
+#pragma unroll
+                for (int t = 16 * j; t < 16 * j + 16; ++t) {
+                    run *= gs[t * ld + e];
+                    ks[t * ld + e] *= run;
+                    qs[t * ld + e] *= run;
+                }
+                if (j < 3) between_blocks[j - 1][e] = run;
+            }
+            __syncthreads();
+            if (tid < 64) between_blocks[2][tid] = between_blocks[0][tid] * between_blocks[1][tid];
+            __syncthreads();
+            if (tid < 192)
+                for (int e = 0; e < nd4; e += 4) {
+                    ulonglong2 l[4];
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) l[x] = *reinterpret_cast<const ulonglong2*>(ends + (s_at + x) * ld + e);
+                    if (gap >= 0) {
+                        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(&between_blocks[gap][e]);
+#pragma unroll
+                        for (int x = 0; x < 4; ++x) { l[x].x = mul2(l[x].x, w.x); l[x].y = mul2(l[x].y, w.y); }
+                    }
+#pragma unroll
+                    for (int y = 0; y < 2; ++y) {
+                        const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(ks + (t_at + 8 * y) * ld + e);
+                        const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(qs + (t_at + 8 * y) * ld + e);
+#pragma unroll
+                        for (int x = 0; x < 4; ++x) {
+                            fa[x][y] = fma2(l[x].y, k.y, fma2(l[x].x, k.x, fa[x][y]));
+                            fm[x][y] = fma2(l[x].y, q.y, fma2(l[x].x, q.x, fm[x][y]));
+                        }
+                    }
+                }
         }
+        if (tid < 192)
+#pragma unroll
+            for (int x = 0; x < 4; ++x)
+#pragma unroll
+                for (int y = 0; y < 2; ++y) {
+                    float lo, hi;
+                    one(fa[x][y], lo, hi);
+                    at[(s_at + x) * DC_LD + t_at + 8 * y] = lo + hi;
+                    one(fm[x][y], lo, hi);
+                    ps[(s_at + x) * DC_LD + t_at + 8 * y] = lo + hi;
+                }
         __syncthreads();
         for (int i = tid; i < DC * DC; i += 256) {
             Mo[i] = ps[(i & 63) * DC_LD + (i >> 6)];
@@ -975,7 +1041,7 @@ static int delta_chunked(const float* qn, const float* kn, const float* decay, c
     float* Qg = Kc + (PC ? ch : (size_t)pass * G) * DC * D4;
     float* U = Qg + (PC ? ch * DC * D4 : 0);
     float* LS = U + ch * DC * V;
-    int region = PC ? 3 * DC * DC_LD : 2 * DC * (D4 + 4);
+    int region = PC ? (3 * DC + 48) * DC_LD : 2 * DC * (D4 + 4);
     if (region < DC * DC_COLS) region = DC * DC_COLS;
     const size_t smem1 = ((size_t)region + DC * DC_LD + DC * (PC ? DC_LD : DC_PLD)) * sizeof(float);
     const int tiles = D4 <= 128 ? 1 : 2;
