@@ -855,7 +855,10 @@ __device__ __forceinline__ float head_square_sum(const float (&x)[E], const floa
 // all), keys and values of one size: a warp holds a head in registers, E neighbouring elements of each half a lane, so that a pair's
 // two elements meet in one lane; the sines and cosines of a block's tokens are formed once, in shared memory, before the wait for the
 // product.  (Element by element through shared memory, every head with the trigonometry of its own: 2,778 tokens of 20 heads of 128
-// unrotated 23 us, of 24 rotated and normed 33; now 12 and 15.)  What rmsnorm_rows_kernel says about __restrict__ holds for src.
+// unrotated 23 us, of 24 rotated and normed 33.)  A token a
+// block, two from 2,048 on, and two heads a warp in flight; us, with up to four tokens a block and one head: 2,778 tokens of 20 heads of
+// 128 15.1 and 21.0, 2,565 of 24 rotated 17.2 and 25.6, 1,301 of 32 heads of 64 10.4 and 18.7, 700 of 24 8.3 and 9.4, 8,192 43.1 and 42.7
+// (four tokens 43.8).  The last tokens come first, as in the norm of many rows.  What rmsnorm_rows_kernel says about __restrict__ holds for src.
 template <typename T, int E>
 __global__ void __launch_bounds__(256)
 head_norm_rows_kernel(const T* src, int row_stride, T* q_out, int q_out_stride, int nh, int nkv, const float* __restrict__ inv_freq,
@@ -865,11 +868,11 @@ head_norm_rows_kernel(const T* src, int row_stride, T* q_out, int q_out_stride, 
                       HeadWriteExtras ex, int T_, int TB) {
     constexpr int HD = 64 * E, HALF = 32 * E;
     struct alignas(E * sizeof(T)) Piece { T v[E]; };
-    __shared__ float2 turn[4][HALF];                 // (cosine, sine) times the magnitude
-    __shared__ size_t page_at[4];
-    __shared__ float temp[4];
+    __shared__ float2 turn[2][HALF];                 // (cosine, sine) times the magnitude
+    __shared__ size_t page_at[2];
+    __shared__ float temp[2];
     pdl_trigger();
-    const int t0 = blockIdx.x * TB, n_tok = min(TB, T_ - t0), lane = threadIdx.x & 31;
+    const int t0 = (gridDim.x - 1 - blockIdx.x) * TB, n_tok = min(TB, T_ - t0), lane = threadIdx.x & 31;      // the last tokens first
     if (threadIdx.x < n_tok) {
         const int t = t0 + threadIdx.x, pos = tok_pos[t];
         if (write_kv) page_at[threadIdx.x] = ((size_t)block_table[(size_t)seq_slot[tok_seq[t]] * max_pages + pos / RF_PAGE] * nkv * RF_PAGE + pos % RF_PAGE) * HD;
@@ -884,11 +887,22 @@ head_norm_rows_kernel(const T* src, int row_stride, T* q_out, int q_out_stride, 
     __syncthreads();
     pdl_wait();
     const int heads = write_kv ? nh + (ex.v_is_k ? 1 : 2) * nkv : nh;
-    for (int i = threadIdx.x >> 5; i < n_tok * heads; i += 8) {
-        const int t = i / heads, head = i - t * heads;
-        const bool is_v = head >= nh + nkv;
+    constexpr int N = 2;                                 // heads of a warp in flight
+    for (int i0 = threadIdx.x >> 5; i0 < n_tok * heads; i0 += 8 * N) {
+    Piece first[N], second[N];
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+        const int i = min(i0 + 8 * n, n_tok * heads - 1), t = i / heads, head = i - t * heads;
         const T* from = src + (size_t)(t0 + t) * row_stride + (size_t)head * HD + lane * E;
-        const Piece a = *reinterpret_cast<const Piece*>(from), b = *reinterpret_cast<const Piece*>(from + HALF);
+        first[n] = *reinterpret_cast<const Piece*>(from);
+        second[n] = *reinterpret_cast<const Piece*>(from + HALF);
+    }
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+        const int i = i0 + 8 * n, t = i / heads, head = i - t * heads;
+        if (i >= n_tok * heads) continue;
+        const bool is_v = head >= nh + nkv;
+        const Piece a = first[n], b = second[n];
         float x[E], y[E];
 #pragma unroll
         for (int j = 0; j < E; ++j) {
@@ -934,6 +948,7 @@ head_norm_rows_kernel(const T* src, int row_stride, T* q_out, int q_out_stride, 
         for (int j = 0; j < E; ++j) { c.v[j] = Cvt<T>::from_f32(x[j] * scale); d.v[j] = Cvt<T>::from_f32(y[j] * scale); }
         *reinterpret_cast<Piece*>(dst) = c;
         *reinterpret_cast<Piece*>(dst + HALF) = d;
+    }
     }
 }
 
@@ -1562,7 +1577,7 @@ static int launch_head_norm_kv_write(const void* src, int row_stride, int n_part
         const size_t piece = e * sizeof(T);
         auto fits = [&](const void* ptr, long long stride) { return reinterpret_cast<uintptr_t>(ptr) % piece == 0 && stride % e == 0; };
         if (fits(src, row_stride) && (nh == 0 || fits(q_out, q_out_stride)) && (!write_kv || (fits(k_pages, 0) && fits(v_pages, 0)))) {
-            const int tb = T_ >= 4 * 296 ? 4 : (T_ >= 2 * 296 ? 2 : 1);
+            const int tb = T_ >= 2048 ? 2 : 1;          // (what a block's start costs is worth sharing only with blocks for every slot and more)
             auto go = [&](auto kernel) {
                 rf_launch(kernel, dim3((T_ + tb - 1) / tb), dim3(256), 0, st, reinterpret_cast<const T*>(src), row_stride, reinterpret_cast<T*>(q_out),
                           q_out_stride, nh, nkv, inv_freq, tok_seq, tok_pos, seq_slot, block_table, max_pages, reinterpret_cast<T*>(k_pages),
