@@ -322,8 +322,9 @@ __device__ __forceinline__ float row_sum_256(float (&acc)[256 / TPR], float* par
 // block; up to 1,024 wide a row is one warp's, and no barrier stands between a row's loads and its stores.  Memory is the bound
 // (6 or 8 bytes an element).  The sum is the one of a block of 256 threads a row, which up to 1,024 wide is also the few-row form's:
 // there a token's norm does not depend on the number of rows.  The blocks take the last rows first: L2 still holds what the product
-// before wrote last (between the products of a prompt of 33,361 x 896 39.6 -> 36.8 us a launch).  Measured (us; a block a row, each row read twice): 33,361 x 896 78 -> 27
-// (6.6 TB/s), 8,192 x 5,120 60 -> 43, 2,048 x 3,584 10.8 -> 10.9; a sum by one warp's own tree took as long within 1 %.
+// before wrote last (between the products of a prompt of 33,361 x 896 39.6 -> 36.8 us a launch).  Measured (us; a block a row, each row
+// read twice): 33,361 x 896 78 -> 27 (6.6 TB/s), 8,192 x 5,120 60 -> 43, 2,048 x 3,584 10.8 -> 10.9; a sum by one warp's own tree took as
+// long within 1 %.
 // (h without __restrict__: loads through const __restrict__ pointers may be moved up across the wait for the kernel before.)
 template <typename T, int TPR>
 __global__ void __launch_bounds__(256, 5)
@@ -855,10 +856,10 @@ __device__ __forceinline__ float head_square_sum(const float (&x)[E], const floa
 // all), keys and values of one size: a warp holds a head in registers, E neighbouring elements of each half a lane, so that a pair's
 // two elements meet in one lane; the sines and cosines of a block's tokens are formed once, in shared memory, before the wait for the
 // product.  (Element by element through shared memory, every head with the trigonometry of its own: 2,778 tokens of 20 heads of 128
-// unrotated 23 us, of 24 rotated and normed 33.)  A token a
-// block, two from 2,048 on, and two heads a warp in flight; us, with up to four tokens a block and one head: 2,778 tokens of 20 heads of
-// 128 15.1 and 21.0, 2,565 of 24 rotated 17.2 and 25.6, 1,301 of 32 heads of 64 10.4 and 18.7, 700 of 24 8.3 and 9.4, 8,192 43.1 and 42.7
-// (four tokens 43.8).  The last tokens come first, as in the norm of many rows.  What rmsnorm_rows_kernel says about __restrict__ holds for src.
+// unrotated 23 us, of 24 rotated and normed 33.)  A token a block, two from 2,048 on, and two heads a warp in flight; us, with up to
+// four tokens a block and one head: 2,778 tokens of 20 heads of 128 15.1 and 21.0, 2,565 of 24 rotated 17.2 and 25.6, 1,301 of 32
+// heads of 64 10.4 and 18.7, 700 of 24 8.3 and 9.4, 8,192 43.1 and 42.7 (four tokens 43.8).  The last tokens come first, as in the
+// norm of many rows.  What rmsnorm_rows_kernel says about __restrict__ holds for src.
 template <typename T, int E>
 __global__ void __launch_bounds__(256)
 head_norm_rows_kernel(const T* src, int row_stride, T* q_out, int q_out_stride, int nh, int nkv, const float* __restrict__ inv_freq,
