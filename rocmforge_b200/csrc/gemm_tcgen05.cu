@@ -35,15 +35,18 @@
 // Row tile y of the grid is (group, first row, end row) of grp.tiles (grp.tiles[0] tiles exist; the others return at
 // once); its rows of X, sorted by group, meet rows group * group_n + ... of the stacked weights W [groups * group_n, K];
 // rows of the tile beyond its end belong to the next group and are computed but not stored.
-// BM (weights as rows): weight rows of a tile, 128 or 64.  EW: epilogue warps, 4, or 8 that share the tile's columns.
-template <int BN, bool SWAP, int STAGES, bool NORM = false, bool GROUPED = false, int BM = TC_BM, int EW = 4>
+// BM (weights as rows): weight rows of a tile, 128 or 64.  EW: epilogue warps, 4, or 8 that share the tile's columns.  MODE: the one
+// mode that the function is compiled for (EPI_REGLU: any gated unit but silu's), or EPI_ANY: what the mode is, is then asked here.
+template <int BN, bool SWAP, int STAGES, bool NORM = false, bool GROUPED = false, int BM = TC_BM, int EW = 4, int MODE = EPI_ANY>
 __global__ void __launch_bounds__(64 + 32 * EW, SWAP ? (BN == 16 && STAGES <= 4 ? 3 : 2) : 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, TcParams p,
                typename std::conditional<NORM, TcNorm, TcNoNorm>::type norm_arg,
                typename std::conditional<GROUPED, TcGroup, TcNoNorm>::type grp_arg) {
     static_assert(!(GROUPED && (SWAP || NORM)), "grouped products are tokens-as-rows and carry no norm");
     static_assert(BM == TC_BM || (SWAP && !NORM && BM == 64), "tiles of 64 weight rows");
+    static_assert(MODE == EPI_ANY || (SWAP && !NORM), "a mode of its own");
     static_assert(EW == 4 || (SWAP && !NORM && EW == 8 && BN >= 32), "eight epilogue warps share the columns");
+    const int mode = MODE != EPI_ANY ? MODE : p.mode;
     // the variant without the norm never looks at this (every use below sits behind ``NORM &&``)
     const TcNorm& pn = *reinterpret_cast<const TcNorm*>(&norm_arg);
     constexpr uint32_t A_BYTES = BM * TC_BK * 2;
@@ -170,7 +173,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
         const bool ok = mbar_wait(smem_u32(&bars[2 * STAGES]), 0, &abort_flag);
         tcgen05_fence_after();
-        if (ok && n_kb > 0 && !(NORM && p.mode == EPI_RESNORM)) {
+        if (ok && n_kb > 0 && !(NORM && mode == EPI_RESNORM)) {
             // index along map A's rows (64 rows lie in the first 16 lanes of each quarter; the other lanes hold nothing)
             const int row_a = BM == 64 ? (lane < 16 ? coord_a + quarter * 16 + lane : p.N) : coord_a + quarter * 32 + lane;
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16);
@@ -185,7 +188,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     // lane = token m, registers = 32 consecutive weight rows n
                     if constexpr (GROUPED) {
                         const TcGroup& grp = *reinterpret_cast<const TcGroup*>(&grp_arg);
-                        if (p.mode == EPI_CLAMPGLU) {
+                        if (mode == EPI_CLAMPGLU) {
                             epilogue_clamped_glu<CH>(p, r, row_a, tile_b * BN + c0, grp.row_scale, grp.limit, grp.alpha);
                             continue;
                         }
@@ -194,13 +197,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 } else {
                     // lane = weight row n, registers = consecutive tokens m
                     const int n = row_a, m0 = tile_b * BN + c0;
-                    const float b = (p.bias && n < p.N && p.mode != EPI_RESNORM) ? load_vec(p.bias, p.bias_is_f32, n) : 0.f;
+                    const float b = (p.bias && n < p.N && mode != EPI_RESNORM) ? load_vec(p.bias, p.bias_is_f32, n) : 0.f;
                     if (m0 >= p.M) break;                // the tile's other columns are padding, not tokens
                     if (NORM && pn.ss_in) {
 #pragma unroll
                         for (int j = 0; j < CH; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * rstd_s[c0 + j]);
                     }
-                    if (p.mode == EPI_SWIGLU) {
+                    if (mode == EPI_SWIGLU) {
                         // gate in even lanes, up in the odd lane beside it.  Two tokens at a time: the even lane
                         // finishes token j (it gets that token's up), the odd lane token j + 1 (it gets its gate),
                         // so every lane evaluates one silu per pair of tokens and every lane stores.
@@ -215,7 +218,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                                 reinterpret_cast<__nv_bfloat16*>(p.out)[(size_t)m * p.ldo + (n >> 1)] =
                                     __float2bfloat16_rn(silu_fast(g) * u);
                         }
-                    } else if (epi_gated(p.mode)) {      // the same exchange for another unit
+                    } else if (epi_gated(mode)) {      // the same exchange for another unit
                         const bool odd = lane & 1;
                         with_gated_unit(p.mode, p.limit, p.alpha, [&](auto unit) {
 #pragma unroll
@@ -234,19 +237,19 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         // 1.2 us, half of a small product's time at 64 tokens)
                         const int m_cnt = min(CH, p.M - m0);
                         const size_t o0 = (size_t)m0 * p.ldo + n;
-                        if (p.mode == EPI_STORE) {
+                        if (mode == EPI_STORE) {
                             __nv_bfloat16* ob = reinterpret_cast<__nv_bfloat16*>(p.out) + o0;
 #pragma unroll
                             for (int j = 0; j < CH; ++j)
                                 if (j < m_cnt) ob[(size_t)j * p.ldo] = __float2bfloat16_rn(__uint_as_float(r[j]) + b);
-                        } else if (p.mode == EPI_RESIDUAL) {
+                        } else if (mode == EPI_RESIDUAL) {
                             float* of = reinterpret_cast<float*>(p.out) + o0;
 #pragma unroll
                             for (int j = 0; j < CH; ++j)
                                 if (j < m_cnt) of[(size_t)j * p.ldo] += __uint_as_float(r[j]) + b;
                         } else {                         // F32, or a split's partial sums (PARTIAL, RESNORM)
                             float* of = reinterpret_cast<float*>(p.out) + o0 +
-                                        (p.mode == EPI_F32 ? (size_t)0 : (size_t)split * p.partial_stride);
+                                        (mode == EPI_F32 ? (size_t)0 : (size_t)split * p.partial_stride);
 #pragma unroll
                             for (int j = 0; j < CH; ++j)
                                 if (j < m_cnt) of[(size_t)j * p.ldo] = __uint_as_float(r[j]) + b;
@@ -256,7 +259,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
         }
     }
-    if (NORM && p.mode == EPI_RESNORM) {
+    if (NORM && mode == EPI_RESNORM) {
         // ---- the K splits of an output tile are one thread-block cluster (along grid.z).  Every CTA owns BN / S of the
         // tile's tokens: the others push their partial sums of those tokens into its shared memory, it adds them in
         // rank order to the 32-bit stream and prepares the norm.  Nothing goes through global memory, and the order of
@@ -352,14 +355,14 @@ static int sm_count() {
     return n;
 }
 
-template <int BN, bool SWAP, int STAGES, bool NORM = false, bool GROUPED = false, int BM = TC_BM, int EW = 4>
+template <int BN, bool SWAP, int STAGES, bool NORM = false, bool GROUPED = false, int BM = TC_BM, int EW = 4, int MODE = EPI_ANY>
 static int launch_cfg(const CUtensorMap& ma, const CUtensorMap& mb, const TcParams& p, dim3 grid, cudaStream_t st,
                       const TcNorm* norm = nullptr, int cluster_z = 1, const TcGroup* group = nullptr) {
     constexpr size_t smem = (size_t)STAGES * (BM * TC_BK * 2 + BN * TC_BK * 2) + (2 * STAGES + 1) * 8 + 16 + 1024;
     static PerDevice<bool> devices;
     bool& configured = devices.here();
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN, SWAP, STAGES, NORM, GROUPED, BM, EW>,
+        cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN, SWAP, STAGES, NORM, GROUPED, BM, EW, MODE>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         configured = true;
@@ -381,17 +384,66 @@ static int launch_cfg(const CUtensorMap& ma, const CUtensorMap& mb, const TcPara
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = g_rf_pdl ? 2 : 1;
-        cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<BN, SWAP, STAGES, NORM, GROUPED, BM, EW>, ma, mb, p, extra, grp);
+        cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<BN, SWAP, STAGES, NORM, GROUPED, BM, EW, MODE>, ma, mb, p, extra, grp);
         if (e != cudaSuccess) return (int)e;
         RF_LAUNCH_CHECK();
         return 0;
     }
-    rf_launch(gemm_tc_kernel<BN, SWAP, STAGES, NORM, GROUPED, BM, EW>, grid, dim3(64 + 32 * EW), smem, st, ma, mb, p, extra, grp);
+    rf_launch(gemm_tc_kernel<BN, SWAP, STAGES, NORM, GROUPED, BM, EW, MODE>, grid, dim3(64 + 32 * EW), smem, st, ma, mb, p, extra, grp);
     RF_LAUNCH_CHECK();
     return 0;
 }
 
+// The forms that products of few tokens take beside the general one (tiles of 128 weight rows, four epilogue warps).
+//
+// half: tiles of 64 weight rows where tiles of 128 leave SMs without one and K is whole.  wide: eight epilogue warps; where a number
+// costs more than an add and a store to a whole line, so not for partial sums (64 tokens x 4,608 x 3,584 9.9 us, 10.4 with eight).
+//
+// Each of them is compiled for one mode.  The other products of a step run the general form, so the instructions of another function
+// come from L2 anew in every layer, about 1 us with all modes in it: in chains of one function these forms won throughout, but steps
+// of 17 to 40 tokens of a model 1,536 wide became up to 8 % slower.  (The general form itself, in a function for silu alone, costs such
+// steps 1 to 5 %.)  Gated units and bfloat16 rows gain enough; 32-bit rows and sums into the stream stay with the general form.
+// Whole decode steps, us, the general form alone, these forms with all modes in them, and so:
+//     896 wide (0.5B)   8 tokens 628, 625, 606; 24 684, 699, 677; 64 788, 768, 752; 65 903, 951, 902; 128 996, 992, 956
+//     1,536 wide        8 tokens 435, 433, 422; 24 481, 511, 485; 40 532, 560, 534; 64 576, 568, 554; 128 747, 713, 701
+//     Ludusun's design  8 tokens 288, 266, 263; 24 315, 316, 306; 64 420, 409, 400; 128 587, 567, 563
+//     (behind the general form still: 640 wide, 16 tokens, 303 and 313; 768 wide, 12 tokens, 306 and 315)
+// With 17 to 32 tokens a gated product gains nothing over the general form's warm instructions (24 tokens, 768 wide 336, 342 in half
+// tiles), bfloat16 rows do (Ludusun, 17 tokens: 305, 295).  And activations of less than 128 KB come slowly into tiles that reach beyond
+// 128 KB: 65 tokens x 9,728 x 896 10.4 us, in half tiles 11.9 (80 tokens 10.4, 10.1); 33 x 17,920 x 1,536 13.6, 14.7 (43: 13.7, 12.8).
+// Beyond a tile an SM half tiles cost: their rows meet as many token bytes (8 tokens x 32,000 x 2,048 23.4, 27.7).
+struct SkinnyForm { bool half, wide; };
+static SkinnyForm skinny_form(int M, int N, int bn, int ldx, int mode, int splits, bool normed_rows, int sms) {
+    const long long row = (long long)ldx * 2, edge = 128 << 10;
+    const bool slow_tile = bn >= 64 && M * row < edge && bn * row > edge;
+    if (normed_rows || splits != 1 || slow_tile || !(mode == EPI_STORE || epi_gated(mode))) return {false, false};
+    const bool half = (long long)((N + TC_BM - 1) / TC_BM) * ((M + bn - 1) / bn) <= sms && (bn != 32 || mode == EPI_STORE);
+    return {half, !half && bn >= 64};
+}
+static int skinny_tokens(int M) { return M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128)); }      // tokens of a tile
+
+template <int MODE>
+static int launch_special(SkinnyForm form, int bn, const CUtensorMap& ma, const CUtensorMap& mb, const TcParams& p, dim3 grid, cudaStream_t st) {
+    if (form.half) {
+        if (bn == 16) return launch_cfg<16, true, 11, false, false, 64, 4, MODE>(ma, mb, p, grid, st);
+        if constexpr (MODE == EPI_STORE)
+            if (bn == 32) return launch_cfg<32, true, 9, false, false, 64, 8, MODE>(ma, mb, p, grid, st);
+        if (bn == 64) return launch_cfg<64, true, 6, false, false, 64, 8, MODE>(ma, mb, p, grid, st);
+        if (bn == 128) return launch_cfg<128, true, 4, false, false, 64, 8, MODE>(ma, mb, p, grid, st);
+    } else {
+        if (bn == 64) return launch_cfg<64, true, 4, false, false, TC_BM, 8, MODE>(ma, mb, p, grid, st);
+        if (bn == 128) return launch_cfg<128, true, 3, false, false, TC_BM, 8, MODE>(ma, mb, p, grid, st);
+    }
+    return RF_ERR_BAD_ARG;                               // (skinny_form names no other)
+}
+
 extern "C" {
+
+// The form of a product of few tokens on a GPU of ``sms`` SMs: 1 tiles of 64 weight rows, 2 eight epilogue warps, 0 the general one.
+int rf_gemm_tc_skinny_form(int M, int N, int ldx, int mode, int splits, int normed_rows, int sms) {
+    const SkinnyForm f = skinny_form(M, N, skinny_tokens(M), ldx, mode, splits, normed_rows != 0, sms);
+    return f.half ? 1 : f.wide ? 2 : 0;
+}
 
 // Whether the tensor-core kernel takes this product (else the caller uses the CUDA-core kernel).
 int rf_gemm_tc_supported(int M, int N, int K, int mode) {
@@ -495,18 +547,10 @@ static int gemm_skinny(const void* X, int ldx, const void* W, const void* bias, 
     static_assert(sizeof(TcParams) + sizeof(TcNorm) <= 128, "two tensor maps and these must stay within 384 bytes");
     CUtensorMap ma, mb;
     int e;
-    const int bn = M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128));
+    const int bn = skinny_tokens(M);
     const bool normed_rows = ss_in || mode == EPI_RESNORM;
-    // Tiles of 64 weight rows where tiles of 128 leave SMs without one and K is whole (us with the norm before it, 128 and 64 rows:
-    // 64 tokens x 9,728 x 896 8.7, 8.4; 8 tokens x 9,728 x 896 8.1, 7.2, x 16,384 x 2,048 15.6, 14.2, x 4,096 x 2,048 12.3, 9.6).  Beyond
-    // a tile an SM they cost: half a tile's rows meet as many token bytes (8 tokens x 32,000 x 2,048 23.4, 27.7; 64 x 37,888 x 3,584
-    // 46.6, 50.7; 8 x 27,648 x 5,120 48.2, 48.3).
-    const bool half_tiles = !normed_rows && splits == 1 && (N + TC_BM - 1) / TC_BM * ((M + bn - 1) / bn) <= sm_count();
-    const int bm = half_tiles ? 64 : TC_BM;
-    // Eight epilogue warps where a number costs more than an add and a store to a whole line (us, four and eight: 64 tokens x 9,728 x 896
-    // gated 10.0, 8.7, 128 tokens 14.0, 11.6; 64 tokens x 37,888 x 3,584 47.8, 46.6; 64 x 8,192 x 2,048 in bfloat16 15.3, 14.3; but
-    // partial sums, 64 x 4,608 x 3,584 9.9, 10.4, 64 x 896 x 896 5.1, 5.4, and a head's 32-bit rows, 64 x 151,936 x 896 55.8, 56.6)
-    const bool wide_epilogue = epi_gated(mode) || mode == EPI_STORE;
+    const SkinnyForm form = skinny_form(M, N, bn, ldx, mode, splits, normed_rows, sm_count());
+    const int bm = form.half ? 64 : TC_BM;
     if ((e = make_map(&ma, W, N, K, K, bm)) || (e = make_map(&mb, X, M, K, ldx, bn))) return e;
     dim3 grid((M + bn - 1) / bn, (N + bm - 1) / bm, splits);      // token tiles fastest: they share a weight tile in L2
     // stage counts chosen so that two CTAs share an SM (three with up to 16 tokens: 3 x 4 stages hold as many weight
@@ -522,18 +566,12 @@ static int gemm_skinny(const void* X, int ldx, const void* W, const void* bias, 
         if (bn == 64) return launch_cfg<64, true, 4, true>(ma, mb, p, grid, st, &nrm, cz);
         return launch_cfg<128, true, 3, true>(ma, mb, p, grid, st, &nrm, cz);
     }
-    if (half_tiles) {
-        if (bn == 16) return launch_cfg<16, true, 11, false, false, 64>(ma, mb, p, grid, st);
-        if (bn == 32) return launch_cfg<32, true, 9, false, false, 64, 8>(ma, mb, p, grid, st);
-        if (bn == 64) return launch_cfg<64, true, 6, false, false, 64, 8>(ma, mb, p, grid, st);
-        return launch_cfg<128, true, 4, false, false, 64, 8>(ma, mb, p, grid, st);
+    if (form.half || form.wide) {
+        if (mode == EPI_STORE) return launch_special<EPI_STORE>(form, bn, ma, mb, p, grid, st);
+        if (mode == EPI_SWIGLU) return launch_special<EPI_SWIGLU>(form, bn, ma, mb, p, grid, st);
+        return launch_special<EPI_REGLU>(form, bn, ma, mb, p, grid, st);
     }
     if (bn == 16) return launch_cfg<16, true, 4>(ma, mb, p, grid, st);
-    if (wide_epilogue) {
-        if (bn == 32) return launch_cfg<32, true, 5, false, false, TC_BM, 8>(ma, mb, p, grid, st);
-        if (bn == 64) return launch_cfg<64, true, 4, false, false, TC_BM, 8>(ma, mb, p, grid, st);
-        return launch_cfg<128, true, 3, false, false, TC_BM, 8>(ma, mb, p, grid, st);
-    }
     if (bn == 32) return launch_cfg<32, true, 5>(ma, mb, p, grid, st);
     if (bn == 64) return launch_cfg<64, true, 4>(ma, mb, p, grid, st);
     return launch_cfg<128, true, 3>(ma, mb, p, grid, st);

@@ -10,7 +10,7 @@
 #define TC_THREADS 192
 #define TC_WAIT_LIMIT_NS 2000000000ULL      // 2 s
 
-enum { EPI_STORE = 0, EPI_F32 = 1, EPI_RESIDUAL = 2, EPI_SWIGLU = 3, EPI_PARTIAL = 4, EPI_RESNORM = 5, EPI_CLAMPGLU = 6, EPI_REGLU = 7, EPI_GEGLU = 8 };
+enum { EPI_ANY = -1, EPI_STORE = 0, EPI_F32 = 1, EPI_RESIDUAL = 2, EPI_SWIGLU = 3, EPI_PARTIAL = 4, EPI_RESNORM = 5, EPI_CLAMPGLU = 6, EPI_REGLU = 7, EPI_GEGLU = 8 };
 // the modes whose output is half as wide as the (row-interleaved gate/up) weight
 __host__ __device__ __forceinline__ bool epi_gated(int mode) { return mode == EPI_SWIGLU || mode == EPI_CLAMPGLU || mode == EPI_REGLU || mode == EPI_GEGLU; }
 

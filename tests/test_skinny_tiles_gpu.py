@@ -38,6 +38,24 @@ def test_tiles_of_64_rows(M, N, K, mode):
     torch.testing.assert_close(got.double(), ref, atol=2e-5 + K * 2.0 ** -24, rtol=2e-5 if mode == tc.F32 else 2.0 ** -8)
 
 
+@pytest.mark.parametrize("mode", [tc.STORE, tc.SWIGLU, tc.GEGLU])
+@pytest.mark.parametrize("M,N,K", [
+    (64, 320, 1024), (65, 320, 896), (73, 320, 896), (74, 320, 896),               # around the last rows that end below 128 KB
+    (17, 320, 896), (32, 148 * 128 + 130, 128), (33, 148 * 128 + 2, 136), (65, 148 * 128 + 2, 136)])
+def test_form_for_one_kind_of_output(M, N, K, mode):
+    g = torch.Generator(DEV).manual_seed(M + N + K + mode)
+    x = torch.randn((M, K), generator=g, device=DEV).bfloat16()
+    w = (torch.randn((N, K), generator=g, device=DEV) * K ** -0.5).bfloat16()
+    got = tc.gemm_tc_skinny(x, w, mode=mode)
+    sums = tc.gemm_tc_skinny(x, w, mode=tc.F32)                                    # the general form
+    if mode == tc.STORE:
+        assert torch.equal(got.view(torch.int16), sums.bfloat16().view(torch.int16))
+    else:
+        # the same sums: only the unit's own arithmetic (a few 2^-24) lies between, so at most bfloat16's rounding (2^-9) differs
+        want = UNITS[mode](sums[:, ::2].double(), sums[:, 1::2].double())
+        torch.testing.assert_close(got.double(), want, atol=1e-6, rtol=2.0 ** -8)
+
+
 @pytest.mark.parametrize("M", [8, 32, 64, 100])
 def test_bias_and_numbers_that_are_not_finite(M):
     g = torch.Generator(DEV).manual_seed(M)
