@@ -3,7 +3,7 @@ from .basic import (PAGE, embed, add_rmsnorm, rope_kv_write, swiglu, gemm_simt, 
                     attention_f32_token_supported, f32_token_splits, F32_PROMPT_FROM, argmax, sample, set_sample_cached, advance_decode, gather_tokens,
                     attention_decode, attention_decode_supported, attention_decode_scratch, DECODE_CHUNK,
                     attention_prefill, attention_prefill_supported, PREFILL_TILE,
-                    attention_decode_warps, attention_decode_formed, decode_splits, decode_pages,
+                    attention_decode_warps, attention_decode_formed, decode_forms_queries, decode_splits, decode_pages,
                     attention_prefill_tc, attention_prefill_tc_supported, PREFILL_TC_TILE)
 from .basic import (relu2, add_row, branch_norm_add, head_norm_kv_write, gemm_simt_grouped, retention_prepare,
                     retention_scan, retention_gate, retention_chunked, RETENTION_CHUNK, moe_route, moe_sort, moe_combine, moe_gather, MOE_TILE_SMALL, MOE_TILE_LARGE, MOE_TILE_TC)

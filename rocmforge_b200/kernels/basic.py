@@ -714,6 +714,25 @@ def decode_pages(longest: int, window: int | None) -> int:
     return pages
 
 
+def decode_forms_queries(B: int, n_kv_heads: int, head_dim: int, longest: int, span: int | None, product_ctas: int, sms: int) -> bool:
+    """Whether a decode step's attention forms its queries, keys and values from the q|k|v product's partial sums itself
+    (``attention_decode_formed``) instead of having them written by a kernel between; ``product_ctas``: CTAs of that product.
+
+    It saves a launch, and gains by it where its CTAs find room beside the product's, so that their first tiles, positions and pages are at
+    hand when the sums arrive.  Heads of 64 always do (steps of 0.5B's shape and of 32 heads on 8, batch 1 to 64, contexts of 100 to
+    16,000: 0.925 to 0.999 of the time).  Heads of 128 take tiles of 16 keys, no more of them than a CTA has warps (at most a CTA
+    an SM: eight warps), and either the attention's CTAs are at most half the SMs or both kernels' together about 2.5 an SM.  us a layer
+    gained, at 148 SMs (product's + attention's CTAs): 7B's shape batch 2 (288 + 64) 0.9, 4 (288 + 64) 1.6, 5 (288 + 80) 0.4, but 6
+    (288 + 96) -1.3, 8 (288 + 128) -0.9; 14B's batch 2 (280 + 64) 2.2, 3 (280 + 96) 1.1, 4 (280 + 128) -0.3; 32 heads on 4 of 4,096
+    batch 6 (280 + 96) -0.2, 8 (280 + 128) -1.5; 48 on 8 of 6,144 batch 2 (384 + 64) 4.2, 3 (384 + 96) -4.8; 16 on 2 of 2,048 batch 16
+    (160 + 128) 1.2; 8 on 1 of 1,024 batch 32 (60 + 128) 1.5."""
+    if head_dim <= 64:
+        return True
+    splits = decode_splits(B, n_kv_heads, longest, span, head_dim)
+    ctas, tiles = B * n_kv_heads * splits, -(-decode_pages(longest, span) // splits) * PAGE // 16
+    return head_dim == 128 and tiles <= 8 and ctas <= sms and (ctas <= sms // 2 or product_ctas + ctas <= 51 * sms // 20)
+
+
 def attention_decode_warps(q: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: int, k_pages, v_pages,
                            tok_seq, tok_pos, seq_slot, block_table, scale: float, window: int | None,
                            splits: int | None = None, warps: int | None = None,

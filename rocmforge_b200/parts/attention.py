@@ -325,12 +325,8 @@ class GQAAttention(Mixer):
 
     def _attend_from_product(self, ctx, y, view):
         """A decode step in two launches: the K-split product, and the attention that adds up its partial sums, turns queries and
-        keys and writes the cache; None where a step needs more than that kernel does, or gains nothing by it.
-
-        It gains where its CTAs find room beside the product's and so have their first tiles, positions and pages at hand when the sums
-        arrive: heads of 64, and heads of 128 in tiles of 16 keys where those are no more than a CTA's warps.  A whole step, us, with the
-        writer between and without it: 0.5B batch 64 960, 929; 7B batch 1 2,440, 2,409 (tiles of 32 2,461); but 7B batch 8 2,542, 2,568
-        (tiles of 16 2,595) and batch 64 3,325, 3,354."""
+        keys and writes the cache; None where a step needs more than that kernel does, or gains nothing by it
+        (``kernels.decode_forms_queries``)."""
         tc, w = kernels.tensor_core, self.qkv.weight
         rot = (self.position.rotation() if self.position is not None else None) or {}
         heads = (self.n_heads, self.n_kv_heads, self.head_dim)
@@ -339,21 +335,19 @@ class GQAAttention(Mixer):
                 and not self.keep_first and not self.sink and rot.get("inv_freq") is not None and rot["rot_dim"] == self.head_dim
                 and not rot.get("interleaved", False) and kernels.attention_decode_supported(*heads)):
             return None
-        longest, span = ctx.model_cache_limit if ctx.replayed else ctx.max_end, self.window or self.chunk
-        splits = kernels.decode_splits(ctx.B, self.n_kv_heads, longest, span, self.head_dim)
-        tiles = -(-kernels.decode_pages(longest, span) // splits) * kernels.PAGE // 16
-        if self.head_dim > 128 or (self.head_dim == 128 and (tiles > 8 or ctx.B * self.n_kv_heads * splits > sm_count(ctx.device))):
-            return None
         if not ctx.uses_tensor_cores(y.x if isinstance(y, ScaledRows) else y, w, tc.PARTIAL):
             return None
         sums = tc.split_k_for(w.shape[0], w.shape[1], tokens=ctx.T)
-        if sums == 1:
+        longest, span = ctx.model_cache_limit if ctx.replayed else ctx.max_end, self.window or self.chunk
+        if sums == 1 or not kernels.decode_forms_queries(ctx.B, self.n_kv_heads, self.head_dim, longest, span,
+                                                         (w.shape[0] + 127) // 128 * sums, sm_count(ctx.device)):
             return None
         x, row_ss = ctx.unpack_rows(y, w, tc.PARTIAL)
         parts = tc.gemm_tc_skinny(x, w, mode=tc.PARTIAL, splits=sums, row_ss=row_ss)
         return kernels.attention_decode_formed(
             parts, *heads, rot["inv_freq"], view.k_pages, view.v_pages, ctx.tok_seq, ctx.tok_pos, ctx.seq_slot, view.block_table, self.scale,
-            self.window, bias=self.qkv.bias, chunk=self.chunk, splits=splits)
+            self.window, bias=self.qkv.bias, chunk=self.chunk,
+            splits=kernels.decode_splits(ctx.B, self.n_kv_heads, longest, span, self.head_dim))
 
     def attend(self, ctx, q, view):
         """Attention of the step's tokens over the cache; q is the first heads*head_dim columns of ``q``."""

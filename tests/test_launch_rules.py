@@ -83,3 +83,20 @@ def test_forms_of_products_of_few_tokens():
     assert [of(M, 9728, 896, tc.SWIGLU) for M in (64, 65, 73, 74, 128)] == [1, 0, 0, 1, 1]
     assert [of(M, 17920, 1536, tc.SWIGLU) for M in (33, 42, 43, 64)] == [0, 0, 1, 1]
     assert [of(M, 40000, 896, tc.STORE) for M in (65, 74)] == [0, 2]
+
+
+def test_when_decode_attention_forms_its_own_queries():
+    """Heads of 64 always; heads of 128 where the attention's CTAs find room beside the q|k|v product's."""
+    def takes(B, heads, kv, width, longest=512, span=None, hd=128):
+        N = (heads + 2 * kv) * hd
+        product = (N + 127) // 128 * tc.split_k_for(N, width, 148, tokens=B)
+        return basic.decode_forms_queries(B, kv, hd, longest, span, product, 148)
+    from rocmforge_b200.kernels import tensor_core as tc
+    assert all(takes(B, 14, 2, 896, n, hd=64) for B in (1, 8, 64, 128) for n in (512, 1024, 16384))
+    assert [B for B in range(1, 17) if takes(B, 28, 4, 3584)] == [1, 2, 3, 4, 5]          # 7B; at 6 and 8 the writer's step is shorter
+    assert [B for B in range(1, 17) if takes(B, 28, 4, 3584, 1024)] == [1, 2]
+    assert [B for B in range(1, 9) if takes(B, 40, 8, 5120)] == [1, 2, 3]                 # 14B
+    assert [B for B in range(1, 9) if takes(B, 48, 8, 6144)] == [1, 2]
+    assert [B for B in range(1, 33) if takes(B, 16, 2, 2048)] == list(range(1, 17))
+    assert not any(takes(B, 28, 4, 3584, 8192) for B in (1, 2, 8, 64)) and takes(1, 28, 4, 3584, 8192, 128)
+    assert not takes(1, 16, 2, 4096, hd=256)
