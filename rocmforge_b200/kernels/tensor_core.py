@@ -223,20 +223,25 @@ def gemm_tc_grouped(x: torch.Tensor, w: torch.Tensor, tiles: torch.Tensor, max_t
 
 
 def split_k_for(N: int, K: int, sm_count: Optional[int] = None, tokens: Optional[int] = None) -> int:
-    """K splits of a skinny product, from N and K (never from the batch's content), so that about two CTAs per SM stream
-    the weight and every split keeps at least 4 blocks of 64, of a K of at most 16 blocks 8 / 3 (the products of 14 blocks of the
-    0.5B shape in 3, 4, 5, 7 splits, a decode step, us: batch 1 676, 645, 629, 624, batch 16 723, 677, 662, 666, batch 64 922, 880, 862,
-    864; longer K in finer splits gains nothing, K of 2,048 in 8, 10, 12: Ludusun batch 8 275, 275, 281).  ``tokens``: a step of at most 16 tokens fits three CTAs on an
-    SM, and a weight with long K ranges is then cut for three per SM (splits of at least 16 blocks; the down projection of
-    the 7B shape 10 -> 15: a decode step at batch 8 2.624 -> 2.603 ms, at batch 1 2.560 -> 2.530 ms; with 32 or 64 tokens,
-    two CTAs per SM, the same cut costs 0.16 ms).  The short K ranges of q|k|v and o gain nothing from more splits."""
+    """K splits of a skinny product, from N and K (never from the batch's content): about two CTAs per SM stream the weight, and a split
+    has at least 4 blocks of 64 or, where K has at most 16 blocks, 2 while that makes no more than a CTA per SM (the last split has
+    what is left).  ``tokens``: a step of at most 16 tokens fits three CTAs on an SM, and a weight with long K ranges is then cut
+    for three per SM (splits of at least 16 blocks; the down projection of the 7B shape 10 -> 15: a decode step at batch 8 2.624 ->
+    2.603 ms, at batch 1 2.560 -> 2.530 ms; with 32 or 64 tokens, two CTAs per SM, the same cut costs 0.16 ms).
+
+    A short K in splits of 4, 8 / 3 and 2 blocks, whole decode steps of 12 layers with that width, us: 8 blocks, batch 1 261, 259, 252,
+    64 356, 358, 354; 10 blocks, batch 16 320, 310, 290, 128 473, 463, 438; 12 blocks, batch 16 321, 318, 301, 64 382, 379, 373; 14 blocks,
+    batch 16 348, 312, 311, 128 485, 474, 482; 16 blocks, batch 16 334, 323, 322, 64 412, 401, 400, 128 500, 514, 514; Ludusun's
+    design 1,024 wide, batch 16 195, 199, 197, 64 272, 276, 273.  Beyond a CTA per SM (48 tiles of 16 blocks) the finer splits cost:
+    batch 64 620, 623, 623.  From 24 blocks on splits of 4 are as good as any (1,536 wide, batch 16, of 4 and 3 blocks: 410, 413)."""
     sm_count = sm_count or device_sm_count()
     tiles = (N + 127) // 128
     kb = (K + 63) // 64
     if tiles >= 2 * sm_count or kb < 8:
         return 1
     want = max(1, (2 * sm_count) // tiles)
-    splits = max(1, min(want, kb // 4 if kb > 16 else kb * 3 // 8))
+    splits = kb // 4 if kb > 16 else max(kb // 4, min(kb // 2, sm_count // tiles))
+    splits = max(1, min(want, splits))
     if tokens is not None and tokens <= 16:
         splits = max(splits, min((3 * sm_count) // tiles, kb // 16))
     per = (kb + splits - 1) // splits
@@ -303,9 +308,10 @@ def gemm_tc_skinny(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor
 
 def resnorm_splits(N: int, K: int) -> int:
     """K splits of the product that finishes the residual update itself: the splits of a tile are one thread-block
-    cluster, so a power of two up to 8, as near the ordinary rule as that allows; from N and K alone."""
-    want = split_k_for(N, K)
+    cluster, so a power of two up to 8, as near the ordinary rule as that allows, of at least 4 blocks of 64 (nothing
+    reads the partial sums of more of them later); from N and K alone."""
     kb = (K + 63) // 64
+    want = min(split_k_for(N, K), max(1, kb // 4))
     s = 1
     while s * 2 <= min(want, 8) and (s * 2 - 1) * ((kb + s * 2 - 1) // (s * 2)) < kb:
         s *= 2
