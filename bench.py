@@ -232,36 +232,19 @@ def decode_rate(model, prompts, steps, warmup, check=16):
             "mean_ctx": mean_ctx, "t0": t0, "t1": t1, "checked_steps": checked}
 
 
-def ablation(model, batch, steps=32, prompt_len=PROMPT_LEN):
-    """Where a replayed decode step's time goes: every kind of kernel in turn is replaced by a stand-in that launches
-    nothing and returns a buffer of the right shape, the step's graph is captured anew and timed.  The difference to
-    the whole step is what that kernel costs inside the chain (with its overlaps), which a profiler's serialised,
-    cold-cache replay does not show.  Results are garbage while a stand-in is in place; only the time is read."""
+def ablation_cases(cfg, device):
+    """[(name, [(module, attribute, stand-in)])]: every kind of kernel of a decode step with stand-ins that launch nothing and return a
+    buffer of the right shape."""
     import torch
     from rocmforge_b200 import kernels
     from rocmforge_b200.kernels import tensor_core as tc
-    from rocmforge_b200.engine.graph import DecodeRunner
-    cfg = model.config
-    L = cfg.num_hidden_layers
     buffers = {}
 
     def buffer(key, shape, dtype):
+        key = (key, shape, dtype)
         if key not in buffers:
-            buffers[key] = torch.zeros(shape, dtype=dtype, device=model.device)
+            buffers[key] = torch.zeros(shape, dtype=dtype, device=device)
         return buffers[key]
-
-    def run():
-        cache = model.new_cache(max_tokens=batch * (prompt_len + 256), max_slots=batch)
-        runner = DecodeRunner(model, cache)
-        slots = [cache.alloc_slot() for _ in range(batch)]
-        for s in slots:                                  # prompt_len cached positions (their content does not matter)
-            cache.prepare([s], [prompt_len])
-            cache.commit([s], [prompt_len])
-        runner.greedy_loop(slots, [1] * batch, 4)
-        torch.cuda.synchronize()
-        _, start, end, _ = runner.greedy_loop(slots, [1] * batch, steps)
-        torch.cuda.synchronize()
-        return start.elapsed_time(end) / steps * 1e3     # us a step
 
     def no_norm(h, weight, eps, dt, pending=None, rows=None, out=None):
         return buffer(("norm", rows is None), (h.shape[0] if rows is None else rows.shape[0], h.shape[1]), dt)
@@ -269,15 +252,15 @@ def ablation(model, batch, steps=32, prompt_len=PROMPT_LEN):
     def no_rope(qkv, nh, nkv, hd, inv, *a, **kw):
         return buffer("q", (qkv.shape[1] if qkv.dim() == 3 else qkv.shape[0], nh * hd), torch.bfloat16)
 
-    def no_attention(q, nh, nkv, hd, *a, **kw):
-        return buffer("o", (q.shape[0], nh * hd), torch.bfloat16)
+    def no_attention(q, nh, nkv, hd, *a, **kw):          # q: rows, or a stack of partial sums that the attention adds up itself
+        return buffer("o", (q.shape[-2], nh * hd), torch.bfloat16)
 
     real_skinny, real_resnorm = tc.gemm_tc_skinny, tc.gemm_tc_skinny_resnorm
 
     def without(pred):
-        def f(x, w, bias=None, *, mode=tc.STORE, splits=1, out=None, row_ss=None):
+        def f(x, w, bias=None, *, mode=tc.STORE, splits=1, out=None, row_ss=None, **unit):
             if not pred(w, mode):
-                return real_skinny(x, w, bias, mode=mode, splits=splits, out=out, row_ss=row_ss)
+                return real_skinny(x, w, bias, mode=mode, splits=splits, out=out, row_ss=row_ss, **unit)
             if out is not None:
                 return out
             M, N = x.shape[0], w.shape[0]
@@ -294,18 +277,44 @@ def ablation(model, batch, steps=32, prompt_len=PROMPT_LEN):
 
     H, I, V = cfg.hidden_size, cfg.intermediate_size, cfg.vocab_size
     QKV = (cfg.num_attention_heads + 2 * cfg.num_key_value_heads) * cfg.head_dim
-    cases = [("norm kernels (first layer and final norm when the others are fused)", [(kernels, "add_rmsnorm", no_norm)]),
-             ("rotation + cache write", [(kernels, "rope_kv_write", no_rope)]),
-             ("attention", [(kernels, "attention_decode_warps", no_attention)]),
-             ("q|k|v product", without(lambda w, m: w.shape[0] == QKV and m == tc.PARTIAL)),
-             ("o product", without(lambda w, m: tuple(w.shape) == (H, cfg.num_attention_heads * cfg.head_dim))),
-             ("gate/up product", without(lambda w, m: m == tc.SWIGLU)),
-             ("down product", without(lambda w, m: tuple(w.shape) == (H, I))),
-             ("output matrix (per step)", without(lambda w, m: w.shape[0] == V)),
-             ("all products", without(lambda w, m: True))]
+    return [("norm kernels (first layer and final norm when the others are fused)", [(kernels, "add_rmsnorm", no_norm)]),
+            ("rotation + cache write (nothing where the attention does both itself)", [(kernels, "rope_kv_write", no_rope)]),
+            ("attention (with rotation and cache write where it does them itself)",
+             [(kernels, "attention_decode_warps", no_attention), (kernels, "attention_decode_formed", no_attention)]),
+            ("q|k|v product", without(lambda w, m: w.shape[0] == QKV and m == tc.PARTIAL)),
+            ("o product", without(lambda w, m: tuple(w.shape) == (H, cfg.num_attention_heads * cfg.head_dim))),
+            ("gate/up product", without(lambda w, m: m == tc.SWIGLU)),
+            ("down product", without(lambda w, m: tuple(w.shape) == (H, I))),
+            ("output matrix (per step)", without(lambda w, m: w.shape[0] == V)),
+            ("all products", without(lambda w, m: True))]
+
+
+def ablation(model, batch, steps=32, prompt_len=PROMPT_LEN):
+    """Where a replayed decode step's time goes: every kind of kernel in turn is replaced by a stand-in that launches
+    nothing and returns a buffer of the right shape, the step's graph is captured anew and timed.  The difference to
+    the whole step is what that kernel costs inside the chain (with its overlaps), which a profiler's serialised,
+    cold-cache replay does not show.  Results are garbage while a stand-in is in place; only the time is read."""
+    import torch
+    from rocmforge_b200.engine.graph import DecodeRunner
+    cfg = model.config
+    L = cfg.num_hidden_layers
+
+    def run():
+        cache = model.new_cache(max_tokens=batch * (prompt_len + 256), max_slots=batch)
+        runner = DecodeRunner(model, cache)
+        slots = [cache.alloc_slot() for _ in range(batch)]
+        for s in slots:                                  # prompt_len cached positions (their content does not matter)
+            cache.prepare([s], [prompt_len])
+            cache.commit([s], [prompt_len])
+        runner.greedy_loop(slots, [1] * batch, 4)
+        torch.cuda.synchronize()
+        _, start, end, _ = runner.greedy_loop(slots, [1] * batch, steps)
+        torch.cuda.synchronize()
+        return start.elapsed_time(end) / steps * 1e3     # us a step
+
     whole = run()
     rows = [{"kernel": "whole step", "us_per_step": round(whole, 1)}]
-    for name, patches in cases:
+    for name, patches in ablation_cases(cfg, model.device):
         saved = [(module, attr, getattr(module, attr)) for module, attr, _ in patches]
         for module, attr, stand_in in patches:
             setattr(module, attr, stand_in)
