@@ -17,7 +17,7 @@ pytestmark = pytest.mark.gpu
 def test_stand_ins_take_a_kernels_launches_away(tmp_path, heads, kv_heads, head_dim, batch, formed):
     L = 2
     write_tiny(dict(TINY_D, num_hidden_layers=L, hidden_size=1024, num_attention_heads=heads, num_key_value_heads=kv_heads, head_dim=head_dim,
-                    intermediate_size=2048), str(tmp_path), "bfloat16")
+                    intermediate_size=1536), str(tmp_path), "bfloat16")
     model = rf.LLM(str(tmp_path), dtype="bfloat16").model
     cache = model.new_cache(max_tokens=batch * 128, max_slots=batch)
     slots = [cache.alloc_slot() for _ in range(batch)]
