@@ -152,12 +152,12 @@ class DeviceDescriptor:
             self._busy = True
 
     def views(self, T: int, B: int, R: int, extras=(), decode_extras: bool = False):
-        key = (T, B, R, extras, decode_extras)
-        got = self._views.get(key)
+        key = (T, B, R, tuple(map(tuple, extras)), decode_extras) if T == B else None
+        got = None if key is None else self._views.get(key)
         if got is None:
             lay, _ = StepBatch.layout(T, B, R, extras, decode_extras)
             got = {name: self.dev[o:o + n] for name, (o, n) in lay.items()}
-            if T == B:                                 # a decode step's: prompts' sizes hardly ever come again
+            if key is not None:                        # a decode step's: prompts' sizes hardly ever come again
                 if len(self._views) >= 64:
                     self._views.clear()
                 self._views[key] = got

@@ -267,3 +267,13 @@ def test_rollback_gives_back_what_a_failed_step_took():
     assert c.free_pages() == free and c.length(s) == 70
     c.prepare([s], [1]); c.commit([s], [1])           # the slot goes on as if nothing had happened
     invariant(c)
+
+
+def test_descriptor_views_are_kept_for_decode_steps_only():
+    from rocmforge_b200.engine.batch import DeviceDescriptor
+    desc = DeviceDescriptor("cpu", capacity=256)
+    one = desc.views(3, 3, 3, (("tiles", 4),))
+    assert desc.views(3, 3, 3, [("tiles", 4)]) is one and desc.views(3, 3, 3, [["tiles", 4]]) is one
+    assert desc.views(3, 3, 3) is not one and "seeds" in desc.views(3, 3, 3, decode_extras=True)
+    assert desc.views(5, 3, 3, [("tiles", 4)]) is not desc.views(5, 3, 3, [("tiles", 4)])
+    assert one["tiles"].numel() == 4 and one["tokens"].data_ptr() == desc.dev.data_ptr()
