@@ -13,7 +13,7 @@ indexed by slot, zeroed when the slot is handed out.
 from __future__ import annotations
 
 from dataclasses import dataclass
-from typing import Dict, List, Optional, Sequence
+from typing import Dict, List, Optional, Sequence, Tuple
 
 import numpy as np
 import torch
@@ -28,6 +28,14 @@ PAGE = 64
 
 def pages_for(n_tokens: int) -> int:
     return (n_tokens + PAGE - 1) // PAGE
+
+
+def upload_spans(dirty: Dict[int, List[int]], width: int) -> List[Tuple[int, int]]:
+    """[first, last) entries of the flattened block table to copy for the changed entries ``dirty`` (slot -> [lo, hi)): all of them and what
+    lies between in one span, unless that is far more than they are."""
+    spans = [(slot * width + lo, slot * width + hi) for slot, (lo, hi) in dirty.items()]
+    first, last = min(a for a, _ in spans), max(b for _, b in spans)
+    return [(first, last)] if last - first <= 4096 + 4 * sum(b - a for a, b in spans) else spans
 
 
 class KVGroup:
@@ -131,12 +139,7 @@ class KVGroup:
         if not self._dirty:
             return
         if self.table_dev.is_cuda:
-            # the changed entries and what lies between them in one copy, unless that is far more than they are
-            W = self.max_pages_per_seq
-            spans = [(slot * W + lo, slot * W + hi) for slot, (lo, hi) in self._dirty.items()]
-            first, last = min(a for a, _ in spans), max(b for _, b in spans)
-            if last - first <= 4096 + 4 * sum(b - a for a, b in spans):
-                spans = [(first, last)]
+            spans = upload_spans(self._dirty, self.max_pages_per_seq)
             n = sum(b - a for a, b in spans)
             if self._upload_done is None:
                 self._upload_done = torch.cuda.Event()

@@ -269,6 +269,25 @@ def test_rollback_gives_back_what_a_failed_step_took():
     invariant(c)
 
 
+def test_upload_spans_cover_the_changes():
+    from rocmforge_b200.cache.sequence_cache import upload_spans
+    assert upload_spans({3: [2, 5]}, 10) == [(32, 35)]
+    assert upload_spans({7: [0, 1], 2: [9, 10], 4: [3, 4]}, 10) == [(29, 71)]          # in one copy with what lies between
+    assert upload_spans({0: [0, 1], 1: [0, 1]}, 4103) == [(0, 4104)] and upload_spans({0: [0, 1], 1: [0, 1]}, 4104) == [(0, 1), (4104, 4105)]
+    rng = random.Random(5)
+    for _ in range(200):
+        width = rng.choice([1, 7, 64, 5000])
+        dirty = {}
+        for slot in rng.sample(range(300), rng.randint(1, 8)):
+            lo = rng.randrange(width)
+            dirty[slot] = [lo, rng.randint(lo + 1, width)]
+        spans = upload_spans(dirty, width)
+        for slot, (lo, hi) in dirty.items():
+            assert any(a <= slot * width + lo and slot * width + hi <= b for a, b in spans)
+        changed = sum(hi - lo for lo, hi in dirty.values())
+        assert sum(b - a for a, b in spans) <= changed or (len(spans) == 1 and spans[0][1] - spans[0][0] <= 4096 + 4 * changed)
+
+
 def test_descriptor_views_are_kept_for_decode_steps_only():
     from rocmforge_b200.engine.batch import DeviceDescriptor
     desc = DeviceDescriptor("cpu", capacity=256)
