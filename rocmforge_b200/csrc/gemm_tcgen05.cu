@@ -402,7 +402,9 @@ static int launch_cfg(const CUtensorMap& ma, const CUtensorMap& mb, const TcPara
 // Each of them is compiled for one mode.  The other products of a step run the general form, so the instructions of another function
 // come from L2 anew in every layer, about 1 us with all modes in it: in chains of one function these forms won throughout, but steps
 // of 17 to 40 tokens of a model 1,536 wide became up to 8 % slower.  (The general form itself, in a function for silu alone, costs such
-// steps 1 to 5 %.)  Gated units and bfloat16 rows gain enough; 32-bit rows and sums into the stream stay with the general form.
+// steps 1 to 5 %.)  Gated units and bfloat16 rows gain enough; sums into the stream stay with the general form, and 32-bit rows but for
+// up to 16 tokens and a K of 1,024 and more, where a few rows' long sums wait for one SM's ring (Figalix's design, 32-bit rows in the
+// general form and in half tiles: 8 tokens 469, 460; but 24 tokens 560, 564).
 // Whole decode steps, us, the general form alone, these forms with all modes in them, and so:
 //     896 wide (0.5B)   8 tokens 628, 625, 606; 24 684, 699, 677; 64 788, 768, 752; 65 903, 951, 902; 128 996, 992, 956
 //     1,536 wide        8 tokens 435, 433, 422; 24 481, 511, 485; 40 532, 560, 534; 64 576, 568, 554; 128 747, 713, 701
@@ -413,10 +415,11 @@ static int launch_cfg(const CUtensorMap& ma, const CUtensorMap& mb, const TcPara
 // 128 KB: 65 tokens x 9,728 x 896 10.4 us, in half tiles 11.9 (80 tokens 10.4, 10.1); 33 x 17,920 x 1,536 13.6, 14.7 (43: 13.7, 12.8).
 // Beyond a tile an SM half tiles cost: their rows meet as many token bytes (8 tokens x 32,000 x 2,048 23.4, 27.7).
 struct SkinnyForm { bool half, wide; };
-static SkinnyForm skinny_form(int M, int N, int bn, int ldx, int mode, int splits, bool normed_rows, int sms) {
+static SkinnyForm skinny_form(int M, int N, int K, int bn, int ldx, int mode, int splits, bool normed_rows, int sms) {
     const long long row = (long long)ldx * 2, edge = 128 << 10;
     const bool slow_tile = bn >= 64 && M * row < edge && bn * row > edge;
-    if (normed_rows || splits != 1 || slow_tile || !(mode == EPI_STORE || epi_gated(mode))) return {false, false};
+    const bool rows_f32 = mode == EPI_F32 && bn == 16 && K >= 1024;
+    if (normed_rows || splits != 1 || slow_tile || !(mode == EPI_STORE || epi_gated(mode) || rows_f32)) return {false, false};
     const bool half = (long long)((N + TC_BM - 1) / TC_BM) * ((M + bn - 1) / bn) <= sms && (bn != 32 || mode == EPI_STORE);
     return {half, !half && bn >= 64};
 }
@@ -424,8 +427,9 @@ static int skinny_tokens(int M) { return M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64
 
 template <int MODE>
 static int launch_special(SkinnyForm form, int bn, const CUtensorMap& ma, const CUtensorMap& mb, const TcParams& p, dim3 grid, cudaStream_t st) {
-    if (form.half) {
-        if (bn == 16) return launch_cfg<16, true, 11, false, false, 64, 4, MODE>(ma, mb, p, grid, st);
+    if (form.half && bn == 16) return launch_cfg<16, true, 11, false, false, 64, 4, MODE>(ma, mb, p, grid, st);
+    if constexpr (MODE == EPI_F32) return RF_ERR_BAD_ARG;
+    else if (form.half) {
         if constexpr (MODE == EPI_STORE)
             if (bn == 32) return launch_cfg<32, true, 9, false, false, 64, 8, MODE>(ma, mb, p, grid, st);
         if (bn == 64) return launch_cfg<64, true, 6, false, false, 64, 8, MODE>(ma, mb, p, grid, st);
@@ -440,8 +444,8 @@ static int launch_special(SkinnyForm form, int bn, const CUtensorMap& ma, const 
 extern "C" {
 
 // The form of a product of few tokens on a GPU of ``sms`` SMs: 1 tiles of 64 weight rows, 2 eight epilogue warps, 0 the general one.
-int rf_gemm_tc_skinny_form(int M, int N, int ldx, int mode, int splits, int normed_rows, int sms) {
-    const SkinnyForm f = skinny_form(M, N, skinny_tokens(M), ldx, mode, splits, normed_rows != 0, sms);
+int rf_gemm_tc_skinny_form(int M, int N, int K, int ldx, int mode, int splits, int normed_rows, int sms) {
+    const SkinnyForm f = skinny_form(M, N, K, skinny_tokens(M), ldx, mode, splits, normed_rows != 0, sms);
     return f.half ? 1 : f.wide ? 2 : 0;
 }
 
@@ -549,7 +553,7 @@ static int gemm_skinny(const void* X, int ldx, const void* W, const void* bias, 
     int e;
     const int bn = skinny_tokens(M);
     const bool normed_rows = ss_in || mode == EPI_RESNORM;
-    const SkinnyForm form = skinny_form(M, N, bn, ldx, mode, splits, normed_rows, sm_count());
+    const SkinnyForm form = skinny_form(M, N, K, bn, ldx, mode, splits, normed_rows, sm_count());
     const int bm = form.half ? 64 : TC_BM;
     if ((e = make_map(&ma, W, N, K, K, bm)) || (e = make_map(&mb, X, M, K, ldx, bn))) return e;
     dim3 grid((M + bn - 1) / bn, (N + bm - 1) / bm, splits);      // token tiles fastest: they share a weight tile in L2
@@ -567,6 +571,7 @@ static int gemm_skinny(const void* X, int ldx, const void* W, const void* bias, 
         return launch_cfg<128, true, 3, true>(ma, mb, p, grid, st, &nrm, cz);
     }
     if (form.half || form.wide) {
+        if (mode == EPI_F32) return launch_special<EPI_F32>(form, bn, ma, mb, p, grid, st);
         if (mode == EPI_STORE) return launch_special<EPI_STORE>(form, bn, ma, mb, p, grid, st);
         if (mode == EPI_SWIGLU) return launch_special<EPI_SWIGLU>(form, bn, ma, mb, p, grid, st);
         return launch_special<EPI_REGLU>(form, bn, ma, mb, p, grid, st);

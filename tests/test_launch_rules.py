@@ -69,14 +69,16 @@ def test_forms_of_products_of_few_tokens():
     from rocmforge_b200.csrc import build
     from rocmforge_b200.kernels import tensor_core as tc
     form = build.load("gemm_tcgen05").rf_gemm_tc_skinny_form
-    of = lambda M, N, K, mode, splits=1, normed=0: form(M, N, K, mode, splits, normed, 148)
+    of = lambda M, N, K, mode, splits=1, normed=0: form(M, N, K, K, mode, splits, normed, 148)
     for mode in (tc.STORE, tc.SWIGLU, tc.REGLU, tc.GEGLU, tc.CLAMPGLU):
         assert [of(M, 9728, 2048, mode) for M in (1, 16, 33, 64, 65, 128)] == [1] * 6
         assert [of(M, 148 * 128 + 2, 2048, mode) for M in (1, 16, 17, 32, 33, 64, 65, 128)] == [0, 0, 0, 0, 2, 2, 2, 2]
         assert of(8, 9728, 2048, mode, normed=1) == 0
     assert [of(M, 17920, 1536, tc.SWIGLU) for M in (17, 24, 32)] == [0, 0, 0]          # was up to 8 % of a step slower in half tiles
     assert [of(M, 2304, 2048, tc.STORE) for M in (17, 32)] == [1, 1]
-    for mode in (tc.F32, tc.RESIDUAL, tc.PARTIAL, tc.RESNORM):
+    assert [of(M, N, K, tc.F32) for M, N, K in ((1, 16, 1024), (16, 64, 2048), (16, 64, 1016), (17, 64, 2048), (64, 64, 2048), (8, 32000, 2048))
+            ] == [1, 1, 0, 0, 0, 0]
+    for mode in (tc.RESIDUAL, tc.PARTIAL, tc.RESNORM):
         assert all(of(M, 9728, 2048, mode) == 0 for M in (1, 17, 64, 128))
     assert of(64, 4608, 3584, tc.PARTIAL, splits=8) == 0
     # activations of less than 128 KB in a tile that reaches beyond 128 KB
