@@ -268,7 +268,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             // what a page takes.  (us, with one number an instruction, rounded by integer additions, and so: 64 prompts of 16..1,024
             // tokens, 14 heads of 64 166.5, 152.5; one of 8,192 227, 208; 2,048 tokens, 28 heads of 128 42.9, 38.9.  Four CTAs an SM in
             // place of two, heads of 64 and halves of a page at a time, changed nothing; pages left out for warps that see none
-            // of their keys cost 3 %.)
+            // of their keys cost 3 %.  Of earlier forms: a share of the exponentials as a polynomial on the FMA pipe 763 -> 734 TFLOP/s at 8,192
+            // tokens, two softmax threads a row 763 -> 435.)
             Two sum01 = two(0.f, 0.f), sum23 = sum01;
             const Two sl22 = two(sl2, sl2), nref2 = two(nref, nref);
             uint32_t pk[AT_BN / 2];

@@ -319,8 +319,9 @@ int rf_delta_scan(const float* qn, const float* kn, const float* kq, const float
 // The solve kernel then takes the tokens in blocks of 16.  Inside a block it walks, for every s, over t with k_s P(s, t) in registers
 // (four lanes share s, 16 channels each at a time).  Between two blocks P(s, t) is the product from s to its block's end, times that of
 // the whole blocks between, times that from t's block's start to t: keys and queries are scaled so once, and what remains are plain
-// products over the channels.  It leaves G o q and P(s, end) o k for the other two kernels, which are the same otherwise.  (16 heads of 128 x 128: 2,048 tokens
-// 669 us token by token, 250 in chunks; three prompts of 1,365, 700 and 500 321; walking over all later tokens, not a block's, 284, 370.)
+// products over the channels.  It leaves G o q and P(s, end) o k for the other two kernels, which are the same otherwise.  (16 heads of
+// 128 x 128: 2,048 tokens 669 us token by token, 250 in chunks; three prompts of 1,365, 700 and 500 321; walking over all later tokens, not
+// a block's, 284, 370.)
 // A warp's own stream of instructions bounds all three (issue slots 40 to 60 % busy), so they work on two numbers an instruction wherever
 // there is one, and the solve kernel on two tokens at a time (us, one number and one token at a time: 309 and 413; one decay per head,
 // 2,048 tokens 224, now 220).
@@ -490,8 +491,8 @@ delta_chunk_solve_kernel(const float* __restrict__ qn, const float* __restrict__
                 }
                 if (d >= D) go[d] = 0.f;
             }
-                    __syncthreads();                          // keys, queries and decays have been read as they are
-            if (tid < 192) {                          // a thread per channel and block after the first: k_t and q_t times the decays from its start
+            __syncthreads();                          // keys, queries and decays have been read as they are
+            if (tid < 192) {                          // a thread per channel and block after the first: k_t, q_t times the decays from its start
                 const int j = 1 + (tid >> 6), e = tid & 63;
                 float run = 1.f;
 #pragma unroll

@@ -890,66 +890,72 @@ head_norm_rows_kernel(const T* src, int row_stride, T* q_out, int q_out_stride, 
     const int heads = write_kv ? nh + (ex.v_is_k ? 1 : 2) * nkv : nh;
     constexpr int N = 2;                                 // heads of a warp in flight
     for (int i0 = threadIdx.x >> 5; i0 < n_tok * heads; i0 += 8 * N) {
-    Piece first[N], second[N];
+        Piece first[N], second[N];
 #pragma unroll
-    for (int n = 0; n < N; ++n) {
-        const int i = min(i0 + 8 * n, n_tok * heads - 1), t = i / heads, head = i - t * heads;
-        const T* from = src + (size_t)(t0 + t) * row_stride + (size_t)head * HD + lane * E;
-        first[n] = *reinterpret_cast<const Piece*>(from);
-        second[n] = *reinterpret_cast<const Piece*>(from + HALF);
-    }
-#pragma unroll
-    for (int n = 0; n < N; ++n) {
-        const int i = i0 + 8 * n, t = i / heads, head = i - t * heads;
-        if (i >= n_tok * heads) continue;
-        const bool is_v = head >= nh + nkv;
-        const Piece a = first[n], b = second[n];
-        float x[E], y[E];
-#pragma unroll
-        for (int j = 0; j < E; ++j) {
-            x[j] = Cvt<T>::to_f32(a.v[j]); y[j] = Cvt<T>::to_f32(b.v[j]);
-            if (ex.bias != nullptr) {
-                x[j] += load_vec(ex.bias, ex.bias_is_f32, head * HD + lane * E + j);
-                y[j] += load_vec(ex.bias, ex.bias_is_f32, head * HD + HALF + lane * E + j);
-            }
+        for (int n = 0; n < N; ++n) {
+            const int i = min(i0 + 8 * n, n_tok * heads - 1), t = i / heads, head = i - t * heads;
+            const T* from = src + (size_t)(t0 + t) * row_stride + (size_t)head * HD + lane * E;
+            first[n] = *reinterpret_cast<const Piece*>(from);
+            second[n] = *reinterpret_cast<const Piece*>(from + HALF);
         }
-        const bool normed = unit_norm && !is_v;
-        const void* nw = normed ? (head < nh ? q_norm_w : k_norm_w) : nullptr;
-        if (normed && !ex.norm_after) {
-            const float r = rsqrtf(head_square_sum<E>(x, y) / (float)HD + eps);
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+            const int i = i0 + 8 * n, t = i / heads, head = i - t * heads;
+            if (i >= n_tok * heads) continue;
+            const bool is_v = head >= nh + nkv;
+            const Piece a = first[n], b = second[n];
+            float x[E], y[E];
 #pragma unroll
             for (int j = 0; j < E; ++j) {
-                if (nw != nullptr) { x[j] *= load_vec(nw, norm_w_is_f32, lane * E + j); y[j] *= load_vec(nw, norm_w_is_f32, HALF + lane * E + j); }
-                x[j] *= r; y[j] *= r;
+                x[j] = Cvt<T>::to_f32(a.v[j]); y[j] = Cvt<T>::to_f32(b.v[j]);
+                if (ex.bias != nullptr) {
+                    x[j] += load_vec(ex.bias, ex.bias_is_f32, head * HD + lane * E + j);
+                    y[j] += load_vec(ex.bias, ex.bias_is_f32, head * HD + HALF + lane * E + j);
+                }
             }
-        }
-        if (rotated && !is_v) {
+            const bool normed = unit_norm && !is_v;
+            const void* nw = normed ? (head < nh ? q_norm_w : k_norm_w) : nullptr;
+            if (normed && !ex.norm_after) {
+                const float r = rsqrtf(head_square_sum<E>(x, y) / (float)HD + eps);
 #pragma unroll
-            for (int j = 0; j < E; ++j) {
-                const float2 c = turn[t][lane * E + j];
-                const float u = x[j] * c.x - y[j] * c.y;
-                y[j] = y[j] * c.x + x[j] * c.y;
-                x[j] = u;
+                for (int j = 0; j < E; ++j) {
+                    if (nw != nullptr) {
+                        x[j] *= load_vec(nw, norm_w_is_f32, lane * E + j);
+                        y[j] *= load_vec(nw, norm_w_is_f32, HALF + lane * E + j);
+                    }
+                    x[j] *= r; y[j] *= r;
+                }
             }
-        }
-        if (normed && ex.norm_after) {
-            const float r = rsqrtf(head_square_sum<E>(x, y) / (float)HD + eps);
+            if (rotated && !is_v) {
 #pragma unroll
-            for (int j = 0; j < E; ++j) {
-                x[j] *= r; y[j] *= r;
-                if (nw != nullptr) { x[j] *= load_vec(nw, norm_w_is_f32, lane * E + j); y[j] *= load_vec(nw, norm_w_is_f32, HALF + lane * E + j); }
+                for (int j = 0; j < E; ++j) {
+                    const float2 c = turn[t][lane * E + j];
+                    const float u = x[j] * c.x - y[j] * c.y;
+                    y[j] = y[j] * c.x + x[j] * c.y;
+                    x[j] = u;
+                }
             }
-        }
-        const float scale = head < nh ? temp[t] : 1.f;
-        T* dst = (head < nh ? q_out + (size_t)(t0 + t) * q_out_stride + (size_t)head * HD
-                  : !is_v ? k_pages + page_at[t] + (size_t)(head - nh) * RF_PAGE * HD
-                          : v_pages + page_at[t] + (size_t)(head - nh - nkv) * RF_PAGE * HD) + lane * E;
-        Piece c, d;
+            if (normed && ex.norm_after) {
+                const float r = rsqrtf(head_square_sum<E>(x, y) / (float)HD + eps);
 #pragma unroll
-        for (int j = 0; j < E; ++j) { c.v[j] = Cvt<T>::from_f32(x[j] * scale); d.v[j] = Cvt<T>::from_f32(y[j] * scale); }
-        *reinterpret_cast<Piece*>(dst) = c;
-        *reinterpret_cast<Piece*>(dst + HALF) = d;
-    }
+                for (int j = 0; j < E; ++j) {
+                    x[j] *= r; y[j] *= r;
+                    if (nw != nullptr) {
+                        x[j] *= load_vec(nw, norm_w_is_f32, lane * E + j);
+                        y[j] *= load_vec(nw, norm_w_is_f32, HALF + lane * E + j);
+                    }
+                }
+            }
+            const float scale = head < nh ? temp[t] : 1.f;
+            T* dst = (head < nh ? q_out + (size_t)(t0 + t) * q_out_stride + (size_t)head * HD
+                      : !is_v ? k_pages + page_at[t] + (size_t)(head - nh) * RF_PAGE * HD
+                              : v_pages + page_at[t] + (size_t)(head - nh - nkv) * RF_PAGE * HD) + lane * E;
+            Piece c, d;
+#pragma unroll
+            for (int j = 0; j < E; ++j) { c.v[j] = Cvt<T>::from_f32(x[j] * scale); d.v[j] = Cvt<T>::from_f32(y[j] * scale); }
+            *reinterpret_cast<Piece*>(dst) = c;
+            *reinterpret_cast<Piece*>(dst + HALF) = d;
+        }
     }
 }
 

@@ -159,11 +159,9 @@ __device__ __forceinline__ float at_exp2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// (The latent attention's) weights are rounded to bfloat16 with integer arithmetic (add half an ulp, keep the upper 16 bits): the
-// conversion instruction shares the special-function unit with ex2.  Two variants that measured SLOWER here
-// and were dropped: a share of the exponentials as a polynomial on the FMA pipe (763 -> 734 TFLOP/s at 8,192
-// tokens), and two softmax threads per row (763 -> 435): the softmax warps lack neither ex2 throughput nor
-// threads; what helped was letting the next page's scores be computed while they work (see issue_s).
+// The latent prompt attention rounds its weights to bfloat16 with integer arithmetic (add half an ulp, keep the upper 16 bits).  The
+// other prompt attention did so too, and became 9 % faster by the conversion instruction and two numbers an instruction (its comment has
+// the figures); here neither has been tried.
 __device__ __forceinline__ uint32_t at_pack_bf16x2(float a, float b) {      // a, b >= 0 and finite
     return __byte_perm(__float_as_uint(a) + 0x8000u, __float_as_uint(b) + 0x8000u, 0x7632);
 }
