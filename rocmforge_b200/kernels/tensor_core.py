@@ -224,23 +224,27 @@ def gemm_tc_grouped(x: torch.Tensor, w: torch.Tensor, tiles: torch.Tensor, max_t
 
 def split_k_for(N: int, K: int, sm_count: Optional[int] = None, tokens: Optional[int] = None) -> int:
     """K splits of a skinny product, from N and K (never from the batch's content): about two CTAs per SM stream the weight, and a split
-    has at least 4 blocks of 64 or, where K has at most 16 blocks, 2 while that makes no more than a CTA per SM (the last split has
-    what is left).  ``tokens``: a step of at most 16 tokens fits three CTAs on an SM, and a weight with long K ranges is then cut
+    has at least 4 blocks of 64 or, where K has at most 16 blocks, 2 while that makes no more than a CTA per SM and, beyond 32 tokens,
+    no more than 6 stacks to add up (the last split has what is left).  ``tokens``: a step of at most 16 tokens fits three CTAs on an SM, and a weight with long K ranges is then cut
     for three per SM (splits of at least 16 blocks; the down projection of the 7B shape 10 -> 15: a decode step at batch 8 2.624 ->
     2.603 ms, at batch 1 2.560 -> 2.530 ms; with 32 or 64 tokens, two CTAs per SM, the same cut costs 0.16 ms).
 
     A short K in splits of 4, 8 / 3 and 2 blocks, whole decode steps of 12 layers with that width, us: 8 blocks, batch 1 261, 259, 252,
     64 356, 358, 354; 10 blocks, batch 16 320, 310, 290, 128 473, 463, 438; 12 blocks, batch 16 321, 318, 301, 64 382, 379, 373; 14 blocks,
     batch 16 348, 312, 311, 128 485, 474, 482; 16 blocks, batch 16 334, 323, 322, 64 412, 401, 400, 128 500, 514, 514; Ludusun's
-    design 1,024 wide, batch 16 195, 199, 197, 64 272, 276, 273.  Beyond a CTA per SM (48 tiles of 16 blocks) the finer splits cost:
-    batch 64 620, 623, 623.  From 24 blocks on splits of 4 are as good as any (1,536 wide, batch 16, of 4 and 3 blocks: 410, 413)."""
+    design 1,024 wide, batch 16 195, 199, 197, 64 272, 276, 273.  4, 5 and 7 splits of 14 blocks in 0.5B's step with contexts of 900, where
+    more CTAs add up the same stacks: batch 8 625, 607, 604, 64 817, 816, 826.  Beyond a CTA per SM (48 tiles of 16 blocks) finer splits
+    cost: batch 64 620, 623, 623.  From 24 blocks on splits of 4 are as good as any (1,536 wide, batch 16, of 4 and 3 blocks: 410, 413)."""
     sm_count = sm_count or device_sm_count()
     tiles = (N + 127) // 128
     kb = (K + 63) // 64
     if tiles >= 2 * sm_count or kb < 8:
         return 1
     want = max(1, (2 * sm_count) // tiles)
-    splits = kb // 4 if kb > 16 else max(kb // 4, min(kb // 2, sm_count // tiles))
+    splits = kb // 4
+    if kb <= 16:
+        finer = kb // 2 if tokens is not None and tokens <= 32 else min(kb // 2, 6)
+        splits = max(splits, min(finer, sm_count // tiles))
     splits = max(1, min(want, splits))
     if tokens is not None and tokens <= 16:
         splits = max(splits, min((3 * sm_count) // tiles, kb // 16))

@@ -106,14 +106,17 @@ def test_when_decode_attention_forms_its_own_queries():
 
 def test_k_splits_of_a_short_k():
     from rocmforge_b200.kernels import tensor_core as tc
-    for tokens in (1, 16, 64, 128):
+    for tokens in (1, 16, 17, 32):
         assert [tc.split_k_for(1024, 64 * kb, 148, tokens) for kb in range(7, 18)] == [1, 4, 3, 5, 4, 6, 5, 7, 5, 8, 4]
+    for tokens in (33, 64, 128, None):                    # at most six stacks
+        assert [tc.split_k_for(1024, 64 * kb, 148, tokens) for kb in range(7, 18)] == [1, 4, 3, 5, 4, 6, 5, 5, 5, 6, 4]
     for N in (896, 1152, 1536, 2304, 3112, 4608, 6144, 9728, 18944, 40000):
         for K in (512, 520, 576, 640, 704, 768, 832, 896, 960, 1000, 1024):
-            s, kb, tiles = tc.split_k_for(N, K, 148, 64), (K + 63) // 64, (N + 127) // 128
-            per = -(-kb // s)
-            assert (s - 1) * per < kb, "no split is empty"
-            assert s == 1 or (tiles * s <= 2 * 148 and per >= 2)
-            assert tiles * s <= 148 or kb // s >= 4 or s <= kb // 4, "more than a CTA per SM: at least four blocks a split"
+            for tokens in (8, 32, 64):
+                s, kb, tiles = tc.split_k_for(N, K, 148, tokens), (K + 63) // 64, (N + 127) // 128
+                per = -(-kb // s)
+                assert (s - 1) * per < kb, "no split is empty"
+                assert s == 1 or (tiles * s <= 2 * 148 and per >= 2)
+                assert tiles * s <= 148 or s <= kb // 4, "more than a CTA per SM: at least four blocks a split"
     # the product that finishes the residual update: splits of four blocks and more, as many as form a cluster
     assert [tc.resnorm_splits(n, n) for n in (512, 768, 896, 1024, 2048, 3584)] == [2, 2, 2, 4, 8, 8]
