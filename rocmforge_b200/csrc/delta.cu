@@ -322,9 +322,9 @@ int rf_delta_scan(const float* qn, const float* kn, const float* kq, const float
 // products over the channels.  It leaves G o q and P(s, end) o k for the other two kernels, which are the same otherwise.  (16 heads of
 // 128 x 128: 2,048 tokens 669 us token by token, 250 in chunks; three prompts of 1,365, 700 and 500 321; walking over all later tokens, not
 // a block's, 284, 370.)
-// A warp's own stream of instructions bounds all three (issue slots 40 to 60 % busy), so they work on two numbers an instruction wherever
-// there is one, and the solve kernel on two tokens at a time (us, one number and one token at a time: 309 and 413; one decay per head,
-// 2,048 tokens 224, now 220).
+// A warp's own stream of instructions bounds all three (issue slots 38 to 45 % busy, two to four warps a scheduler), so they work on two
+// numbers an instruction wherever there is one, and the solve kernel on two tokens at a time (us, one number and one token at a time: 309
+// and 413; one decay per head, 2,048 tokens 224, now 220).
 // Decays are multiplied on as running products, never divided by and never taken the logarithm of: 0 and 1 need no special case.
 // Everything is 32-bit.  The chunk table (built on the host with the step) is first[B+1] (index of each sequence's first
 // chunk), then (sequence, first row) per chunk.
